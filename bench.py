@@ -298,7 +298,7 @@ def hard_roofline(hard, peak64):
     ms = sum(h[0] for h in hard)
     ex = [h[1] for h in hard]
     alg = sum(h[2] for h in hard)
-    out = {"kernel": "k_hard_bundles<256,2> (one launch per tree step)", "bound": "fp64",
+    out = {"kernel": "k_hard_bundles<128,3> (one launch per tree step)", "bound": "fp64",
            "launch_ms": ms / len(hard), "unit": "TFLOP/s", "peak": peak64,
            "peak_source": "measured (FP64 FMA microbenchmark p3t_probe_fma_peak)",
            "algorithmic_tflops": alg / (ms * 1e-3) / 1e12,

@@ -156,14 +156,13 @@ def tune_heavy_steps(P, disk, grid=HEAVY_GRID, steps=HEAVY_STEPS):
 
 
 # (member slots, CTAs per SM, clusters above the slots in the wide launch)
-BUNDLE_GRID = ((256, 2, 0), (256, 2, 1), (128, 3, 1), (128, 4, 1))
+BUNDLE_GRID = ((128, 3, 0), (128, 3, 1), (256, 2, 1))
 
 
 def tune_wide(g, istep=1, reps=2, grid=BUNDLE_GRID):
     """Times the bundled hard launch from one restored state for each bundle
     shape (p3t_set_hard_bundle) and placement of the clusters above it
-    (p3t_set_hard_wide: concurrent wide launch or one per CTA in the main
-    launch); installs the fastest.  Returns (best, {choice: ms})."""
+    (p3t_set_hard_wide); installs the fastest.  Returns (best, {choice: ms})."""
     lib = g.lib
     _lib.check(lib.p3t_state_snapshot(0), "p3t_state_snapshot")
     table = {}

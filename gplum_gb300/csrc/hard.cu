@@ -12,6 +12,7 @@
 #include "../../include/gplum_p3t.h"
 #include "p3t_capi_internal.cuh"
 #include "p3t_engine.cuh"
+#include "p3t_exact.cuh"
 #include "p3t_phys.cuh"
 
 namespace p3t {
@@ -84,6 +85,17 @@ struct FragParams {
     unsigned long long seed;
 };
 
+// What a cluster's integration keeps for its end: start time of the log, the
+// energy its collisions dissipated, fragments and collisions made (bundle form).
+struct ClusterRec {
+    long long t0, n_frag;
+    double ed, edd;
+    int n_col;
+};
+
+// parameters at their neutral value, whose operations are exact no-ops
+enum : int { PL_EPS2 = 1, PL_EPS2_SUN = 2, PL_M_SUN = 4 };
+
 struct HardArgs {
     State S;
     Params P;
@@ -104,9 +116,10 @@ struct HardArgs {
     FragRec *frags;      // [frag_cap] fragments of this launch
     int32_t *n_frags;    // fragments made so far
     int frag_base, frag_cap;  // hard slots frag_base + k hold fragment k
-    int wide;                 // bundle form: clusters above BCAP_MAIN in k_hard_wide (1) or run_cluster (0)
+    int wide_cap;             // bundle form: members of a cluster k_hard_wide takes as a lone wide bundle at most
+    int plain;                // PL_* bits
+    ClusterRec *crec;         // [n_clusters]
     int max_steps;            // block steps a cluster may take in one tree step (ST_ITER_CAP beyond)
-    int lone_in;              // bundle form: the lone tier runs in the bundle CTAs (1) or in k_hard_lone (0)
     unsigned long long *phase_cycles;  // optional [HP_N]: clock cycles per phase of the bundle loop, all CTAs
     unsigned long long *live; // optional [2]: pair terms evaluated (predicted/corrected, full), bundle form
 };
@@ -297,7 +310,7 @@ struct FragCtx {
 // merge-list update (src/hermite.h:395-423).  One lane.  Without a fragment
 // context (or with a_frag = 0) this is perfect accretion.  Returns the
 // number of fragments, whose hard slots are written to X->out_slots.
-__device__ int collide(const Params &P, const Hard &H, int imp, int tar, double &edisp, double &edisp_d,
+__device__ __noinline__ int collide(const Params &P, const Hard &H, int imp, int tar, double &edisp, double &edisp_d,
                        ColRec &rec, const FragCtx *X) {
     rec.id_imp = H.id[imp];
     rec.id_tar = H.id[tar];
@@ -1278,6 +1291,7 @@ struct HardBufs {
     DevBuf<FragRec> frags;
     DevBuf<int32_t> n_frags, fgslot, fidx;
     DevBuf<long long> fmap;
+    DevBuf<ClusterRec> crec;
     DevBuf<unsigned long long> live;  // [2] pair terms evaluated by the last launch
     DevBuf<unsigned long long> phase;  // [HP_N] clock cycles per bundle phase (when profiled)
     DevBuf<int32_t> iso;               // isolated bodies: flags, positions, list, count
@@ -1319,8 +1333,8 @@ static double g_edisp[2] = {0., 0.};
 static int g_warp_min = 8, g_cta_min = 64;
 static int g_hard_mode = 0;  // 0: bundles, 1: thread/warp/CTA tiers
 static float g_heavy = 6.75f;  // predicted log2(1 + block steps) from which a cluster runs alone (0: never)
-static int g_wide = 1;        // clusters above the bundle capacity: wide lone bundles (1) or one per CTA (0)
-static int g_bcap = 256, g_bocc = 2;  // bundle member slots and CTAs per SM (256/2, 128/3, 128/4)
+static int g_wide = 1;        // clusters above 256 members: wide lone bundles (1) or one per CTA (0)
+static int g_bcap = 128;      // bundle member slots (128: three CTAs per SM, 256: one)
 static FragParams g_frag = {0., 9.426627927538057e-12, 10, 0, 0ULL};  // off (a_frag = 0)
 static int g_frag_cap = 0;  // fragment slots of the current launch
 static int g_max_steps = MAX_BLOCK_STEPS;  // block-step cap per cluster and tree step
@@ -1457,7 +1471,6 @@ int p3t_set_hard_bundle(int member_slots, int ctas_per_sm) {
     const bool ok = (member_slots == 256 && ctas_per_sm == 2) || (member_slots == 128 && (ctas_per_sm == 3 || ctas_per_sm == 4));
     if (!ok) return ST_BAD_INDEX;
     g_bcap = member_slots;
-    g_bocc = ctas_per_sm;
     return 0;
 }
 
@@ -1509,7 +1522,7 @@ int p3t_hard_enqueue(void) {
     if ((r = B.reserve(E.n_members + g_frag_cap)) || (r = B.order.reserve(nc)) || (r = B.queue.reserve(4)) ||
         (r = B.n_cols.reserve(1)) || (r = B.cl_edisp.reserve(2 * (size_t)nc + 2)) ||
         (r = B.cols.reserve(4096)) || (r = B.frags.reserve(g_frag_cap + 1)) || (r = B.n_frags.reserve(1)) ||
-        (r = B.live.reserve(2)))
+        (r = B.live.reserve(2)) || (r = B.crec.reserve(nc)))
         return r;
     cudaMemsetAsync(B.n_frags.p, 0, sizeof(int32_t), c->stream);
     cudaMemsetAsync(B.live.p, 0, 2 * sizeof(unsigned long long), c->stream);
@@ -1536,6 +1549,9 @@ int p3t_hard_enqueue(void) {
         } else {
             prio = sched_priority(c, nc, &pmin, &pscale);
         }
+        // members a bundle can admit (with fragmentation it keeps room for a
+        // collision's fragments)
+        const int main_cap = g_bcap - (g_frag.a_frag > 0. ? 2 * g_frag.n_frag_max : 0);
         // heavy clusters: learned prediction of log2(1 + block steps) >= g_heavy;
         // lone ones: >= g_lone (the lone form is perfect accretion only)
         int heavy_key = 2147483647, lone_key = 2147483647;
@@ -1543,7 +1559,7 @@ int p3t_hard_enqueue(void) {
             heavy_key = std::min(ORDER_NB - 1, (int)((g_heavy - pmin) * pscale));
         if (prio && (int)g_prio.size() != nc && g_lone > 0.f && g_frag.a_frag <= 0. && g_hard_mode == 0)
             lone_key = std::max(0, std::min(ORDER_NB - 1, (int)((g_lone - pmin) * pscale)));
-        { P3T_COUNT_LAUNCH(); k_order_bins<<<(nc + 255) / 256, 256, 0, c->stream>>>(E.cl_cnt.p, prio, nc, g_hard_mode, g_bcap, g_warp_min, g_cta_min,
+        { P3T_COUNT_LAUNCH(); k_order_bins<<<(nc + 255) / 256, 256, 0, c->stream>>>(E.cl_cnt.p, prio, nc, g_hard_mode, main_cap, g_warp_min, g_cta_min,
                                                               pmin, pscale, heavy_key, lone_key, LCAP, B.bin.p,
                                                               B.hist.p, B.ntier.p + 3); }
         { P3T_COUNT_LAUNCH(); k_order_scan<<<1, 1024, 0, c->stream>>>(B.hist.p, B.ntier.p); }
@@ -1626,7 +1642,9 @@ int p3t_hard_integrate(int istep) {
         A.n_frags = B.n_frags.p;
         A.frag_base = E.n_members;
         A.frag_cap = g_frag_cap;
-        A.wide = g_wide;
+        A.wide_cap = g_wide ? BCAP_WIDE : BCAP_MAIN;
+        A.plain = (P.eps2 == 0. ? PL_EPS2 : 0) | (P.eps2_sun == 0. ? PL_EPS2_SUN : 0) | (P.m_sun == 1. ? PL_M_SUN : 0);
+        A.crec = B.crec.p;
         A.max_steps = g_max_steps;
         A.live = B.live.p;
         A.phase_cycles = g_hard_profile ? B.phase.p : nullptr;
@@ -1641,25 +1659,18 @@ int p3t_hard_integrate(int istep) {
             static cudaStream_t s_wide = nullptr, s_lone = nullptr;
             static cudaEvent_t ev_done = nullptr, ev_lone = nullptr;
             const int smem_w = (int)sizeof(BundleSmem<BCAP_WIDE>);
-            static_assert(sizeof(BundleSmem<BCAP_WIDE>) <= 200 * 1024, "the wide bundle fits an SM");
-            static_assert(sizeof(LoneSmem<bundle_threads(256)>) <= sizeof(BundleSmem<256>) &&
-                              sizeof(LoneSmem<BT>) <= 200 * 1024 && sizeof(LoneSmem<LONE_T>) <= LONE_EXCL_SMEM,
-                          "lone state fits the shared memory it borrows");
-            // the lone tier in the bundle CTAs: k_hard_lone with no CTAs of its own
+            static_assert(sizeof(BundleSmem<BCAP_WIDE>) <= 226 * 1024 && sizeof(BundleSmem<256>) <= 226 * 1024,
+                          "a large bundle fits an SM");
+            static_assert(sizeof(BundleSmem<128>) <= 75 * 1024, "three bundles of 128 slots fit an SM");
+            static_assert(sizeof(LoneSmem<LONE_T>) <= LONE_EXCL_SMEM, "the lone state fits its request");
             const bool lone = g_lone > 0.f && g_frag.a_frag <= 0.;
-            A.lone_in = (lone && g_lone_ctas == 0) ? 1 : 0;
-            int smem = g_bcap == 128 ? (int)sizeof(BundleSmem<128>) : (int)sizeof(BundleSmem<256>);
-            if (A.lone_in && g_bcap == 128) smem = std::max(smem, (int)sizeof(LoneSmem<BT>));
             if (!attr) {
-                if ((r = cuda_status(cudaFuncSetAttribute(k_hard_bundles<256, 2>,
+                if ((r = cuda_status(cudaFuncSetAttribute(k_hard_bundles<256, 1>,
                                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                           (int)sizeof(BundleSmem<256>)))) ||
-                    (r = cuda_status(cudaFuncSetAttribute(
-                         k_hard_bundles<128, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)std::max(sizeof(BundleSmem<128>), sizeof(LoneSmem<BT>))))) ||
-                    (r = cuda_status(cudaFuncSetAttribute(
-                         k_hard_bundles<128, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)std::max(sizeof(BundleSmem<128>), sizeof(LoneSmem<BT>))))) ||
+                    (r = cuda_status(cudaFuncSetAttribute(k_hard_bundles<128, 3>,
+                                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          (int)sizeof(BundleSmem<128>)))) ||
                     (r = cuda_status(cudaFuncSetAttribute(k_hard_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                           smem_w))) ||
                     (r = cuda_status(cudaFuncSetAttribute(k_hard_lone, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1671,10 +1682,10 @@ int p3t_hard_integrate(int istep) {
                     return r;
                 attr = true;
             }
-            // the lone clusters (with CTAs of their own) and the clusters above
-            // BCAP_MAIN bodies on streams of their own, started first so that
-            // they hold SMs from the beginning (no launch when there are none)
-            bool lone_k = lone && g_lone_ctas > 0;
+            // the lone clusters and the clusters above a bundle's slots on
+            // streams of their own, started first so that they hold SMs from
+            // the beginning (no launch when there are none)
+            bool lone_k = lone;
             if ((r = cuda_status(cudaEventRecord(g_ev_launch[0], c->stream)))) return r;
             // The wide and lone CTAs must hold their SMs before the persistent
             // bundle CTAs fill every SM (with a cross-stream event the bundle
@@ -1682,15 +1693,15 @@ int p3t_hard_integrate(int istep) {
             // library stream has drained; its tier sizes then give the wide
             // grid, and both kernels are submitted before the bundle kernel
             // with no dependency left to resolve.
-            int wide_ctas = 0;
-            if (A.wide || lone_k) {
-                int nt[3] = {0, 0, 0};
-                if ((r = d2h(c, nt, B.ntier.p, sizeof(nt)))) return r;  // synchronizes the stream
-                wide_ctas = A.wide ? std::min(nt[0], std::max(1, sms / 16)) : 0;
-                if (nt[2] == 0) lone_k = false;
-            }
+            int nt[3] = {0, 0, 0};
+            if ((r = d2h(c, nt, B.ntier.p, sizeof(nt)))) return r;  // synchronizes the stream
+            const int wide_ctas = std::min(nt[0], std::max(1, sms / 8));
+            if (nt[2] == 0) lone_k = false;
             if (lone_k) {
-                { P3T_COUNT_LAUNCH(); k_hard_lone<<<g_lone_ctas, LONE_T, LONE_EXCL_SMEM, s_lone>>>(A); }
+                // CTAs of their own hold an SM each; without, they share SMs with bundles
+                const int lc = g_lone_ctas > 0 ? g_lone_ctas : sms;
+                const int sm = g_lone_ctas > 0 ? LONE_EXCL_SMEM : (int)sizeof(LoneSmem<LONE_T>);
+                { P3T_COUNT_LAUNCH(); k_hard_lone<<<lc, LONE_T, sm, s_lone>>>(A); }
                 if ((r = cuda_status(cudaGetLastError())) || (r = cuda_status(cudaEventRecord(ev_lone, s_lone))))
                     return r;
             }
@@ -1698,14 +1709,13 @@ int p3t_hard_integrate(int istep) {
                 { P3T_COUNT_LAUNCH(); k_hard_wide<<<wide_ctas, WT, smem_w, s_wide>>>(A); }
                 if ((r = cuda_status(cudaGetLastError()))) return r;
             }
-            // persistent: g_bocc CTAs per SM (fewer when there are few clusters)
-            const int blocks = std::max(1, std::min(sms * g_bocc, (nc + 3) / 4));
+            // persistent: as many CTAs as the SMs hold (fewer when there are few clusters)
+            const int per_sm = g_bcap == 128 ? 3 : 1;
+            const int blocks = std::max(1, std::min(sms * per_sm, (nc + 3) / 4));
             if (g_bcap == 256)
-                { P3T_COUNT_LAUNCH(); k_hard_bundles<256, 2><<<blocks, bundle_threads(256), smem, c->stream>>>(A); }
-            else if (g_bocc == 3)
-                { P3T_COUNT_LAUNCH(); k_hard_bundles<128, 3><<<blocks, BT, smem, c->stream>>>(A); }
+                { P3T_COUNT_LAUNCH(); k_hard_bundles<256, 1><<<blocks, bundle_threads(256), (int)sizeof(BundleSmem<256>), c->stream>>>(A); }
             else
-                { P3T_COUNT_LAUNCH(); k_hard_bundles<128, 4><<<blocks, BT, smem, c->stream>>>(A); }
+                { P3T_COUNT_LAUNCH(); k_hard_bundles<128, 3><<<blocks, bundle_threads(128), (int)sizeof(BundleSmem<128>), c->stream>>>(A); }
             if ((r = cuda_status(cudaGetLastError()))) return r;
             if (wide_ctas > 0 && ((r = cuda_status(cudaEventRecord(ev_done, s_wide))) ||
                                   (r = cuda_status(cudaStreamWaitEvent(c->stream, ev_done, 0)))))

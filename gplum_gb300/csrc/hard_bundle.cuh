@@ -1,37 +1,48 @@
 // Lane-dense form of the hard part: one CTA integrates a "bundle" of many
-// clusters at once.
+// clusters at once, all of their state in shared memory.
 //
-// FP64 runs at 1/64 of the FP32 rate on this GPU, and a warp instruction
-// occupies the FP64 pipe for all 32 lanes whether or not they are active.  A
-// warp (or thread) per cluster leaves most lanes idle: a cluster has a few
-// active members per block step, and a serial pair loop per member has one
-// live partner in several.  Here the CTA keeps up to BCAP members of up to
-// bmaxcl(BCAP) clusters in shared memory and advances every cluster by one block
-// step per iteration, so each phase runs over the union of the bundle's
-// work items:
-//   - member phases (predict, correct, time steps) over all members or all
-//     active members of all clusters;
-//   - pair phases over (target, partner) items: an FP32 distance prefilter
-//     (with a per-cluster margin proven below) packs the live pairs into a
-//     ring in (target, partner) order; their FP64 terms are computed one pair
-//     per thread; the terms are then added to each target's accumulators in
-//     partner order, which is the summation order of the reference loop
-//     (src/gravity_hard.h:203-367), so the sums are bit-identical;
-//   - collision detection over unordered member pairs, FP32 prefilter, FP64
-//     R for the survivors and a per-cluster lexicographic (R, pair) minimum.
-// Finished clusters leave the bundle and the queue refills it, so the CTA
-// stays full until the queue is empty.  The main 256-slot bundle runs one
-// thread per slot (bundle_threads: 8 warps, 2 CTAs per SM at 128 registers):
-// the member phases are long dependent FP64 chains, and twice the warps of a
-// 128-thread bundle keep the FP64 pipe busier (55 % vs 47 % of cycles,
-// 10-11 % less time at 1M bodies).  Clusters larger than BCAP_MAIN run
-// concurrently in k_hard_wide: alone in a wide bundle of BCAP_WIDE slots, or
-// beyond that in the one-cluster-per-CTA form (run_cluster<128>).
-//
-// The global per-slot arrays (struct Hard) stay the state of record; shared
-// memory mirrors the fields that other members read (positions, velocities,
-// predicted state, masses, radii, ids, flags) and is refreshed after every
-// phase that changes them.
+// What bounds it.  An FP64 instruction holds its warp for 64 cycles whatever
+// its active lanes, with no overlap inside the warp, and an SM takes one per
+// 19 cycles from all its warps.  So (1) the launch's throughput is the number
+// of FP64 warp instructions, and (2) the span of a long chain of block steps
+// (hundreds of steps of a close pair) is the number of dependent FP64
+// instructions of one step, plus whatever the phases wait for in between.
+// Hence:
+//   - The CTA keeps up to BCAP members of up to bmaxcl(BCAP) clusters and
+//     advances every cluster by one block step per iteration, so each phase
+//     runs over the union of the bundle's work items, one lane per item:
+//     predictor per (member, component), pair terms per live (target, partner)
+//     pair, the targets' sun force in warps of its own beside them, sums and
+//     corrector per (target, component), the time-step criteria per target.
+//   - The members' state of record is shared memory (42 doubles a slot): a
+//     block step makes no trip to global memory.  The arrays of struct Hard
+//     are written only around a collision, which works on them.
+//   - Roots, reciprocals and quotients run on the integer pipe
+//     (p3t_exact.cuh), comparisons of positive doubles on their bits, products
+//     by powers of two (a block step's length) fused into the following sum
+//     where the product is exact; every rounding is that of the plain form.
+//   - When a pass has few items, the three components of an item sit in lanes
+//     of their own (bundle_terms_split), which shortens the chain; when it has
+//     many, one lane takes an item, which is the fewest instructions.
+//   - The live pairs are listed once per block step, for its three passes (a
+//     margin covers the corrector's displacement, which is checked; a pass
+//     that cannot rely on the list makes its own).
+// Measured against the form that kept the members in global memory (256 slots,
+// 2 CTAs per SM, the library's roots, a list per pass): a block step of a lone
+// pair 35 -> 15 us, of a 60-body cluster 49 -> 30 us; the hard launch of a tree
+// step 39 -> 26 ms on the 1,048,576-body ring (throughput-bound, 16 M member
+// steps), 19 -> 10 ms at 50,000 bodies and 28 -> 14 ms on the 2 M-body wide
+// disk (both bound by their longest chains).
+// Why 128 slots: three such CTAs fill an SM's shared memory (74 KB each), and
+// three independent bundles overlap one's waits with the others' FP64 work; a
+// bundle of 256 slots fits once per SM.
+// Pair terms are added to each target in partner order, the summation order
+// of the reference loop (src/gravity_hard.h:203-367), so the sums are
+// bit-identical to the one-cluster-per-team form; pairs beyond the cutoff
+// contribute exact +-0 terms to accumulators that start at +0.
+// Finished clusters leave the bundle and the queue refills it.  Clusters
+// larger than a bundle run concurrently in k_hard_wide: alone in a wide
+// bundle of BCAP_WIDE slots, or beyond that in the one-cluster-per-CTA form.
 //
 // Prefilter margins.  FP32 coordinates are taken relative to the cluster's
 // first member, u = fl32(x - ref).  While every stored |x - ref| component
@@ -43,64 +54,79 @@
 // exact R < 1 has FP32 d^2 <= thr_c (r_i + r_j)_32^2 with
 // thr_c = (1.000001 + err / (2 min f r_p))^2 * 1.000001 (both rounded up to
 // FP32).  Pairs above the thresholds are therefore beyond the cutoff (their
-// terms are exact zeros) or have R > 1, so skipping them is exact; pairs below
-// them but beyond the cutoff contribute exact +-0 terms to accumulators that
-// start at +0, which leaves every sum unchanged.
+// terms are exact zeros) or have R > 1, so skipping them is exact.  The list
+// made from the predicted positions serves the corrected ones too: it holds
+// the pairs up to thr_f (1 + 1/64)^2, and every corrected component is
+// checked to lie within r_out / 128 of its prediction.
 #pragma once
 
 namespace p3t {
 
-constexpr int BT = 128;      // threads of a bundle (one CTA) unless bundle_threads says otherwise
-constexpr int BPT = 4;       // (target, partner) items a thread tests per round of bundle_pairs
-constexpr int BCAP_MAIN = 256;  // member slots of a bundle
-constexpr int BCAP_WIDE = 512;  // member slots of the wide form (clusters of 257..512 bodies, one at a time)
-// clusters in a bundle at once: half its member slots, at most one per thread
-__host__ __device__ constexpr int bmaxcl(int cap) { return cap / 2 < 128 ? cap / 2 : 128; }
-// threads of a bundle of `cap` member slots: one per slot for the main
-// 256-slot form (8 warps; twice the warps per SM of 128 at 2 CTAs per SM,
-// for the FP64 dependency chains), 128 for the others
-__host__ __device__ constexpr int bundle_threads(int cap) { return cap == 256 ? 256 : (cap == 512 ? 512 : 128); }
+constexpr int BPT = 4;          // (target, partner) items a thread tests per round of bundle_build
+constexpr int BCAP_MAIN = 256;  // members a cluster may have to stay out of the one-per-CTA form without k_hard_wide
+constexpr int BCAP_WIDE = 512;  // member slots of the wide form (one cluster at a time)
+// clusters in a bundle at once
+__host__ __device__ constexpr int bmaxcl(int cap) { return cap > 256 ? 8 : cap / 2; }
+__host__ __device__ constexpr int bundle_threads(int cap) { return cap >= 256 ? 256 : 128; }
+// pair terms held at once, entries of the live-pair list
+__host__ __device__ constexpr int bundle_terms_cap(int cap) { return 256; }
+__host__ __device__ constexpr int bundle_list_cap(int cap) { return cap >= 256 ? 2048 : 1024; }
 constexpr int BSURV = 64;    // colliding-pair candidates kept per block step
 constexpr int BCLAIM = 8;    // clusters claimed from the queue at a time
 
 enum : int { CF_COL = 1, CF_FIN = 2, CF_FRESH = 4, CF_EXACT = 8 };
 enum : unsigned char { MF_ACT = 1, MF_TGT = 2 };
+// fields of a member slot (three components from each vector's first); F_N*:
+// the running pass's forces of a target, in the order of F_AS..F_JD
+enum : int {
+    F_POS = 0, F_VEL = 3, F_AS = 6, F_JS = 9, F_AD = 12, F_JD = 15, F_MASS = 18, F_ROI, F_TH, F_DT, F_TE, F_ACC0,
+    F_KEEP = 24,  // the fields above persist between block steps
+    F_XP = 24, F_VP = 27, F_NAS = 30, F_NJS = 33, F_NAD = 36, F_NJD = 39, F_N = 42,
+    F_PHS = F_XP, F_PHD = F_XP + 1  // potentials of a full pass (the predicted state is dead then)
+};
 
 template <int BCAP>
 struct BundleSmem {
-    static constexpr int NT = bundle_threads(BCAP);  // threads of the bundle
-    // member mirror (pool slot p)
-    double pos[3 * BCAP], vel[3 * BCAP], xp[3 * BCAP], vp[3 * BCAP];
-    double mass[BCAP], roi[BCAP], fr[BCAP];
-    double acc[7 * BCAP];  // force accumulators of the running pair phase
-    double term[7 * NT];   // FP64 pair terms of one drain
-    long long id[BCAP];
-    float pos32[3 * BCAP], xp32[3 * BCAP], roi32[BCAP], fr32[BCAP];
-    int gslot[BCAP];
-    int pfx[BCAP + 1];
-    int ring[(BPT + 1) * NT];  // live pair items: a round's BPT per thread beyond a part drain
-    int seg[NT + 1];
-    short tgt[BCAP], cl[BCAP], owner[BCAP];
-    unsigned char dead[BCAP], merged[BCAP], flag[BCAP];
+    static constexpr int S = BCAP;
+    static constexpr int NT = bundle_threads(BCAP);
+    static constexpr int NCL = bmaxcl(BCAP);
+    static constexpr int TC = bundle_terms_cap(BCAP);
+    static constexpr int LC = bundle_list_cap(BCAP);
+    double d[F_N][S];     // member state by field and slot
+    double term[6 * TC];  // pair terms of one drain
     // clusters (bundle index k)
-    double c_ts[bmaxcl(BCAP)], c_ref[3 * bmaxcl(BCAP)], c_ed[bmaxcl(BCAP)], c_edd[bmaxcl(BCAP)];
-    unsigned long long c_key[bmaxcl(BCAP)], c_red[4 * bmaxcl(BCAP)];
-    long long c_pb[bmaxcl(BCAP)], c_work[bmaxcl(BCAP)], c_t0[bmaxcl(BCAP)];
-    long long c_label[bmaxcl(BCAP)], c_fragn[bmaxcl(BCAP)];  // id_cluster, fragments made (KOMINAMI)
-    int c_n0[bmaxcl(BCAP)], c_addn[bmaxcl(BCAP)], c_addg[bmaxcl(BCAP)];  // members at admission; new fragments (count, first slot)
-    float c_thrf[bmaxcl(BCAP)], c_thrc[bmaxcl(BCAP)], c_E32[bmaxcl(BCAP)];
-    int c_idx[bmaxcl(BCAP)], c_off[bmaxcl(BCAP)], c_n[bmaxcl(BCAP)], c_goff[bmaxcl(BCAP)], c_steps[bmaxcl(BCAP)], c_ncol[bmaxcl(BCAP)];
-    int c_flags[bmaxcl(BCAP)], c_imp[bmaxcl(BCAP)], c_tar[bmaxcl(BCAP)];
+    double c_ts[NCL], c_ref[3][NCL];
+    unsigned long long c_key[NCL], c_tm[NCL], c_R[NCL];  // min th + dt, min th, min R of the step
+    long long c_pb[NCL], c_work[NCL];
     // colliding-pair candidates
     double sv_R[BSURV];
     long long sv_p[BSURV];
+    unsigned long long live[2];
+    float x32[3][S], roi32[S], fr32[S];  // prefilter copies (x32: of the running pass's positions)
+    int hmov[S];                         // high word of r_out / 128
+    int gslot[S], pfx[S + 1];
+    unsigned list[LC];  // live pairs of the pass: target index << 16 | partner slot, in (target, partner) order
+    float c_thrf[NCL], c_thrc[NCL], c_E32[NCL];
+    int c_idx[NCL], c_off[NCL], c_n[NCL], c_goff[NCL], c_steps[NCL], c_flags[NCL], c_n0[NCL], c_act[NCL];
+    int c_imp[NCL], c_tar[NCL], c_addn[NCL], c_addg[NCL];
     int sv_k[BSURV];
     // claimed, not yet admitted clusters
     int pend_c[BCLAIM], pend_n[BCLAIM];
     int ws[NT / 32];
     int used, ncl, fresh_k, fresh_p, n_sv, n_pend, i_pend, exhausted, any, grew, phase;
+    int ln, moved, any_dead;  // list entries; a corrected position left the list's margin; dead members
+    short tgt[S], cl[S], owner[S], eqc[S], twh[S], twn[S], segb[S], sege[S];
+    unsigned char dead[S], merged[S], flag[S];
     long long ph_acc[HP_N], ph_t;  // optional per-phase clock counts (thread 0)
 };
+
+// the bundle of this CTA, by its symbol: functions that are not inlined keep
+// shared-memory loads (a reference passed to them would make them generic)
+template <int BCAP>
+__device__ __forceinline__ BundleSmem<BCAP> &bundle_smem() {
+    extern __shared__ __align__(16) unsigned char bundle_raw[];
+    return *reinterpret_cast<BundleSmem<BCAP> *>(bundle_raw);
+}
 
 // the end of a phase of the bundle loop (after its barrier): thread 0 adds
 // the clock cycles since the last mark to the phase's count
@@ -112,11 +138,37 @@ struct BundleSmem {
             B.ph_t = t_;                                       \
         }                                                      \
     } while (0)
+// member- and cluster-parallel loops over the bundle
+#define FOR_SLOTS(p) for (int p = threadIdx.x; p < B.used; p += BT)
+#define FOR_CLUSTERS(k) for (int k = threadIdx.x; k < B.ncl; k += BT)
 
 __device__ __forceinline__ unsigned long long dbits(double x) {
     return (unsigned long long)__double_as_longlong(x);
 }
 __device__ __forceinline__ double bitsd(unsigned long long b) { return __longlong_as_double((long long)b); }
+__device__ __forceinline__ int dhi(double x) { return __double2hiint(x); }
+// a < b, min for doubles >= +0: by their bits (the FP64 pipe's comparison
+// costs an FP64 instruction)
+__device__ __forceinline__ bool plt(double a, double b) { return dbits(a) < dbits(b); }
+__device__ __forceinline__ double pmin(double a, double b) { return plt(b, a) ? b : a; }
+// +0 for a zero of either sign: the sum +0 + x
+__device__ __forceinline__ double from_zero(double x) { return (dbits(x) << 1) == 0ULL ? 0. : x; }
+// a normal power of two whose products with it are exact
+__device__ __forceinline__ bool is_pow2(double x) {
+    const unsigned h = (unsigned)dhi(x);
+    return __double2loint(x) == 0 && (h & 0x800fffffu) == 0u && h - 0x10000000u < 0x60000000u;
+}
+
+template <int BCAP>
+__device__ __forceinline__ V3 bld(const BundleSmem<BCAP> &B, int f, int p) {
+    return v3(B.d[f][p], B.d[f + 1][p], B.d[f + 2][p]);
+}
+template <int BCAP>
+__device__ __forceinline__ void bst(BundleSmem<BCAP> &B, int f, int p, V3 v) {
+    B.d[f][p] = v.x;
+    B.d[f + 1][p] = v.y;
+    B.d[f + 2][p] = v.z;
+}
 
 // exclusive block-wide prefix sum of v over NT threads; all threads must call
 template <int NT>
@@ -142,172 +194,65 @@ __device__ __forceinline__ int bscan(int v, int *ws, int &total) {
     return off + x - v;
 }
 
-// FP32 copy of a position relative to the cluster origin, with the bound check
+// FP32 copy of component c of a position relative to the cluster origin, with
+// the bound check
 template <int BCAP>
-__device__ __forceinline__ void st32b(BundleSmem<BCAP> &B, float *dst, int p, V3 x, int k) {
-    const float u0 = (float)(x.x - B.c_ref[3 * k]), u1 = (float)(x.y - B.c_ref[3 * k + 1]),
-                u2 = (float)(x.z - B.c_ref[3 * k + 2]);
-    dst[3 * p] = u0;
-    dst[3 * p + 1] = u1;
-    dst[3 * p + 2] = u2;
-    const float E = B.c_E32[k];
-    if (!(fabsf(u0) < E && fabsf(u1) < E && fabsf(u2) < E)) atomicOr(&B.c_flags[k], CF_EXACT);
+__device__ __forceinline__ void st32b(BundleSmem<BCAP> &B, int c, int p, double x, int k) {
+    const float u = (float)(x - B.c_ref[c][k]);
+    B.x32[c][p] = u;
+    if (!(fabsf(u) < B.c_E32[k])) atomicOr(&B.c_flags[k], CF_EXACT);
+}
+template <int BCAP>
+__device__ __forceinline__ float bd2_32(const BundleSmem<BCAP> &B, int s, int t) {
+    const float dx = B.x32[0][s] - B.x32[0][t], dy = B.x32[1][s] - B.x32[1][t], dz = B.x32[2][s] - B.x32[2][t];
+    return dx * dx + dy * dy + dz * dz;
 }
 
-// mirror every field of slot p from the state of record (global slot g)
+// ---- targets and live pairs -------------------------------------------------
+// ordered list of the occupied slots whose flag has `bit`, and the prefix of
+// their partner counts (pfx; pfx[count] = total); returns the count
 template <int BCAP>
-__device__ __forceinline__ void mirror_all(BundleSmem<BCAP> &B, const Hard &H, int p, int g, int k, bool with32) {
-    const V3 x = ld3(H.pos, g);
-    st3(B.pos, p, x);
-    st3(B.vel, p, ld3(H.vel, g));
-    st3(B.xp, p, ld3(H.xp, g));
-    st3(B.vp, p, ld3(H.vp, g));
-    B.mass[p] = H.mass[g];
-    B.roi[p] = H.r_out_inv[g];
-    const double fr = H.f[g] * H.r_planet[g];
-    B.fr[p] = fr;
-    B.fr32[p] = (float)fr;
-    B.roi32[p] = (float)H.r_out_inv[g];
-    B.id[p] = H.id[g];
-    B.dead[p] = (unsigned char)H.dead[g];
-    B.merged[p] = (unsigned char)H.merged[g];
-    B.gslot[p] = g;
-    B.cl[p] = (short)k;
-    if (with32) {
-        st32b(B, B.pos32, p, x, k);
-        st32b(B, B.xp32, p, ld3(H.xp, g), k);
-    }
-}
-
-// ---- pair phases ------------------------------------------------------------
-// ordered list of the occupied slots whose flag has `bit`
-template <int BCAP>
-__device__ int bundle_list(BundleSmem<BCAP> &B, unsigned char bit) {
-    constexpr int BT = BundleSmem<BCAP>::NT;
-    constexpr int PER = BCAP / BT;
+__device__ __forceinline__ int bundle_targets(BundleSmem<BCAP> &B, unsigned char bit) {
+    constexpr int BT = BundleSmem<BCAP>::NT, PER = BCAP / BT;
     const int base = threadIdx.x * PER;
-    int c = 0;
+    int v = 0;  // partner count << 10 | targets
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int p = base + j;
-        if (p < B.used && (B.flag[p] & bit)) c++;
+        if (p < B.used && (B.flag[p] & bit)) v += (B.c_n[B.cl[p]] << 10) | 1;
     }
     int tot;
-    int off = bscan<BT>(c, B.ws, tot);
+    int off = bscan<BT>(v, B.ws, tot);
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int p = base + j;
-        if (p < B.used && (B.flag[p] & bit)) B.tgt[off++] = (short)p;
+        if (p < B.used && (B.flag[p] & bit)) {
+            B.tgt[off & 1023] = (short)p;
+            B.pfx[off & 1023] = off >> 10;
+            off += (B.c_n[B.cl[p]] << 10) | 1;
+        }
     }
+    if (threadIdx.x == 0) B.pfx[tot & 1023] = tot >> 10;
     __syncthreads();
-    return tot;
+    return tot & 1023;
 }
 
-// the seven terms (acc_d xyz, jerk_d xyz, -phi_d) of target s from partner t,
-// the arithmetic of hard_force for one pair
+// The live pairs from item `base` of the targets' (target, partner) items on,
+// until the items end or the list is full: B.list[0..B.ln).  Returns the next
+// item.  mode 0: full (pos of both); 1: predicted i and j; 2: corrected i,
+// predicted j.  exact: FP64 tests for every cluster.  Ends with a barrier.
 template <int BCAP>
-__device__ __forceinline__ void pair_terms(const Params &P, const BundleSmem<BCAP> &B, int mode, int s, int t, double *o) {
-    V3 xi, vi, xj, vj;
-    if (mode == 1) { xi = ld3(B.xp, s); vi = ld3(B.vp, s); }
-    else { xi = ld3(B.pos, s); vi = ld3(B.vel, s); }
-    if (mode == 0) { xj = ld3(B.pos, t); vj = ld3(B.vel, t); }
-    else { xj = ld3(B.xp, t); vj = ld3(B.vp, t); }
-    const V3 dr = xj - xi;
-    double dr2 = dot(dr, dr);
-    dr2 += P.eps2;
-    const double r_out_inv = dmin(B.roi[s], B.roi[t]);
-    const V3 dv = vj - vi;
-    const double rij = sqrt(dr2);
-    const double rinv = 1. / rij;
-    const double r2inv = rinv * rinv;
-    const double r3inv = r2inv * rinv;
-    const double mj = B.mass[t];
-    const double mr3 = mj * r3inv;
-    const double alpha = dot(dr, dv) * r2inv;
-    double Wc = 0.;
-    if (mode == 0) Wc = 1. - cut_W(P, rij, r_out_inv);
-    const double Kc = 1. - cut_K(P, rij, r_out_inv);
-    const double dKdt = cut_dKdt(P, rij, r_out_inv, alpha);
-    const double alpha_c = alpha * Kc;
-    const V3 a = mr3 * Kc * dr;
-    const V3 j = mr3 * (Kc * dv - (3. * alpha_c + dKdt) * dr);
-    o[0] = a.x; o[1] = a.y; o[2] = a.z;
-    o[3] = j.x; o[4] = j.y; o[5] = j.z;
-    o[6] = (mode == 0) ? -(mj * rinv * Wc) : 0.;
-}
-
-// terms of ring[0..m), then in-order addition into the targets' accumulators
-template <int BCAP>
-__device__ void bundle_drain(const Params &P, BundleSmem<BCAP> &B, const int *ring, int mode, int m) {
+__device__ __forceinline__ int bundle_build(const HardArgs &A, BundleSmem<BCAP> &B, int mode, int nt, int base, bool exact) {
     constexpr int BT = BundleSmem<BCAP>::NT;
-    const int q = threadIdx.x;
-    int sq = -1;
-    if (q < m) {
-        const int e = ring[q];
-        sq = e >> 16;
-        double o[7];
-        pair_terms(P, B, mode, sq, e & 0xffff, o);
-#pragma unroll
-        for (int c = 0; c < 7; c++) B.term[c * BT + q] = o[c];
-    }
-    const int head = (q < m) && (q == 0 || (ring[q - 1] >> 16) != sq);
-    int nseg;
-    const int off = bscan<BT>(head, B.ws, nseg);
-    if (head) B.seg[off] = q;
-    if (q == 0) B.seg[nseg] = m;
-    __syncthreads();
-    const int ncomp = (mode == 0) ? 7 : 6;
-    for (int it = q; it < ncomp * nseg; it += BT) {
-        const int j = it / ncomp, c = it - ncomp * j;
-        const int a = B.seg[j], b = B.seg[j + 1];
-        const int s = ring[a] >> 16;
-        double acc = B.acc[c * BCAP + s];
-        for (int k = a; k < b; k++) acc += B.term[c * BT + k];
-        B.acc[c * BCAP + s] = acc;
-    }
-    __syncthreads();
-}
-
-// mode 0: full (pos/vel, with phi); 1: predicted i and j; 2: corrected i,
-// predicted j -- for the nt targets in B.tgt
-template <int BCAP>
-__device__ void bundle_pairs(const HardArgs &A, BundleSmem<BCAP> &B, int mode, int nt) {
-    constexpr int BT = BundleSmem<BCAP>::NT;
-    const int tid = threadIdx.x;
-    constexpr int PER = BCAP / BT;
-    for (int i = tid; i < nt; i += BT) {
-        const int s = B.tgt[i];
-#pragma unroll
-        for (int c = 0; c < 7; c++) B.acc[c * BCAP + s] = 0.;
-    }
-    // partner-count prefix over the targets
-    int total;
-    {
-        const int base = tid * PER;
-        int c = 0;
-#pragma unroll
-        for (int j = 0; j < PER; j++)
-            if (base + j < nt) c += B.c_n[B.cl[B.tgt[base + j]]];
-        int off = bscan<BT>(c, B.ws, total);
-#pragma unroll
-        for (int j = 0; j < PER; j++)
-            if (base + j < nt) {
-                B.pfx[base + j] = off;
-                off += B.c_n[B.cl[B.tgt[base + j]]];
-            }
-        if (tid == 0) B.pfx[nt] = total;
-        __syncthreads();
-    }
-    const float *xi32 = (mode == 1) ? B.xp32 : B.pos32;
-    const float *xj32 = (mode == 0) ? B.pos32 : B.xp32;
-    // rounds of BPT consecutive items per thread (the ring stays in (target,
-    // partner) order); full drains of BT items as the ring fills
-    int ring_n = 0;
-    long long n_live = 0;
-    for (int base = 0; base < total; base += BPT * BT) {
-        const int f0 = base + BPT * tid;
-        int e[BPT], nl = 0;
-        unsigned lv = 0u;
+    const int tid = threadIdx.x, total = B.pfx[nt];
+    const float mg = mode == 0 ? 1.f : 1.033f;  // (1 + 1/64)^2 and the product's rounding
+    for (int i = tid; i < nt; i += BT) B.segb[i] = B.sege[i] = 0;
+    int n = 0;
+    while (base < total && n + BPT * BT <= BundleSmem<BCAP>::LC) {
+        const int per = (total - base <= BT) ? 1 : BPT;  // few items: one a thread
+        const int f0 = base + per * tid;
+        unsigned e[BPT], lv = 0u;
+        int nl = 0;
         if (f0 < total) {
             int lo = 0, hi = nt - 1;
             while (lo < hi) {
@@ -318,91 +263,373 @@ __device__ void bundle_pairs(const HardArgs &A, BundleSmem<BCAP> &B, int mode, i
 #pragma unroll
             for (int u = 0; u < BPT; u++) {
                 const int f = f0 + u;
-                e[u] = 0;
-                if (f >= total) continue;
+                e[u] = 0u;
+                if (u >= per || f >= total) continue;
                 while (B.pfx[lo + 1] <= f) lo++;
                 const int s = B.tgt[lo], k = B.cl[s];
                 const int t = B.c_off[k] + (f - B.pfx[lo]);
                 int live = 0;
-                if (B.id[s] != B.id[t]) {
-                    if (!(B.c_flags[k] & CF_EXACT)) {
+                if (B.eqc[s] != B.eqc[t]) {
+                    if (!exact && !(B.c_flags[k] & CF_EXACT)) {
                         const float rf = fminf(B.roi32[s], B.roi32[t]);
-                        live = d2_32(xi32, s, xj32, t) * (rf * rf) <= B.c_thrf[k];
+                        live = bd2_32(B, s, t) * (rf * rf) <= B.c_thrf[k] * mg;
                     } else {
-                        const V3 xi = ld3((mode == 1) ? B.xp : B.pos, s);
-                        const V3 dr = ld3((mode == 0) ? B.pos : B.xp, t) - xi;
+                        const V3 dr = bld(B, mode == 0 ? F_POS : F_XP, t) - bld(B, mode == 1 ? F_XP : F_POS, s);
                         double dr2 = dot(dr, dr);
                         dr2 += A.P.eps2;
-                        const double r = dmin(B.roi[s], B.roi[t]);
-                        live = !(dr2 * r * r > 1.000001);
+                        const double r = pmin(B.d[F_ROI][s], B.d[F_ROI][t]);
+                        live = !(dr2 * r * r > (mode == 1 ? 1.033 : 1.000001));
                     }
                 }
-                e[u] = (s << 16) | t;
+                e[u] = ((unsigned)lo << 16) | (unsigned)t;
                 lv |= (unsigned)live << u;
                 nl += live;
             }
         }
         int cnt;
-        int off = ring_n + bscan<BT>(nl, B.ws, cnt);
+        int off = n + bscan<BT>(nl, B.ws, cnt);
 #pragma unroll
         for (int u = 0; u < BPT; u++)
-            if ((lv >> u) & 1u) B.ring[off++] = e[u];
-        ring_n += cnt;
-        n_live += cnt;
-        __syncthreads();
-        int head = 0;
-        while (ring_n - head >= BT) {
-            const long long t0 = (A.phase_cycles && tid == 0) ? clock64() : 0;
-            bundle_drain(A.P, B, B.ring + head, mode, BT);
-            if (A.phase_cycles && tid == 0) B.ph_acc[HP_DRAIN] += clock64() - t0;
-            head += BT;
+            if ((lv >> u) & 1u) B.list[off++] = e[u];
+        n += cnt;
+        base += per * BT;
+    }
+    if (tid == 0) B.ln = n;
+    __syncthreads();
+    // each target's run of the list
+    for (int q = tid; q < n; q += BT) {
+        const int ti = B.list[q] >> 16;
+        const int tp = q > 0 ? (int)(B.list[q - 1] >> 16) : -1;
+        if (ti != tp) {
+            B.segb[ti] = (short)q;
+            if (tp >= 0) B.sege[tp] = (short)q;
         }
-        if (head > 0) {
-            // the rest (fewer than BT items, at or beyond BT) to the front
-            const int rest = ring_n - head;
-            if (tid < rest) B.ring[tid] = B.ring[head + tid];
-            ring_n = rest;
+        if (q == n - 1) B.sege[ti] = (short)n;
+    }
+    return base;
+}
+
+// ---- pair terms ---------------------------------------------------------------
+// where a pair sits in the cutoff function's range: x = (gamma - y) /
+// (gamma - 1) < 0 inside gamma r_out (K = 0), >= 1 beyond r_out (K = 1)
+__device__ __forceinline__ bool kx_near(double x) { return dhi(x) < 0 && (dbits(x) << 1) != 0ULL; }
+__device__ __forceinline__ bool kx_far(double x) { return dhi(x) >= 0x3ff00000; }
+
+// 1 - K and the bracket 140 x^3 (x-1)^3 r_out_inv / (1 - gamma) of dK/dt for a
+// pair that is not near; the operand order of cut_Kx and cut_dKdt
+__device__ __forceinline__ void kx_mid(const Params &P, double x, double r_out_inv, double &Kc, double &dKdr) {
+    const double x2 = x * x, x_1 = x - 1.;
+    const bool near = kx_near(x), far = kx_far(x);
+    const double K = (((-20. * x + 70.) * x - 84.) * x + 35.) * x2 * x2;
+    const double D = 140. * x * x * x * x_1 * x_1 * x_1 * r_out_inv * P.g_1_inv;
+    Kc = near ? 1. : (far ? 0. : 1. - K);
+    dKdr = (near || far) ? 0. : D;
+}
+
+// the seven terms (acc_d xyz, jerk_d xyz, phi_d) of target s from partner t:
+// the arithmetic of hard_force for one pair.  Near pairs (K = 0, 1 - K = 1,
+// dK/dt = 0) need 37 FP64 operations, the others 63.
+template <int BCAP>
+__device__ __forceinline__ void pair_terms(const HardArgs &A, const BundleSmem<BCAP> &B, int fi, int fj, bool phi,
+                                           int s, int t, bool mine, double *o, int st) {
+    const Params &P = A.P;
+    const V3 dr = bld(B, fj, t) - bld(B, fi, s);
+    double dr2 = dot(dr, dr);
+    if (!(A.plain & PL_EPS2)) dr2 += P.eps2;
+    const double r_out_inv = pmin(B.d[F_ROI][s], B.d[F_ROI][t]);
+    const V3 dv = bld(B, fj + 3, t) - bld(B, fi + 3, s);
+    const double rij = sqrt_rn(dr2);
+    const double rinv = rcp_rn(rij);
+    const double r2inv = rinv * rinv;
+    const double mj = B.d[F_MASS][t];
+    const double mr3 = mj * (r2inv * rinv);
+    const double alpha = dot(dr, dv) * r2inv;
+    if (phi && mine) {
+        const double Wc = 1. - cut_W(P, rij, r_out_inv);
+        o[6 * st] = mj * rinv * Wc;
+    }
+    const double x = (P.gamma - rij * r_out_inv) * P.g_1_inv;
+    double b = 3. * alpha, mk = mr3;
+    V3 kv = dv;
+    if (!__all_sync(0xffffffffu, kx_near(x))) {
+        double Kc, dKdr;
+        kx_mid(P, x, r_out_inv, Kc, dKdr);
+        b = 3. * (alpha * Kc) + alpha * rij * dKdr;
+        kv = Kc * dv;
+        mk = mr3 * Kc;
+    }
+    if (!mine) return;
+    o[0] = mk * dr.x; o[st] = mk * dr.y; o[2 * st] = mk * dr.z;
+    o[3 * st] = mr3 * (kv.x - b * dr.x);
+    o[4 * st] = mr3 * (kv.y - b * dr.y);
+    o[5 * st] = mr3 * (kv.z - b * dr.z);
+}
+
+// sun_force (p3t_phys.cuh) of target s into its running forces
+template <int BCAP>
+__device__ __forceinline__ void sun_terms(const HardArgs &A, BundleSmem<BCAP> &B, int fi, bool phi, int s) {
+    const Params &P = A.P;
+    const V3 x = bld(B, fi, s), v = bld(B, fi + 3, s);
+    double r2 = dot(x, x);
+    if (!(A.plain & PL_EPS2_SUN)) r2 += P.eps2_sun;
+    const double r2inv = rcp_rn(r2);
+    const double rinv = sqrt_rn(r2inv);
+    double mr3 = rinv * r2inv;
+    if (!(A.plain & PL_M_SUN)) mr3 = P.m_sun * mr3;
+    const double alpha = dot(x, v) * r2inv;
+    if (phi) B.d[F_PHS][s] = -P.m_sun * rinv;
+    const V3 dr = v3(-x.x, -x.y, -x.z), dv = v3(-v.x, -v.y, -v.z);
+    bst(B, F_NAS, s, mr3 * dr);
+    bst(B, F_NJS, s, mr3 * (dv - 3. * alpha * dr));
+}
+
+// terms of list[q0..q1) and, with sun, the targets' sun force: one lane an item
+template <int BCAP>
+__device__ __forceinline__ void bundle_terms(const HardArgs &A, BundleSmem<BCAP> &B, int fi, int fj, bool phi, int q0,
+                                             int np, int ns, int st) {
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    const int np32 = (np + 31) & ~31;  // pairs and sun forces in different warps
+    const int lane = threadIdx.x & 31;
+    for (int w0 = threadIdx.x - lane; w0 < np32 + ns; w0 += BT) {  // whole warps
+        const int it = w0 + lane;
+        if (w0 < np32) {
+            const unsigned e = B.list[q0 + min(it, np - 1)];
+            pair_terms(A, B, fi, fj, phi, B.tgt[e >> 16], e & 0xffffu, it < np, B.term + it, st);
+        } else if (it < np32 + ns) {
+            sun_terms(A, B, fi, phi, B.tgt[it - np32]);
+        }
+    }
+}
+
+// The same with the components of an item in three lanes of four (at most
+// NT / 4 items): each lane computes its component's differences and products,
+// the sums of three are gathered by shuffles in the order of dot().
+template <int BCAP>
+__device__ __forceinline__ void bundle_terms_split(const HardArgs &A, BundleSmem<BCAP> &B, int fi, int fj, int q0,
+                                                   int np, int ns, int st) {
+    const Params &P = A.P;
+    const int np8 = (np + 7) & ~7;
+    const int it = threadIdx.x >> 2, c = min((int)(threadIdx.x & 3), 2);
+    const int w8 = it & ~7;  // the warp's first item
+    if (w8 >= np8 + ns) return;
+    constexpr unsigned ALL = 0xffffffffu;
+    const bool sun = w8 >= np8;
+    const bool mine = (threadIdx.x & 3) < 3 && (sun ? it < np8 + ns : it < np);
+    auto dot3 = [&](double p) {
+        const double a = __shfl_sync(ALL, p, 0, 4), b = __shfl_sync(ALL, p, 1, 4), d = __shfl_sync(ALL, p, 2, 4);
+        return a + b + d;
+    };
+    if (!sun) {
+        const unsigned e = B.list[q0 + min(it, np - 1)];
+        const int s = B.tgt[e >> 16], t = e & 0xffffu;
+        const double dr = B.d[fj + c][t] - B.d[fi + c][s];
+        double dr2 = dot3(dr * dr);
+        if (!(A.plain & PL_EPS2)) dr2 += P.eps2;
+        const double r_out_inv = pmin(B.d[F_ROI][s], B.d[F_ROI][t]);
+        const double dv = B.d[fj + 3 + c][t] - B.d[fi + 3 + c][s];
+        const double rv = dot3(dr * dv);
+        const double rij = sqrt_rn(dr2);
+        const double rinv = rcp_rn(rij);
+        const double r2inv = rinv * rinv;
+        const double mr3 = B.d[F_MASS][t] * (r2inv * rinv);
+        const double alpha = rv * r2inv;
+        const double x = (P.gamma - rij * r_out_inv) * P.g_1_inv;
+        double b = 3. * alpha, kv = dv, mk = mr3;
+        if (!__all_sync(ALL, kx_near(x))) {
+            double Kc, dKdr;
+            kx_mid(P, x, r_out_inv, Kc, dKdr);
+            b = 3. * (alpha * Kc) + alpha * rij * dKdr;
+            kv = Kc * dv;
+            mk = mr3 * Kc;
+        }
+        const double a = mk * dr, j = mr3 * (kv - b * dr);
+        if (mine) {
+            B.term[c * st + it] = a;
+            B.term[(3 + c) * st + it] = j;
+        }
+    } else {
+        const int s = B.tgt[min(it - np8, ns - 1)];
+        const double x = B.d[fi + c][s], v = B.d[fi + 3 + c][s];
+        double r2 = dot3(x * x);
+        const double xv = dot3(x * v);
+        if (!(A.plain & PL_EPS2_SUN)) r2 += P.eps2_sun;
+        const double r2inv = rcp_rn(r2);
+        const double rinv = sqrt_rn(r2inv);
+        double mr3 = rinv * r2inv;
+        if (!(A.plain & PL_M_SUN)) mr3 = P.m_sun * mr3;
+        const double alpha = xv * r2inv;
+        const double a = mr3 * -x, j = mr3 * (-v - 3. * alpha * -x);
+        if (mine) {
+            B.d[F_NAS + c][s] = a;
+            B.d[F_NJS + c][s] = j;
+        }
+    }
+}
+
+// ---- sums and corrector ---------------------------------------------------------
+// component c of FPHard::correct (src/particle.h:1208-1274) for target slot s:
+// correct()'s roundings with 2 J0, -2 Am and, for a power-of-two Dt, the
+// products by Dt fused where they are exact.  last: also a2 and a3, over the
+// step's starting acc and jerk (which nothing reads after it).
+template <int BCAP>
+__device__ __forceinline__ void correct_comp(BundleSmem<BCAP> &B, int s, int c, double as, double js, double ad,
+                                             double jd, bool last) {
+    const int k = B.cl[s];
+    const double Dt = B.c_ts[k] - B.d[F_TH][s];
+    const double J0_s = Dt * B.d[F_JS + c][s], J1_s = Dt * js, Am_s = as - B.d[F_AS + c][s];
+    const double A2_s = 3. * Am_s - fma(2., J0_s, J1_s);
+    const double A3_s = fma(-2., Am_s, J1_s + J0_s);
+    const double J0_d = B.d[F_JD + c][s] * Dt, J1_d = jd * Dt, Am_d = ad - B.d[F_AD + c][s];
+    const double A2_d = 3. * Am_d - fma(2., J0_d, J1_d);
+    const double A3_d = fma(-2., Am_d, J1_d + J0_d);
+    const double A2 = A2_s + A2_d, A3 = A3_s + A3_d;
+    const double dx = 1.6666666666666667e-2 * (Dt * Dt) * (5. * A2 + 3. * 1.1666666666666667e-3 * A3);
+    const double dv = 8.3333333333333333e-2 * Dt * fma(4., A2, 3. * A3);
+    B.d[F_POS + c][s] = B.d[F_XP + c][s] + dx;
+    B.d[F_VEL + c][s] = B.d[F_VP + c][s] + dv;
+    if ((dhi(dx) & 0x7fffffff) >= B.hmov[s]) B.moved = 1;
+    if (last) {
+        const double Di = recip_pow2_or_div(Dt), Di2 = Di * Di, Di3 = Di2 * Di;
+        const double t2 = 2. * Di2, t3 = 6. * Di3;
+        B.d[F_AS + c][s] = t2 * (A2_s + 3. * A3_s);
+        B.d[F_JS + c][s] = t3 * A3_s;
+        B.d[F_AD + c][s] = (2. * (A2_d + 3. * A3_d)) * Di2;
+        B.d[F_JD + c][s] = (6. * A3_d) * Di3;
+    }
+}
+
+// mergeAccJerk (src/hermite.h:36-83) of merged target s: twins in insertion order
+template <int BCAP>
+__device__ __noinline__ void bundle_merge(int s) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    V3 a = B.d[F_MASS][s] * bld(B, F_NAD, s), j = B.d[F_MASS][s] * bld(B, F_NJD, s);
+    double m = B.d[F_MASS][s];
+    for (int k = B.twh[s], g = 0; k >= 0 && g < BCAP; k = B.twn[k], g++) {
+        addto(a, B.d[F_MASS][k] * bld(B, F_NAD, k));
+        addto(j, B.d[F_MASS][k] * bld(B, F_NJD, k));
+        m += B.d[F_MASS][k];
+    }
+    const double mi = 1. / m;
+    a = a * mi;
+    j = j * mi;
+    bst(B, F_NAD, s, a);
+    bst(B, F_NJD, s, j);
+    for (int k = B.twh[s], g = 0; k >= 0 && g < BCAP; k = B.twn[k], g++) {
+        bst(B, F_NAD, k, a);
+        bst(B, F_NJD, k, j);
+    }
+}
+
+// One force pass over the nt targets: list, terms, in-order sums into the
+// targets' running forces, mergeAccJerk for merged targets (in a full pass
+// those with twins).  corr 1, 2: then the first or second correction.  phi: the
+// potentials too (a full pass at a cluster's end).  Ends with a barrier.
+template <int BCAP, bool FULL>
+__device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> &B, int mode, int nt, bool want_phi,
+                                            int corr, bool &listed) {
+    constexpr int BT = BundleSmem<BCAP>::NT, TC = BundleSmem<BCAP>::TC;
+    const int tid = threadIdx.x;
+    const bool phi = FULL && want_phi;
+    const int fi = mode == 1 ? F_XP : F_POS, fj = FULL ? F_POS : F_XP;
+    const int st = phi ? (6 * TC) / 7 : TC;  // terms held at once
+    const bool merge = B.any_dead != 0;
+    const bool exact = mode == 2 && B.moved != 0;
+    if (exact) listed = false;
+    int base = 0;
+    bool first = true, more = true;
+    while (more) {
+        if (!listed) {
+            base = bundle_build(A, B, mode, nt, base, exact);
+            more = base < B.pfx[nt];
+            listed = first && !more && !exact;
+        } else {
+            more = false;
+        }
+        const int n = B.ln;
+        if (tid == 0) B.live[mode == 0 ? 1 : 0] += n;
+        int q0 = 0;
+        do {
+            const int np = min(n - q0, st), ns = first ? nt : 0;
+            if (!phi && ((np + 7) & ~7) + ns <= BT / 4) bundle_terms_split(A, B, fi, fj, q0, np, ns, st);
+            else bundle_terms(A, B, fi, fj, phi, q0, np, ns, st);
+            __syncthreads();
+            HP_MARK(HP_PAIRS);
+            const bool end = q0 + np >= n && !more;
+            const bool fuse = corr && end && !merge;
+            for (int it = tid; it < 3 * nt; it += BT) {
+                const int t = it / 3, c = it - 3 * t, s = B.tgt[t];
+                double ad = first ? 0. : B.d[F_NAD + c][s], jd = first ? 0. : B.d[F_NJD + c][s];
+                int k = max((int)B.segb[t], q0) - q0;
+                const int ke = min((int)B.sege[t], q0 + np) - q0;
+                if (first && k < ke) {
+                    ad = from_zero(B.term[c * st + k]);
+                    jd = from_zero(B.term[(3 + c) * st + k]);
+                    k++;
+                }
+                for (; k < ke; k++) {
+                    ad += B.term[c * st + k];
+                    jd += B.term[(3 + c) * st + k];
+                }
+                B.d[F_NAD + c][s] = ad;
+                B.d[F_NJD + c][s] = jd;
+                if (fuse) correct_comp(B, s, c, B.d[F_NAS + c][s], B.d[F_NJS + c][s], ad, jd, corr == 2);
+            }
+            if (phi)
+                for (int t = tid; t < nt; t += BT) {
+                    const int s = B.tgt[t];
+                    double ph = first ? 0. : B.d[F_PHD][s];
+                    const int ke = min((int)B.sege[t], q0 + np) - q0;
+                    for (int k = max((int)B.segb[t], q0) - q0; k < ke; k++) ph -= B.term[6 * st + k];
+                    B.d[F_PHD][s] = ph;
+                }
+            __syncthreads();
+            first = false;
+            q0 += np;
+        } while (q0 < n);
+    }
+    if (merge) {
+        for (int t = tid; t < nt; t += BT) {
+            const int s = B.tgt[t];
+            if (mode == 0 ? (B.merged[s] && B.twh[s] >= 0) : (!B.dead[s] && B.merged[s])) bundle_merge<BCAP>(s);
+        }
+        __syncthreads();
+        if (corr) {
+            for (int it = tid; it < 3 * nt; it += BT) {
+                const int t = it / 3, c = it - 3 * t, s = B.tgt[t];
+                correct_comp(B, s, c, B.d[F_NAS + c][s], B.d[F_NJS + c][s], B.d[F_NAD + c][s], B.d[F_NJD + c][s],
+                             corr == 2);
+            }
             __syncthreads();
         }
     }
-    if (ring_n > 0) {
-        const long long t0 = (A.phase_cycles && tid == 0) ? clock64() : 0;
-        bundle_drain(A.P, B, B.ring, mode, ring_n);
-        if (A.phase_cycles && tid == 0) B.ph_acc[HP_DRAIN] += clock64() - t0;
-    }
-    if (A.live && tid == 0) atomicAdd(&A.live[mode == 0 ? 1 : 0], (unsigned long long)n_live);
+    HP_MARK(HP_CORRECT);
 }
 
-// sun force and the accumulated pair sums of the targets to the state of
-// record, then mergeAccJerk for the merged targets (merge_sel 1: active
-// phase, merged alive targets; 2: all merged targets with twins)
+// a full pass over the flagged slots' targets: FP32 copies of their clusters'
+// positions, then the pass
 template <int BCAP>
-__device__ void bundle_finalize(const HardArgs &A, BundleSmem<BCAP> &B, int mode, int nt, int merge_sel) {
+__device__ __noinline__ int bundle_full(const HardArgs &A, bool phi) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     constexpr int BT = BundleSmem<BCAP>::NT;
-    const Hard &H = A.H;
-    for (int i = threadIdx.x; i < nt; i += BT) {
-        const int s = B.tgt[i], g = B.gslot[s];
-        V3 xi, vi, as, js;
-        if (mode == 1) { xi = ld3(B.xp, s); vi = ld3(B.vp, s); }
-        else { xi = ld3(B.pos, s); vi = ld3(B.vel, s); }
-        if (mode == 0) {
-            double phs;
-            sun_force(A.P, xi, vi, as, js, &phs);
-            H.phi_s[g] = phs;
-            H.phi_d[g] = B.acc[6 * BCAP + s];
-        } else {
-            sun_force(A.P, xi, vi, as, js, nullptr);
-        }
-        st3(H.acc_s, g, as);
-        st3(H.jerk_s, g, js);
-        st3(H.acc_d, g, v3(B.acc[s], B.acc[BCAP + s], B.acc[2 * BCAP + s]));
-        st3(H.jerk_d, g, v3(B.acc[3 * BCAP + s], B.acc[4 * BCAP + s], B.acc[5 * BCAP + s]));
+    FOR_SLOTS(p) {
+        if (!(B.flag[p] & MF_TGT)) continue;
+        const int k = B.cl[p];
+#pragma unroll 1
+        for (int c = 0; c < 3; c++) st32b(B, c, p, B.d[F_POS + c][p], k);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt; i += BT) {
-        const int s = B.tgt[i], g = B.gslot[s];
-        const bool m = (merge_sel == 1) ? (!B.dead[s] && B.merged[s]) : (B.merged[s] && H.tw_head[g] >= 0);
-        if (m) merge_acc_jerk(H, g);
+    const int nt = bundle_targets(B, MF_TGT);
+    bool listed = false;
+    bundle_pass<BCAP, true>(A, B, 0, nt, phi, 0, listed);
+    return nt;
+}
+
+// the running forces of the targets become their state
+template <int BCAP>
+__device__ __forceinline__ void bundle_take(BundleSmem<BCAP> &B, int nt) {
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    for (int it = threadIdx.x; it < 12 * nt; it += BT) {
+        const int t = it / 12, f = it - 12 * t, s = B.tgt[t];
+        B.d[F_AS + f][s] = B.d[F_NAS + f][s];
     }
     __syncthreads();
 }
@@ -411,45 +638,81 @@ __device__ void bundle_finalize(const HardArgs &A, BundleSmem<BCAP> &B, int mode
 // unordered pairs {a, b} of each cluster, balanced over members: member a
 // takes b = a + d (mod n) for d = 1..n/2 (the pair at distance n/2 once)
 template <int BCAP>
-__device__ void bundle_detect(const HardArgs &A, BundleSmem<BCAP> &B, bool second) {
+__device__ __forceinline__ void bundle_detect(const HardArgs &A, BundleSmem<BCAP> &B, bool second) {
     constexpr int BT = BundleSmem<BCAP>::NT;
-    for (int p = threadIdx.x; p < B.used; p += BT) {
+    FOR_SLOTS(p) {
         if (B.dead[p]) continue;
         const int k = B.cl[p];
         const int o = B.c_off[k], n = B.c_n[k], a = p - o;
         const bool exact = (B.c_flags[k] & CF_EXACT) != 0;
-        const float thr = B.c_thrc[k];
+        const float thr = B.c_thrc[k], fr = B.fr32[p];
         for (int d = 1; 2 * d <= n; d++) {
             if (2 * d == n && a >= d) break;
             int b = a + d;
             if (b >= n) b -= n;
             const int q = o + b;
-            if (B.dead[q]) continue;
             if (!exact) {
-                const float rs = B.fr32[p] + B.fr32[q];
-                if (d2_32(B.xp32, p, B.xp32, q) > thr * (rs * rs)) continue;
+                const float rs = fr + B.fr32[q];
+                if (bd2_32(B, p, q) > thr * (rs * rs)) continue;
             }
+            if (B.dead[q]) continue;
             const int lo = (a < b) ? a : b, hi = (a < b) ? b : a;
-            const V3 dr = ld3(B.xp, o + lo) - ld3(B.xp, o + hi);
+            const int gl = B.gslot[o + lo], gh = B.gslot[o + hi];
+            const V3 dr = bld(B, F_XP, o + lo) - bld(B, F_XP, o + hi);
             const double d2 = dot(dr, dr);
-            const double r2 = B.fr[o + lo] + B.fr[o + hi];
+            const double r2 = A.H.f[gl] * A.H.r_planet[gl] + A.H.f[gh] * A.H.r_planet[gh];
             if (d2 > r2 * r2 * 1.000001) continue;
             const double R = sqrt(d2) / r2;
             if (!(R < 1.)) continue;
             const long long pp = (long long)lo * n + hi;
             if (!second) {
-                atomicMin(&B.c_key[k], dbits(R));
+                atomicMin(&B.c_R[k], dbits(R));
                 const int i = atomicAdd(&B.n_sv, 1);
                 if (i < BSURV) {
                     B.sv_k[i] = k;
                     B.sv_R[i] = R;
                     B.sv_p[i] = pp;
                 }
-            } else if (dbits(R) == B.c_key[k]) {
-                atomicMin(&B.c_pb[k], pp);
+            } else if (dbits(R) == B.c_R[k]) {
+                atomicMin((unsigned long long *)&B.c_pb[k], (unsigned long long)pp);
             }
         }
     }
+}
+
+// the colliding pair of each cluster that has one (the smallest R, then the
+// first ordered pair), and the block step of its alive members
+template <int BCAP>
+__device__ __noinline__ void bundle_collisions_found(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    if (B.n_sv <= BSURV) {
+        for (int i = threadIdx.x; i < B.n_sv; i += BT)
+            if (dbits(B.sv_R[i]) == B.c_R[B.sv_k[i]])
+                atomicMin((unsigned long long *)&B.c_pb[B.sv_k[i]], (unsigned long long)B.sv_p[i]);
+    } else {
+        bundle_detect(A, B, true);
+    }
+    __syncthreads();
+    FOR_CLUSTERS(k) {
+        if (B.c_R[k] < dbits(1.)) {
+            B.c_flags[k] |= CF_COL;
+            const int o = B.c_off[k], n = B.c_n[k];
+            const int a = (int)(B.c_pb[k] / n), b = (int)(B.c_pb[k] % n);
+            if (B.d[F_MASS][o + a] < B.d[F_MASS][o + b]) { B.c_imp[k] = o + a; B.c_tar[k] = o + b; }
+            else { B.c_imp[k] = o + b; B.c_tar[k] = o + a; }
+            B.c_act[k] = 0;
+        }
+    }
+    __syncthreads();
+    FOR_SLOTS(p) {
+        const int k = B.cl[p];
+        if (!(B.c_flags[k] & CF_COL)) continue;
+        B.d[F_DT][p] = B.c_ts[k] - B.d[F_TH][p];
+        B.flag[p] = B.dead[p] ? 0 : (MF_ACT | MF_TGT);
+        if (!B.dead[p]) atomicAdd(&B.c_act[k], 1);
+    }
+    __syncthreads();
 }
 
 // ---- bundle lifecycle ---------------------------------------------------------------
@@ -459,7 +722,8 @@ __device__ void bundle_detect(const HardArgs &A, BundleSmem<BCAP> &B, bool secon
 // predicted long chains of block steps), one at a time and alone in the
 // bundle, so their iterations stay short; phase 1: the rest, packed.
 template <int BCAP>
-__device__ void bundle_refill(const HardArgs &A, BundleSmem<BCAP> &B) {
+__device__ __noinline__ void bundle_refill(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     const int lane = threadIdx.x & 31;
     const int n_heavy = A.n_tier[3];
     if (threadIdx.x < 32) {
@@ -541,9 +805,23 @@ __device__ void bundle_refill(const HardArgs &A, BundleSmem<BCAP> &B) {
     __syncthreads();
 }
 
-// load the fresh clusters (bundle indices fresh_k..ncl-1, slots fresh_p..used-1)
+// the start of a block step for the clusters from k0 on: the step's time and
+// the collision keys
 template <int BCAP>
-__device__ void bundle_load(const HardArgs &A, BundleSmem<BCAP> &B) {
+__device__ __forceinline__ void bundle_open(BundleSmem<BCAP> &B, int k) {
+    B.c_ts[k] = bitsd(B.c_key[k]);
+    B.c_R[k] = dbits(1.);
+    B.c_pb[k] = 0x7fffffffffffffffLL;
+    B.c_flags[k] &= ~CF_COL;
+    B.c_act[k] = 0;
+    B.c_steps[k]++;
+}
+
+// load the fresh clusters (bundle indices fresh_k..ncl-1, slots
+// fresh_p..used-1), their first full force and the time of their first step
+template <int BCAP>
+__device__ __noinline__ void bundle_load(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     constexpr int BT = BundleSmem<BCAP>::NT;
     const Hard &H = A.H;
     const int tid = threadIdx.x;
@@ -553,18 +831,20 @@ __device__ void bundle_load(const HardArgs &A, BundleSmem<BCAP> &B) {
         const int goff = A.off[c];
         B.c_goff[k] = goff;
         const V3 r0 = ld3(A.S.pos, A.members[goff]);
-        B.c_ref[3 * k] = r0.x; B.c_ref[3 * k + 1] = r0.y; B.c_ref[3 * k + 2] = r0.z;
-        B.c_steps[k] = 0; B.c_ncol[k] = 0; B.c_work[k] = 0;
-        B.c_label[k] = A.S.id_cluster[A.members[goff]];
-        B.c_fragn[k] = 0;
+        B.c_ref[0][k] = r0.x; B.c_ref[1][k] = r0.y; B.c_ref[2][k] = r0.z;
+        B.c_steps[k] = 0; B.c_work[k] = 0;
         B.c_n0[k] = B.c_n[k];
         B.c_addn[k] = 0;
-        B.c_ed[k] = 0.; B.c_edd[k] = 0.;
-        B.c_t0[k] = A.times ? global_ns() : 0;
-        B.c_red[4 * k] = 0ULL;                 // max |x - ref| component
-        B.c_red[4 * k + 1] = 0ULL;             // max |v| component
-        B.c_red[4 * k + 2] = 0ULL;             // max r_out_inv
-        B.c_red[4 * k + 3] = dbits(1.e300);    // min f r_planet
+        ClusterRec &R = A.crec[c];
+        R.t0 = A.times ? global_ns() : 0;
+        R.ed = R.edd = 0.;
+        R.n_frag = 0;
+        R.n_col = 0;
+        // maxima of |x - ref| and |v| components and of r_out_inv, minimum of f r_planet
+        B.c_key[k] = 0ULL;
+        B.c_tm[k] = 0ULL;
+        B.c_R[k] = 0ULL;
+        B.c_pb[k] = (long long)dbits(1.e300);
     }
     __syncthreads();
     for (int p = p0 + tid; p < p1; p += BT) {
@@ -575,306 +855,218 @@ __device__ void bundle_load(const HardArgs &A, BundleSmem<BCAP> &B) {
             else hi = mid - 1;
         }
         const int k = lo, g = B.c_goff[k] + (p - B.c_off[k]), i = A.members[g];
-        // FPHard(const FPGrav&), src/particle.h:1096-1116
-        st3(H.pos, g, ld3(A.S.pos, i)); st3(H.vel, g, ld3(A.S.vel, i));
-        st3(H.acc_s, g, ld3(A.S.acc_s, i)); st3(H.jerk_s, g, ld3(A.S.jerk_s, i));
-        st3(H.acc_d, g, ld3(A.S.acc_d, i)); st3(H.jerk_d, g, ld3(A.S.jerk_d, i));
-        const V3 z = v3(0., 0., 0.);
-        st3(H.x0, g, z); st3(H.v0, g, z); st3(H.a0_s, g, z); st3(H.j0_s, g, z); st3(H.a0_d, g, z);
-        st3(H.j0_d, g, z); st3(H.xp, g, z); st3(H.vp, g, z); st3(H.a2_s, g, z); st3(H.a3_s, g, z);
-        st3(H.a2_d, g, z); st3(H.a3_d, g, z);
-        H.phi_d[g] = A.S.phi_d[i]; H.phi_s[g] = A.S.phi_s[i];
-        H.mass[g] = A.S.mass[i]; H.r_planet[g] = A.S.r_planet[i]; H.f[g] = A.S.f[i];
-        H.r_out_inv[g] = A.S.r_out_inv[i];
-        H.time_c[g] = A.S.time[i]; H.th[g] = 0.; H.dt[g] = A.S.dt[i]; H.acc0[g] = A.S.acc0[i];
-        H.id[g] = A.S.id[i];
+        // FPHard(const FPGrav&), src/particle.h:1096-1116 (the forces come
+        // from the first full pass)
+        const V3 x = ld3(A.S.pos, i), v = ld3(A.S.vel, i);
+        const double mass = A.S.mass[i], rp = A.S.r_planet[i], f = A.S.f[i], roi = A.S.r_out_inv[i], dt = A.S.dt[i];
+        const double acc0 = A.S.acc0[i], tc = A.S.time[i];
+        const int64_t id = A.S.id[i];
+        bst(B, F_POS, p, x);
+        bst(B, F_VEL, p, v);
+        B.d[F_MASS][p] = mass;
+        B.d[F_ROI][p] = roi;
+        B.d[F_TH][p] = 0.;
+        B.d[F_DT][p] = dt;
+        B.d[F_TE][p] = 0. + dt;
+        B.d[F_ACC0][p] = acc0;
+        H.mass[g] = mass; H.r_planet[g] = rp; H.f[g] = f; H.r_out_inv[g] = roi;
+        H.time_c[g] = tc; H.acc0[g] = acc0; H.id[g] = id;
         H.dead[g] = 0; H.merged[g] = 0;
         H.tw_head[g] = H.tw_tail[g] = H.tw_next[g] = -1;
-        mirror_all(B, H, p, g, k, false);
-        B.owner[p] = -1;
-        B.flag[p] = 0;
-        const V3 x = ld3(H.pos, g), v = ld3(H.vel, g);
-        const double ext = dmax(fabs(x.x - B.c_ref[3 * k]), dmax(fabs(x.y - B.c_ref[3 * k + 1]),
-                                                                  fabs(x.z - B.c_ref[3 * k + 2])));
+        const double fr = f * rp;
+        B.fr32[p] = (float)fr;
+        B.roi32[p] = (float)roi;
+        // the high word of a double just below r_out / 128
+        B.hmov[p] = (int)(__float_as_uint(0.0078f / B.roi32[p]) >> 3) + (896 << 20);
+        B.gslot[p] = g;
+        B.cl[p] = (short)k;
+        B.eqc[p] = (short)p;
+        B.owner[p] = B.twh[p] = B.twn[p] = -1;
+        B.dead[p] = B.merged[p] = 0;
+        const double ext = dmax(fabs(x.x - B.c_ref[0][k]), dmax(fabs(x.y - B.c_ref[1][k]), fabs(x.z - B.c_ref[2][k])));
         const double vm = dmax(fabs(v.x), dmax(fabs(v.y), fabs(v.z)));
-        atomicMax(&B.c_red[4 * k], dbits(ext));
-        atomicMax(&B.c_red[4 * k + 1], dbits(vm));
-        atomicMax(&B.c_red[4 * k + 2], dbits(B.roi[p]));
-        atomicMin(&B.c_red[4 * k + 3], dbits(B.fr[p]));
+        atomicMax(&B.c_key[k], dbits(ext));
+        atomicMax(&B.c_tm[k], dbits(vm));
+        atomicMax(&B.c_R[k], dbits(roi));
+        atomicMin((unsigned long long *)&B.c_pb[k], dbits(fr));
     }
     __syncthreads();
     for (int k = k0 + tid; k < k1; k += BT) {
         // coordinate bound, then the prefilter thresholds (see the header)
-        const double E = (bitsd(B.c_red[4 * k]) + 2. * bitsd(B.c_red[4 * k + 1]) * A.t_end) * 1.0001 + 1.e-30;
+        const double E = (bitsd(B.c_key[k]) + 2. * bitsd(B.c_tm[k]) * A.t_end) * 1.0001 + 1.e-30;
         const double err = 3.e-7 * E;
-        const double rmax = bitsd(B.c_red[4 * k + 2]), frmin = bitsd(B.c_red[4 * k + 3]);
+        const double rmax = bitsd(B.c_R[k]), frmin = bitsd((unsigned long long)B.c_pb[k]);
         const double tf = 1.000001 + 1.0001 * err * rmax;
         const double tc = 1.000001 + 1.0001 * err / (2. * frmin);
         B.c_thrf[k] = __double2float_ru(tf * tf * 1.000001);
         B.c_thrc[k] = (frmin > 0.) ? __double2float_ru(tc * tc * 1.000001) : __int_as_float(0x7f800000);
         B.c_E32[k] = __double2float_rd(E);
+        B.c_key[k] = dbits(1.e10);
     }
+    for (int p = tid; p < p1; p += BT) B.flag[p] = p < p0 ? 0 : MF_TGT;
     __syncthreads();
-    for (int p = tid; p < p1; p += BT) {
-        if (p < p0) {
-            B.flag[p] = 0;
-            continue;
-        }
-        st32b(B, B.pos32, p, ld3(B.pos, p), B.cl[p]);
-        B.flag[p] = MF_TGT;
-    }
+    for (int p = p0 + tid; p < p1; p += BT) atomicMin(&B.c_key[B.cl[p]], dbits(B.d[F_TE][p]));
+    const int nt = bundle_full<BCAP>(A, false);
+    bundle_take(B, nt);
+    for (int k = k0 + tid; k < k1; k += BT) bundle_open(B, k);
+    if (tid == 0) B.n_sv = B.moved = 0;
     __syncthreads();
 }
 
-// member-parallel loop over the occupied slots
-#define FOR_SLOTS(p) for (int p = threadIdx.x; p < B.used; p += BT)
-#define FOR_CLUSTERS(k) for (int k = threadIdx.x; k < B.ncl; k += BT)
-
-// A cluster made fragments (KOMINAMI): its member range grows by them, the
-// clusters after it move up, and every slot is mirrored again from the
-// state of record (fragments are rare; owners are remapped).
+// every field of slot p from the state of record (global slot g), after a collision
 template <int BCAP>
-__device__ void bundle_grow(const HardArgs &A, BundleSmem<BCAP> &B) {
-    constexpr int BT = BundleSmem<BCAP>::NT;
-    const Hard &H = A.H;
+__device__ __forceinline__ void bundle_reload(BundleSmem<BCAP> &B, const Hard &H, int p, int g, int k) {
+    bst(B, F_POS, p, ld3(H.pos, g));
+    bst(B, F_VEL, p, ld3(H.vel, g));
+    B.d[F_MASS][p] = H.mass[g];
+    B.d[F_ROI][p] = H.r_out_inv[g];
+    B.d[F_TH][p] = H.th[g];
+    B.d[F_DT][p] = H.dt[g];
+    B.d[F_TE][p] = 0.;
+    B.d[F_ACC0][p] = H.acc0[g];
+    B.fr32[p] = (float)(H.f[g] * H.r_planet[g]);
+    B.roi32[p] = (float)H.r_out_inv[g];
+    B.hmov[p] = (int)(__float_as_uint(0.0078f / B.roi32[p]) >> 3) + (896 << 20);
+    B.dead[p] = (unsigned char)H.dead[g];
+    B.merged[p] = (unsigned char)H.merged[g];
+    B.gslot[p] = g;
+    B.cl[p] = (short)k;
+    for (int f = F_AS; f < F_MASS; f++) B.d[f][p] = 0.;
+}
+
+// Slot p's new place: its persistent fields move to slot q (>= 0) with the
+// cluster index k and its cluster's shift dp; every thread calls it, PER slots each.
+template <int BCAP>
+__device__ __forceinline__ void bundle_move(BundleSmem<BCAP> &B, const int *mv_new, const int *mv_k, const int *mv_d) {
+    constexpr int BT = BundleSmem<BCAP>::NT, PER = BCAP / BT;
+    const int tid = threadIdx.x;
+#pragma unroll 1
+    for (int f = 0; f < F_KEEP; f += 8) {
+        double v[PER][8];
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+            if (mv_new[j] >= 0)
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[j][u] = B.d[f + u][tid + j * BT];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+            if (mv_new[j] >= 0)
+#pragma unroll
+                for (int u = 0; u < 8; u++) B.d[f + u][mv_new[j]] = v[j][u];
+    }
+    float r32[PER], f32[PER];
+    int gs[PER], hm[PER], lk[PER][4], dm[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++)
+        if (mv_new[j] >= 0) {
+            const int p = tid + j * BT;
+            auto sh = [&](int x) { return x >= 0 ? x + mv_d[j] : -1; };
+            r32[j] = B.roi32[p]; f32[j] = B.fr32[p];
+            gs[j] = B.gslot[p]; hm[j] = B.hmov[p];
+            lk[j][0] = sh(B.owner[p]); lk[j][1] = sh(B.eqc[p]); lk[j][2] = sh(B.twh[p]); lk[j][3] = sh(B.twn[p]);
+            dm[j] = B.dead[p] | (B.merged[p] << 8);
+        }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; j++)
+        if (mv_new[j] >= 0) {
+            const int q = mv_new[j];
+            B.roi32[q] = r32[j]; B.fr32[q] = f32[j];
+            B.gslot[q] = gs[j]; B.hmov[q] = hm[j];
+            B.cl[q] = (short)mv_k[j];
+            B.owner[q] = (short)lk[j][0]; B.eqc[q] = (short)lk[j][1]; B.twh[q] = (short)lk[j][2];
+            B.twn[q] = (short)lk[j][3];
+            B.dead[q] = (unsigned char)(dm[j] & 0xff);
+            B.merged[q] = (unsigned char)(dm[j] >> 8);
+        }
+    __syncthreads();
+}
+
+// A cluster made fragments (KOMINAMI): its member range grows by them and the
+// clusters after it move up.
+template <int BCAP>
+__device__ __noinline__ void bundle_grow(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    constexpr int BT = BundleSmem<BCAP>::NT, PER = BCAP / BT;
     const int tid = threadIdx.x;
     static_assert(bmaxcl(BCAP) <= BT, "one thread per bundle cluster");
     const int add = (tid < B.ncl) ? B.c_addn[tid] : 0;
-    const int nn = (tid < B.ncl) ? B.c_n[tid] + add : 0;
+    const int my_n = (tid < B.ncl) ? B.c_n[tid] : 0;
     int tot;
-    const int noff = bscan<BT>(nn, B.ws, tot);
-    constexpr int PER = BCAP / BT;
-    int mv_new[PER], mv_g[PER], mv_k[PER], mv_own[PER];
-    int my_old_n = 0, my_addg = 0;
-    if (tid < B.ncl) {
-        my_old_n = B.c_n[tid];
-        my_addg = B.c_addg[tid];
-    }
-    __syncthreads();
+    const int noff = bscan<BT>(my_n + add, B.ws, tot);
     if (tot > BCAP) {  // no room: the fragments cannot be integrated here
         if (tid == 0) atomicOr(A.status, ST_CLUSTER_TOO_BIG);
         return;
     }
     if (tid < B.ncl) B.c_key[tid] = (unsigned long long)(unsigned)noff;  // new offsets, by cluster
     __syncthreads();
+    int mv_new[PER], mv_k[PER], mv_d[PER];
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int p = tid + j * BT;
         mv_new[j] = -1;
         if (p < B.used) {
             const int k = B.cl[p];
-            const int no = (int)B.c_key[k];
-            mv_new[j] = no + (p - B.c_off[k]);
-            mv_g[j] = B.gslot[p];
             mv_k[j] = k;
-            mv_own[j] = (B.owner[p] >= 0) ? no + (B.owner[p] - B.c_off[k]) : -1;
+            mv_d[j] = (int)B.c_key[k] - B.c_off[k];
+            mv_new[j] = p + mv_d[j];
         }
     }
     __syncthreads();
+    bundle_move(B, mv_new, mv_k, mv_d);
     if (tid < B.ncl) {
         B.c_off[tid] = noff;
-        B.c_n[tid] = nn;
+        B.c_n[tid] = my_n + add;
         // fragments are smaller than the members the prefilter margins were
         // set for: exact FP64 tests for this cluster from here on
         if (add > 0) B.c_flags[tid] |= CF_EXACT;
+        for (int i = 0; i < add; i++) {
+            const int q = noff + my_n + i;
+            bundle_reload(B, A.H, q, B.c_addg[tid] + i, tid);
+            B.eqc[q] = (short)q;
+            B.owner[q] = B.twh[q] = B.twn[q] = -1;
+        }
     }
     if (tid == 0) B.used = tot;
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        if (mv_new[j] < 0) continue;
-        mirror_all(B, H, mv_new[j], mv_g[j], mv_k[j], true);
-        B.owner[mv_new[j]] = (short)mv_own[j];
-    }
-    if (tid < B.ncl)
-        for (int i = 0; i < add; i++) {
-            const int q = noff + my_old_n + i;
-            mirror_all(B, H, q, my_addg + i, tid, true);
-            B.owner[q] = -1;
-        }
-    __syncthreads();
 }
 
-// one block step of every cluster in the bundle (timeIntegrate_multi body,
-// src/hermite.h:224-479)
+// the collisions of the block step: the colliding clusters' state goes to
+// the state of record, one thread per cluster resolves the collision on it,
+// and their members come back with a full force and first time steps
 template <int BCAP>
-__device__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> &B) {
+__device__ __noinline__ void bundle_collide(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     constexpr int BT = BundleSmem<BCAP>::NT;
     const Params &P = A.P;
     const Hard &H = A.H;
-    // makeActiveList: ts = min over alive members of th + dt
-    FOR_CLUSTERS(k) {
-        B.c_steps[k]++;
-        B.c_key[k] = dbits(1.e10);
-    }
-    __syncthreads();
     FOR_SLOTS(p) {
-        if (B.dead[p]) continue;
+        if (!(B.c_flags[B.cl[p]] & CF_COL)) continue;
         const int g = B.gslot[p];
-        atomicMin(&B.c_key[B.cl[p]], dbits(H.th[g] + H.dt[g]));
+        st3(H.pos, g, bld(B, F_POS, p));
+        st3(H.vel, g, bld(B, F_VEL, p));
+        H.th[g] = B.d[F_TH][p];
+        H.dt[g] = B.d[F_DT][p];
+        H.phi_d[g] = 0.;
+        H.phi_s[g] = 0.;
     }
-    __syncthreads();
-    FOR_CLUSTERS(k) {
-        B.c_ts[k] = bitsd(B.c_key[k]);
-        B.c_key[k] = dbits(1.);
-        B.c_pb[k] = 0x7fffffffffffffffLL;
-    }
-    if (threadIdx.x == 0) B.n_sv = 0;
-    __syncthreads();
-    HP_MARK(HP_TS);
-    // predict every member
-    FOR_SLOTS(p) {
-        const int g = B.gslot[p], k = B.cl[p];
-        V3 xp, vp;
-        predict(H, g, B.c_ts[k] - H.th[g], xp, vp);
-        st3(B.xp, p, xp);
-        st3(B.vp, p, vp);
-        st32b(B, B.xp32, p, xp, k);
-    }
-    __syncthreads();
-    HP_MARK(HP_PREDICT);
-    // collisionDetermination, src/hermite.h:98-196
-    bundle_detect(A, B, false);
-    __syncthreads();
-    if (B.n_sv <= BSURV) {
-        for (int i = threadIdx.x; i < B.n_sv; i += BT)
-            if (dbits(B.sv_R[i]) == B.c_key[B.sv_k[i]]) atomicMin(&B.c_pb[B.sv_k[i]], B.sv_p[i]);
-    } else {
-        bundle_detect(A, B, true);
-    }
-    __syncthreads();
-    FOR_CLUSTERS(k) {
-        int fl = B.c_flags[k] & ~CF_COL;
-        if (B.c_key[k] < dbits(1.)) {
-            fl |= CF_COL;
-            const int o = B.c_off[k], n = B.c_n[k];
-            const int a = (int)(B.c_pb[k] / n), b = (int)(B.c_pb[k] % n);
-            if (B.mass[o + a] < B.mass[o + b]) { B.c_imp[k] = o + a; B.c_tar[k] = o + b; }
-            else { B.c_imp[k] = o + b; B.c_tar[k] = o + a; }
-        }
-        B.c_flags[k] = fl;
-    }
-    __syncthreads();
-    HP_MARK(HP_DETECT);
-    // the active set (every alive member on a collision) and the twins of
-    // active merged members
-    FOR_SLOTS(p) {
-        const int k = B.cl[p], g = B.gslot[p];
-        const bool col = (B.c_flags[k] & CF_COL) != 0;
-        if (col) H.dt[g] = B.c_ts[k] - H.th[g];
-        unsigned char f = 0;
-        if (!B.dead[p] && (col || H.th[g] + H.dt[g] == B.c_ts[k])) {
-            f = MF_ACT | MF_TGT;
-            atomicAdd((unsigned long long *)&B.c_work[k], (unsigned long long)B.c_n[k]);
-        }
-        B.flag[p] = f;
-    }
-    __syncthreads();
-    FOR_SLOTS(p) {
-        const int ow = B.owner[p];
-        if (B.dead[p] && ow >= 0 && (B.flag[ow] & MF_ACT)) B.flag[p] |= MF_TGT;
-    }
-    __syncthreads();
-    const int nt = bundle_list(B, MF_TGT);
-    HP_MARK(HP_ACTIVE);
-    bundle_pairs(A, B, 1, nt);
-    HP_MARK(HP_PAIRS);
-    bundle_finalize(A, B, 1, nt, 1);
-    HP_MARK(HP_FINAL);
-    for (int it = 0; it < 2; it++) {
-        // FPHard::correct, one thread per (target, component): correct()'s
-        // arithmetic component by component
-        for (int i = threadIdx.x; i < 3 * nt; i += BT) {
-            const int t = i / 3, d = i - 3 * t;
-            const int s = B.tgt[t], g = B.gslot[s], k = B.cl[s];
-            const int gd = 3 * g + d;
-            // every input first (one round trip to the state of record)
-            const double th = H.th[g], as = H.acc_s[gd], a0s = H.a0_s[gd], j0s = H.j0_s[gd], js = H.jerk_s[gd];
-            const double ad = H.acc_d[gd], a0d = H.a0_d[gd], j0d = H.j0_d[gd], jd = H.jerk_d[gd];
-            const double xp = H.xp[gd], vp = H.vp[gd];
-            const double Dt = B.c_ts[k] - th;
-            const double Dt2 = Dt * Dt, Di = recip_pow2_or_div(Dt), Di2 = Di * Di, Di3 = Di2 * Di;
-            const double Am_s = as - a0s, J0_s = Dt * j0s, J1_s = Dt * js;
-            const double A2_s = 3. * Am_s - (J1_s + 2. * J0_s);
-            const double A3_s = -2. * Am_s + (J1_s + J0_s);
-            H.a2_s[gd] = 2. * Di2 * (A2_s + 3. * A3_s);
-            H.a3_s[gd] = 6. * Di3 * A3_s;
-            const double Am_d = ad - a0d, J0_d = j0d * Dt, J1_d = jd * Dt;
-            const double A2_d = 3. * Am_d - (J1_d + 2. * J0_d);
-            const double A3_d = -2. * Am_d + (J1_d + J0_d);
-            H.a2_d[gd] = 2. * (A2_d + 3. * A3_d) * Di2;
-            H.a3_d[gd] = 6. * A3_d * Di3;
-            const double A2 = A2_s + A2_d, A3 = A3_s + A3_d;
-            const double x = xp + 1.6666666666666667e-2 * Dt2 * (5. * A2 + 3. * 1.1666666666666667e-3 * A3);
-            const double v = vp + 8.3333333333333333e-2 * Dt * (4. * A2 + 3. * A3);
-            H.pos[gd] = x;
-            H.vel[gd] = v;
-            B.pos[3 * s + d] = x;
-            B.vel[3 * s + d] = v;
-            const float u = (float)(x - B.c_ref[3 * k + d]);
-            B.pos32[3 * s + d] = u;
-            if (!(fabsf(u) < B.c_E32[k])) atomicOr(&B.c_flags[k], CF_EXACT);
-        }
-        __syncthreads();
-        HP_MARK(HP_CORRECT);
-        bundle_pairs(A, B, 2, nt);
-        HP_MARK(HP_PAIRS);
-        bundle_finalize(A, B, 2, nt, 1);
-        HP_MARK(HP_FINAL);
-    }
-    // time and calcDeltat: the two criteria of a target (planets, sun) in a
-    // pair of lanes, exchanged by a shuffle; the even lane goes on with the
-    // target's time and dt_hermite's step choice
-    for (int base = 0; base < 2 * nt; base += BT) {
-        const int i = base + threadIdx.x, t = i >> 1;
-        const bool act = i < 2 * nt;
-        int s = 0, g = 0, k = 0;
-        bool upd = false;
-        double crit = 0.;
-        if (act) {
-            s = B.tgt[t];
-            g = B.gslot[s];
-            k = B.cl[s];
-            upd = !(B.c_flags[k] & CF_COL) && !B.dead[s];
-            if (upd) {
-                // one code path for both lanes (the inputs chosen by parity)
-                const bool sun = (i & 1) != 0;
-                crit = dt4th(sun ? P.eta_sun : P.eta, P.alpha2, sun ? 0. : H.acc0[g], ld3(sun ? H.acc_s : H.acc_d, g),
-                             ld3(sun ? H.jerk_s : H.jerk_d, g), ld3(sun ? H.a2_s : H.a2_d, g),
-                             ld3(sun ? H.a3_s : H.a3_d, g));
-            }
-        }
-        const double other = __shfl_xor_sync(0xffffffffu, crit, 1);
-        if (act && !(i & 1)) {
-            H.th[g] += B.c_ts[k] - H.th[g];
-            if (upd) H.dt[g] = dt_next_hermite(P, H.th[g], H.dt[g], dmin(crit, other));
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt; i += BT) {
-        const int s = B.tgt[i], k = B.cl[s];
-        if (B.dead[s] && B.owner[s] >= 0 && !(B.c_flags[k] & CF_COL)) H.dt[B.gslot[s]] = H.dt[B.gslot[B.owner[s]]];
-    }
-    if (threadIdx.x == 0) B.any = 0;
-    __syncthreads();
-    HP_MARK(HP_DT);
-    // collisions: one thread per colliding cluster
     if (threadIdx.x == 0) B.grew = 0;
     __syncthreads();
     FOR_CLUSTERS(k) {
         B.c_addn[k] = 0;
         if (!(B.c_flags[k] & CF_COL)) continue;
-        B.any = 1;
         ColRec rec;
         double e1 = 0., e2 = 0.;
-        const int o = B.c_off[k], n = B.c_n[k];
+        const int o = B.c_off[k], n = B.c_n[k], c = B.c_idx[k];
+        ClusterRec &R = A.crec[c];
         int fs[32];
-        FragCtx X{&A, &B.gslot[o], n, B.c_idx[k], B.c_label[k], &B.c_fragn[k], fs};
+        FragCtx X{&A, &B.gslot[o], n, c, A.S.id_cluster[A.members[B.c_goff[k]]], &R.n_frag, fs};
         const int nf = collide(P, H, B.gslot[B.c_imp[k]], B.gslot[B.c_tar[k]], e1, e2, rec, &X);
-        B.c_ed[k] += e1;
-        B.c_edd[k] += e2;
-        rec.cluster = B.c_idx[k];
-        rec.seq = B.c_ncol[k]++;
+        R.ed += e1;
+        R.edd += e2;
+        rec.cluster = c;
+        rec.seq = R.n_col++;
         rec.n = B.c_n0[k];
         const int slot = atomicAdd(A.n_cols, 1);
         if (slot < A.col_cap) A.cols[slot] = rec;
@@ -885,61 +1077,250 @@ __device__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> &B) {
             B.grew = 1;
             for (int i = 0; i < nf; i++) A.frags[fs[i] - A.frag_base].n0 = B.c_n0[k];
         }
-        // twin owners (pool slots) from the merge lists
-        for (int j = 0; j < n; j++) B.owner[o + j] = -1;
-        for (int j = 0; j < n; j++) {
-            const int gj = B.gslot[o + j];
-            if (!H.merged[gj]) continue;
-            for (int t = H.tw_head[gj], gg = 0; t >= 0 && gg < 4096; t = H.tw_next[t], gg++)
-                for (int q = 0; q < n; q++)
-                    if (B.gslot[o + q] == t) {
-                        B.owner[o + q] = (short)(o + j);
-                        break;
-                    }
-        }
     }
-    __syncthreads();
-    if (B.grew) bundle_grow(A, B);
-    __syncthreads();
-    if (B.any) {
-        FOR_SLOTS(p) {
-            const int k = B.cl[p];
-            B.flag[p] = 0;
-            if (!(B.c_flags[k] & CF_COL)) continue;
-            mirror_all(B, H, p, B.gslot[p], k, true);
-            B.flag[p] = MF_TGT;
-        }
-        __syncthreads();
-        const int nc = bundle_list(B, MF_TGT);
-        bundle_pairs(A, B, 0, nc);
-        bundle_finalize(A, B, 0, nc, 2);
-        for (int i = threadIdx.x; i < nc; i += BT) {
-            const int s = B.tgt[i], g = B.gslot[s];
-            if (!B.dead[s])
-                H.dt[g] = dt_initial(P, H.th[g], H.dt[g], H.acc0[g], ld3(H.acc_d, g), ld3(H.jerk_d, g),
-                                     ld3(H.acc_s, g), ld3(H.jerk_s, g));
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < nc; i += BT) {
-            const int s = B.tgt[i], g = B.gslot[s];
-            if (B.merged[s])
-                for (int t = H.tw_head[g], gg = 0; t >= 0 && gg < 4096; t = H.tw_next[t], gg++) H.dt[t] = H.dt[g];
-        }
-        __syncthreads();
-    }
-    HP_MARK(HP_COLLIDE);
-    // getSystemTime, src/hermite.h:25-35
-    FOR_CLUSTERS(k) B.c_key[k] = dbits(1.e10);
+    __threadfence_block();
     __syncthreads();
     FOR_SLOTS(p) {
-        if (!B.dead[p]) atomicMin(&B.c_key[B.cl[p]], dbits(H.th[B.gslot[p]]));
+        const int k = B.cl[p];
+        B.flag[p] = 0;
+        if (!(B.c_flags[k] & CF_COL)) continue;
+        const int g = B.gslot[p], o = B.c_off[k], n = B.c_n[k];
+        bundle_reload(B, H, p, g, k);
+        // the merge lists as slots: twins, their owner, equal ids
+        auto slot_of = [&](int t) {
+            if (t >= 0)
+                for (int q = 0; q < n; q++)
+                    if (B.gslot[o + q] == t) return o + q;
+            return -1;
+        };
+        B.twh[p] = (short)slot_of(H.tw_head[g]);
+        B.twn[p] = (short)slot_of(H.tw_next[g]);
+        const int64_t id = H.id[g];
+        int own = -1, eq = p;
+        for (int q = n - 1; q >= 0; q--) {
+            const int gj = B.gslot[o + q];
+            if (H.id[gj] == id) eq = o + q;
+            if (H.merged[gj])
+                for (int t = H.tw_head[gj], gg = 0; t >= 0 && gg < 4096; t = H.tw_next[t], gg++)
+                    if (t == g) own = o + q;
+        }
+        B.owner[p] = (short)own;
+        B.eqc[p] = (short)eq;
+        if (B.dead[p]) B.any_dead = 1;
     }
-    if (threadIdx.x == 0) B.any = 0;
+    __syncthreads();
+    if (B.grew) bundle_grow<BCAP>(A);
+    FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_COL) ? MF_TGT : 0;
+    __syncthreads();
+    const int nc = bundle_full<BCAP>(A, false);
+    bundle_take(B, nc);
+    for (int i = threadIdx.x; i < nc; i += BT) {
+        const int s = B.tgt[i];
+        if (B.dead[s]) continue;
+        B.d[F_DT][s] = dt_initial(P, B.d[F_TH][s], B.d[F_DT][s], B.d[F_ACC0][s], bld(B, F_AD, s), bld(B, F_JD, s),
+                                  bld(B, F_AS, s), bld(B, F_JS, s));
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nc; i += BT) {
+        const int s = B.tgt[i];
+        if (B.merged[s])
+            for (int t = B.twh[s], gg = 0; t >= 0 && gg < BCAP; t = B.twn[t], gg++) B.d[F_DT][t] = B.d[F_DT][s];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nc; i += BT) {
+        const int s = B.tgt[i];
+        B.d[F_TE][s] = B.d[F_TH][s] + B.d[F_DT][s];
+    }
+    __syncthreads();
+}
+
+// dt_next_hermite by the exponents: its halvings of a power of two against
+// the time's lowest set bit and the criterion's exponent
+__device__ __forceinline__ double dt_next_bits(const Params &P, double time, double dt, double dt_1) {
+    const double dmax_ = 0.5 * P.dt_tree;
+    if (!is_pow2(dt) || !is_pow2(dmax_) || !(dhi(time) >= 0 && dhi(time) < 0x7fe00000) || dhi(dt_1) < 0)
+        return dt_next_hermite(P, time, dt, dt_1);
+    const int ed = dhi(dt) >> 20;
+    int e = min(ed + 1, dhi(dmax_) >> 20);
+    const unsigned long long b = dbits(time), m = (b & ((1ULL << 52) - 1)) | (1ULL << 52);
+    if (b != 0ULL) {  // time a multiple of 2^e: e at most its lowest set bit's exponent
+        const int et = (int)(b >> 52);
+        if (et == 0) return dt_next_hermite(P, time, dt, dt_1);
+        e = min(e, et - 52 + (__ffsll((long long)m) - 1));
+    }
+    if (e < 64) return dt_next_hermite(P, time, dt, dt_1);
+    const int e1 = dhi(dt_1) >> 20;
+    while (e1 < e && ed - 1 < e) e--;  // dt_1 < 2^e: its exponent is smaller
+    const double next = __hiloint2double(e << 20, 0);
+    return plt(next, 2. * P.dt_min) ? P.dt_min : next;
+}
+
+// dt4th's last expression (p3t_phys.cuh), from the norms and squares
+__device__ __forceinline__ double dt4th_of(double eta, double Acc, double Jerk, double Snap, double Crac, double Jerk2,
+                                           double Snap2) {
+    return (dbits(Jerk) << 1) != 0ULL ? eta * sqrt_rn(div_rn(Acc * Snap + Jerk2, Jerk * Crac + Snap2))
+                                      : 1.7976931348623157e308;
+}
+
+// time and calcDeltat (src/particle.h:1276-1314) of the targets, and their
+// running forces into the state.  The two criteria (planets, sun) of a target
+// in a pair of lanes; when there are few targets, the four norms of each in
+// lanes of their own.
+template <int BCAP>
+__device__ __forceinline__ void bundle_dt(const HardArgs &A, BundleSmem<BCAP> &B, int nt) {
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    constexpr unsigned ALL = 0xffffffffu;
+    const Params &P = A.P;
+    const bool wide = 8 * nt <= BT;
+    const int sh = wide ? 3 : 1, L = 1 << sh;  // lanes a target
+    for (int base = 0; base < L * nt; base += BT) {
+        const int i = base + threadIdx.x;
+        if (i - (i & 31) >= L * nt) break;  // no target in this warp
+        const int t = min(i >> sh, nt - 1), r = i & (L - 1);
+        const bool act = i < L * nt;
+        const int s = B.tgt[t], k = B.cl[s];
+        double crit;
+        if (wide) {
+            const int sun = r >> 2, w = r & 3;
+            // acc and jerk as the last pass left them, snap and crackle as the corrector did
+            const int f = (w < 2) ? (sun ? F_NAS : F_NAD) + 3 * w : (sun ? F_AS : F_AD) + 3 * (w - 2);
+            const V3 v = bld(B, f, s);
+            double n2 = dot(v, v);
+            if (w == 0 && !sun) {
+                const double a0 = B.d[F_ACC0][s];
+                n2 = n2 + P.alpha2 * a0 * a0;
+            }
+            const double nn = sqrt_rn(n2);
+            const double Acc = __shfl_sync(ALL, nn, 0, 4), Jerk = __shfl_sync(ALL, nn, 1, 4),
+                         Snap = __shfl_sync(ALL, nn, 2, 4), Crac = __shfl_sync(ALL, nn, 3, 4);
+            const double Jerk2 = __shfl_sync(ALL, n2, 1, 4), Snap2 = __shfl_sync(ALL, n2, 2, 4);
+            crit = dt4th_of(sun ? P.eta_sun : P.eta, Acc, Jerk, Snap, Crac, Jerk2, Snap2);
+        } else {
+            // dt4th (p3t_phys.cuh), a norm after the other
+            const int sun = r;
+            double n2[4];
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                const V3 v = bld(B, (w < 2) ? (sun ? F_NAS : F_NAD) + 3 * w : (sun ? F_AS : F_AD) + 3 * (w - 2), s);
+                n2[w] = dot(v, v);
+            }
+            const double a0 = sun ? 0. : B.d[F_ACC0][s];
+            n2[0] = n2[0] + P.alpha2 * a0 * a0;
+            double nn[4];
+#pragma unroll 1
+            for (int w = 0; w < 4; w++) nn[w] = sqrt_rn(n2[w]);
+            crit = dt4th_of(sun ? P.eta_sun : P.eta, nn[0], nn[1], nn[2], nn[3], n2[1], n2[2]);
+        }
+        const double other = __shfl_xor_sync(ALL, crit, L / 2);
+        if (act) {
+            for (int f = r; f < 12; f += L) B.d[F_AS + f][s] = B.d[F_NAS + f][s];
+            if (r == 0) {
+                const double th0 = B.d[F_TH][s], th = th0 + (B.c_ts[k] - th0);
+                B.d[F_TH][s] = th;
+                double dt = B.d[F_DT][s];
+                if (!(B.c_flags[k] & CF_COL) && !B.dead[s]) {
+                    dt = dt_next_bits(P, th, dt, dmin(crit, other));
+                    B.d[F_DT][s] = dt;
+                }
+                B.d[F_TE][s] = th + dt;
+            }
+        }
+    }
+    __syncthreads();
+    if (B.any_dead) {  // a twin's block step is its target's
+        for (int i = threadIdx.x; i < nt; i += BT) {
+            const int s = B.tgt[i], k = B.cl[s];
+            if (B.dead[s] && B.owner[s] >= 0 && !(B.c_flags[k] & CF_COL)) B.d[F_DT][s] = B.d[F_DT][B.owner[s]];
+        }
+        __syncthreads();
+    }
+}
+
+// one block step of every cluster in the bundle (timeIntegrate_multi body,
+// src/hermite.h:224-479), whose time bundle_open has set
+template <int BCAP>
+__device__ __forceinline__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> &B) {
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    // FPHard::predict (src/particle.h:1183-1206), one lane per (member,
+    // component): predict()'s roundings, the products by a power-of-two Dt
+    // fused where they are exact.  The active set: the alive members whose
+    // step ends now.
+    const int used = B.used, lane = threadIdx.x & 31;
+    for (int w0 = threadIdx.x - lane; w0 < 3 * used; w0 += BT) {  // whole warps
+        const int it = min(w0 + lane, 3 * used - 1);
+        const int c = it >= 2 * used ? 2 : (it >= used ? 1 : 0), p = it - c * used, k = B.cl[p];
+        const double ts = B.c_ts[k], Dt = ts - B.d[F_TH][p];
+        const double x = B.d[F_POS + c][p], v = B.d[F_VEL + c][p];
+        const double a = B.d[F_AS + c][p] + B.d[F_AD + c][p], j = B.d[F_JS + c][p] + B.d[F_JD + c][p];
+        const double hD = Dt * 0.5, u = fma(0.5, a, 1.6666666666666667e-1 * Dt * j);
+        double xp, vp;
+        if (__all_sync(0xffffffffu, is_pow2(Dt))) {
+            xp = fma(Dt, fma(Dt, u, v), x);
+            vp = fma(Dt, fma(hD, j, a), v);
+        } else {
+            xp = x + Dt * (v + Dt * u);
+            vp = v + Dt * (a + hD * j);
+        }
+        if (w0 + lane >= 3 * used) continue;
+        B.d[F_XP + c][p] = xp;
+        B.d[F_VP + c][p] = vp;
+        st32b(B, c, p, xp, k);
+        if (c == 0) {
+            const bool act = !B.dead[p] && dbits(B.d[F_TE][p]) == dbits(ts);
+            B.flag[p] = act ? (MF_ACT | MF_TGT) : 0;
+            if (act) atomicAdd(&B.c_act[k], 1);
+        }
+    }
+    __syncthreads();
+    HP_MARK(HP_PREDICT);
+    // collisionDetermination, src/hermite.h:98-196
+    bundle_detect(A, B, false);
+    __syncthreads();
+    const bool col = B.n_sv > 0;
+    if (col) bundle_collisions_found<BCAP>(A);
+    HP_MARK(HP_DETECT);
+    if (B.any_dead) {  // the twins of active merged members
+        FOR_SLOTS(p) {
+            const int ow = B.owner[p];
+            if (B.dead[p] && ow >= 0 && (B.flag[ow] & MF_ACT)) B.flag[p] |= MF_TGT;
+        }
+        __syncthreads();
+    }
+    const int nt = bundle_targets(B, MF_TGT);
+    HP_MARK(HP_ACTIVE);
+    // predicted forces and first correction, corrected forces and second
+    // correction, corrected forces
+    bool listed = false;
+#pragma unroll 1
+    for (int ps = 0; ps < 3; ps++) bundle_pass<BCAP, false>(A, B, ps == 0 ? 1 : 2, nt, false, (ps + 1) % 3, listed);
+    FOR_CLUSTERS(k) {
+        B.c_work[k] += (long long)B.c_act[k] * B.c_n[k];
+        B.c_key[k] = B.c_tm[k] = dbits(1.e10);
+    }
+    bundle_dt(A, B, nt);
+    HP_MARK(HP_DT);
+    if (col) bundle_collide<BCAP>(A);
+    HP_MARK(HP_COLLIDE);
+    // getSystemTime (src/hermite.h:25-35) and makeActiveList's next time
+    // (src/hermite.h:4-24): the minima of th and th + dt over the alive members
+    if (threadIdx.x == 0) B.any = B.n_sv = B.moved = 0;
+    if (col) {
+        FOR_CLUSTERS(k) B.c_key[k] = B.c_tm[k] = dbits(1.e10);
+        __syncthreads();
+    }
+    FOR_SLOTS(p) {
+        if (B.dead[p]) continue;
+        const int k = B.cl[p];
+        atomicMin(&B.c_tm[k], dbits(B.d[F_TH][p]));
+        atomicMin(&B.c_key[k], dbits(B.d[F_TE][p]));
+    }
     __syncthreads();
     FOR_CLUSTERS(k) {
-        const double time = bitsd(B.c_key[k]);
-        if (time < A.t_end && B.c_steps[k] >= A.max_steps) atomicOr(A.status, ST_ITER_CAP);
-        if (!(time < A.t_end) || B.c_steps[k] >= A.max_steps) {
+        const bool going = B.c_tm[k] < dbits(A.t_end);
+        if (going && B.c_steps[k] < A.max_steps) {
+            bundle_open(B, k);
+        } else {
+            if (going) atomicOr(A.status, ST_ITER_CAP);
             B.c_flags[k] |= CF_FIN;
             B.any = 1;
         }
@@ -950,135 +1331,153 @@ __device__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> &B) {
 
 // final forces, write-back and removal of the finished clusters
 template <int BCAP>
-__device__ void bundle_retire(const HardArgs &A, BundleSmem<BCAP> &B) {
-    constexpr int BT = BundleSmem<BCAP>::NT;
+__device__ __noinline__ void bundle_retire(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    constexpr int BT = BundleSmem<BCAP>::NT, PER = BCAP / BT;
     const Hard &H = A.H;
     const int tid = threadIdx.x;
     FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_FIN) ? MF_TGT : 0;
     __syncthreads();
-    const int nt = bundle_list(B, MF_TGT);
-    bundle_pairs(A, B, 0, nt);
-    bundle_finalize(A, B, 0, nt, 2);
+    const int nt = bundle_full<BCAP>(A, true);
     // write back to FPGrav, with resetTime (src/hard.h:768-787)
     for (int i = tid; i < nt; i += BT) {
         const int s = B.tgt[i], g = B.gslot[s], k = B.cl[s];
+        const double th = B.d[F_TH][s], dt = B.d[F_DT][s];
+        const V3 x = bld(B, F_POS, s), v = bld(B, F_VEL, s), as = bld(B, F_NAS, s), js = bld(B, F_NJS, s),
+                 ad = bld(B, F_NAD, s), jd = bld(B, F_NJD, s);
+        const double phd = B.d[F_PHD][s], phs = B.d[F_PHS][s];
         if (g >= A.frag_base) {  // a fragment: joins the system after the launch
             A.frags[g - A.frag_base].n_cl = B.c_n[k];
+            st3(H.pos, g, x); st3(H.vel, g, v); st3(H.acc_s, g, as); st3(H.jerk_s, g, js);
+            st3(H.acc_d, g, ad); st3(H.jerk_d, g, jd);
+            H.phi_d[g] = phd; H.phi_s[g] = phs; H.th[g] = th; H.dt[g] = dt;
             continue;
         }
         const int idx = A.members[g];
-        st3(A.S.pos, idx, ld3(H.pos, g)); st3(A.S.vel, idx, ld3(H.vel, g));
-        st3(A.S.acc_s, idx, ld3(H.acc_s, g)); st3(A.S.jerk_s, idx, ld3(H.jerk_s, g));
-        st3(A.S.acc_d, idx, ld3(H.acc_d, g)); st3(A.S.jerk_d, idx, ld3(H.jerk_d, g));
-        A.S.phi_d[idx] = H.phi_d[g]; A.S.phi_s[idx] = H.phi_s[g];
-        A.S.mass[idx] = H.mass[g]; A.S.r_planet[idx] = H.r_planet[g];
-        A.S.time[idx] = H.time_c[g] + H.th[g]; A.S.dt[idx] = H.dt[g];
+        st3(A.S.pos, idx, x); st3(A.S.vel, idx, v);
+        st3(A.S.acc_s, idx, as); st3(A.S.jerk_s, idx, js);
+        st3(A.S.acc_d, idx, ad); st3(A.S.jerk_d, idx, jd);
+        A.S.phi_d[idx] = phd; A.S.phi_s[idx] = phs;
+        A.S.mass[idx] = B.d[F_MASS][s]; A.S.r_planet[idx] = H.r_planet[g];
+        A.S.time[idx] = H.time_c[g] + th; A.S.dt[idx] = dt;
         A.S.id[idx] = H.id[g];
-        A.S.dead[idx] = H.dead[g]; A.S.merged[idx] = H.merged[g];
+        A.S.dead[idx] = B.dead[s]; A.S.merged[idx] = B.merged[s];
         A.S.n_cluster[idx] = B.c_n[k];
     }
     FOR_CLUSTERS(k) {
         if (!(B.c_flags[k] & CF_FIN)) continue;
         const int c = B.c_idx[k];
-        A.cl_edisp[2 * c] = (B.c_ncol[k] > 0) ? B.c_ed[k] : 0.;
-        A.cl_edisp[2 * c + 1] = (B.c_ncol[k] > 0) ? B.c_edd[k] : 0.;
+        const ClusterRec &R = A.crec[c];
+        A.cl_edisp[2 * c] = (R.n_col > 0) ? R.ed : 0.;
+        A.cl_edisp[2 * c + 1] = (R.n_col > 0) ? R.edd : 0.;
         if (A.cost) {
             A.cost[2 * c] = B.c_steps[k];
             A.cost[2 * c + 1] = B.c_work[k];
         }
         if (A.times) {
-            A.times[2 * c] = B.c_t0[k];
+            A.times[2 * c] = R.t0;
             A.times[2 * c + 1] = global_ns();
         }
     }
-    __syncthreads();
     // compaction: kept clusters move down, in order
     int keep = 0, nk = 0, nkeep = 0, noff = 0, tot = 0;
-    int t_idx = 0, t_n = 0, t_goff = 0, t_steps = 0, t_ncol = 0, t_flags = 0;
-    double t_ref0 = 0., t_ref1 = 0., t_ref2 = 0., t_ed = 0., t_edd = 0.;
-    long long t_work = 0, t_t0 = 0;
+    int t_idx = 0, t_n = 0, t_goff = 0, t_steps = 0, t_flags = 0, t_n0 = 0;
+    double t_ts = 0., t_ref0 = 0., t_ref1 = 0., t_ref2 = 0.;
+    long long t_work = 0;
     float t_thrf = 0.f, t_thrc = 0.f, t_E = 0.f;
-    long long t_label = 0, t_fragn = 0;
-    int t_n0 = 0;
     if (tid < B.ncl) {
         keep = !(B.c_flags[tid] & CF_FIN);
         t_idx = B.c_idx[tid]; t_n = B.c_n[tid]; t_goff = B.c_goff[tid];
-        t_steps = B.c_steps[tid]; t_ncol = B.c_ncol[tid]; t_flags = B.c_flags[tid];
-        t_ref0 = B.c_ref[3 * tid]; t_ref1 = B.c_ref[3 * tid + 1]; t_ref2 = B.c_ref[3 * tid + 2];
-        t_ed = B.c_ed[tid]; t_edd = B.c_edd[tid]; t_work = B.c_work[tid]; t_t0 = B.c_t0[tid];
+        t_steps = B.c_steps[tid]; t_flags = B.c_flags[tid]; t_n0 = B.c_n0[tid];
+        t_ts = B.c_ts[tid]; t_ref0 = B.c_ref[0][tid]; t_ref1 = B.c_ref[1][tid]; t_ref2 = B.c_ref[2][tid];
+        t_work = B.c_work[tid];
         t_thrf = B.c_thrf[tid]; t_thrc = B.c_thrc[tid]; t_E = B.c_E32[tid];
-        t_label = B.c_label[tid]; t_fragn = B.c_fragn[tid]; t_n0 = B.c_n0[tid];
     }
     static_assert(bmaxcl(BCAP) <= BT, "one thread per bundle cluster");
-    nk = bscan<BT>(keep, B.ws, nkeep);
-    noff = bscan<BT>(keep ? t_n : 0, B.ws, tot);
-    // slots: read the old placement before anything moves
-    constexpr int PER = BCAP / BT;
-    int mv_new[PER], mv_g[PER], mv_k[PER], mv_own[PER];
+    noff = bscan<BT>(keep ? (t_n << 10) | 1 : 0, B.ws, tot);
+    nk = noff & 1023;
+    noff >>= 10;
+    nkeep = tot & 1023;
+    tot >>= 10;
+    // old -> new offset and index per kept cluster, through c_key (free here)
+    if (tid < B.ncl)
+        B.c_key[tid] = keep ? ((unsigned long long)(unsigned)noff | ((unsigned long long)(unsigned)nk << 32)) : ~0ULL;
     __syncthreads();
-    if (keep) {
-        // old -> new offset per kept cluster, through c_key (free here)
-        B.c_key[tid] = (unsigned long long)(unsigned)noff | ((unsigned long long)(unsigned)nk << 32);
-    }
-    __syncthreads();
+    int mv_new[PER], mv_k[PER], mv_d[PER];
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int p = tid + j * BT;
         mv_new[j] = -1;
         if (p < B.used) {
             const int k = B.cl[p];
-            if (!(B.c_flags[k] & CF_FIN)) {
-                const int no = (int)(B.c_key[k] & 0xffffffffULL), kk = (int)(B.c_key[k] >> 32);
-                mv_new[j] = no + (p - B.c_off[k]);
-                mv_g[j] = B.gslot[p];
-                mv_k[j] = kk;
-                mv_own[j] = (B.owner[p] >= 0) ? no + (B.owner[p] - B.c_off[k]) : -1;
+            const unsigned long long key = B.c_key[k];
+            if (key != ~0ULL) {
+                mv_k[j] = (int)(key >> 32);
+                mv_d[j] = (int)(key & 0xffffffffULL) - B.c_off[k];
+                mv_new[j] = p + mv_d[j];
             }
         }
     }
     __syncthreads();
+    if (nkeep > 0) bundle_move(B, mv_new, mv_k, mv_d);
     if (keep) {
         B.c_idx[nk] = t_idx; B.c_off[nk] = noff; B.c_n[nk] = t_n; B.c_goff[nk] = t_goff;
-        B.c_steps[nk] = t_steps; B.c_ncol[nk] = t_ncol; B.c_flags[nk] = t_flags;
-        B.c_ref[3 * nk] = t_ref0; B.c_ref[3 * nk + 1] = t_ref1; B.c_ref[3 * nk + 2] = t_ref2;
-        B.c_ed[nk] = t_ed; B.c_edd[nk] = t_edd; B.c_work[nk] = t_work; B.c_t0[nk] = t_t0;
+        B.c_steps[nk] = t_steps; B.c_flags[nk] = t_flags; B.c_n0[nk] = t_n0;
+        B.c_ts[nk] = t_ts; B.c_ref[0][nk] = t_ref0; B.c_ref[1][nk] = t_ref1; B.c_ref[2][nk] = t_ref2;
+        B.c_work[nk] = t_work;
         B.c_thrf[nk] = t_thrf; B.c_thrc[nk] = t_thrc; B.c_E32[nk] = t_E;
-        B.c_label[nk] = t_label; B.c_fragn[nk] = t_fragn; B.c_n0[nk] = t_n0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int p = tid + j * BT;
-        if (mv_new[j] >= 0 && mv_new[j] != p) {
-            mirror_all(B, H, mv_new[j], mv_g[j], mv_k[j], true);
-            B.owner[mv_new[j]] = (short)mv_own[j];
-        } else if (mv_new[j] >= 0) {
-            B.cl[p] = (short)mv_k[j];
-            B.owner[p] = (short)mv_own[j];
-        }
+        B.c_R[nk] = dbits(1.);
+        B.c_pb[nk] = 0x7fffffffffffffffLL;
+        B.c_act[nk] = 0;
+        B.c_addn[nk] = 0;
     }
     if (tid == 0) {
         B.ncl = nkeep;
         B.used = tot;
+        B.any_dead = 0;
+    }
+    __syncthreads();
+    FOR_SLOTS(p) {
+        if (B.dead[p]) B.any_dead = 1;
     }
     __syncthreads();
 }
 
-// The clusters above BCAP_MAIN bodies (the queue's tier 0), concurrently
-// with k_hard_bundles: one CTA takes one at a time -- up to BCAP_WIDE bodies
-// (fragment room included) as a lone wide bundle, the lane-dense form, larger
-// ones in the one-cluster-per-CTA form.  Same arithmetic, bit for bit, as
-// every other form.
+template <int BCAP>
+__device__ __forceinline__ void bundle_init(BundleSmem<BCAP> &B) {
+    if (threadIdx.x == 0) {
+        B.used = B.ncl = B.n_pend = B.i_pend = B.exhausted = B.phase = 0;
+        B.n_sv = B.moved = B.any = B.any_dead = 0;
+        B.live[0] = B.live[1] = 0ULL;
+        for (int k = 0; k < HP_N; k++) B.ph_acc[k] = 0;
+        B.ph_t = clock64();
+    }
+}
+template <int BCAP>
+__device__ __forceinline__ void bundle_close(const HardArgs &A, BundleSmem<BCAP> &B) {
+    if (threadIdx.x == 0 && A.live) {
+        atomicAdd(&A.live[0], B.live[0]);
+        atomicAdd(&A.live[1], B.live[1]);
+    }
+    if (A.phase_cycles && threadIdx.x == 0)
+        for (int k = 0; k < HP_N; k++) atomicAdd(&A.phase_cycles[k], (unsigned long long)B.ph_acc[k]);
+}
+
+// The clusters above a bundle's slots (the queue's tier 0), concurrently with
+// k_hard_bundles: one CTA takes one at a time -- up to A.wide_cap bodies
+// (fragment room included) as a lone wide bundle, larger ones in the
+// one-cluster-per-CTA form.  Same arithmetic, bit for bit, as every other form.
 constexpr int WT = bundle_threads(BCAP_WIDE);  // threads of a wide CTA (it holds its SM)
-__global__ void __launch_bounds__(WT, 1) k_hard_wide(HardArgs A) {
-    extern __shared__ __align__(16) unsigned char bundle_smem[];
-    BundleSmem<BCAP_WIDE> &B = *reinterpret_cast<BundleSmem<BCAP_WIDE> *>(bundle_smem);
+__global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ HardArgs A) {
+    constexpr int BCAP = BCAP_WIDE;
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     __shared__ double red_d[WT / 32];
     __shared__ long long red_l[WT / 32];
     __shared__ int q_sh;
     const int tid = threadIdx.x;
     Team<WT> tm{tid, red_d, red_l};
     const int room = (A.frag.a_frag > 0.) ? 2 * A.frag.n_frag_max : 0;
+    bundle_init(B);
     for (int guard = 0; guard < (1 << 30); guard++) {
         if (tid == 0) q_sh = atomicAdd(&A.queue[0], 1);
         __syncthreads();
@@ -1087,7 +1486,7 @@ __global__ void __launch_bounds__(WT, 1) k_hard_wide(HardArgs A) {
         if (q >= A.n_tier[0]) break;
         const int c = A.order[q];
         const int n = A.cnt[c];
-        if (n + room > BCAP_WIDE) {
+        if (n > A.wide_cap || n + room > BCAP_WIDE) {
             run_cluster<WT>(A, c, tm);
             continue;
         }
@@ -1098,104 +1497,43 @@ __global__ void __launch_bounds__(WT, 1) k_hard_wide(HardArgs A) {
             B.c_n[0] = n;
             B.c_flags[0] = CF_FRESH;
             B.used = n;
-            B.fresh_k = 0;
-            B.fresh_p = 0;
-            B.n_pend = B.i_pend = 0;
-            B.exhausted = 1;
-            B.phase = 1;
+            B.fresh_k = B.fresh_p = 0;
+            B.any_dead = 0;
         }
         __syncthreads();
-        bundle_load(A, B);
-        {
-            const int nt = bundle_list(B, MF_TGT);
-            bundle_pairs(A, B, 0, nt);
-            bundle_finalize(A, B, 0, nt, 2);
-        }
+        bundle_load<BCAP>(A);
         // bundle_step advances the cluster by one block step; it retires when done
         for (int it = 0; it < A.max_steps + 8; it++) {
             bundle_step(A, B);
-            if (B.any) bundle_retire(A, B);
+            if (B.any) bundle_retire<BCAP>(A);
             if (B.ncl == 0) break;
         }
         __syncthreads();
     }
+    bundle_close(A, B);
 }
 
-// one CTA: (without k_hard_wide) the clusters above BCAP one at a time, then
 // bundles of BCAP member slots until the queue is empty; OCC CTAs per SM
 template <int BCAP, int OCC>
-__global__ void __launch_bounds__(bundle_threads(BCAP), OCC) k_hard_bundles(HardArgs A) {
-    constexpr int BT = BundleSmem<BCAP>::NT;
-    extern __shared__ __align__(16) unsigned char bundle_smem[];
-    BundleSmem<BCAP> &B = *reinterpret_cast<BundleSmem<BCAP> *>(bundle_smem);
-    __shared__ double red_d[BT / 32];
-    __shared__ long long red_l[BT / 32];
-    __shared__ int q_sh;
-    const int tid = threadIdx.x;
-    const long long t_k0 = A.phase_cycles ? clock64() : 0;
-    const Team<BT> tm{tid, red_d, red_l};
-    if (!A.wide) {
-        for (int guard = 0; guard < (1 << 30); guard++) {
-            if (tid == 0) q_sh = atomicAdd(&A.queue[0], 1);
-            __syncthreads();
-            const int q = q_sh;
-            __syncthreads();
-            if (q >= A.n_tier[0]) break;
-            run_cluster<BT>(A, A.order[q], tm);
-        }
-    }
-    // the lone tier: each cluster integrated alone by the whole CTA, the
-    // bundle's shared memory holding its state (the predicted longest chains
-    // start first, beside bundles on the other CTA slots of the SM)
-    if (A.lone_in) {
-        LoneSmem<BT> &L = *reinterpret_cast<LoneSmem<BT> *>(bundle_smem);
-        for (int guard = 0; guard < (1 << 30); guard++) {
-            if (tid == 0) q_sh = atomicAdd(&A.queue[3], 1);
-            __syncthreads();
-            const int q = q_sh;
-            __syncthreads();
-            if (q >= A.n_tier[2]) break;
-            const int c = A.order[A.n_tier[0] + A.n_tier[1] + q];
-            if (A.cnt[c] > LCAP) {  // the lone tier holds at most LCAP members
-                if (tid == 0) atomicOr(A.status, ST_CLUSTER_TOO_BIG);
-                continue;
-            }
-            lone_cluster<BT>(A, c, L, tm, red_d);
-        }
-    }
-    if (tid == 0) {
-        B.used = 0;
-        B.ncl = 0;
-        B.n_pend = 0;
-        B.i_pend = 0;
-        B.exhausted = 0;
-        B.phase = 0;
-        for (int k = 0; k < HP_N; k++) B.ph_acc[k] = 0;
-        B.ph_t = clock64();
-        B.ph_acc[HP_LONE] = B.ph_t - t_k0;  // the clusters above the slots, the lone tier
-    }
+__global__ void __launch_bounds__(bundle_threads(BCAP), OCC) k_hard_bundles(const __grid_constant__ HardArgs A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    bundle_init(B);
     __syncthreads();
     for (int guard = 0; guard < (1 << 30); guard++) {
-        if (tid == 0) {
+        if (threadIdx.x == 0) {
             B.fresh_k = B.ncl;
             B.fresh_p = B.used;
         }
         __syncthreads();
-        bundle_refill(A, B);
+        bundle_refill<BCAP>(A);
         if (B.ncl == 0) break;
-        if (B.fresh_k < B.ncl) {
-            bundle_load(A, B);
-            const int nt = bundle_list(B, MF_TGT);
-            bundle_pairs(A, B, 0, nt);
-            bundle_finalize(A, B, 0, nt, 2);
-        }
+        if (B.fresh_k < B.ncl) bundle_load<BCAP>(A);
         HP_MARK(HP_ADMIT);
         bundle_step(A, B);
-        if (B.any) bundle_retire(A, B);
+        if (B.any) bundle_retire<BCAP>(A);
         HP_MARK(HP_RETIRE);
     }
-    if (A.phase_cycles && tid == 0)
-        for (int k = 0; k < HP_N; k++) atomicAdd(&A.phase_cycles[k], (unsigned long long)B.ph_acc[k]);
+    bundle_close(A, B);
 }
 
 #undef FOR_SLOTS

@@ -236,8 +236,8 @@ int p3t_hard_fetch(int col_cap, long long *col_pairs, double *edisp);
 int p3t_set_hard_tiers(int warp_min, int cta_min);
 /* Execution form of the hard launch: 0 (default) bundles -- each CTA holds
  * the members of many clusters in shared memory and advances them together,
- * so FP64 work is spread over all lanes; clusters above the bundle capacity
- * (256 members) run one per CTA.  1: the size tiers of p3t_set_hard_tiers.
+ * so FP64 work is spread over all lanes; clusters above a bundle's slots run
+ * alone (p3t_set_hard_wide).  1: the size tiers of p3t_set_hard_tiers.
  * Both give identical results.  No counterpart in GPLUM's interface. */
 int p3t_set_hard_mode(int mode);
 /* Bundle form with the learned order: clusters whose predicted
@@ -246,15 +246,16 @@ int p3t_set_hard_mode(int mode);
  * bundle (default 6.75, about 110 block steps; set by the autotuner from
  * whole runs; 0 turns it off).  Results do not depend on it. */
 int p3t_set_hard_heavy(float log2_steps);
-/* Bundle form: the clusters above the bundle's member slots run in a second,
- * concurrent launch as lone bundles of up to 512 slots, one per CTA of 512
- * threads holding its SM, submitted before the bundle kernel (1, default), or
- * one cluster per CTA inside the main launch (0).  Results are bit-identical;
- * set by the autotuner. */
+/* Bundle form: clusters above the bundle's member slots run in a second,
+ * concurrent launch of CTAs that hold their SM, submitted before the bundle
+ * kernel, one cluster at a time: as lone bundles up to 512 members (1,
+ * default) or up to 256 (0); larger ones in the one-cluster-per-CTA form.
+ * Results are bit-identical; set by the autotuner. */
 int p3t_set_hard_wide(int on);
-/* Bundle form: member slots per bundle and resident CTAs per SM -- 256/2
- * (default), 128/3 or 128/4 (clusters above the slot count go to the wide
- * or one-per-CTA form).  Results are bit-identical; set by the autotuner. */
+/* Bundle form: member slots per bundle and CTAs per SM asked for -- 128/3
+ * (default), 128/4 or 256/2; a bundle keeps all of its members' state in
+ * shared memory, so at most three CTAs of 128 slots or one of 256 fit an SM,
+ * and a launch uses as many.  Results are bit-identical; set by the autotuner. */
 int p3t_set_hard_bundle(int member_slots, int ctas_per_sm);
 /* Bundle form with the learned order: clusters whose predicted
  * log2(1 + block steps) is at least log2_steps and that have at most 64
@@ -263,10 +264,9 @@ int p3t_set_hard_bundle(int member_slots, int ctas_per_sm);
  * independent parts of a block step (members x components, target x partner
  * pair terms, the sun force, the two time-step criteria) spread over the
  * CTA's threads -- which shortens a block step's chain of FP64 operations
- * (the longest chains of block steps set the launch's span).  ctas = 0: the
- * lone clusters run first in the bundle kernel's own CTAs (256 threads, beside
- * bundles on the SM's other CTA slot); ctas > 0: in a kernel of that many
- * 128-thread CTAs of their own, each holding a whole SM.  Perfect accretion
+ * (the longest chains of block steps set the launch's span).  ctas = 0: one
+ * 128-thread CTA per SM, beside bundles; ctas > 0: that many, each holding a
+ * whole SM.  Perfect accretion
  * only (with fragmentation the clusters stay in the bundles); a block step
  * with a collision runs in the one-cluster-per-CTA form's loop and the lone
  * form goes on from its result.  log2_steps = 0:
@@ -285,11 +285,11 @@ int p3t_set_walk(int form);
 /* Per-phase clock counts of the bundle form's loop (off by default; on, each
  * CTA's thread 0 reads the SM clock at the barriers that end the phases):
  * p3t_hard_phase_cycles writes, summed over the CTAs of the last launch, the
- * cycles of: 0 clusters above the slots and the lone tier, 1 admission
- * (claim, load, first force), 2 block time, 3 prediction, 4 collision
- * detection, 5 active set, 6 pair terms, 7 their sums, 8 correction, 9 time
- * steps, 10 collisions, 11 system time, 12 retirement, 13 of which (in
- * 1, 6, 12) the pair-term drains; n >= 14.  No
+ * cycles of: 1 admission (claim, load), 3 prediction and active set, 4
+ * collision detection, 5 target list, 6 pair lists and terms with the sun
+ * force (those of admission and retirement too), 8 their sums and the
+ * correction, 9 time steps, 10 collisions, 11 system and block time, 12
+ * retirement; 0, 2, 7 and 13 stay zero; n >= 14.  No
  * counterpart in GPLUM's interface (its CALC_WTIME timers are per call). */
 int p3t_set_hard_profile(int on);
 int p3t_hard_phase_cycles(unsigned long long *out, int n);
