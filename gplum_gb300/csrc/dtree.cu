@@ -16,20 +16,29 @@
 //     body box, or size^2 > theta^2 d^2 (d: cell centre of mass to the
 //     group's body box); opened leaves give EPJ entries, unopened cells SPJ
 //     entries (quadrupole about the centre of mass).
-// Steps: bounding box (two-stage reduction); keys; a stable LSD radix sort of
-// (key, index) in 8 passes of 8 bits; the tree one level at a time (a scan of
-// "a new 3-bit digit starts here" over the sorted keys gives the children,
-// contiguous, in level order); moments and boxes bottom-up (leaves sum their
-// bodies in key order, as the host builder; inner nodes combine children by
-// the parallel-axis rule); groups; and the walks, split into (group, node of
-// the upper three levels) tasks taken in pre-order, each walking its subtree
-// with the host builder's stack discipline (count, then fill), so the
-// concatenated lists equal the host builder's entry for entry (SPJ entries
-// name the same cells; node numbers are in level order here).  By default the
-// walk is breadth first instead, one CTA per group over an order-keeping
-// frontier (k_walk_bfs), giving the same lists; the task walk is its
-// fallback.  The lists go straight into the resident soft-force buffers.  Compiled with -fmad=false so the box and
-// opening arithmetic rounds as the host builder's (-ffp-contract=off).
+// Steps: bounding box; keys; a stable LSD radix sort of (key, index) in 8
+// passes of 8 bits, one launch each (k_radix_pass); the nodes of every level
+// at once from the sorted keys (k_node_levels: which levels' nodes a body
+// heads follows from the common prefixes of the keys around it); groups;
+// moments and boxes bottom-up (leaves sum their bodies in key order, as the
+// host builder; inner nodes combine children by the parallel-axis rule); and
+// the walks, breadth first, one CTA per group over an order-keeping frontier
+// (k_walk_bfs), with the walk of (group, node of the upper three levels) tasks
+// as the fallback, taken in pre-order, each walking its subtree with the host
+// builder's stack discipline (count, then fill).  Both give the host
+// builder's lists entry for entry (SPJ entries name the same cells; node
+// numbers are in level order here).  The lists go straight into the resident
+// soft-force buffers.  The host waits three times a build, for the sizes of
+// the node table, of the group table and of the lists.  Compiled with
+// -fmad=false so the box and opening arithmetic rounds as the host builder's
+// (-ffp-contract=off).
+//
+// Small builds are bound by launches and waits, large ones by memory passes.
+// With the nodes one level at a time (five launches, a scan and a host wait for
+// each of the up to 21 levels), a sort of three to five launches a pass and a
+// second sort for the launch order, a build took 179 launches and 1.10 ms at
+// 3000 bodies, 2.68 ms at 1,048,576 (ring) and 4.11 ms at 2,097,152 (0.3-3 AU);
+// now about 30 launches, 0.36, 1.48 and 2.42 ms.
 #include <algorithm>
 #include <cstdint>
 #include <vector>
@@ -53,58 +62,58 @@ struct TNodeF {
     int first, count, child0, nchild;
 };
 
-constexpr int RADIX_TILE = 4096;  // keys per radix block (256 threads x 16)
+constexpr int RADIX_T = 256, RADIX_K = 8, RADIX_TILE = RADIX_T * RADIX_K;  // keys of a radix tile
+constexpr int MAX_LEVEL = 21;                                             // levels below the root
 constexpr int WALK_STACK = 256;
 
 // ---- bounding box and keys ------------------------------------------------------
-__global__ void k_bbox_partial(const double *pos, int n, double *part) {
+// root cube as the host builder: out = {base.xyz, size, scale}; anchored at
+// the lower corner, so a thin axis is not cut at coarse levels.  The last CTA
+// to finish combines the partial boxes.
+__global__ void __launch_bounds__(256) k_bbox(const double *pos, int n, double *part, unsigned *done, double *out) {
     __shared__ double s[6][256];
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        for (int d = 0; d < 3; d++) {
-            lo[d] = fmin(lo[d], pos[3 * i + d]);
-            hi[d] = fmax(hi[d], pos[3 * i + d]);
+    __shared__ bool last;
+    const int tid = threadIdx.x;
+    double b[6] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
+    auto reduce = [&]() {
+        for (int d = 0; d < 6; d++) s[d][tid] = b[d];
+        __syncthreads();
+        for (int o = 128; o > 0; o >>= 1) {
+            if (tid < o)
+                for (int d = 0; d < 3; d++) {
+                    s[d][tid] = fmin(s[d][tid], s[d][tid + o]);
+                    s[3 + d][tid] = fmax(s[3 + d][tid], s[3 + d][tid + o]);
+                }
+            __syncthreads();
         }
-    for (int d = 0; d < 3; d++) {
-        s[d][threadIdx.x] = lo[d];
-        s[3 + d][threadIdx.x] = hi[d];
+    };
+    for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x)
+        for (int d = 0; d < 3; d++) {
+            const double x = pos[3 * i + d];
+            b[d] = fmin(b[d], x);
+            b[3 + d] = fmax(b[3 + d], x);
+        }
+    reduce();
+    if (tid < 6) {
+        __stcg(&part[6 * blockIdx.x + tid], s[tid][0]);
+        __threadfence();
     }
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int d = 0; d < 3; d++) {
-                s[d][threadIdx.x] = fmin(s[d][threadIdx.x], s[d][threadIdx.x + o]);
-                s[3 + d][threadIdx.x] = fmax(s[3 + d][threadIdx.x], s[3 + d][threadIdx.x + o]);
-            }
-        __syncthreads();
-    }
-    if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = s[threadIdx.x][0];
-}
-
-// root cube as the host builder: out = {base.xyz, size, scale} (one block of
-// 256); anchored at the lower corner, so a thin axis is not cut at coarse levels
-__global__ void k_bbox_root(const double *part, int nblk, double *out) {
-    __shared__ double s[6][256];
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int b = threadIdx.x; b < nblk; b += 256)
-        for (int d = 0; d < 3; d++) {
-            lo[d] = fmin(lo[d], part[6 * b + d]);
-            hi[d] = fmax(hi[d], part[6 * b + 3 + d]);
-        }
-    for (int d = 0; d < 3; d++) {
-        s[d][threadIdx.x] = lo[d];
-        s[3 + d][threadIdx.x] = hi[d];
+    if (tid == 0) {
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+        if (last) *done = 0u;
+        __threadfence();
     }
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int d = 0; d < 3; d++) {
-                s[d][threadIdx.x] = fmin(s[d][threadIdx.x], s[d][threadIdx.x + o]);
-                s[3 + d][threadIdx.x] = fmax(s[3 + d][threadIdx.x], s[3 + d][threadIdx.x + o]);
-            }
-        __syncthreads();
-    }
-    if (threadIdx.x) return;
+    if (!last) return;
+    for (int d = 0; d < 6; d++) b[d] = d < 3 ? 1e300 : -1e300;
+    for (int k = tid; k < (int)gridDim.x; k += 256)
+        for (int d = 0; d < 3; d++) {
+            b[d] = fmin(b[d], __ldcg(&part[6 * k + d]));
+            b[3 + d] = fmax(b[3 + d], __ldcg(&part[6 * k + 3 + d]));
+        }
+    reduce();
+    if (tid) return;
     double ext = 0.;
     for (int d = 0; d < 3; d++) ext = fmax(ext, s[3 + d][0] - s[d][0]);
     const double size = ext * 1.0001 + 1e-300;
@@ -123,141 +132,302 @@ __device__ __forceinline__ unsigned long long spread21(unsigned long long v) {
     return v;
 }
 
-__global__ void k_keys(const double *pos, int n, const double *root, unsigned long long *key, int *idx) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    unsigned long long c[3];
-    for (int d = 0; d < 3; d++) {
-        const double u = (pos[3 * i + d] - root[d]) * root[4];
-        long long v = (long long)u;
-        v = v < 0 ? 0 : (v > (1 << 21) - 1 ? (1 << 21) - 1 : v);
-        c[d] = (unsigned long long)v;
+// keys and the counts of each of their eight digits (ghist[8][256], zeroed)
+__global__ void __launch_bounds__(256) k_keys(const double *pos, int n, const double *root, unsigned long long *key,
+                                              int *idx, unsigned *ghist) {
+    __shared__ unsigned h[8][256];
+    const int tid = threadIdx.x;
+    for (int p = 0; p < 8; p++) h[p][tid] = 0u;
+    __syncthreads();
+    const double b0 = root[0], b1 = root[1], b2 = root[2], sc = root[4];
+    for (int base = blockIdx.x * RADIX_TILE; base < min(n, (int)(blockIdx.x + 1) * RADIX_TILE); base += 256) {
+        const int i = base + tid;
+        const unsigned in = __ballot_sync(0xffffffffu, i < n);
+        if (i >= n) continue;
+        unsigned long long c[3];
+        for (int d = 0; d < 3; d++) {
+            const double u = (pos[3 * i + d] - (d == 0 ? b0 : (d == 1 ? b1 : b2))) * sc;
+            long long v = (long long)u;
+            v = v < 0 ? 0 : (v > (1 << 21) - 1 ? (1 << 21) - 1 : v);
+            c[d] = (unsigned long long)v;
+        }
+        const unsigned long long k = (spread21(c[0]) << 2) | (spread21(c[1]) << 1) | spread21(c[2]);
+        key[i] = k;
+        idx[i] = i;
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+            const int d = (int)(k >> (8 * p)) & 255;
+            int same;
+            const unsigned all = __match_all_sync(in, d, &same);
+            if (!same) atomicAdd(&h[p][d], 1u);
+            else if ((tid & 31) == __ffs(all) - 1) atomicAdd(&h[p][d], (unsigned)__popc(all));
+        }
     }
-    key[i] = (spread21(c[0]) << 2) | (spread21(c[1]) << 1) | spread21(c[2]);
-    idx[i] = i;
+    __syncthreads();
+    for (int p = 0; p < 8; p++)
+        if (h[p][tid]) atomicAdd(&ghist[256 * p + tid], h[p][tid]);
 }
 
 // ---- stable LSD radix sort of (key, index) -----------------------------------------
-__global__ void __launch_bounds__(256) k_radix_hist(const unsigned long long *key, int n, int shift, int nblk,
-                                                    int *hist) {
-    __shared__ int h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const int base = blockIdx.x * RADIX_TILE;
-    for (int j = threadIdx.x; j < RADIX_TILE; j += 256) {
-        const int k = base + j;
-        if (k < n) atomicAdd(&h[(key[k] >> shift) & 255], 1);
-    }
-    __syncthreads();
-    hist[threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];  // digit-major
-}
-
-// scatter of one tile in 16 rounds of 256 keys; within a round, keys with the
-// same digit keep their order (warp match + per-warp counts)
-__global__ void __launch_bounds__(256) k_radix_scatter(const unsigned long long *key, const int *idx, int n,
-                                                       int shift, int nblk, const int *offs,
-                                                       unsigned long long *key_out, int *idx_out) {
-    __shared__ int cnt[8][256];
-    __shared__ int run[256];
+// One pass over an 8-bit digit in one launch: a tile ranks its keys by digit
+// (warp match, per-warp counts, so equal digits keep their order), publishes
+// its digit counts, sums its predecessors' by decoupled look-back (one thread
+// a digit) and writes its keys digit by digit from shared memory, so that keys
+// are read and written once a pass.  200,000 keys: 11.7 us a pass (ncu) against
+// 29 us in three to five launches (counts, scan, scatter).
+__global__ void __launch_bounds__(RADIX_T) k_radix_pass(const unsigned long long *__restrict__ key,
+                                                        const int *__restrict__ idx, int n, int ntiles, int shift,
+                                                        const unsigned *__restrict__ ghist, unsigned long long *st,
+                                                        unsigned *ticket, unsigned epoch, int *status,
+                                                        unsigned long long *__restrict__ key_out,
+                                                        int *__restrict__ idx_out) {
+    constexpr int NW = RADIX_T / 32;
+    __shared__ unsigned long long sk[RADIX_TILE];
+    __shared__ int si[RADIX_TILE], wc[NW][256], dstart[256], dbase[256], ws[2][NW], sh_tile;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    for (int j = 0; j < 8; j++) cnt[j][tid] = 0;
-    run[tid] = offs[tid * nblk + blockIdx.x];
+    const int tile = lb_tile(ticket, ntiles, &sh_tile);
+    for (int j = 0; j < NW; j++) wc[j][tid] = 0;
     __syncthreads();
-    const int base = blockIdx.x * RADIX_TILE;
-    for (int r = 0; r < RADIX_TILE / 256; r++) {
-        const int k = base + r * 256 + tid;
-        const bool valid = k < n;
-        unsigned long long kv = 0;
-        int iv = 0, d = 256;
-        if (valid) {
-            kv = key[k];
-            iv = idx[k];
-            d = (int)((kv >> shift) & 255);
-        }
+    const int base = tile * RADIX_TILE, cnt = min(RADIX_TILE, n - base);
+    unsigned long long kv[RADIX_K];
+    int iv[RADIX_K], rk[RADIX_K];
+#pragma unroll
+    for (int r = 0; r < RADIX_K; r++) {
+        const int q = w * (32 * RADIX_K) + r * 32 + lane;
+        kv[r] = q < cnt ? key[base + q] : 0ULL;
+        iv[r] = q < cnt ? idx[base + q] : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < RADIX_K; r++) {
+        const bool valid = w * (32 * RADIX_K) + r * 32 + lane < cnt;
+        const int d = valid ? (int)(kv[r] >> shift) & 255 : 256;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid && rank == 0) cnt[w][d] = __popc(peers);
-        __syncthreads();
-        if (valid) {
-            int off = run[d] + rank;
-            for (int ww = 0; ww < w; ww++) off += cnt[ww][d];
-            key_out[off] = kv;
-            idx_out[off] = iv;
+        const int before = __popc(peers & ((1u << lane) - 1u));
+        int pre = 0;
+        if (valid) pre = wc[w][d];
+        __syncwarp();
+        if (valid && before == 0) wc[w][d] = pre + __popc(peers);
+        __syncwarp();
+        rk[r] = pre + before;
+    }
+    __syncthreads();
+    // thread d: the digit's keys in the tile, by warp
+    int total = 0;
+#pragma unroll
+    for (int j = 0; j < NW; j++) {
+        const int c = wc[j][tid];
+        wc[j][tid] = total;
+        total += c;
+    }
+    unsigned long long *const mine = st + (size_t)tile * 256 + tid;
+    lb_put(mine, epoch, tile == 0 ? LB_PREFIX : LB_SUM, (unsigned)total);
+    // exclusive sums over the digits: of the tile's counts and of all keys'
+    const int g = (int)ghist[tid];
+    int x = total, y = g;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, x, o), b = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) {
+            x += a;
+            y += b;
         }
-        __syncthreads();
-        int add = 0;
-        for (int ww = 0; ww < 8; ww++) {
-            add += cnt[ww][tid];
-            cnt[ww][tid] = 0;
+    }
+    if (lane == 31) {
+        ws[0][w] = x;
+        ws[1][w] = y;
+    }
+    __syncthreads();
+    int ds = x - total, gs = y - g;
+    for (int k = 0; k < w; k++) {
+        ds += ws[0][k];
+        gs += ws[1][k];
+    }
+    unsigned ex = 0;
+    for (int p = tile - 1; p >= 0; p--) {
+        unsigned flag;
+        ex += lb_get(st + (size_t)p * 256 + tid, epoch, flag, status);
+        if (flag == LB_PREFIX) break;
+    }
+    if (tile > 0) lb_put(mine, epoch, LB_PREFIX, ex + (unsigned)total);
+    dstart[tid] = ds;
+    dbase[tid] = gs + (int)ex - ds;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RADIX_K; r++) {
+        if (w * (32 * RADIX_K) + r * 32 + lane >= cnt) continue;
+        const int d = (int)(kv[r] >> shift) & 255;
+        const int q = dstart[d] + wc[w][d] + rk[r];
+        sk[q] = kv[r];
+        si[q] = iv[r];
+    }
+    __syncthreads();
+    for (int q = tid; q < cnt; q += RADIX_T) {
+        const unsigned long long k = sk[q];
+        // (a prefix that the wait's limit cut short stays inside the arrays)
+        const int o = min(max(dbase[(int)(k >> shift) & 255] + q, 0), n - 1);
+        key_out[o] = k;
+        idx_out[o] = si[q];
+    }
+}
+
+// ---- the nodes of every level --------------------------------------------------------
+// 3-bit digits that two keys share from the top (21: equal)
+__device__ __forceinline__ int common_digits(unsigned long long a, unsigned long long b) {
+    const unsigned long long x = a ^ b;
+    return x == 0ULL ? MAX_LEVEL : (__clzll((long long)x) - 1) / 3;
+}
+
+// The levels whose node body k (in key order) heads.  The cell of level L
+// around k is a node when the cell of level L - 1 around k holds more than
+// `limit` bodies, and k heads it when it does not hold k - 1: L from
+// common_digits(k - 1, k) + 1 on, up to one below the deepest cell around k of
+// more than `limit` bodies (MAX_LEVEL at most).  A cell of level l around k
+// holds more than `limit` bodies when some limit + 1 consecutive keys around k
+// share l digits.  lo > hi: none.  The root is always a node, headed by body 0.
+__device__ __forceinline__ void head_levels(const unsigned long long *__restrict__ key, int n, int k, int limit,
+                                            int &lo, int &hi) {
+    const unsigned long long me = key[k];
+    lo = k == 0 ? 0 : common_digits(key[k - 1], me) + 1;
+    int m = -1;  // deepest level of a cell of more than `limit` bodies around k
+    if (limit <= 16) {
+        for (int j = max(0, k - limit); j <= k && j + limit < n; j++) m = max(m, common_digits(key[j], key[j + limit]));
+    } else {
+        // bodies around k in the cell of level l, up to `limit` on each side,
+        // by bisection; the deepest level by bisection
+        int a = -1, b = MAX_LEVEL;
+        while (a < b) {
+            const int l = (a + b + 1) >> 1;
+            int p = max(0, k - limit), q = k;
+            while (p < q) {
+                const int mid = (p + q) >> 1;
+                if (common_digits(key[mid], me) >= l) q = mid;
+                else p = mid + 1;
+            }
+            const int first = p;
+            p = k;
+            q = min(n - 1, k + limit);
+            while (p < q) {
+                const int mid = (p + q + 1) >> 1;
+                if (common_digits(key[mid], me) >= l) p = mid;
+                else q = mid - 1;
+            }
+            if (p - first + 1 > limit) a = l;
+            else b = l - 1;
         }
-        run[tid] += add;
-        __syncthreads();
+        m = a;
     }
+    hi = m >= 0 ? min(m, MAX_LEVEL - 1) + 1 : (k == 0 ? 0 : -1);
 }
 
-// ---- tree, one level at a time -------------------------------------------------------
-__global__ void k_root_node(TNode *nd, int *parent, const double *root, int n, int limit, int *enode) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0) {
-        nd[0].first = 0;
-        nd[0].count = n;
-        nd[0].child0 = -1;
-        nd[0].nchild = 0;
-        nd[0].size = root[3];
-        parent[0] = -1;
+// per body its levels, per block and level the bodies that head a node
+// (cnt[level][block]); blocks of 256 bodies
+__global__ void __launch_bounds__(256) k_node_levels(const unsigned long long *__restrict__ key, int n, int limit,
+                                                     unsigned short *lev, int *cnt) {
+    __shared__ int wc[8][MAX_LEVEL + 1];
+    const int k = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int lo = 1, hi = 0;
+    if (k < n) {
+        head_levels(key, n, k, limit, lo, hi);
+        lev[k] = (unsigned short)(lo | ((hi + 1) << 8));
     }
-    if (k < n) enode[k] = (n > limit) ? 0 : -1;
-}
-
-__global__ void k_lvl_heads(const unsigned long long *key, const int *enode, const TNode *nd, int n, int shift,
-                            int *head) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int p = enode[k];
-    int h = 0;
-    if (p >= 0) h = (k == nd[p].first) || (((key[k] >> shift) & 7ULL) != ((key[k - 1] >> shift) & 7ULL));
-    head[k] = h;
-}
-
-__global__ void k_lvl_make(const int *enode, const int *head, const int *hs, int n, int base, TNode *nd,
-                           int *parent, int *enode_next) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int p = enode[k];
-    if (p < 0) {
-        enode_next[k] = -1;
-        return;
+    for (int L = 0; L <= MAX_LEVEL; L++) {
+        const unsigned b = __ballot_sync(0xffffffffu, lo <= L && L <= hi);
+        if (lane == 0) wc[w][L] = __popc(b);
     }
-    const int c = base + hs[k] + head[k] - 1;
-    enode_next[k] = c;
-    if (head[k]) {
-        nd[c].first = k;
-        nd[c].size = nd[p].size * 0.5;
-        nd[c].child0 = -1;
-        nd[c].nchild = 0;
-        parent[c] = p;
-        if (k == nd[p].first) nd[p].child0 = c;
+    __syncthreads();
+    if (threadIdx.x <= MAX_LEVEL) {
+        int c = 0;
+        for (int j = 0; j < 8; j++) c += wc[j][threadIdx.x];
+        cnt[threadIdx.x * gridDim.x + blockIdx.x] = c;
     }
 }
-
-__global__ void k_lvl_count(int base, int m, TNode *nd, const int *parent) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    const int c = base + t, p = parent[c];
-    const int end = (t + 1 < m && parent[c + 1] == p) ? nd[c + 1].first : nd[p].first + nd[p].count;
-    nd[c].count = end - nd[c].first;
-    if (nd[p].child0 == c) {
-        int j = 1;
-        while (t + j < m && parent[c + j] == p && j < 8) j++;
-        nd[p].nchild = j;
+// their exclusive sums, level after level: the number of each block's first
+// node of a level; lstart[level] (and, last, the node count)
+struct LevelScan {
+    const int *cnt;
+    int *off, *lstart;
+    int nblk;
+    __device__ int operator()(int, int i) const { return cnt[i]; }
+    __device__ void operator()(int, int i, int prefix, int) const {
+        off[i] = prefix;
+        if (i % nblk == 0) lstart[i / nblk] = prefix;
     }
-}
+    __device__ void total(int, int t) const { lstart[MAX_LEVEL + 1] = t; }
+};
 
-__global__ void k_lvl_split(int n, int level, int limit, const TNode *nd, int *enode) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int c = enode[k];
-    if (c >= 0 && !(nd[c].count > limit && level < 21)) enode[k] = -1;
+// The nodes: body k writes those it heads, numbered in level order.  A node
+// with a deeper one headed by the same body is split, the body's deepest is
+// a leaf.  nch (zeroed) counts children; leaves and each level's inner nodes
+// are listed (list[nn..]: the inner nodes of level L from lstart[L] on;
+// icnt[L] of them; icnt[MAX_LEVEL + 1] leaves).
+__global__ void __launch_bounds__(256) k_nodes(const unsigned long long *__restrict__ key, int n,
+                                               const unsigned short *__restrict__ lev, const int *__restrict__ off,
+                                               const int *__restrict__ lstart, const double *__restrict__ root, int nn,
+                                               TNode *nd, int *parent, int *nch, int *list, int *icnt) {
+    __shared__ int wc[8][MAX_LEVEL + 1];
+    const int k = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int lo = 1, hi = 0;
+    unsigned long long me = 0;
+    if (k < n) {
+        lo = lev[k] & 255;
+        hi = (lev[k] >> 8) - 1;
+        me = key[k];
+    }
+    for (int L = 0; L <= MAX_LEVEL; L++) {
+        const unsigned b = __ballot_sync(0xffffffffu, lo <= L && L <= hi);
+        if (lane == 0) wc[w][L] = __popc(b);
+    }
+    __syncthreads();
+    const unsigned lt = (1u << lane) - 1u;
+    double size = root[3];
+    int up = 0, leaf = -1;  // heads of the level above up to k; this body's leaf
+    for (int L = 0; L <= MAX_LEVEL; L++, size *= 0.5) {
+        const bool head = lo <= L && L <= hi, inner = head && L < hi;
+        const unsigned b = __ballot_sync(0xffffffffu, head), bi = __ballot_sync(0xffffffffu, inner);
+        int c = off[L * gridDim.x + blockIdx.x] + __popc(b & lt);
+        for (int j = 0; j < w; j++) c += wc[j][L];
+        int at = 0;
+        if (bi) {
+            if (lane == 0) at = atomicAdd(&icnt[L], __popc(bi));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(bi & lt);
+        }
+        if (head) {
+            // its end: the first later key outside the cell
+            const int sh = 3 * (MAX_LEVEL - L);
+            const unsigned long long pre = L == 0 ? 0ULL : me >> sh;
+            int p = k, step = 1;  // key[p] inside
+            while (p + step < n && (L == 0 || (key[p + step] >> sh) == pre)) {
+                p += step;
+                step *= 2;
+            }
+            int q = min(p + step, n);  // n or outside
+            while (q - p > 1) {
+                const int mid = (p + q) >> 1;
+                if (L == 0 || (key[mid] >> sh) == pre) p = mid;
+                else q = mid;
+            }
+            TNode &N = nd[c];
+            N.first = k;
+            N.count = q - k;
+            N.size = size;
+            // a split node's first child is headed by the same body, one level down
+            N.child0 = -1;
+            const int par = L == 0 ? -1 : up - 1;
+            parent[c] = par;
+            if (L > 0) atomicAdd(&nch[par], 1);
+            if (L > lo) nd[par].child0 = c;
+            if (inner) list[nn + lstart[L] + at] = c;
+            else leaf = c;
+        }
+        up = c + (head ? 1 : 0);
+    }
+    const unsigned bl = __ballot_sync(0xffffffffu, leaf >= 0);
+    if (bl) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&icnt[MAX_LEVEL + 1], __popc(bl));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bl & lt);
+        if (leaf >= 0) list[at] = leaf;
+    }
 }
 
 // ---- moments and boxes, bottom-up -------------------------------------------------------
@@ -266,8 +436,8 @@ constexpr int LEAF_B = 8;  // bodies of a leaf loaded at once (leaves hold at mo
 // builder's sums), an inner node combines its children in child order by the
 // parallel-axis rule.  Children are read through L2 (ld.cg): they may have
 // been written by other CTAs of the same launch.
-__device__ void node_moments(int c, TNode *nd, SPJRec *spj, const int *order, const double *pos, const double *mass,
-                             const double *rs) {
+__device__ void node_moments(int c, TNode *nd, TNodeF *nf, SPJRec *spj, const int *order, const double *pos,
+                             const double *mass, const double *rs) {
     TNode &N = nd[c];
     const int nchild = __ldcg(&N.nchild), child0 = __ldcg(&N.child0);
     double m = 0., cx = 0., cy = 0., cz = 0., q[6] = {0., 0., 0., 0., 0., 0.};
@@ -367,14 +537,31 @@ __device__ void node_moments(int c, TNode *nd, SPJRec *spj, const int *order, co
     S.pos[1] = cy;
     S.pos[2] = cz;
     S.xx = q[0]; S.yy = q[1]; S.zz = q[2]; S.xy = q[3]; S.xz = q[4]; S.yz = q[5];
+    // the walk's FP32 copy
+    TNodeF F;
+    for (int d = 0; d < 3; d++) {
+        F.ilo[d] = (float)ilo[d];
+        F.ihi[d] = (float)ihi[d];
+        F.olo[d] = (float)olo[d];
+        F.ohi[d] = (float)ohi[d];
+    }
+    F.com[0] = (float)cx;
+    F.com[1] = (float)cy;
+    F.com[2] = (float)cz;
+    F.size = (float)N.size;
+    F.first = N.first;
+    F.count = N.count;
+    F.child0 = child0;
+    F.nchild = nchild;
+    nf[c] = F;
 }
 
 // one level (nodes lo..hi-1) per launch, deepest level first
-__global__ void k_moments(int lo, int hi, TNode *nd, SPJRec *spj, const int *order, const double *pos,
+__global__ void k_moments(int lo, int hi, TNode *nd, TNodeF *nf, SPJRec *spj, const int *order, const double *pos,
                           const double *mass, const double *rs) {
     const int c = lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= hi) return;
-    node_moments(c, nd, spj, order, pos, mass, rs);
+    node_moments(c, nd, nf, spj, order, pos, mass, rs);
 }
 
 // Moments in lane-dense launches: every leaf at once from a compacted list
@@ -382,60 +569,62 @@ __global__ void k_moments(int lo, int hi, TNode *nd, SPJRec *spj, const int *ord
 // level at a time, deepest first.  A launch over all nodes of a level, or one
 // climbing thread per finished child, left most lanes of the FP64 pipe's warp
 // instructions idle (ncu: 23 % lane efficiency for the climbing form).
-__global__ void k_leaf_flag(int nn, const TNode *nd, int *flag) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < nn) flag[c] = nd[c].nchild == 0;
-}
-// leaves to the front of `list` (ascending), inner nodes to the back in
-// ascending node order (so each level's inner nodes are one run; inner node c
-// sits at nn - 1 - (c - pos[c]) counted from the back); count = leaves
-__global__ void k_leaf_list(int nn, const int *flag, const int *pos, int *list, int *count) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nn) return;
-    if (flag[c]) list[pos[c]] = c;
-    else list[nn - 1 - (c - pos[c])] = c;
-    if (c == nn - 1) *count = pos[c] + flag[c];
-}
-__global__ void k_moments_leaves(const int *list, const int *count, TNode *nd, SPJRec *spj, const int *order,
-                                 const double *pos, const double *mass, const double *rs) {
+__global__ void k_moments_leaves(const int *list, const int *count, TNode *nd, TNodeF *nf, SPJRec *spj,
+                                 const int *order, const double *pos, const double *mass, const double *rs) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= *count) return;
-    node_moments(list[t], nd, spj, order, pos, mass, rs);
+    node_moments(list[t], nd, nf, spj, order, pos, mass, rs);
 }
-// the inner nodes of level [lo, hi): their run in the back of `list` (from
-// the leaf-position scan: inner nodes below c number c - lpos[c])
-__global__ void k_moments_inner(int lo, int hi, int nn, const int *list, const int *lpos, const int *flag, TNode *nd,
-                                SPJRec *spj, const int *order, const double *pos, const double *mass, const double *rs) {
-    const int a = lo - lpos[lo];                                 // inner nodes before the level
-    const int b = (hi < nn) ? hi - lpos[hi] : nn - (lpos[nn - 1] + flag[nn - 1]);  // ... and up to its end
+// the inner nodes of a level (inner: their list, icnt: how many)
+__global__ void k_moments_inner(const int *inner, const int *icnt, TNode *nd, TNodeF *nf, SPJRec *spj,
+                                const int *order, const double *pos, const double *mass, const double *rs) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a + t >= b) return;
-    node_moments(list[nn - 1 - (a + t)], nd, spj, order, pos, mass, rs);
+    if (t >= *icnt) return;
+    node_moments(inner[t], nd, nf, spj, order, pos, mass, rs);
+}
+// the inner nodes of levels from..to (deepest first) in one CTA, level after
+// level: runs of levels of few nodes -- the top of the tree, and the deep
+// chains around close pairs -- whose launches would cost more than their work
+constexpr int TOP_T = 128, TOP_NODES = 128;
+__global__ void __launch_bounds__(TOP_T) k_moments_run(int from, int to, const int *lstart, const int *inner, const int *icnt,
+                                                       TNode *nd, TNodeF *nf, SPJRec *spj, const int *order,
+                                                       const double *pos, const double *mass, const double *rs) {
+    for (int L = from; L >= to; L--) {
+        for (int t = threadIdx.x; t < icnt[L]; t += TOP_T)
+            node_moments(inner[lstart[L] + t], nd, nf, spj, order, pos, mass, rs);
+        __threadfence();
+        __syncthreads();
+    }
 }
 
 // ---- groups ---------------------------------------------------------------------------------
-__global__ void k_group_mark(int nn, const TNode *nd, const int *parent, int ngl, int *gmark) {
+// also the children counts into the node records
+__global__ void k_group_mark(int nn, TNode *nd, const int *parent, const int *nch, int ngl, int *gmark) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nn) return;
-    const TNode &N = nd[c];
-    const bool cand = N.count <= ngl || N.nchild == 0;
+    TNode &N = nd[c];
+    const int m = nch[c];
+    N.nchild = m;
+    const bool cand = N.count <= ngl || m == 0;
     const bool top = (c == 0) || nd[parent[c]].count > ngl;
     if (cand && top) gmark[N.first] = c + 1;
 }
-
-__global__ void k_group_flag(const int *gmark, int n, int *flag) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) flag[k] = gmark[k] > 0;
-}
-
-__global__ void k_group_fill(const int *gmark, const int *gpos, int n, int ng, int *gnode, int *i_off) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n && gmark[k] > 0) {
-        gnode[gpos[k]] = gmark[k] - 1;
-        i_off[gpos[k]] = k;
+// the groups in key order (a scan over the bodies): node and first body
+struct GroupScan {
+    const int *gmark;
+    int *gnode, *i_off, *ng;
+    int n;
+    __device__ int operator()(int, int k) const { return gmark[k] > 0; }
+    __device__ void operator()(int, int k, int prefix, int v) const {
+        if (!v) return;
+        gnode[prefix] = gmark[k] - 1;
+        i_off[prefix] = k;
     }
-    if (k == 0) i_off[ng] = n;
-}
+    __device__ void total(int, int t) const {
+        i_off[t] = n;
+        *ng = t;
+    }
+};
 
 // ---- walk --------------------------------------------------------------------------------------
 __device__ __forceinline__ bool box_overlap(const double *alo, const double *ahi, const double *blo,
@@ -469,26 +658,6 @@ __device__ __forceinline__ bool cell_open(const TNode &C, const double *gilo, co
                                           const double *golo, const double *gohi, double theta2) {
     const bool near = box_overlap(C.olo, C.ohi, gilo, gihi) || box_overlap(golo, gohi, C.ilo, C.ihi);
     return near || (C.size * C.size > theta2 * box_dist2(gilo, gihi, C.com));
-}
-
-__global__ void k_node_f32(const TNode *nd, int nn, TNodeF *nf) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nn) return;
-    const TNode &N = nd[c];
-    TNodeF F;
-    for (int d = 0; d < 3; d++) {
-        F.ilo[d] = (float)N.ilo[d];
-        F.ihi[d] = (float)N.ihi[d];
-        F.olo[d] = (float)N.olo[d];
-        F.ohi[d] = (float)N.ohi[d];
-        F.com[d] = (float)N.com[d];
-    }
-    F.size = (float)N.size;
-    F.first = N.first;
-    F.count = N.count;
-    F.child0 = N.child0;
-    F.nchild = N.nchild;
-    nf[c] = F;
 }
 
 // Ternary comparisons on FP32 copies of doubles (each within 2^-24 relative
@@ -800,6 +969,28 @@ __global__ void __launch_bounds__(BFS_T) k_walk_bfs(const TNode *nd, const TNode
     }
 }
 
+// What the host reads after the walk: lists' sizes, frontier items, whether a
+// frontier or the store overflowed, the status bits so far.
+struct WalkInfo {
+    unsigned long long cursor;
+    int n[2], overflow, status;
+};
+// the groups' list offsets from their counts (scan y = 0: EPJ, 1: SPJ)
+struct WalkScan {
+    const int *jc, *sc;
+    int *j_off, *s_off;
+    int ng;
+    WalkInfo *info;
+    const int *status;
+    __device__ int operator()(int y, int g) const { return y ? sc[g] : jc[g]; }
+    __device__ void operator()(int y, int g, int prefix, int) const { (y ? s_off : j_off)[g] = prefix; }
+    __device__ void total(int y, int t) const {
+        (y ? s_off : j_off)[ng] = t;
+        info->n[y] = t;
+        if (y == 0) info->status = *(const volatile int *)status;
+    }
+};
+
 // fill pass: group g's entries from its stored frontier, in frontier order
 __global__ void __launch_bounds__(BFS_T) k_walk_bfs_fill(const TNodeF *nf, int ng, const int *len, const long long *off,
                                                          const int *store, const int *order, const int *j_off,
@@ -847,34 +1038,56 @@ __global__ void k_walk_group_off(const int *jo, const int *so, int ng, int ntop,
     s_off[g] = (g < ng) ? so[(long long)g * ntop] : ns;
 }
 
-// launch order of the soft kernel: largest groups first (key: weight desc, group asc)
-__global__ void k_group_weight(int ng, const int *i_off, const int *j_off, const int *s_off,
-                               unsigned long long *key, int *idx) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ng) return;
-    const long long ni = i_off[g + 1] - i_off[g];
-    const long long nj = (j_off[g + 1] - j_off[g]) + 2LL * (s_off[g + 1] - s_off[g]);
-    const long long w = ((ni + 31) / 32) * 32 * nj;
-    const unsigned long long wc = (unsigned long long)(w < (1LL << 43) ? w : (1LL << 43) - 1);
-    key[g] = (((1ULL << 43) - 1 - wc) << 20) | (unsigned long long)g;
-    idx[g] = g;
+// Launch order of the soft kernel: groups by descending weight class (eight
+// classes an octave; the order inside a class is arbitrary, and no result
+// depends on it), a counting sort by one CTA.  A full sort of the weights was 40
+// launches.
+constexpr int GO_T = 1024, GO_BINS = 1024;
+__global__ void __launch_bounds__(GO_T) k_group_order(int ng, const int *i_off, const int *j_off, const int *s_off,
+                                                      int *order) {
+    __shared__ int h[GO_BINS], ws[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    auto bin = [&](int g) {
+        const long long ni = i_off[g + 1] - i_off[g];
+        const long long nj = (j_off[g + 1] - j_off[g]) + 2LL * (s_off[g + 1] - s_off[g]);
+        const float wt = (float)(((ni + 31) / 32) * 32 * nj + 1);
+        const int b = (int)(__float_as_uint(wt) >> 20) - (127 << 3);
+        return GO_BINS - 1 - min(max(b, 0), GO_BINS - 1);
+    };
+    h[tid] = 0;
+    __syncthreads();
+    for (int g = tid; g < ng; g += GO_T) atomicAdd(&h[bin(g)], 1);
+    __syncthreads();
+    const int c = h[tid];
+    int x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[w] = x;
+    __syncthreads();
+    for (int k = 0; k < w; k++) x += ws[k];
+    h[tid] = x - c;
+    __syncthreads();
+    for (int g = tid; g < ng; g += GO_T) order[atomicAdd(&h[bin(g)], 1)] = g;
 }
 
 // ---- host side ----------------------------------------------------------------------------------
 struct DTree {
     DevBuf<double> part, root;
     DevBuf<unsigned long long> key, key2;
-    DevBuf<int> idx, idx2, hist, hoff, head, hs, enode, enode2, parent, gmark, gflag, gpos, gnode;
+    DevBuf<unsigned> ghist, done;
+    DevBuf<unsigned short> lev;
+    DevBuf<int> idx, idx2, lcnt, loff, lstart, nch, list, parent, gmark, gnode, ng;
     DevBuf<TNode> nd;
     DevBuf<TNodeF> nf;
     DevBuf<int> top, pc, tasks;
     DevBuf<unsigned char> ostat;
-    DevBuf<int> bjc, bsc, blen, bstore, bover;  // breadth-first walk
-    DevBuf<int> arrived;                        // leaf flags, positions and list of the moments
+    DevBuf<int> bjc, bsc, blen, bstore;  // breadth-first walk
+    DevBuf<WalkInfo> binfo;
     DevBuf<long long> boff;
-    DevBuf<unsigned long long> bcur;
     long long bstore_cap = 1LL << 24;
-    size_t node_cap = 0;
     std::vector<int> level_start;
     int n_nodes = 0, n_groups = 0;
 };
@@ -885,54 +1098,12 @@ static int g_walk_last = -1;  // the form the last build's lists came from
 static int g_walk_cap = BFS_CAP;  // frontier items a group's CTA may hold (lower: more groups take the task walk)
 static int g_moments_up = 1;  // moments: leaves in one launch, then inner nodes per level (1); all nodes per level (0)
 
-// (key, idx) sorted in place by key, stably (8 passes of 8 bits over `bits`)
-static int radix_sort(Context *c, DTree &T, unsigned long long *&key, int *&idx, unsigned long long *&key2,
-                      int *&idx2, int n, int bits) {
-    const int nblk = (n + RADIX_TILE - 1) / RADIX_TILE;
-    int r = 0;
-    if ((r = T.hist.reserve(256 * (size_t)nblk)) || (r = T.hoff.reserve(256 * (size_t)nblk + 1))) return r;
-    for (int shift = 0; shift < bits; shift += 8) {
-        { P3T_COUNT_LAUNCH(); k_radix_hist<<<nblk, 256, 0, c->stream>>>(key, n, shift, nblk, T.hist.p); }
-        if ((r = g_eng.scan(T.hist.p, T.hoff.p, 256 * nblk, nullptr))) return r;  // stream-ordered, no host wait
-        { P3T_COUNT_LAUNCH(); k_radix_scatter<<<nblk, 256, 0, c->stream>>>(key, idx, n, shift, nblk, T.hoff.p, key2, idx2); }
-        std::swap(key, key2);
-        std::swap(idx, idx2);
-    }
-    return cuda_status(cudaGetLastError());
-}
-
-// node storage that keeps its contents when it grows
-static int grow_nodes(Context *c, DTree &T, size_t need) {
-    if (need <= T.node_cap) return 0;
-    const size_t cap = std::max(need, T.node_cap * 2);
-    TNode *np = nullptr;
-    int *pp = nullptr;
-    int r = cuda_status(cudaMalloc(&np, cap * sizeof(TNode)));
-    if (r) return r;
-    if ((r = cuda_status(cudaMalloc(&pp, cap * sizeof(int))))) {
-        cudaFree(np);
-        return r;
-    }
-    if (T.node_cap) {
-        cudaMemcpyAsync(np, T.nd.p, T.node_cap * sizeof(TNode), cudaMemcpyDeviceToDevice, c->stream);
-        cudaMemcpyAsync(pp, T.parent.p, T.node_cap * sizeof(int), cudaMemcpyDeviceToDevice, c->stream);
-        cudaStreamSynchronize(c->stream);
-    }
-    T.nd.release();
-    T.parent.release();
-    T.nd.p = np;
-    T.nd.cap = cap * sizeof(TNode);
-    T.parent.p = pp;
-    T.parent.cap = cap * sizeof(int);
-    T.node_cap = cap;
-    return 0;
-}
-
 static inline int nblocks(long long n, int t = 256) { return (int)std::max<long long>(1, (n + t - 1) / t); }
 
 // Builds the tree of the state's bodies and writes the group lists and the
-// SPJ array into the resident soft-force set.
-static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_limit) {
+// SPJ array into the resident soft-force set.  *status: the status bits that the
+// breadth-first walk's end had seen, -1 when the task walk ran (its own come later).
+static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_limit, int *status) {
     Engine &E = g_eng;
     DTree &T = g_dt;
     DevSet &d = c->res;
@@ -940,115 +1111,125 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
     if (n <= 0 || theta <= 0. || n_leaf_limit < 1 || n_group_limit < 1) return ST_BAD_INDEX;
     const int limit = std::min(n_leaf_limit, n_group_limit);
     int r = 0;
-    const int pb = std::min(1024, nblocks(n));
-    if ((r = T.part.reserve(6 * (size_t)pb)) || (r = T.root.reserve(8)) || (r = T.key.reserve(n)) ||
-        (r = T.key2.reserve(n)) || (r = T.idx.reserve(n)) || (r = T.idx2.reserve(n)) || (r = T.head.reserve(n)) ||
-        (r = T.hs.reserve(n)) || (r = T.enode.reserve(n)) || (r = T.enode2.reserve(n)) ||
-        (r = T.gmark.reserve(n)) || (r = T.gflag.reserve(n)) || (r = T.gpos.reserve(n)))
-        return r;
-    // 1. root cube, keys, sort
-    { P3T_COUNT_LAUNCH(); k_bbox_partial<<<pb, 256, 0, c->stream>>>(E.S.pos, n, T.part.p); }
-    { P3T_COUNT_LAUNCH(); k_bbox_root<<<1, 256, 0, c->stream>>>(T.part.p, pb, T.root.p); }
-    { P3T_COUNT_LAUNCH(); k_keys<<<nblocks(n), 256, 0, c->stream>>>(E.S.pos, n, T.root.p, T.key.p, T.idx.p); }
-    unsigned long long *key = T.key.p, *key2 = T.key2.p;
-    int *idx = T.idx.p, *idx2 = T.idx2.p;
-    if ((r = radix_sort(c, T, key, idx, key2, idx2, n, 64))) return r;  // 8 passes: back in T.key / T.idx
-    // 2. levels
-    if ((r = grow_nodes(c, T, (size_t)n / 4 + 1024))) return r;
-    { P3T_COUNT_LAUNCH(); k_root_node<<<nblocks(n), 256, 0, c->stream>>>(T.nd.p, T.parent.p, T.root.p, n, limit, T.enode.p); }
-    T.level_start.assign(1, 0);
-    int base = 1;
-    int *en = T.enode.p, *en2 = T.enode2.p;
-    for (int level = 0; level < 21; level++) {
-        { P3T_COUNT_LAUNCH(); k_lvl_heads<<<nblocks(n), 256, 0, c->stream>>>(key, en, T.nd.p, n, 3 * (20 - level), T.head.p); }
-        int m = 0;
-        if ((r = E.scan(T.head.p, T.hs.p, n, &m))) return r;
-        if (m == 0) break;
-        if ((r = grow_nodes(c, T, (size_t)base + m))) return r;
-        T.level_start.push_back(base);
-        { P3T_COUNT_LAUNCH(); k_lvl_make<<<nblocks(n), 256, 0, c->stream>>>(en, T.head.p, T.hs.p, n, base, T.nd.p, T.parent.p, en2); }
-        { P3T_COUNT_LAUNCH(); k_lvl_count<<<nblocks(m), 256, 0, c->stream>>>(base, m, T.nd.p, T.parent.p); }
-        { P3T_COUNT_LAUNCH(); k_lvl_split<<<nblocks(n), 256, 0, c->stream>>>(n, level + 1, limit, T.nd.p, en2); }
-        std::swap(en, en2);
-        base += m;
+    const int pb = std::min(512, nblocks(n)), rt = (n + RADIX_TILE - 1) / RADIX_TILE, lbk = nblocks(n);
+    if (!T.done.p) {
+        if ((r = T.done.reserve(1))) return r;
+        cudaMemsetAsync(T.done.p, 0, T.done.cap, c->stream);
     }
-    T.level_start.push_back(base);
+    if ((r = T.part.reserve(6 * (size_t)pb)) || (r = T.root.reserve(8)) || (r = T.key.reserve(n)) ||
+        (r = T.key2.reserve(n)) || (r = T.idx.reserve(n)) || (r = T.idx2.reserve(n)) || (r = d.i_idx.reserve(n)) ||
+        (r = T.ghist.reserve(8 * 256)) || (r = T.lev.reserve(n)) ||
+        (r = T.lcnt.reserve((MAX_LEVEL + 1) * (size_t)lbk)) || (r = T.loff.reserve((MAX_LEVEL + 1) * (size_t)lbk)) ||
+        (r = T.lstart.reserve(MAX_LEVEL + 2)) || (r = T.gmark.reserve(n)) || (r = T.ng.reserve(1)))
+        return r;
+    // 1. root cube, keys, sort (the last pass writes the order into the group lists' bodies)
+    cudaMemsetAsync(T.ghist.p, 0, 8 * 256 * sizeof(unsigned), c->stream);
+    { P3T_COUNT_LAUNCH(); k_bbox<<<pb, 256, 0, c->stream>>>(E.S.pos, n, T.part.p, T.done.p, T.root.p); }
+    { P3T_COUNT_LAUNCH(); k_keys<<<rt, 256, 0, c->stream>>>(E.S.pos, n, T.root.p, T.key.p, T.idx.p, T.ghist.p); }
+    for (int p = 0; p < 8; p++) {
+        const bool odd = p & 1;
+        if ((r = E.lb.reserve(c, 256 * (size_t)rt))) return r;
+        { P3T_COUNT_LAUNCH(); k_radix_pass<<<rt, RADIX_T, 0, c->stream>>>(odd ? T.key2.p : T.key.p, odd ? T.idx2.p : T.idx.p, n, rt, 8 * p,
+                                                                     T.ghist.p + 256 * p, E.lb.st.p, E.lb.ticket.p,
+                                                                     E.lb.epoch, c->status, odd ? T.key.p : T.key2.p,
+                                                                     p == 7 ? d.i_idx.p : (odd ? T.idx.p : T.idx2.p)); }
+    }
+    const unsigned long long *key = T.key.p;
+    const int *idx = d.i_idx.p;
+    // 2. nodes of every level
+    { P3T_COUNT_LAUNCH(); k_node_levels<<<lbk, 256, 0, c->stream>>>(key, n, limit, T.lev.p, T.lcnt.p); }
+    if ((r = launch_scan_lb(c, E.lb, LevelScan{T.lcnt.p, T.loff.p, T.lstart.p, lbk},
+                            LevelScan{T.lcnt.p, T.loff.p, T.lstart.p, lbk}, (MAX_LEVEL + 1) * lbk)))
+        return r;
+    int ls[MAX_LEVEL + 2];
+    if ((r = d2h(c, ls, T.lstart.p, sizeof ls))) return r;
+    const int base = ls[MAX_LEVEL + 1];
+    if (base < 1 || base > (MAX_LEVEL + 1) * (long long)n) return ST_ITER_CAP;
+    T.level_start.assign(1, 0);
+    for (int L = 1; L <= MAX_LEVEL + 1 && ls[L] > T.level_start.back(); L++) T.level_start.push_back(ls[L]);
     T.n_nodes = base;
-    if ((r = d.spj.reserve(base))) return r;
-    // 3. moments, bottom-up in one launch (or one launch per level, deepest first)
+    if ((r = T.nd.reserve(base)) || (r = T.parent.reserve(base)) || (r = T.nch.reserve((size_t)base + MAX_LEVEL + 2)) ||
+        (r = T.list.reserve(2 * (size_t)base)) || (r = T.nf.reserve(base)) || (r = d.spj.reserve(base)) ||
+        (r = T.gnode.reserve(base + 1)) || (r = d.i_off.reserve(base + 1)))
+        return r;
+    int *icnt = T.nch.p + base;
+    cudaMemsetAsync(T.nch.p, 0, ((size_t)base + MAX_LEVEL + 2) * sizeof(int), c->stream);
+    cudaMemsetAsync(T.gmark.p, 0, n * sizeof(int), c->stream);
+    { P3T_COUNT_LAUNCH(); k_nodes<<<lbk, 256, 0, c->stream>>>(key, n, T.lev.p, T.loff.p, T.lstart.p, T.root.p, base, T.nd.p, T.parent.p,
+                                                       T.nch.p, T.list.p, icnt); }
+    // 3. groups in Morton order (their count comes back while the moments run)
+    { P3T_COUNT_LAUNCH(); k_group_mark<<<nblocks(base), 256, 0, c->stream>>>(base, T.nd.p, T.parent.p, T.nch.p, n_group_limit, T.gmark.p); }
+    {
+        const GroupScan gs{T.gmark.p, T.gnode.p, d.i_off.p, T.ng.p, n};
+        if ((r = launch_scan_lb(c, E.lb, gs, gs, n))) return r;
+    }
+    // 4. moments: the leaves in one launch, then the inner nodes level by level
+    // (or all nodes level by level), deepest first
+    const int nlev_all = (int)T.level_start.size() - 1;
     if (g_moments_up) {
-        if ((r = T.arrived.reserve(3 * (size_t)base + 1))) return r;
-        int *flag = T.arrived.p, *lpos = T.arrived.p + base, *list = T.arrived.p + 2 * base, *cnt = list + base;
-        { P3T_COUNT_LAUNCH(); k_leaf_flag<<<nblocks(base), 256, 0, c->stream>>>(base, T.nd.p, flag); }
-        if ((r = E.scan(flag, lpos, base, nullptr))) return r;
-        { P3T_COUNT_LAUNCH(); k_leaf_list<<<nblocks(base), 256, 0, c->stream>>>(base, flag, lpos, list, cnt); }
-        { P3T_COUNT_LAUNCH(); k_moments_leaves<<<nblocks(base, 128), 128, 0, c->stream>>>(list, cnt, T.nd.p, d.spj.p, idx,
-                                                                                      E.S.pos, E.S.mass,
+        { P3T_COUNT_LAUNCH(); k_moments_leaves<<<nblocks(base, 128), 128, 0, c->stream>>>(T.list.p, icnt + MAX_LEVEL + 1, T.nd.p, T.nf.p,
+                                                                                      d.spj.p, idx, E.S.pos, E.S.mass,
                                                                                       E.S.r_search); }
-        for (int L = (int)T.level_start.size() - 2; L >= 0; L--) {
-            const int lo = T.level_start[L], hi = T.level_start[L + 1];
-            { P3T_COUNT_LAUNCH(); k_moments_inner<<<nblocks(hi - lo, 128), 128, 0, c->stream>>>(lo, hi, base, list, lpos, flag,
-                                                                                           T.nd.p, d.spj.p, idx,
-                                                                                           E.S.pos, E.S.mass,
-                                                                                           E.S.r_search); }
+        for (int L = nlev_all - 2; L >= 0;) {  // the deepest level has leaves only
+            int to = L;
+            while (to >= 0 && T.level_start[to + 1] - T.level_start[to] <= TOP_NODES) to--;
+            const int m = T.level_start[L + 1] - T.level_start[L];
+            if (to < L) {  // levels L..to + 1 are small
+                { P3T_COUNT_LAUNCH(); k_moments_run<<<1, TOP_T, 0, c->stream>>>(L, to + 1, T.lstart.p, T.list.p + base, icnt, T.nd.p, T.nf.p,
+                                                                           d.spj.p, idx, E.S.pos, E.S.mass, E.S.r_search); }
+                L = to;
+            } else {
+                { P3T_COUNT_LAUNCH(); k_moments_inner<<<nblocks(m, 128), 128, 0, c->stream>>>(T.list.p + base + T.level_start[L], icnt + L,
+                                                                                         T.nd.p, T.nf.p, d.spj.p, idx,
+                                                                                         E.S.pos, E.S.mass,
+                                                                                         E.S.r_search); }
+                L--;
+            }
         }
     } else {
-        for (int L = (int)T.level_start.size() - 2; L >= 0; L--) {
+        for (int L = nlev_all - 1; L >= 0; L--) {
             const int lo = T.level_start[L], hi = T.level_start[L + 1];
-            { P3T_COUNT_LAUNCH(); k_moments<<<nblocks(hi - lo, 128), 128, 0, c->stream>>>(lo, hi, T.nd.p, d.spj.p, idx, E.S.pos, E.S.mass,
-                                                                    E.S.r_search); }
+            { P3T_COUNT_LAUNCH(); k_moments<<<nblocks(hi - lo, 128), 128, 0, c->stream>>>(lo, hi, T.nd.p, T.nf.p, d.spj.p, idx, E.S.pos,
+                                                                                 E.S.mass, E.S.r_search); }
         }
     }
-    // 4. groups in Morton order
-    cudaMemsetAsync(T.gmark.p, 0, n * sizeof(int), c->stream);
-    { P3T_COUNT_LAUNCH(); k_group_mark<<<nblocks(base), 256, 0, c->stream>>>(base, T.nd.p, T.parent.p, n_group_limit, T.gmark.p); }
-    { P3T_COUNT_LAUNCH(); k_group_flag<<<nblocks(n), 256, 0, c->stream>>>(T.gmark.p, n, T.gflag.p); }
     int ng = 0;
-    if ((r = E.scan(T.gflag.p, T.gpos.p, n, &ng))) return r;
+    if ((r = d2h(c, &ng, T.ng.p, sizeof(int)))) return r;
     T.n_groups = ng;
-    if ((r = T.gnode.reserve(ng + 1)) || (r = d.i_off.reserve(ng + 1)) || (r = d.j_off.reserve(ng + 1)) ||
-        (r = d.s_off.reserve(ng + 1)) || (r = d.i_idx.reserve(n)))
-        return r;
-    { P3T_COUNT_LAUNCH(); k_group_fill<<<nblocks(n), 256, 0, c->stream>>>(T.gmark.p, T.gpos.p, n, ng, T.gnode.p, d.i_off.p); }
-    cudaMemcpyAsync(d.i_idx.p, idx, n * sizeof(int), cudaMemcpyDeviceToDevice, c->stream);
+    if ((r = d.j_off.reserve(ng + 1)) || (r = d.s_off.reserve(ng + 1))) return r;
     // 5. walks: breadth first, one CTA per group; if a frontier outgrows its
     // CTA (or the frontier store), the task walk below
-    if ((r = T.nf.reserve(T.n_nodes))) return r;
-    { P3T_COUNT_LAUNCH(); k_node_f32<<<nblocks(T.n_nodes), 256, 0, c->stream>>>(T.nd.p, T.n_nodes, T.nf.p); }
     bool walked = false;
+    *status = 0;
     if (g_walk_bfs && ng > 0) {
         if ((r = T.bjc.reserve(ng)) || (r = T.bsc.reserve(ng)) || (r = T.blen.reserve(ng)) ||
-            (r = T.boff.reserve(ng)) || (r = T.bover.reserve(1)) || (r = T.bcur.reserve(1)) ||
-            (r = T.bstore.reserve((size_t)T.bstore_cap)))
+            (r = T.boff.reserve(ng)) || (r = T.binfo.reserve(1)) || (r = T.bstore.reserve((size_t)T.bstore_cap)))
             return r;
-        cudaMemsetAsync(T.bover.p, 0, sizeof(int), c->stream);
-        cudaMemsetAsync(T.bcur.p, 0, sizeof(unsigned long long), c->stream);
+        cudaMemsetAsync(T.binfo.p, 0, sizeof(WalkInfo), c->stream);
         { P3T_COUNT_LAUNCH(); k_walk_bfs<<<ng, BFS_T, 0, c->stream>>>(T.nd.p, T.nf.p, T.gnode.p, ng, theta * theta,
                                                                   (float)(theta * theta), T.bjc.p, T.bsc.p, T.blen.p,
-                                                                  T.boff.p, T.bstore.p, T.bcur.p, T.bstore_cap,
-                                                                  T.bover.p, g_walk_cap); }
-        int over = 0;
-        unsigned long long used = 0;
-        int nj = 0, ns = 0;
-        if ((r = E.scan(T.bjc.p, d.j_off.p, ng, &nj)) || (r = E.scan(T.bsc.p, d.s_off.p, ng, &ns)) ||
-            (r = d2h(c, &over, T.bover.p, sizeof(int))) || (r = d2h(c, &used, T.bcur.p, sizeof(used))))
-            return r;
-        if (!over) {
-            if ((r = h2d(c, d.j_off.p + ng, &nj, sizeof(int))) || (r = h2d(c, d.s_off.p + ng, &ns, sizeof(int))) ||
-                (r = d.j_idx.reserve(nj)) || (r = d.s_idx.reserve(ns)))
-                return r;
+                                                                  T.boff.p, T.bstore.p, &T.binfo.p->cursor, T.bstore_cap,
+                                                                  &T.binfo.p->overflow, g_walk_cap); }
+        const WalkScan wsn{T.bjc.p, T.bsc.p, d.j_off.p, d.s_off.p, ng, T.binfo.p, c->status};
+        if ((r = launch_scan_lb(c, E.lb, wsn, wsn, ng, 2))) return r;
+        WalkInfo info;
+        if ((r = d2h(c, &info, T.binfo.p, sizeof info))) return r;
+        *status = info.status;
+        if (!info.overflow) {
+            if ((r = d.j_idx.reserve(info.n[0])) || (r = d.s_idx.reserve(info.n[1]))) return r;
             { P3T_COUNT_LAUNCH(); k_walk_bfs_fill<<<ng, BFS_T, 0, c->stream>>>(T.nf.p, ng, T.blen.p, T.boff.p, T.bstore.p,
                                                                            idx, d.j_off.p, d.s_off.p, d.j_idx.p,
                                                                            d.s_idx.p); }
             walked = true;
-        } else if ((long long)used > T.bstore_cap) {
-            T.bstore_cap = (long long)(used + used / 4);  // room for the next build
+        } else if ((long long)info.cursor > T.bstore_cap) {
+            T.bstore_cap = (long long)(info.cursor + info.cursor / 4);  // room for the next build
         }
     }
     g_walk_last = walked ? 1 : 0;
     // the task walk: the top levels in pre-order (host, from the node table),
     // then (group, top node) pairs: open tests, counts, offsets, entries
     if (!walked) {
+        *status = -1;
         const int nlev = (int)T.level_start.size() - 1;
         const int depth = std::min(g_walk_depth, nlev - 1);
         const int ntop_nodes = T.level_start[depth + 1];
@@ -1099,13 +1280,13 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
         { P3T_COUNT_LAUNCH(); k_walk_class<<<wb, 128, 0, c->stream>>>(T.nd.p, top_d, anc_d, lvl_d, np, ntop, depth, T.ostat.p, idx, 0, jc,
                                                 sc, tflag, nullptr, nullptr, nullptr, nullptr); }
         int ntask = 0;
-        if ((r = E.scan(tflag, tpos, (int)np, &ntask)) || (r = T.tasks.reserve(ntask + 1))) return r;
+        if ((r = g_eng.scan(tflag, tpos, (int)np, &ntask)) || (r = T.tasks.reserve(ntask + 1))) return r;
         { P3T_COUNT_LAUNCH(); k_task_list<<<wb, 128, 0, c->stream>>>(tflag, tpos, np, T.tasks.p); }
         { P3T_COUNT_LAUNCH(); k_walk_tasks<<<nblocks(ntask, 128), 128, 0, c->stream>>>(T.nd.p, T.nf.p, T.gnode.p, top_d, ntop, T.tasks.p,
                                                                  ntask, theta * theta, th2f, idx, 0, jc, sc, nullptr,
                                                                  nullptr, nullptr, nullptr, c->status); }
         int nj = 0, ns = 0;
-        if ((r = E.scan(jc, jo, (int)np, &nj)) || (r = E.scan(sc, so, (int)np, &ns))) return r;
+        if ((r = g_eng.scan(jc, jo, (int)np, &nj)) || (r = g_eng.scan(sc, so, (int)np, &ns))) return r;
         { P3T_COUNT_LAUNCH(); k_walk_group_off<<<nblocks(ng + 1), 256, 0, c->stream>>>(jo, so, ng, ntop, nj, ns, d.j_off.p, d.s_off.p); }
         if ((r = d.j_idx.reserve(nj)) || (r = d.s_idx.reserve(ns))) return r;
         { P3T_COUNT_LAUNCH(); k_walk_class<<<wb, 128, 0, c->stream>>>(T.nd.p, top_d, anc_d, lvl_d, np, ntop, depth, T.ostat.p, idx, 1, jc,
@@ -1114,16 +1295,9 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
                                                                  ntask, theta * theta, th2f, idx, 1, jc, sc, jo, so,
                                                                  d.j_idx.p, d.s_idx.p, c->status); }
     }
-    // 6. the soft kernel's launch order (the bodies' key buffers and the
-    // group-scan scratch are free by now)
+    // 6. the soft kernel's launch order
     if ((r = d.order.reserve(ng))) return r;
-    if (ng > 0) {
-        unsigned long long *k1 = T.key.p, *k2 = T.key2.p;
-        int *i1 = T.gflag.p, *i2 = T.head.p;
-        { P3T_COUNT_LAUNCH(); k_group_weight<<<nblocks(ng), 256, 0, c->stream>>>(ng, d.i_off.p, d.j_off.p, d.s_off.p, k1, i1); }
-        if ((r = radix_sort(c, T, k1, i1, k2, i2, ng, 64))) return r;
-        cudaMemcpyAsync(d.order.p, i1, ng * sizeof(int), cudaMemcpyDeviceToDevice, c->stream);
-    }
+    if (ng > 0) { P3T_COUNT_LAUNCH(); k_group_order<<<1, GO_T, 0, c->stream>>>(ng, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p); }
     d.order_valid = true;
     c->res_groups = ng;
     c->res_spj = base;
@@ -1153,19 +1327,25 @@ int p3t_set_walk_limits(int frontier_cap, long long store_items) {
     return 0;
 }
 
-int p3t_state_tree(double theta, int n_leaf_limit, int n_group_limit) {
+// the lists, with no wait at the end where the build has already read clean
+// status bits (nothing after the breadth-first walk's count pass sets any)
+static int tree_lists(double theta, int n_leaf_limit, int n_group_limit) {
     Context *c = ctx_get(0);
     if (!c || !g_eng.c) return -(int)cudaErrorNoDevice;
-    int r = g_eng.pack_soft();
+    int r = g_eng.pack_soft(), status = -1;
     if (r) return r;
-    if ((r = device_tree(c, theta, n_leaf_limit, n_group_limit))) return r;
-    return read_status(c);
+    if ((r = device_tree(c, theta, n_leaf_limit, n_group_limit, &status))) return r;
+    return status == 0 ? 0 : read_status(c);
+}
+
+int p3t_state_tree(double theta, int n_leaf_limit, int n_group_limit) {
+    const int r = tree_lists(theta, n_leaf_limit, n_group_limit);
+    return r ? r : read_status(g_eng.c);
 }
 
 int p3t_state_tree_soft(double theta, int n_leaf_limit, int n_group_limit) {
-    int r = p3t_state_tree(theta, n_leaf_limit, n_group_limit);
-    if (r) return r;
-    return soft_run_state();
+    const int r = tree_lists(theta, n_leaf_limit, n_group_limit);
+    return r ? r : soft_run_state();
 }
 
 int p3t_tree_lists_counts(long long *counts) {

@@ -33,81 +33,24 @@ __global__ void k_iota(int32_t *p, int n) {
 }
 inline int nb(int n, int t = 256) { return (n + t - 1) / t; }
 
-// Exclusive scan of int32 (block-level Hillis-Steele in shared memory, then
-// block sums scanned recursively).
-__global__ void k_scan_block(const int32_t *in, int32_t *out, int32_t *bsum, int n) {
-    __shared__ int32_t s[1024];
-    const int i = blockIdx.x * 1024 + threadIdx.x;
-    const int32_t v = (i < n) ? in[i] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        int32_t t = (threadIdx.x >= off) ? s[threadIdx.x - off] : 0;
-        __syncthreads();
-        s[threadIdx.x] += t;
-        __syncthreads();
-    }
-    if (i < n) out[i] = s[threadIdx.x] - v;
-    if (threadIdx.x == 1023) bsum[blockIdx.x] = s[1023];
-}
-__global__ void k_scan_add(int32_t *out, const int32_t *bscan, int n) {
-    const int i = blockIdx.x * 1024 + threadIdx.x;
-    if (i < n) out[i] += bscan[blockIdx.x];
-}
-
+// Exclusive scan of int32; total (may be null): its sum, with a host wait.
+struct ScanIn {
+    const int32_t *in;
+    __device__ int operator()(int, int i) const { return in[i]; }
+};
+struct ScanOut {
+    int32_t *out, *sum;
+    __device__ void operator()(int, int i, int prefix, int) const { out[i] = prefix; }
+    __device__ void total(int, int t) const { *sum = t; }
+};
 int Engine::scan(const int32_t *in, int32_t *out, int n, int32_t *total) {
     if (n <= 0) {
         if (total) *total = 0;
         return 0;
     }
-    // levels of block sums live in scan_tmp
-    std::vector<int> sizes;
-    int m = n;
-    size_t need = 0;
-    while (true) {
-        const int blocks = (m + 1023) / 1024;
-        sizes.push_back(m);
-        need += (size_t)blocks * 2;
-        if (blocks <= 1) break;
-        m = blocks;
-    }
-    int r = scan_tmp.reserve(need + 2);
-    if (r) return r;
-    // recursive scan
-    struct Lvl { const int32_t *in; int32_t *out; int32_t *bsum; int n; };
-    std::vector<Lvl> lv;
-    int32_t *tmp = scan_tmp.p;
-    const int32_t *cur_in = in;
-    int32_t *cur_out = out;
-    int cn = n;
-    while (true) {
-        const int blocks = (cn + 1023) / 1024;
-        int32_t *bsum = tmp;
-        int32_t *bscan = tmp + blocks;
-        tmp += 2 * blocks;
-        lv.push_back({cur_in, cur_out, bsum, cn});
-        { P3T_COUNT_LAUNCH(); k_scan_block<<<blocks, 1024, 0, c->stream>>>(cur_in, cur_out, bsum, cn); }
-        if (blocks <= 1) break;
-        cur_in = bsum;
-        cur_out = bscan;
-        cn = blocks;
-    }
-    for (int L = (int)lv.size() - 2; L >= 0; L--) {
-        const int blocks = (lv[L].n + 1023) / 1024;
-        { P3T_COUNT_LAUNCH(); k_scan_add<<<blocks, 1024, 0, c->stream>>>(lv[L].out, lv[L + 1].out, lv[L].n); }
-    }
-    if (total) {
-        // total = out[n-1] + in[n-1]
-        int32_t a = 0, b = 0;
-        if (n > 0) {
-            cudaMemcpyAsync(&a, out + n - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
-            cudaMemcpyAsync(&b, in + n - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
-        }
-        r = cuda_status(cudaStreamSynchronize(c->stream));
-        if (r) return r;
-        *total = a + b;
-    }
-    return cuda_status(cudaGetLastError());
+    int r = scan_tmp.reserve(1);
+    if (r || (r = launch_scan_lb(c, lb, ScanIn{in}, ScanOut{out, scan_tmp.p}, n))) return r;
+    return total ? d2h(c, total, scan_tmp.p, sizeof(int32_t)) : 0;
 }
 
 // ---------------------------------------------------------------------------

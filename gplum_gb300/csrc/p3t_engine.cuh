@@ -2,6 +2,7 @@
 // context and stream).
 #pragma once
 #include "p3t_capi_internal.cuh"
+#include "p3t_lookback.cuh"
 #include "p3t_state.cuh"
 
 namespace p3t {
@@ -14,6 +15,7 @@ struct Engine {
     DevBuf<int32_t> counters, head, flag, cidx, cl_of, cl_cnt, cl_off, cl_fill, members_tmp, members, keep, kpos,
         scan_tmp, tflag, tpos;
     DevBuf<int64_t> cmin;
+    LookBack lb;
     DevBuf<double> epart, et;
     DevBuf<int> icnt;
     // correction pair list: per body its count and first slot; per pair (i, j) and terms
