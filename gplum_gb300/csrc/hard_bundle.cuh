@@ -29,10 +29,12 @@
 //     that cannot rely on the list makes its own).
 // Measured against the form that kept the members in global memory (256 slots,
 // 2 CTAs per SM, the library's roots, a list per pass): a block step of a lone
-// pair 35 -> 15 us, of a 60-body cluster 49 -> 30 us; the hard launch of a tree
-// step 39 -> 26 ms on the 1,048,576-body ring (throughput-bound, 16 M member
-// steps), 19 -> 10 ms at 50,000 bodies and 28 -> 14 ms on the 2 M-body wide
-// disk (both bound by their longest chains).
+// pair 35 -> 13 us, of a 60-body cluster 49 -> 24 us; the hard launch of a tree
+// step 39 -> 24 ms on the 1,048,576-body ring (throughput-bound, 16 M member
+// steps), 19 -> 8.9 ms at 50,000 bodies and 28 -> 12 ms on the 2 M-body wide
+// disk (both bound by their longest chains).  Rare paths are out of line and work
+// loops are not unrolled: what a block step executes has to stay in the
+// instruction cache (inlining them cost 15 % of a lone pair's block step).
 // Why 128 slots: three such CTAs fill an SM's shared memory (74 KB each), and
 // three independent bundles overlap one's waits with the others' FP64 work; a
 // bundle of 256 slots fits once per SM.
@@ -79,7 +81,7 @@ enum : unsigned char { MF_ACT = 1, MF_TGT = 2 };
 // fields of a member slot (three components from each vector's first); F_N*:
 // the running pass's forces of a target, in the order of F_AS..F_JD
 enum : int {
-    F_POS = 0, F_VEL = 3, F_AS = 6, F_JS = 9, F_AD = 12, F_JD = 15, F_MASS = 18, F_ROI, F_TH, F_DT, F_TE, F_ACC0,
+    F_POS = 0, F_VEL = 3, F_AS = 6, F_JS = 9, F_AD = 12, F_JD = 15, F_MASS = 18, F_ROI, F_TH, F_DT, F_TE, F_A02,  // F_TE: th + dt, during a step a target's Dt; F_A02: alpha2 acc0 acc0
     F_KEEP = 24,  // the fields above persist between block steps
     F_XP = 24, F_VP = 27, F_NAS = 30, F_NJS = 33, F_NAD = 36, F_NJD = 39, F_N = 42,
     F_PHS = F_XP, F_PHD = F_XP + 1  // potentials of a full pass (the predicted state is dead then)
@@ -101,6 +103,7 @@ struct BundleSmem {
     // colliding-pair candidates
     double sv_R[BSURV];
     long long sv_p[BSURV];
+    double q_Kc[8], q_D[8];  // a small pass's 1 - K and dK/dt brackets on their way between warps
     unsigned long long live[2];
     float x32[3][S], roi32[S], fr32[S];  // prefilter copies (x32: of the running pass's positions)
     int hmov[S];                         // high word of r_out / 128
@@ -114,7 +117,7 @@ struct BundleSmem {
     int pend_c[BCLAIM], pend_n[BCLAIM];
     int ws[NT / 32];
     int used, ncl, fresh_k, fresh_p, n_sv, n_pend, i_pend, exhausted, any, grew, phase;
-    int ln, moved, any_dead;  // list entries; a corrected position left the list's margin; dead members
+    int ln, nt, moved, any_dead;  // list entries, targets; a corrected position left the list's margin; dead members
     short tgt[S], cl[S], owner[S], eqc[S], twh[S], twn[S], segb[S], sege[S];
     unsigned char dead[S], merged[S], flag[S];
     long long ph_acc[HP_N], ph_t;  // optional per-phase clock counts (thread 0)
@@ -157,6 +160,13 @@ __device__ __forceinline__ double from_zero(double x) { return (dbits(x) << 1) =
 __device__ __forceinline__ bool is_pow2(double x) {
     const unsigned h = (unsigned)dhi(x);
     return __double2loint(x) == 0 && (h & 0x800fffffu) == 0u && h - 0x10000000u < 0x60000000u;
+}
+
+// the minimum over the warp, a word after the other
+__device__ __forceinline__ unsigned long long warp_min64(unsigned long long v) {
+    const unsigned h = __reduce_min_sync(0xffffffffu, (unsigned)(v >> 32));
+    const unsigned l = __reduce_min_sync(0xffffffffu, (unsigned)(v >> 32) == h ? (unsigned)v : ~0u);
+    return ((unsigned long long)h << 32) | l;
 }
 
 template <int BCAP>
@@ -237,6 +247,99 @@ __device__ __forceinline__ int bundle_targets(BundleSmem<BCAP> &B, unsigned char
     return tot & 1023;
 }
 
+// the FP64 test of a pair (rarely run, and kept out of line like the other
+// rare paths: what a block step executes should stay in the instruction cache)
+template <int BCAP>
+__device__ __noinline__ int pair_live_exact(double eps2, int mode, int s, int t) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    const V3 dr = bld(B, mode == 0 ? F_POS : F_XP, t) - bld(B, mode == 1 ? F_XP : F_POS, s);
+    double dr2 = dot(dr, dr);
+    dr2 += eps2;
+    const double r = pmin(B.d[F_ROI][s], B.d[F_ROI][t]);
+    return !(dr2 * r * r > (mode == 1 ? 1.033 : 1.000001));
+}
+// whether target s's pair with t (both of cluster k) is listed
+template <int BCAP>
+__device__ __forceinline__ int pair_live(const HardArgs &A, const BundleSmem<BCAP> &B, int mode, bool exact, int s,
+                                         int t, int k) {
+    if (B.eqc[s] == B.eqc[t]) return 0;
+    if (!exact && !(B.c_flags[k] & CF_EXACT)) {
+        const float rf = fminf(B.roi32[s], B.roi32[t]);
+        // (1 + 1/64)^2 and the product's rounding
+        return bd2_32(B, s, t) * (rf * rf) <= B.c_thrf[k] * (mode == 0 ? 1.f : 1.033f);
+    }
+    return pair_live_exact<BCAP>(A.P.eps2, mode, s, t);
+}
+
+// Targets and pair list of a bundle of at most 32 slots by warp 0, without
+// barriers (seven in the general form; for the chains of clusters that run
+// alone).  More than 128 items: the targets only.
+template <int BCAP>
+__device__ __forceinline__ void bundle_lists_small(const HardArgs &A, BundleSmem<BCAP> &B) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x;
+    auto prefix = [&](int v) {  // inclusive
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(ALL, v, o);
+            if (lane >= o) v += y;
+        }
+        return v;
+    };
+    {
+        const bool tg = lane < B.used && (B.flag[lane] & MF_TGT);
+        const unsigned m = __ballot_sync(ALL, tg);
+        const int cn = tg ? B.c_n[B.cl[lane]] : 0, at = __popc(m & ((1u << lane) - 1u)), nt = __popc(m);
+        const int end = prefix(cn), total = __shfl_sync(ALL, end, 31);
+        if (tg) {
+            B.tgt[at] = (short)lane;
+            B.pfx[at] = end - cn;
+            B.segb[at] = B.sege[at] = 0;
+        }
+        if (lane == 0) B.pfx[nt] = total;
+        __syncwarp();
+        int n = 0;
+        if (total <= 4 * 32) {
+            const int per = total <= 32 ? 1 : 4, f0 = per * lane, f1 = min(f0 + per, total);
+            unsigned lv = 0u;
+            int lo = 0;
+            if (f0 < total) {
+                while (B.pfx[lo + 1] <= f0) lo++;
+                int l = lo;
+#pragma unroll 1
+                for (int f = f0; f < f1; f++) {
+                    while (B.pfx[l + 1] <= f) l++;
+                    const int s = B.tgt[l], k = B.cl[s];
+                    lv |= (unsigned)pair_live(A, B, 1, false, s, B.c_off[k] + (f - B.pfx[l]), k) << (f - f0);
+                }
+            }
+            __syncwarp();
+            const int nl = __popc(lv), stop = prefix(nl);
+            int off = stop - nl;
+            n = __shfl_sync(ALL, stop, 31);
+            for (; lv; lv &= lv - 1u) {
+                const int f = f0 + __ffs((int)lv) - 1;
+                while (B.pfx[lo + 1] <= f) lo++;
+                B.list[off++] = ((unsigned)lo << 16) | (unsigned)(B.c_off[B.cl[B.tgt[lo]]] + (f - B.pfx[lo]));
+            }
+            __syncwarp();
+            for (int q = lane; q < n; q += 32) {
+                const int ti = B.list[q] >> 16;
+                const int tp = q > 0 ? (int)(B.list[q - 1] >> 16) : -1;
+                if (ti != tp) {
+                    B.segb[ti] = (short)q;
+                    if (tp >= 0) B.sege[tp] = (short)q;
+                }
+                if (q == n - 1) B.sege[ti] = (short)n;
+            }
+        }
+        if (lane == 0) {
+            B.ln = n;
+            B.nt = nt;
+        }
+    }
+}
+
 // The live pairs from item `base` of the targets' (target, partner) items on,
 // until the items end or the list is full: B.list[0..B.ln).  Returns the next
 // item.  mode 0: full (pos of both); 1: predicted i and j; 2: corrected i,
@@ -245,58 +348,43 @@ template <int BCAP>
 __device__ __forceinline__ int bundle_build(const HardArgs &A, BundleSmem<BCAP> &B, int mode, int nt, int base, bool exact) {
     constexpr int BT = BundleSmem<BCAP>::NT;
     const int tid = threadIdx.x, total = B.pfx[nt];
-    const float mg = mode == 0 ? 1.f : 1.033f;  // (1 + 1/64)^2 and the product's rounding
+#pragma unroll 1
     for (int i = tid; i < nt; i += BT) B.segb[i] = B.sege[i] = 0;
     int n = 0;
     while (base < total && n + BPT * BT <= BundleSmem<BCAP>::LC) {
         const int per = (total - base <= BT) ? 1 : BPT;  // few items: one a thread
-        const int f0 = base + per * tid;
-        unsigned e[BPT], lv = 0u;
-        int nl = 0;
+        const int f0 = base + per * tid, f1 = min(f0 + per, total);
+        unsigned lv = 0u;
+        int lo = 0;
         if (f0 < total) {
-            int lo = 0, hi = nt - 1;
+            int hi = nt - 1;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
                 if (B.pfx[mid] <= f0) lo = mid;
                 else hi = mid - 1;
             }
-#pragma unroll
-            for (int u = 0; u < BPT; u++) {
-                const int f = f0 + u;
-                e[u] = 0u;
-                if (u >= per || f >= total) continue;
-                while (B.pfx[lo + 1] <= f) lo++;
-                const int s = B.tgt[lo], k = B.cl[s];
-                const int t = B.c_off[k] + (f - B.pfx[lo]);
-                int live = 0;
-                if (B.eqc[s] != B.eqc[t]) {
-                    if (!exact && !(B.c_flags[k] & CF_EXACT)) {
-                        const float rf = fminf(B.roi32[s], B.roi32[t]);
-                        live = bd2_32(B, s, t) * (rf * rf) <= B.c_thrf[k] * mg;
-                    } else {
-                        const V3 dr = bld(B, mode == 0 ? F_POS : F_XP, t) - bld(B, mode == 1 ? F_XP : F_POS, s);
-                        double dr2 = dot(dr, dr);
-                        dr2 += A.P.eps2;
-                        const double r = pmin(B.d[F_ROI][s], B.d[F_ROI][t]);
-                        live = !(dr2 * r * r > (mode == 1 ? 1.033 : 1.000001));
-                    }
-                }
-                e[u] = ((unsigned)lo << 16) | (unsigned)t;
-                lv |= (unsigned)live << u;
-                nl += live;
+            int l = lo;
+#pragma unroll 1
+            for (int f = f0; f < f1; f++) {
+                while (B.pfx[l + 1] <= f) l++;
+                const int s = B.tgt[l], k = B.cl[s];
+                lv |= (unsigned)pair_live(A, B, mode, exact, s, B.c_off[k] + (f - B.pfx[l]), k) << (f - f0);
             }
         }
         int cnt;
-        int off = n + bscan<BT>(nl, B.ws, cnt);
-#pragma unroll
-        for (int u = 0; u < BPT; u++)
-            if ((lv >> u) & 1u) B.list[off++] = e[u];
+        int off = n + bscan<BT>(__popc(lv), B.ws, cnt);
+        for (; lv; lv &= lv - 1u) {  // the live ones, in order
+            const int f = f0 + __ffs((int)lv) - 1;
+            while (B.pfx[lo + 1] <= f) lo++;
+            B.list[off++] = ((unsigned)lo << 16) | (unsigned)(B.c_off[B.cl[B.tgt[lo]]] + (f - B.pfx[lo]));
+        }
         n += cnt;
         base += per * BT;
     }
     if (tid == 0) B.ln = n;
     __syncthreads();
     // each target's run of the list
+#pragma unroll 1
     for (int q = tid; q < n; q += BT) {
         const int ti = B.list[q] >> 16;
         const int tp = q > 0 ? (int)(B.list[q - 1] >> 16) : -1;
@@ -390,6 +478,7 @@ __device__ __forceinline__ void bundle_terms(const HardArgs &A, BundleSmem<BCAP>
     constexpr int BT = BundleSmem<BCAP>::NT;
     const int np32 = (np + 31) & ~31;  // pairs and sun forces in different warps
     const int lane = threadIdx.x & 31;
+#pragma unroll 1
     for (int w0 = threadIdx.x - lane; w0 < np32 + ns; w0 += BT) {  // whole warps
         const int it = w0 + lane;
         if (w0 < np32) {
@@ -466,7 +555,97 @@ __device__ __forceinline__ void bundle_terms_split(const HardArgs &A, BundleSmem
     }
 }
 
+// A pass of at most 8 pairs and 8 targets, the longest chains' block steps: its
+// time is the dependent FP64 operations of one pair, so the independent parts
+// of a pair go to different warps -- 1 - K to warp 0, the bracket of dK/dt to
+// warp 1, dv, the powers of 1/r and the result to warp 2, the sun force to
+// warp 3 -- each with a component per lane (four lanes a pair); the fourth lane
+// takes the scalars of the last products.  26 instead of 46 dependent FP64
+// instructions.  Contains a barrier: every thread of the CTA calls it.
+template <int BCAP>
+__device__ __forceinline__ void bundle_terms_small(const HardArgs &A, BundleSmem<BCAP> &B, int fi, int fj, int q0,
+                                                   int np, int ns, int st) {
+    const Params &P = A.P;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int w = threadIdx.x >> 5, it = (threadIdx.x & 31) >> 2, c4 = threadIdx.x & 3, c = min(c4, 2);
+    auto dot3 = [&](double p) {
+        const double a = __shfl_sync(ALL, p, 0, 4), b = __shfl_sync(ALL, p, 1, 4), d = __shfl_sync(ALL, p, 2, 4);
+        return a + b + d;
+    };
+    double dr = 0., dv = 0., mr3 = 0., alpha = 0., t1 = 0.;
+    if (w < 3 && np > 0) {
+        const unsigned e = B.list[q0 + min(it, np - 1)];
+        const int s = B.tgt[e >> 16], t = e & 0xffffu;
+        dr = B.d[fj + c][t] - B.d[fi + c][s];
+        double dr2 = dot3(dr * dr);
+        if (!(A.plain & PL_EPS2)) dr2 += P.eps2;
+        const double rij = sqrt_rn(dr2);
+        if (w < 2) {
+            const double r_out_inv = pmin(B.d[F_ROI][s], B.d[F_ROI][t]);
+            const double x = (P.gamma - rij * r_out_inv) * P.g_1_inv;
+            const bool near = kx_near(x), far = kx_far(x);
+            double v = w == 0 ? 1. : 0.;  // near: 1 - K = 1, dK/dr = 0
+            if (!__all_sync(ALL, near)) {
+                if (w == 0) {
+                    const double x2 = x * x;
+                    const double K = (((-20. * x + 70.) * x - 84.) * x + 35.) * x2 * x2;
+                    v = near ? 1. : (far ? 0. : 1. - K);
+                } else {
+                    const double x_1 = x - 1.;
+                    const double D = 140. * x * x * x * x_1 * x_1 * x_1 * r_out_inv * P.g_1_inv;
+                    v = (near || far) ? 0. : D;
+                }
+            }
+            if (c4 == 0) (w == 0 ? B.q_Kc : B.q_D)[it] = v;
+        } else {
+            dv = B.d[fj + 3 + c][t] - B.d[fi + 3 + c][s];
+            const double rv = dot3(dr * dv);
+            const double rinv = rcp_rn(rij);
+            const double r2inv = rinv * rinv;
+            mr3 = B.d[F_MASS][t] * (r2inv * rinv);
+            alpha = rv * r2inv;
+            t1 = alpha * rij;
+        }
+    } else if (w == 3 && ns > 0) {
+        const int s = B.tgt[min(it, ns - 1)];
+        const double x = B.d[fi + c][s], v = B.d[fi + 3 + c][s];
+        double r2 = dot3(x * x);
+        const double xv = dot3(x * v);
+        if (!(A.plain & PL_EPS2_SUN)) r2 += P.eps2_sun;
+        const double r2inv = rcp_rn(r2);
+        const double rinv = sqrt_rn(r2inv);
+        double m3 = rinv * r2inv;
+        if (!(A.plain & PL_M_SUN)) m3 = P.m_sun * m3;
+        const double al = xv * r2inv;
+        const double a = m3 * -x, j = m3 * (-v - 3. * al * -x);
+        if (it < ns && c4 < 3) {
+            B.d[F_NAS + c][s] = a;
+            B.d[F_NJS + c][s] = j;
+        }
+    }
+    __syncthreads();
+    if (w == 2 && np > 0) {
+        const double Kc = B.q_Kc[it], D = B.q_D[it];
+        const bool sc = c4 == 3;  // the lane of the scalars
+        // lanes 0-2: 1 - K times dv, times m/r^3, times dr; lane 3: dK/dt, 1 - K times alpha, times 3
+        const double p1 = (sc ? t1 : Kc) * (sc ? D : dv);
+        const double p2 = (sc ? alpha : mr3) * Kc;
+        const double p3 = p2 * (sc ? 3. : dr);
+        const double b = __shfl_sync(ALL, p3 + p1, 3, 4);
+        const double j = mr3 * (p1 - b * dr);
+        if (it < np && !sc) {
+            B.term[c * st + it] = p3;
+            B.term[(3 + c) * st + it] = j;
+        }
+    }
+}
+
 // ---- sums and corrector ---------------------------------------------------------
+// 1 / Dt: recip_pow2_or_div (p3t_phys.cuh) with the division out of line
+__device__ __forceinline__ double recip_dt(double x) {
+    return is_pow2(x) ? bitsd(0x7FE0000000000000ULL - dbits(x)) : ex_outside(1., x, 1);
+}
+
 // component c of FPHard::correct (src/particle.h:1208-1274) for target slot s:
 // correct()'s roundings with 2 J0, -2 Am and, for a power-of-two Dt, the
 // products by Dt fused where they are exact.  last: also a2 and a3, over the
@@ -474,8 +653,7 @@ __device__ __forceinline__ void bundle_terms_split(const HardArgs &A, BundleSmem
 template <int BCAP>
 __device__ __forceinline__ void correct_comp(BundleSmem<BCAP> &B, int s, int c, double as, double js, double ad,
                                              double jd, bool last) {
-    const int k = B.cl[s];
-    const double Dt = B.c_ts[k] - B.d[F_TH][s];
+    const double Dt = B.d[F_TE][s];
     const double J0_s = Dt * B.d[F_JS + c][s], J1_s = Dt * js, Am_s = as - B.d[F_AS + c][s];
     const double A2_s = 3. * Am_s - fma(2., J0_s, J1_s);
     const double A3_s = fma(-2., Am_s, J1_s + J0_s);
@@ -489,12 +667,99 @@ __device__ __forceinline__ void correct_comp(BundleSmem<BCAP> &B, int s, int c, 
     B.d[F_VEL + c][s] = B.d[F_VP + c][s] + dv;
     if ((dhi(dx) & 0x7fffffff) >= B.hmov[s]) B.moved = 1;
     if (last) {
-        const double Di = recip_pow2_or_div(Dt), Di2 = Di * Di, Di3 = Di2 * Di;
+        const double Di = recip_dt(Dt), Di2 = Di * Di, Di3 = Di2 * Di;
         const double t2 = 2. * Di2, t3 = 6. * Di3;
         B.d[F_AS + c][s] = t2 * (A2_s + 3. * A3_s);
         B.d[F_JS + c][s] = t3 * A3_s;
         B.d[F_AD + c][s] = (2. * (A2_d + 3. * A3_d)) * Di2;
         B.d[F_JD + c][s] = (6. * A3_d) * Di3;
+    }
+}
+
+// a power of two to the n-th, and c times 2^e, by the exponent (no range checks)
+__device__ __forceinline__ int pow2_exp(double x) { return ((dhi(x) >> 20) & 0x7ff) - 1023; }
+__device__ __forceinline__ double scale2(double c, int e) {
+    return __hiloint2double(dhi(c) + (e << 20), __double2loint(c));
+}
+
+// 2 x, by the exponent where x is normal and stays so
+__device__ __forceinline__ double twice(double x) {
+    const unsigned e = ((unsigned)dhi(x) >> 20) & 0x7ffu;
+    return e - 1u < 2045u ? __hiloint2double(dhi(x) + (1 << 20), __double2loint(x)) : x + x;
+}
+
+// The sums and the correction of at most NT / 6 targets with the sun's and the
+// planets' halves of a component in a pair of lanes (their operations are the
+// same up to the operands), then position and velocity: 13 and 17 dependent
+// FP64 instructions where one lane a component takes 30 and 42.  The roundings
+// are correct_comp's.
+template <int BCAP>
+__device__ __forceinline__ void sum_correct_split(BundleSmem<BCAP> &B, int nt, int q0, int np, int st, bool last) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int it = min((int)threadIdx.x, 6 * nt - 1);
+    if ((int)(threadIdx.x & ~31u) >= 6 * nt) return;  // no target in this warp
+    const bool mine = threadIdx.x < 6 * nt;
+    const int h = it & 1, t = (it >> 1) / 3, c = (it >> 1) - 3 * t, s = B.tgt[t];
+    double acc, jerk;
+    if (h == 0) {
+        acc = B.d[F_NAS + c][s];
+        jerk = B.d[F_NJS + c][s];
+    } else {
+        acc = jerk = 0.;
+        int q = B.segb[t] - q0;
+        const int qe = B.sege[t] - q0;
+        if (q < qe) {
+            acc = from_zero(B.term[c * st + q]);
+            jerk = from_zero(B.term[(3 + c) * st + q]);
+#pragma unroll 1
+            for (q++; q < qe; q++) {
+                acc += B.term[c * st + q];
+                jerk += B.term[(3 + c) * st + q];
+            }
+        }
+        if (mine) {
+            B.d[F_NAD + c][s] = acc;
+            B.d[F_NJD + c][s] = jerk;
+        }
+    }
+    const int f0 = (h ? F_AD : F_AS) + c, f1 = (h ? F_JD : F_JS) + c;
+    const double Dt = B.d[F_TE][s], j0 = B.d[f1][s], Am = acc - B.d[f0][s];
+    const int ex = pow2_exp(Dt);
+    const bool p2 = is_pow2(Dt) && ex > -256 && ex < 256;  // (the scaled factors stay normal)
+    double A2, A3;
+    if (__all_sync(ALL, p2)) {
+        // products by Dt are exact and commute with the rounding of a sum
+        A2 = fma(-Dt, fma(2., j0, jerk), 3. * Am);
+        A3 = fma(Dt, jerk + j0, -twice(Am));
+    } else {
+        const double J0 = Dt * j0, J1 = Dt * jerk;
+        A2 = 3. * Am - fma(2., J0, J1);
+        A3 = fma(-2., Am, J1 + J0);
+    }
+    const double A2t = A2 + __shfl_xor_sync(ALL, A2, 1), A3t = A3 + __shfl_xor_sync(ALL, A3, 1);
+    // even lane: the position, odd lane: the velocity
+    const double sum = (h ? 4. : 5.) * A2t + (h ? 3. : 3. * 1.1666666666666667e-3) * A3t;
+    double cf;
+    if (p2) cf = scale2(h ? 8.3333333333333333e-2 : 1.6666666666666667e-2, h ? ex : 2 * ex);
+    else cf = h ? 8.3333333333333333e-2 * Dt : 1.6666666666666667e-2 * (Dt * Dt);
+    const double d = cf * sum;
+    const double r = B.d[(h ? F_VP : F_XP) + c][s] + d;
+    if (!mine) return;
+    B.d[(h ? F_VEL : F_POS) + c][s] = r;
+    if (!h && (dhi(d) & 0x7fffffff) >= B.hmov[s]) B.moved = 1;
+    if (last) {
+        const double S = A2 + 3. * A3;
+        double a2, a3;
+        if (p2) {
+            a2 = scale2(2., -2 * ex) * S;
+            a3 = scale2(6., -3 * ex) * A3;
+        } else {
+            const double Di = recip_dt(Dt), Di2 = Di * Di, Di3 = Di2 * Di;
+            a2 = h ? (2. * S) * Di2 : (2. * Di2) * S;
+            a3 = h ? (6. * A3) * Di3 : (6. * Di3) * A3;
+        }
+        B.d[f0][s] = a2;
+        B.d[f1][s] = a3;
     }
 }
 
@@ -550,13 +815,17 @@ __device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> 
         int q0 = 0;
         do {
             const int np = min(n - q0, st), ns = first ? nt : 0;
-            if (!phi && ((np + 7) & ~7) + ns <= BT / 4) bundle_terms_split(A, B, fi, fj, q0, np, ns, st);
+            if (!FULL && np <= 8 && ns <= 8) bundle_terms_small(A, B, fi, fj, q0, np, ns, st);
+            else if (!phi && ((np + 7) & ~7) + ns <= BT / 4) bundle_terms_split(A, B, fi, fj, q0, np, ns, st);
             else bundle_terms(A, B, fi, fj, phi, q0, np, ns, st);
             __syncthreads();
             HP_MARK(HP_PAIRS);
             const bool end = q0 + np >= n && !more;
             const bool fuse = corr && end && !merge;
-            for (int it = tid; it < 3 * nt; it += BT) {
+            if (!FULL && fuse && first && 6 * nt <= BT) sum_correct_split(B, nt, q0, np, st, corr == 2);
+            else
+#pragma unroll 1
+                for (int it = tid; it < 3 * nt; it += BT) {
                 const int t = it / 3, c = it - 3 * t, s = B.tgt[t];
                 double ad = first ? 0. : B.d[F_NAD + c][s], jd = first ? 0. : B.d[F_NJD + c][s];
                 int k = max((int)B.segb[t], q0) - q0;
@@ -566,6 +835,7 @@ __device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> 
                     jd = from_zero(B.term[(3 + c) * st + k]);
                     k++;
                 }
+#pragma unroll 1
                 for (; k < ke; k++) {
                     ad += B.term[c * st + k];
                     jd += B.term[(3 + c) * st + k];
@@ -575,6 +845,7 @@ __device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> 
                 if (fuse) correct_comp(B, s, c, B.d[F_NAS + c][s], B.d[F_NJS + c][s], ad, jd, corr == 2);
             }
             if (phi)
+#pragma unroll 1
                 for (int t = tid; t < nt; t += BT) {
                     const int s = B.tgt[t];
                     double ph = first ? 0. : B.d[F_PHD][s];
@@ -588,12 +859,14 @@ __device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> 
         } while (q0 < n);
     }
     if (merge) {
+#pragma unroll 1
         for (int t = tid; t < nt; t += BT) {
             const int s = B.tgt[t];
             if (mode == 0 ? (B.merged[s] && B.twh[s] >= 0) : (!B.dead[s] && B.merged[s])) bundle_merge<BCAP>(s);
         }
         __syncthreads();
         if (corr) {
+#pragma unroll 1
             for (int it = tid; it < 3 * nt; it += BT) {
                 const int t = it / 3, c = it - 3 * t, s = B.tgt[t];
                 correct_comp(B, s, c, B.d[F_NAS + c][s], B.d[F_NJS + c][s], B.d[F_NAD + c][s], B.d[F_NJD + c][s],
@@ -611,6 +884,7 @@ template <int BCAP>
 __device__ __noinline__ int bundle_full(const HardArgs &A, bool phi) {
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     constexpr int BT = BundleSmem<BCAP>::NT;
+#pragma unroll 1
     FOR_SLOTS(p) {
         if (!(B.flag[p] & MF_TGT)) continue;
         const int k = B.cl[p];
@@ -627,6 +901,7 @@ __device__ __noinline__ int bundle_full(const HardArgs &A, bool phi) {
 template <int BCAP>
 __device__ __forceinline__ void bundle_take(BundleSmem<BCAP> &B, int nt) {
     constexpr int BT = BundleSmem<BCAP>::NT;
+#pragma unroll 1
     for (int it = threadIdx.x; it < 12 * nt; it += BT) {
         const int t = it / 12, f = it - 12 * t, s = B.tgt[t];
         B.d[F_AS + f][s] = B.d[F_NAS + f][s];
@@ -638,14 +913,16 @@ __device__ __forceinline__ void bundle_take(BundleSmem<BCAP> &B, int nt) {
 // unordered pairs {a, b} of each cluster, balanced over members: member a
 // takes b = a + d (mod n) for d = 1..n/2 (the pair at distance n/2 once)
 template <int BCAP>
-__device__ __forceinline__ void bundle_detect(const HardArgs &A, BundleSmem<BCAP> &B, bool second) {
+__device__ __forceinline__ void bundle_detect(const HardArgs &A, BundleSmem<BCAP> &B, bool second, int p0) {
     constexpr int BT = BundleSmem<BCAP>::NT;
-    FOR_SLOTS(p) {
+#pragma unroll 1
+    for (int p = p0; p < B.used; p += BT) {
         if (B.dead[p]) continue;
         const int k = B.cl[p];
         const int o = B.c_off[k], n = B.c_n[k], a = p - o;
         const bool exact = (B.c_flags[k] & CF_EXACT) != 0;
         const float thr = B.c_thrc[k], fr = B.fr32[p];
+#pragma unroll 1
         for (int d = 1; 2 * d <= n; d++) {
             if (2 * d == n && a >= d) break;
             int b = a + d;
@@ -687,13 +964,15 @@ __device__ __noinline__ void bundle_collisions_found(const HardArgs &A) {
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     constexpr int BT = BundleSmem<BCAP>::NT;
     if (B.n_sv <= BSURV) {
+#pragma unroll 1
         for (int i = threadIdx.x; i < B.n_sv; i += BT)
             if (dbits(B.sv_R[i]) == B.c_R[B.sv_k[i]])
                 atomicMin((unsigned long long *)&B.c_pb[B.sv_k[i]], (unsigned long long)B.sv_p[i]);
     } else {
-        bundle_detect(A, B, true);
+        bundle_detect(A, B, true, threadIdx.x);
     }
     __syncthreads();
+#pragma unroll 1
     FOR_CLUSTERS(k) {
         if (B.c_R[k] < dbits(1.)) {
             B.c_flags[k] |= CF_COL;
@@ -705,10 +984,11 @@ __device__ __noinline__ void bundle_collisions_found(const HardArgs &A) {
         }
     }
     __syncthreads();
+#pragma unroll 1
     FOR_SLOTS(p) {
         const int k = B.cl[p];
         if (!(B.c_flags[k] & CF_COL)) continue;
-        B.d[F_DT][p] = B.c_ts[k] - B.d[F_TH][p];
+        B.d[F_DT][p] = B.d[F_TE][p] = B.c_ts[k] - B.d[F_TH][p];
         B.flag[p] = B.dead[p] ? 0 : (MF_ACT | MF_TGT);
         if (!B.dead[p]) atomicAdd(&B.c_act[k], 1);
     }
@@ -826,6 +1106,7 @@ __device__ __noinline__ void bundle_load(const HardArgs &A) {
     const Hard &H = A.H;
     const int tid = threadIdx.x;
     const int k0 = B.fresh_k, k1 = B.ncl, p0 = B.fresh_p, p1 = B.used;
+#pragma unroll 1
     for (int k = k0 + tid; k < k1; k += BT) {
         const int c = B.c_idx[k];
         const int goff = A.off[c];
@@ -847,6 +1128,7 @@ __device__ __noinline__ void bundle_load(const HardArgs &A) {
         B.c_pb[k] = (long long)dbits(1.e300);
     }
     __syncthreads();
+#pragma unroll 1
     for (int p = p0 + tid; p < p1; p += BT) {
         int lo = k0, hi = k1 - 1;
         while (lo < hi) {
@@ -868,7 +1150,7 @@ __device__ __noinline__ void bundle_load(const HardArgs &A) {
         B.d[F_TH][p] = 0.;
         B.d[F_DT][p] = dt;
         B.d[F_TE][p] = 0. + dt;
-        B.d[F_ACC0][p] = acc0;
+        B.d[F_A02][p] = A.P.alpha2 * acc0 * acc0;
         H.mass[g] = mass; H.r_planet[g] = rp; H.f[g] = f; H.r_out_inv[g] = roi;
         H.time_c[g] = tc; H.acc0[g] = acc0; H.id[g] = id;
         H.dead[g] = 0; H.merged[g] = 0;
@@ -891,6 +1173,7 @@ __device__ __noinline__ void bundle_load(const HardArgs &A) {
         atomicMin((unsigned long long *)&B.c_pb[k], dbits(fr));
     }
     __syncthreads();
+#pragma unroll 1
     for (int k = k0 + tid; k < k1; k += BT) {
         // coordinate bound, then the prefilter thresholds (see the header)
         const double E = (bitsd(B.c_key[k]) + 2. * bitsd(B.c_tm[k]) * A.t_end) * 1.0001 + 1.e-30;
@@ -903,11 +1186,14 @@ __device__ __noinline__ void bundle_load(const HardArgs &A) {
         B.c_E32[k] = __double2float_rd(E);
         B.c_key[k] = dbits(1.e10);
     }
+#pragma unroll 1
     for (int p = tid; p < p1; p += BT) B.flag[p] = p < p0 ? 0 : MF_TGT;
     __syncthreads();
+#pragma unroll 1
     for (int p = p0 + tid; p < p1; p += BT) atomicMin(&B.c_key[B.cl[p]], dbits(B.d[F_TE][p]));
     const int nt = bundle_full<BCAP>(A, false);
     bundle_take(B, nt);
+#pragma unroll 1
     for (int k = k0 + tid; k < k1; k += BT) bundle_open(B, k);
     if (tid == 0) B.n_sv = B.moved = 0;
     __syncthreads();
@@ -915,7 +1201,8 @@ __device__ __noinline__ void bundle_load(const HardArgs &A) {
 
 // every field of slot p from the state of record (global slot g), after a collision
 template <int BCAP>
-__device__ __forceinline__ void bundle_reload(BundleSmem<BCAP> &B, const Hard &H, int p, int g, int k) {
+__device__ __forceinline__ void bundle_reload(const HardArgs &A, BundleSmem<BCAP> &B, int p, int g, int k) {
+    const Hard &H = A.H;
     bst(B, F_POS, p, ld3(H.pos, g));
     bst(B, F_VEL, p, ld3(H.vel, g));
     B.d[F_MASS][p] = H.mass[g];
@@ -923,7 +1210,7 @@ __device__ __forceinline__ void bundle_reload(BundleSmem<BCAP> &B, const Hard &H
     B.d[F_TH][p] = H.th[g];
     B.d[F_DT][p] = H.dt[g];
     B.d[F_TE][p] = 0.;
-    B.d[F_ACC0][p] = H.acc0[g];
+    B.d[F_A02][p] = A.P.alpha2 * H.acc0[g] * H.acc0[g];
     B.fr32[p] = (float)(H.f[g] * H.r_planet[g]);
     B.roi32[p] = (float)H.r_out_inv[g];
     B.hmov[p] = (int)(__float_as_uint(0.0078f / B.roi32[p]) >> 3) + (896 << 20);
@@ -1023,7 +1310,7 @@ __device__ __noinline__ void bundle_grow(const HardArgs &A) {
         if (add > 0) B.c_flags[tid] |= CF_EXACT;
         for (int i = 0; i < add; i++) {
             const int q = noff + my_n + i;
-            bundle_reload(B, A.H, q, B.c_addg[tid] + i, tid);
+            bundle_reload(A, B, q, B.c_addg[tid] + i, tid);
             B.eqc[q] = (short)q;
             B.owner[q] = B.twh[q] = B.twn[q] = -1;
         }
@@ -1041,6 +1328,7 @@ __device__ __noinline__ void bundle_collide(const HardArgs &A) {
     constexpr int BT = BundleSmem<BCAP>::NT;
     const Params &P = A.P;
     const Hard &H = A.H;
+#pragma unroll 1
     FOR_SLOTS(p) {
         if (!(B.c_flags[B.cl[p]] & CF_COL)) continue;
         const int g = B.gslot[p];
@@ -1053,6 +1341,7 @@ __device__ __noinline__ void bundle_collide(const HardArgs &A) {
     }
     if (threadIdx.x == 0) B.grew = 0;
     __syncthreads();
+#pragma unroll 1
     FOR_CLUSTERS(k) {
         B.c_addn[k] = 0;
         if (!(B.c_flags[k] & CF_COL)) continue;
@@ -1080,12 +1369,13 @@ __device__ __noinline__ void bundle_collide(const HardArgs &A) {
     }
     __threadfence_block();
     __syncthreads();
+#pragma unroll 1
     FOR_SLOTS(p) {
         const int k = B.cl[p];
         B.flag[p] = 0;
         if (!(B.c_flags[k] & CF_COL)) continue;
         const int g = B.gslot[p], o = B.c_off[k], n = B.c_n[k];
-        bundle_reload(B, H, p, g, k);
+        bundle_reload(A, B, p, g, k);
         // the merge lists as slots: twins, their owner, equal ids
         auto slot_of = [&](int t) {
             if (t >= 0)
@@ -1110,23 +1400,27 @@ __device__ __noinline__ void bundle_collide(const HardArgs &A) {
     }
     __syncthreads();
     if (B.grew) bundle_grow<BCAP>(A);
+#pragma unroll 1
     FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_COL) ? MF_TGT : 0;
     __syncthreads();
     const int nc = bundle_full<BCAP>(A, false);
     bundle_take(B, nc);
+#pragma unroll 1
     for (int i = threadIdx.x; i < nc; i += BT) {
         const int s = B.tgt[i];
         if (B.dead[s]) continue;
-        B.d[F_DT][s] = dt_initial(P, B.d[F_TH][s], B.d[F_DT][s], B.d[F_ACC0][s], bld(B, F_AD, s), bld(B, F_JD, s),
+        B.d[F_DT][s] = dt_initial(P, B.d[F_TH][s], B.d[F_DT][s], H.acc0[B.gslot[s]], bld(B, F_AD, s), bld(B, F_JD, s),
                                   bld(B, F_AS, s), bld(B, F_JS, s));
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = threadIdx.x; i < nc; i += BT) {
         const int s = B.tgt[i];
         if (B.merged[s])
             for (int t = B.twh[s], gg = 0; t >= 0 && gg < BCAP; t = B.twn[t], gg++) B.d[F_DT][t] = B.d[F_DT][s];
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = threadIdx.x; i < nc; i += BT) {
         const int s = B.tgt[i];
         B.d[F_TE][s] = B.d[F_TH][s] + B.d[F_DT][s];
@@ -1134,32 +1428,35 @@ __device__ __noinline__ void bundle_collide(const HardArgs &A) {
     __syncthreads();
 }
 
+__device__ __noinline__ double dt_next_general(const HardArgs &A, double time, double dt, double dt_1) {
+    return dt_next_hermite(A.P, time, dt, dt_1);
+}
 // dt_next_hermite by the exponents: its halvings of a power of two against
 // the time's lowest set bit and the criterion's exponent
-__device__ __forceinline__ double dt_next_bits(const Params &P, double time, double dt, double dt_1) {
+__device__ __forceinline__ double dt_next_bits(const HardArgs &A, double time, double dt, double dt_1) {
+    const Params &P = A.P;
     const double dmax_ = 0.5 * P.dt_tree;
     if (!is_pow2(dt) || !is_pow2(dmax_) || !(dhi(time) >= 0 && dhi(time) < 0x7fe00000) || dhi(dt_1) < 0)
-        return dt_next_hermite(P, time, dt, dt_1);
+        return dt_next_general(A, time, dt, dt_1);
     const int ed = dhi(dt) >> 20;
     int e = min(ed + 1, dhi(dmax_) >> 20);
     const unsigned long long b = dbits(time), m = (b & ((1ULL << 52) - 1)) | (1ULL << 52);
     if (b != 0ULL) {  // time a multiple of 2^e: e at most its lowest set bit's exponent
         const int et = (int)(b >> 52);
-        if (et == 0) return dt_next_hermite(P, time, dt, dt_1);
+        if (et == 0) return dt_next_general(A, time, dt, dt_1);
         e = min(e, et - 52 + (__ffsll((long long)m) - 1));
     }
-    if (e < 64) return dt_next_hermite(P, time, dt, dt_1);
+    if (e < 64) return dt_next_general(A, time, dt, dt_1);
     const int e1 = dhi(dt_1) >> 20;
     while (e1 < e && ed - 1 < e) e--;  // dt_1 < 2^e: its exponent is smaller
     const double next = __hiloint2double(e << 20, 0);
     return plt(next, 2. * P.dt_min) ? P.dt_min : next;
 }
 
-// dt4th's last expression (p3t_phys.cuh), from the norms and squares
-__device__ __forceinline__ double dt4th_of(double eta, double Acc, double Jerk, double Snap, double Crac, double Jerk2,
-                                           double Snap2) {
-    return (dbits(Jerk) << 1) != 0ULL ? eta * sqrt_rn(div_rn(Acc * Snap + Jerk2, Jerk * Crac + Snap2))
-                                      : 1.7976931348623157e308;
+// dmin of two criteria: by their bits unless one is NaN or negative
+__device__ __forceinline__ double dmin_crit(double a, double b) {
+    const unsigned long long inf = 0x7ff0000000000000ULL;
+    return dbits(a) <= inf && dbits(b) <= inf ? pmin(a, b) : dmin(a, b);
 }
 
 // time and calcDeltat (src/particle.h:1276-1314) of the targets, and their
@@ -1173,53 +1470,56 @@ __device__ __forceinline__ void bundle_dt(const HardArgs &A, BundleSmem<BCAP> &B
     const Params &P = A.P;
     const bool wide = 8 * nt <= BT;
     const int sh = wide ? 3 : 1, L = 1 << sh;  // lanes a target
+#pragma unroll 1
     for (int base = 0; base < L * nt; base += BT) {
         const int i = base + threadIdx.x;
         if (i - (i & 31) >= L * nt) break;  // no target in this warp
         const int t = min(i >> sh, nt - 1), r = i & (L - 1);
         const bool act = i < L * nt;
         const int s = B.tgt[t], k = B.cl[s];
-        double crit;
+        double num, den, Jerk;  // dt4th (p3t_phys.cuh): eta sqrt((Acc Snap + Jerk^2) / (Jerk Crac + Snap^2))
+        const int sun = wide ? r >> 2 : r;
         if (wide) {
-            const int sun = r >> 2, w = r & 3;
+            const int w = r & 3;
             // acc and jerk as the last pass left them, snap and crackle as the corrector did
             const int f = (w < 2) ? (sun ? F_NAS : F_NAD) + 3 * w : (sun ? F_AS : F_AD) + 3 * (w - 2);
             const V3 v = bld(B, f, s);
-            double n2 = dot(v, v);
-            if (w == 0 && !sun) {
-                const double a0 = B.d[F_ACC0][s];
-                n2 = n2 + P.alpha2 * a0 * a0;
-            }
+            const double n2 = dot(v, v) + (w == 0 && !sun ? B.d[F_A02][s] : 0.);
             const double nn = sqrt_rn(n2);
-            const double Acc = __shfl_sync(ALL, nn, 0, 4), Jerk = __shfl_sync(ALL, nn, 1, 4),
-                         Snap = __shfl_sync(ALL, nn, 2, 4), Crac = __shfl_sync(ALL, nn, 3, 4);
-            const double Jerk2 = __shfl_sync(ALL, n2, 1, 4), Snap2 = __shfl_sync(ALL, n2, 2, 4);
-            crit = dt4th_of(sun ? P.eta_sun : P.eta, Acc, Jerk, Snap, Crac, Jerk2, Snap2);
+            // even lanes: Acc Snap + Jerk^2, odd lanes: Jerk Crac + Snap^2
+            const double m1 = __shfl_sync(ALL, nn, w & 1, 4), m2 = __shfl_sync(ALL, nn, 2 + (w & 1), 4);
+            const double q2 = __shfl_sync(ALL, n2, 1 + (w & 1), 4);
+            Jerk = __shfl_sync(ALL, nn, 1, 4);
+            const double nd = m1 * m2 + q2;
+            num = __shfl_sync(ALL, nd, 0, 4);
+            den = __shfl_sync(ALL, nd, 1, 4);
         } else {
-            // dt4th (p3t_phys.cuh), a norm after the other
-            const int sun = r;
+            // a norm after the other
             double n2[4];
 #pragma unroll
             for (int w = 0; w < 4; w++) {
                 const V3 v = bld(B, (w < 2) ? (sun ? F_NAS : F_NAD) + 3 * w : (sun ? F_AS : F_AD) + 3 * (w - 2), s);
                 n2[w] = dot(v, v);
             }
-            const double a0 = sun ? 0. : B.d[F_ACC0][s];
-            n2[0] = n2[0] + P.alpha2 * a0 * a0;
+            n2[0] = n2[0] + (sun ? 0. : B.d[F_A02][s]);
             double nn[4];
 #pragma unroll 1
             for (int w = 0; w < 4; w++) nn[w] = sqrt_rn(n2[w]);
-            crit = dt4th_of(sun ? P.eta_sun : P.eta, nn[0], nn[1], nn[2], nn[3], n2[1], n2[2]);
+            num = nn[0] * nn[2] + n2[1];
+            den = nn[1] * nn[3] + n2[2];
+            Jerk = nn[1];
         }
+        const double crit = (dbits(Jerk) << 1) != 0ULL ? (sun ? P.eta_sun : P.eta) * sqrt_rn(div_rn(num, den))
+                                                       : 1.7976931348623157e308;
         const double other = __shfl_xor_sync(ALL, crit, L / 2);
         if (act) {
             for (int f = r; f < 12; f += L) B.d[F_AS + f][s] = B.d[F_NAS + f][s];
             if (r == 0) {
-                const double th0 = B.d[F_TH][s], th = th0 + (B.c_ts[k] - th0);
+                const double th = B.d[F_TH][s] + B.d[F_TE][s];
                 B.d[F_TH][s] = th;
                 double dt = B.d[F_DT][s];
                 if (!(B.c_flags[k] & CF_COL) && !B.dead[s]) {
-                    dt = dt_next_bits(P, th, dt, dmin(crit, other));
+                    dt = dt_next_bits(A, th, dt, dmin_crit(crit, other));
                     B.d[F_DT][s] = dt;
                 }
                 B.d[F_TE][s] = th + dt;
@@ -1228,6 +1528,7 @@ __device__ __forceinline__ void bundle_dt(const HardArgs &A, BundleSmem<BCAP> &B
     }
     __syncthreads();
     if (B.any_dead) {  // a twin's block step is its target's
+#pragma unroll 1
         for (int i = threadIdx.x; i < nt; i += BT) {
             const int s = B.tgt[i], k = B.cl[s];
             if (B.dead[s] && B.owner[s] >= 0 && !(B.c_flags[k] & CF_COL)) B.d[F_DT][s] = B.d[F_DT][B.owner[s]];
@@ -1246,6 +1547,7 @@ __device__ __forceinline__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> 
     // fused where they are exact.  The active set: the alive members whose
     // step ends now.
     const int used = B.used, lane = threadIdx.x & 31;
+#pragma unroll 1
     for (int w0 = threadIdx.x - lane; w0 < 3 * used; w0 += BT) {  // whole warps
         const int it = min(w0 + lane, 3 * used - 1);
         const int c = it >= 2 * used ? 2 : (it >= used ? 1 : 0), p = it - c * used, k = B.cl[p];
@@ -1268,31 +1570,50 @@ __device__ __forceinline__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> 
         if (c == 0) {
             const bool act = !B.dead[p] && dbits(B.d[F_TE][p]) == dbits(ts);
             B.flag[p] = act ? (MF_ACT | MF_TGT) : 0;
-            if (act) atomicAdd(&B.c_act[k], 1);
+            if (act) {
+                B.d[F_TE][p] = Dt;
+                atomicAdd(&B.c_act[k], 1);
+            }
         }
     }
     __syncthreads();
     HP_MARK(HP_PREDICT);
     // collisionDetermination, src/hermite.h:98-196
-    bundle_detect(A, B, false);
+    // beside it, in warp 0, the lists of a small bundle (made again if there is a
+    // collision, whose targets are others)
+    bool listed = false;
+    const bool small = used <= 32 && !B.any_dead;
+    if (!small) bundle_detect(A, B, false, threadIdx.x);
+    else if (threadIdx.x >= 32) bundle_detect(A, B, false, threadIdx.x - 32);
+    else bundle_lists_small(A, B);
     __syncthreads();
     const bool col = B.n_sv > 0;
     if (col) bundle_collisions_found<BCAP>(A);
     HP_MARK(HP_DETECT);
     if (B.any_dead) {  // the twins of active merged members
+#pragma unroll 1
         FOR_SLOTS(p) {
             const int ow = B.owner[p];
-            if (B.dead[p] && ow >= 0 && (B.flag[ow] & MF_ACT)) B.flag[p] |= MF_TGT;
+            if (B.dead[p] && ow >= 0 && (B.flag[ow] & MF_ACT)) {
+                B.flag[p] |= MF_TGT;
+                B.d[F_TE][p] = B.c_ts[B.cl[p]] - B.d[F_TH][p];
+            }
         }
         __syncthreads();
     }
-    const int nt = bundle_targets(B, MF_TGT);
+    int nt;
+    if (small && !col) {
+        nt = B.nt;
+        listed = B.pfx[nt] <= 4 * 32;
+    } else {
+        nt = bundle_targets(B, MF_TGT);
+    }
     HP_MARK(HP_ACTIVE);
     // predicted forces and first correction, corrected forces and second
     // correction, corrected forces
-    bool listed = false;
 #pragma unroll 1
     for (int ps = 0; ps < 3; ps++) bundle_pass<BCAP, false>(A, B, ps == 0 ? 1 : 2, nt, false, (ps + 1) % 3, listed);
+#pragma unroll 1
     FOR_CLUSTERS(k) {
         B.c_work[k] += (long long)B.c_act[k] * B.c_n[k];
         B.c_key[k] = B.c_tm[k] = dbits(1.e10);
@@ -1305,16 +1626,32 @@ __device__ __forceinline__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> 
     // (src/hermite.h:4-24): the minima of th and th + dt over the alive members
     if (threadIdx.x == 0) B.any = B.n_sv = B.moved = 0;
     if (col) {
+#pragma unroll 1
         FOR_CLUSTERS(k) B.c_key[k] = B.c_tm[k] = dbits(1.e10);
         __syncthreads();
     }
-    FOR_SLOTS(p) {
-        if (B.dead[p]) continue;
-        const int k = B.cl[p];
-        atomicMin(&B.c_tm[k], dbits(B.d[F_TH][p]));
-        atomicMin(&B.c_key[k], dbits(B.d[F_TE][p]));
+    if (used <= 32 && B.ncl == 1 && !col) {  // one cluster: by a warp
+        if (threadIdx.x < 32) {
+            const int p = threadIdx.x;
+            const bool in = p < used && !B.dead[p];
+            const unsigned long long th = warp_min64(in ? dbits(B.d[F_TH][p]) : ~0ULL),
+                                     te = warp_min64(in ? dbits(B.d[F_TE][p]) : ~0ULL);
+            if (p == 0) {
+                B.c_tm[0] = min(th, dbits(1.e10));
+                B.c_key[0] = min(te, dbits(1.e10));
+            }
+        }
+    } else {
+#pragma unroll 1
+        FOR_SLOTS(p) {
+            if (B.dead[p]) continue;
+            const int k = B.cl[p];
+            atomicMin(&B.c_tm[k], dbits(B.d[F_TH][p]));
+            atomicMin(&B.c_key[k], dbits(B.d[F_TE][p]));
+        }
     }
     __syncthreads();
+#pragma unroll 1
     FOR_CLUSTERS(k) {
         const bool going = B.c_tm[k] < dbits(A.t_end);
         if (going && B.c_steps[k] < A.max_steps) {
@@ -1336,10 +1673,12 @@ __device__ __noinline__ void bundle_retire(const HardArgs &A) {
     constexpr int BT = BundleSmem<BCAP>::NT, PER = BCAP / BT;
     const Hard &H = A.H;
     const int tid = threadIdx.x;
+#pragma unroll 1
     FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_FIN) ? MF_TGT : 0;
     __syncthreads();
     const int nt = bundle_full<BCAP>(A, true);
     // write back to FPGrav, with resetTime (src/hard.h:768-787)
+#pragma unroll 1
     for (int i = tid; i < nt; i += BT) {
         const int s = B.tgt[i], g = B.gslot[s], k = B.cl[s];
         const double th = B.d[F_TH][s], dt = B.d[F_DT][s];
@@ -1364,6 +1703,7 @@ __device__ __noinline__ void bundle_retire(const HardArgs &A) {
         A.S.dead[idx] = B.dead[s]; A.S.merged[idx] = B.merged[s];
         A.S.n_cluster[idx] = B.c_n[k];
     }
+#pragma unroll 1
     FOR_CLUSTERS(k) {
         if (!(B.c_flags[k] & CF_FIN)) continue;
         const int c = B.c_idx[k];
@@ -1437,6 +1777,7 @@ __device__ __noinline__ void bundle_retire(const HardArgs &A) {
         B.any_dead = 0;
     }
     __syncthreads();
+#pragma unroll 1
     FOR_SLOTS(p) {
         if (B.dead[p]) B.any_dead = 1;
     }
@@ -1520,14 +1861,16 @@ __global__ void __launch_bounds__(bundle_threads(BCAP), OCC) k_hard_bundles(cons
     bundle_init(B);
     __syncthreads();
     for (int guard = 0; guard < (1 << 30); guard++) {
-        if (threadIdx.x == 0) {
-            B.fresh_k = B.ncl;
-            B.fresh_p = B.used;
+        if (guard == 0 || B.any) {  // clusters have left (or none has come yet)
+            if (threadIdx.x == 0) {
+                B.fresh_k = B.ncl;
+                B.fresh_p = B.used;
+            }
+            __syncthreads();
+            bundle_refill<BCAP>(A);
+            if (B.ncl == 0) break;
+            if (B.fresh_k < B.ncl) bundle_load<BCAP>(A);
         }
-        __syncthreads();
-        bundle_refill<BCAP>(A);
-        if (B.ncl == 0) break;
-        if (B.fresh_k < B.ncl) bundle_load<BCAP>(A);
         HP_MARK(HP_ADMIT);
         bundle_step(A, B);
         if (B.any) bundle_retire<BCAP>(A);
