@@ -176,4 +176,63 @@ P3T_HD double div_rn(double a, double b) {
     return ex_double(ex_div_core(ba, bb, ex_rcp32(m32)));
 }
 
+// Powers of 1 / sqrt(x) with one rounding each, within 0.6 units of the last
+// place (a root, a quotient and products round once apiece).  One cubic step
+// from the FP32 approximation y0: y = y0 (1 + e/2 + 3 e^2/8), e = 1 - m y0^2,
+// |e| < 2^-20, leaves 5/16 e^3 < 2^-61; the products keep 62 fraction bits.
+struct InvRoots {
+    double y1, y3, y4, y5;
+};
+// m in [1, 4) as X with 62 fraction bits -> 1 / sqrt(m) with 63
+P3T_HD uint64_t ex_rsqrt63(uint64_t X, uint32_t seed) {
+    const uint64_t Y0 = ex_frac32(seed);
+    const int64_t e = (int64_t)((1ULL << 62) - ex_mulhi(X, Y0 * Y0));
+    const int64_t eh = (int64_t)(int32_t)(e >> 12);
+    const int64_t c = (e >> 1) + ((eh * eh * 3) >> 41);
+    const int64_t d = (int64_t)(c >> 32) * (int64_t)Y0 + (int64_t)(((uint64_t)(uint32_t)c * Y0) >> 32);
+    return ((Y0 << 30) + (uint64_t)d) << 1;
+}
+P3T_HD uint32_t ex_clz_high(uint64_t v) {
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__clz((int)(v >> 32));
+#else
+    return (uint32_t)__builtin_clzll(v);
+#endif
+}
+// v 2^(s - 62), rounded once; v in [2^57, 2^62]
+P3T_HD double ex_pack62(uint64_t v, int32_t s) {
+    const uint32_t n = ex_clz_high(v);
+    v <<= n;
+    return ex_double(((uint64_t)(uint32_t)(1023 - (int32_t)n + s) << 52) + (v >> 11) + ((v >> 10) & 1));
+}
+// operands outside 2^-380 .. 2^380, zero, infinite or NaN: the library's operations
+#ifdef __CUDACC__
+static __device__ __noinline__ InvRoots ex_inv_roots_library(double x) {
+    const double y = 1.0 / sqrt(x), y2 = y * y;
+    return InvRoots{y, y2 * y, y2 * y2, y2 * (y2 * y)};
+}
+#endif
+P3T_HD bool ex_inv_roots_range(double x) { return (uint32_t)(ex_bits(x) >> 52) - 643u < 760u; }
+// WITH_HIGH: y4 and y5 as well
+template <bool WITH_HIGH>
+P3T_HD InvRoots inv_roots_in(double x) {
+    const uint64_t b = ex_bits(x);
+    const uint32_t e = (uint32_t)(b >> 52), odd = (e & 1u) ^ 1u;
+    const uint64_t X = ((b & (EX_ONE - 1)) | EX_ONE) << (10 + odd);
+    const uint32_t m32 = ((127u + odd) << 23) | ((uint32_t)(b >> 29) & 0x7fffffu);
+    const int32_t k = ((int32_t)(e - odd) - 1023) >> 1;
+    const uint64_t Y = ex_rsqrt63(X, ex_rsqrt32(m32));
+    const uint64_t y2 = ex_mulhi(Y, Y), y3 = ex_mulhi(y2 << 1, Y);  // 62 fraction bits
+    InvRoots r;
+    r.y1 = ex_pack62(Y >> 1, -k);
+    r.y3 = ex_pack62(y3, -3 * k);
+    if (WITH_HIGH) {
+        r.y4 = ex_pack62(ex_mulhi(y2 << 1, y2 << 1), -4 * k);
+        r.y5 = ex_pack62(ex_mulhi(y2 << 1, y3 << 1), -5 * k);
+    } else {
+        r.y4 = r.y5 = 0.;
+    }
+    return r;
+}
+
 }  // namespace p3t

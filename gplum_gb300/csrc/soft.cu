@@ -30,8 +30,8 @@
 //   * forces: FP32 with rsqrt + one Newton step, FMA allowed; partial sums of
 //     32 pairs are folded into an error-free (TwoSum) FP32 hi/lo pair, so the
 //     accumulation error does not grow with the list length.
-// FP64 kernel: the same formulas with every quantity in double, plain
-// 1/sqrt -- the "plain FP64" form used as the accuracy and speed baseline.
+// FP64 kernel: the same formulas with every quantity in double, the powers of
+// 1/r rounded once each -- the "plain FP64" form used as the accuracy baseline.
 //
 // Optional candidate emission: every screen hit (j != i) appends j's particle
 // index to the i's row of a [n x cap] candidate table; the device-side
@@ -39,6 +39,7 @@
 #include <mutex>
 
 #include "p3t_common.cuh"
+#include "p3t_exact.cuh"
 #include "p3t_soft.cuh"
 
 namespace p3t {
@@ -843,9 +844,31 @@ __global__ void __launch_bounds__(SB, OCC) soft_mixed_pipe_kernel(SoftArgs A) {
 
 // --------------------------------------------------------------------------
 // plain FP64
+// The FP64 pipe bounds this form: it takes one warp instruction per 19 cycles of
+// the SM, so the pair loops give it the sums, products and the displacements'
+// differences only.  The root, its powers and their roundings are integer
+// arithmetic (p3t_exact.cuh), as are the per-pair maxima and the screen: radii
+// become the keys of their squares, which order as the radii do.  Per warp and
+// list entry 37 -> 12 FP64 instructions (EP-EP) and 52 -> 32 (EP-SP):
+// 30,000 bodies in groups of 64 (174k + 180k list entries) 1.14 -> 0.63 ms.
+__device__ __forceinline__ long long radius_key(double r, double scale) {
+    const long long b = __double_as_longlong(__dmul_rn(__dmul_rn(r, r), scale));
+    return r >= 0. ? b : r < 0. ? -b : 0;  // a NaN radius loses against any other, as in fmax
+}
+// y1 and y3 of max(r2r, ro2), both non-negative
+__device__ __forceinline__ InvRoots ep_roots(double r2r, unsigned long long ro2) {
+    const unsigned long long a = (unsigned long long)__double_as_longlong(r2r);
+    const double r2 = __longlong_as_double((long long)(a > ro2 ? a : ro2));
+    if (ex_inv_roots_range(r2)) return inv_roots_in<false>(r2);
+    return ex_inv_roots_library(fmax(r2r, __longlong_as_double((long long)ro2)));
+}
+__device__ __forceinline__ InvRoots sp_roots(double r2) {
+    return ex_inv_roots_range(r2) ? inv_roots_in<true>(r2) : ex_inv_roots_library(r2);
+}
+
 template <int S, int IPT, bool EMIT>
 __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int ni, D4 *da, D4 *db, D4 *dc,
-                                          int2 *dids, int *sidx, int *scnt, double *redd, int *redi) {
+                                          longlong2 *dk, int2 *dids, int *sidx, int *scnt, double *redd, int *redi) {
     constexpr int W = SB / S;
     const int tid = threadIdx.x;
     const int sub = tid / W, lane = tid % W;
@@ -854,7 +877,8 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
     const int s0 = A.s_off[g], ns = A.s_off[g + 1] - s0;
     const double eps2 = A.eps2_d;
 
-    double xi[IPT], yi[IPT], zi[IPT], roi[IPT], rsi[IPT];
+    double xi[IPT], yi[IPT], zi[IPT];
+    long long roi[IPT], rsi[IPT];
     int idi[IPT], rki[IPT], pid[IPT], li[IPT];
     bool vi[IPT];
     double ax[IPT], ay[IPT], az[IPT], ap[IPT];
@@ -868,7 +892,7 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
         if ((unsigned)p >= (unsigned)A.n_iptcl) { atomicOr(A.status, ST_BAD_INDEX); p = 0; vi[k] = false; }
         pid[k] = p;
         xi[k] = A.iptcl[p].x; yi[k] = A.iptcl[p].y; zi[k] = A.iptcl[p].z;
-        roi[k] = A.i_r_out[p]; rsi[k] = A.i_r_search[p];
+        roi[k] = radius_key(A.i_r_out[p], 1.); rsi[k] = radius_key(A.i_r_search[p], 1.0201);
         idi[k] = A.iptcl[p].id_local; rki[k] = A.iptcl[p].rank;
         ax[k] = ay[k] = az[k] = ap[k] = 0.;
         ngb[k] = 0; rk[k] = 0; idmax[k] = -1; idmin[k] = INT32_MAX_;
@@ -885,7 +909,7 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
             if ((unsigned)p >= (unsigned)A.n_ptcl) { atomicOr(A.status, ST_BAD_INDEX); p = 0; }
             const SoftPtcl &r = A.ptcl[p];
             da[tid] = D4c(r.x, r.y, r.z, A.mass[p]);
-            db[tid] = D4c(A.r_out[p], A.r_search[p], 0., 0.);
+            dk[tid] = make_longlong2(radius_key(A.r_out[p], 1.), radius_key(A.r_search[p], 1.0201));
             dids[tid] = make_int2(r.id_local, r.rank);
             if (EMIT) sidx[tid] = p;
         }
@@ -893,21 +917,21 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
         const int jb = sub * (TJ / S), je = wact ? min(jb + TJ / S, nt) : jb;
         for (int jj = jb; jj < je; jj++) {
             const D4 a = da[jj];
-            const D4 b = db[jj];
+            const longlong2 b = dk[jj];
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
                 const double rx = xi[k] - a.x, ry = yi[k] - a.y, rz = zi[k] - a.z;
-                const double ro = fmax(roi[k], b.x), rs = fmax(rsi[k], b.y);
-                const double r2r = rx * rx + ry * ry + rz * rz + eps2;
-                const double r2 = fmax(r2r, ro * ro);
-                const double ri = 1.0 / sqrt(r2);
-                const double mr = a.w * ri;
-                const double mr3 = mr * ri * ri;
+                const unsigned long long ro2 = (unsigned long long)llabs(max(roi[k], b.x));
+                const unsigned long long rs2 = (unsigned long long)llabs(max(rsi[k], b.y));
+                double r2r = rx * rx + ry * ry + rz * rz;
+                if (eps2 != 0.) r2r += eps2;
+                const InvRoots w = ep_roots(r2r, ro2);
+                const double mr3 = a.w * w.y3;
                 ax[k] += mr3 * rx;
                 ay[k] += mr3 * ry;
                 az[k] += mr3 * rz;
-                ap[k] += mr;
-                if (r2r < rs * rs * 1.0201) {
+                ap[k] += a.w * w.y1;
+                if ((unsigned long long)__double_as_longlong(r2r) < rs2) {
                     const int idj = dids[jj].x, rkj = dids[jj].y;
                     if ((idi[k] != idj || rki[k] != rkj) && vi[k]) {
                         ngb[k] += 1;
@@ -945,20 +969,20 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
                 const double rx = a.x - xi[k], ry = a.y - yi[k], rz = a.z - zi[k];
-                const double r2 = rx * rx + ry * ry + rz * rz + eps2;
-                const double ri = 1.0 / sqrt(r2);
-                const double r2i = ri * ri, r3i = r2i * ri, r4i = r2i * r2i, r5i = r2i * r3i;
+                double r2 = rx * rx + ry * ry + rz * rz;
+                if (eps2 != 0.) r2 += eps2;
+                const InvRoots w = sp_roots(r2);
                 const double qrx = q1.x * rx + q2.x * ry + q2.z * rz;
                 const double qry = q1.y * ry + q2.y * rz + q2.x * rx;
                 const double qrz = q1.z * rz + q2.z * rx + q2.y * ry;
                 const double rqr = q1.w + qrx * rx + qry * ry + qrz * rz;
-                const double rqr4 = rqr * r4i;
+                const double rqr4 = rqr * w.y4;
                 const double meff = a.w + 0.5 * rqr4;
-                const double meff3 = (a.w + 2.5 * rqr4) * r3i;
-                ax[k] += r5i * qrx - meff3 * rx;
-                ay[k] += r5i * qry - meff3 * ry;
-                az[k] += r5i * qrz - meff3 * rz;
-                ap[k] += meff * ri;
+                const double meff3 = (a.w + 2.5 * rqr4) * w.y3;
+                ax[k] += w.y5 * qrx - meff3 * rx;
+                ay[k] += w.y5 * qry - meff3 * ry;
+                az[k] += w.y5 * qrz - meff3 * rz;
+                ap[k] += meff * w.y1;
             }
         }
     }
@@ -1005,8 +1029,9 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
 }
 
 template <bool EMIT>
-__global__ void __launch_bounds__(SB, 2) soft_f64_kernel(SoftArgs A) {
+__global__ void __launch_bounds__(SB, 4) soft_f64_kernel(SoftArgs A) {
     __shared__ D4 da[TJ], db[TJ], dc[TJ];
+    __shared__ longlong2 dk[TJ];
     __shared__ int2 dids[TJ];
     __shared__ int sidx[EMIT ? TJ : 1];
     __shared__ int scnt[EMIT ? 2 * SB : 1];
@@ -1018,13 +1043,13 @@ __global__ void __launch_bounds__(SB, 2) soft_f64_kernel(SoftArgs A) {
     for (int ib = 0; ib < ni_all; ib += span) {
         const int ni = min(span, ni_all - ib);
         if (ni > A.t_ipt2)
-            group_f64<1, 2, EMIT>(A, g, ib, ni, da, db, dc, dids, sidx, scnt, redd, redi);
+            group_f64<1, 2, EMIT>(A, g, ib, ni, da, db, dc, dk, dids, sidx, scnt, redd, redi);
         else if (ni > A.t_s1)
-            group_f64<1, 1, EMIT>(A, g, ib, ni, da, db, dc, dids, sidx, scnt, redd, redi);
+            group_f64<1, 1, EMIT>(A, g, ib, ni, da, db, dc, dk, dids, sidx, scnt, redd, redi);
         else if (ni > A.t_s2)
-            group_f64<2, 1, EMIT>(A, g, ib, ni, da, db, dc, dids, sidx, scnt, redd, redi);
+            group_f64<2, 1, EMIT>(A, g, ib, ni, da, db, dc, dk, dids, sidx, scnt, redd, redi);
         else
-            group_f64<4, 1, EMIT>(A, g, ib, ni, da, db, dc, dids, sidx, scnt, redd, redi);
+            group_f64<4, 1, EMIT>(A, g, ib, ni, da, db, dc, dk, dids, sidx, scnt, redd, redi);
         __syncthreads();
     }
 }
