@@ -48,6 +48,8 @@ Context *ctx_get(int device) {
         return nullptr;
     }
     cudaMemsetAsync(c->status, 0, sizeof(int), c->stream);
+    int v = 0;
+    c->reads_host = cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) == cudaSuccess && v;
     // default parameters: FPGrav defaults, src/particle.h:917-961
     const double def[21] = {0., 0., 1., 1. / 32., 1. / 8192., 0.01, 0.001, 0.01, 0.001, 1.,
                             0.5, 2., 8., 1., 4., 1., 4., 0., 0., 0., 5.049667e6};
@@ -218,6 +220,17 @@ SoftArgs make_args(Context *c, DevSet &d, int n_group, int n_ptcl, int n_spj, bo
     return A;
 }
 
+// The staged EPJ records of a resident problem -> the soft kernels' arrays.
+static cudaError_t pack_bodies(Context *c, DevSet &d, int n) {
+    if (n <= 0) return cudaSuccess;
+    PackArgs A{};
+    A.one.epj = d.epj_stage.p;
+    A.one.nj = n;
+    A.n_walk = 1;
+    A.ptcl = d.ptcl.p; A.mass = d.mass.p; A.r_out = d.r_out.p; A.r_search = d.r_search.p;
+    return launch_pack_walks(A, n, c->stream);
+}
+
 // Launch order: largest groups first (less tail imbalance).
 // launch order of the groups: most pair work first (i-slots in whole warps x
 // list entries, a superparticle counted twice)
@@ -339,8 +352,7 @@ int p3t_upload_particles(int n, const void *epj) {
         (r = d.acc64.reserve(n)))
         return r;
     if ((r = h2d(c, d.epj_stage.p, epj, (size_t)n * sizeof(EPJRec)))) return r;
-    r = cuda_status(launch_pack_epj(d.epj_stage.p, n, d.ptcl.p, d.mass.p, d.r_out.p, d.r_search.p, c->stream));
-    if (r) return r;
+    if ((r = cuda_status(pack_bodies(c, d, n)))) return r;
     c->res_n = n;
     return 0;
 }
@@ -441,8 +453,7 @@ int p3t_soft_force_host(int n, const void *epj, int n_group, const int *i_off, c
         return e;
     };
     if ((r = u.issue())) return fail(r);
-    if ((r = cuda_status(launch_pack_epj(d.epj_stage.p, n, d.ptcl.p, d.mass.p, d.r_out.p, d.r_search.p, c->stream))))
-        return fail(r);
+    if ((r = cuda_status(pack_bodies(c, d, n)))) return fail(r);
     c->res_n = n;
     c->res_groups = n_group;
     c->res_spj = n_spj;

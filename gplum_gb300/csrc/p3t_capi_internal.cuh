@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "p3t_common.cuh"
+#include "p3t_soft.cuh"
 
 namespace p3t {
 
@@ -28,41 +29,53 @@ struct DevBuf {
 // One set of device buffers for a soft-force problem.
 struct DevSet {
     DevBuf<EPJRec> epj_stage;
-    DevBuf<EPIRec> epi_stage;
     DevBuf<SoftPtcl> iptcl;
     DevBuf<double> i_r_out, i_r_search;
     DevBuf<SoftPtcl> ptcl;
     DevBuf<double> mass, r_out, r_search;
     DevBuf<SPJRec> spj;
+    DevBuf<SoftSplit> isplit, jsplit;
+    DevBuf<SpjPack> spjp;
     DevBuf<int> i_off, i_idx, j_off, j_idx, s_off, s_idx, order;
     DevBuf<ForceRec> force;
     DevBuf<D4> acc64;
     DevBuf<int> cand;
     bool order_valid = false;
     void release() {
-        epj_stage.release(); epi_stage.release(); iptcl.release(); i_r_out.release(); i_r_search.release(); ptcl.release(); mass.release(); r_out.release();
-        r_search.release(); spj.release(); i_off.release(); i_idx.release(); j_off.release(); j_idx.release();
+        epj_stage.release(); iptcl.release(); i_r_out.release(); i_r_search.release(); ptcl.release(); mass.release(); r_out.release();
+        r_search.release(); spj.release(); isplit.release(); jsplit.release(); spjp.release(); i_off.release(); i_idx.release(); j_off.release(); j_idx.release();
         s_off.release(); s_idx.release(); order.release(); force.release(); acc64.release(); cand.release();
     }
 };
 
 constexpr int MAX_TAGS = 8;
 
-// State of one in-flight multiwalk dispatch.
+// State of one in-flight multiwalk dispatch (or of the functor calls).
 struct WalkSlot {
     DevSet d;
-    void *h_in = nullptr;
+    void *h_tab = nullptr;  // pinned: a copy of the status word, then the walks' records table
+    size_t h_tab_cap = 0;
+    void *h_in = nullptr;  // pinned: records that the device cannot read in place
     size_t h_in_cap = 0;
-    void *h_out = nullptr;
+    void *h_out = nullptr;  // pinned: the forces, written by the kernel
     size_t h_out_cap = 0;
-    cudaEvent_t done = nullptr;
+    cudaEvent_t read = nullptr, done = nullptr;  // the caller's records read; the forces there
     int n_i = 0;
     bool busy = false;
-    int status = 0;
+    void release() {
+        d.release();
+        if (h_tab) cudaFreeHost(h_tab);
+        if (h_in) cudaFreeHost(h_in);
+        if (h_out) cudaFreeHost(h_out);
+        if (read) cudaEventDestroy(read);
+        if (done) cudaEventDestroy(done);
+        *this = WalkSlot();
+    }
 };
 
 struct Context {
     int device = 0;
+    bool reads_host = false;  // the device reads any host memory in place (it walks the host's page tables)
     cudaStream_t stream = nullptr;
     int *status = nullptr;  // device status bits
     double params[21];
@@ -78,6 +91,8 @@ struct Context {
     // index-form multiwalk: EPJ/SPJ arrays resident across dispatches
     DevSet idx;
     int idx_nj = 0, idx_ns = 0;
+    float idx_eps2 = 0.f;  // what idx.spjp was packed with
+    int idx_trace = -1;
     // pinned staging
     void *h_stage = nullptr;
     size_t h_stage_cap = 0;
@@ -86,6 +101,7 @@ struct Context {
     void *h_order = nullptr;  // group launch order on its way to the device
     size_t h_order_cap = 0;
     WalkSlot walk[MAX_TAGS];
+    WalkSlot fun;  // the single-group functor calls
 
     void release() {
         res.release();
@@ -95,13 +111,8 @@ struct Context {
         if (h_order) cudaFreeHost(h_order);
         h_stage = h_out = h_order = nullptr;
         h_stage_cap = h_out_cap = h_order_cap = 0;
-        for (auto &w : walk) {
-            w.d.release();
-            if (w.h_in) cudaFreeHost(w.h_in);
-            if (w.h_out) cudaFreeHost(w.h_out);
-            if (w.done) cudaEventDestroy(w.done);
-            w = WalkSlot();
-        }
+        for (auto &w : walk) w.release();
+        fun.release();
     }
 };
 
@@ -122,7 +133,6 @@ int h2d(Context *c, void *dst, const void *src, size_t bytes);
 // stream (a non-blocking stream, which plain cudaMemcpy does not wait for).
 int d2h(Context *c, void *dst, const void *src, size_t bytes);
 
-struct SoftArgs;
 SoftArgs make_args(Context *c, DevSet &d, int n_group, int n_ptcl, int n_spj, bool accumulate);
 int set_group_order(Context *c, DevSet &d, int n_group, const int *i_off_h, const int *j_off_h, const int *s_off_h);
 bool is_pinned(const void *p);

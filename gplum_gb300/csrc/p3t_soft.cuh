@@ -61,17 +61,55 @@ struct SoftArgs {
     // per-device buffers (stream-ordered, grown on demand).
     SoftSplit *isplit, *jsplit;
     SpjPack *spjp;
+    int packed;       // 1: the scratch is filled already (launch_pack_walks)
+    const int *gate;  // optional device word: non-zero and the mixed kernels return at once
 };
+
+// One walk's records and where its packed entries start.  The records may lie
+// in device memory or in host memory that the device reads in place (pinned,
+// or any memory where the device walks the host's page tables).  They start on
+// 8-byte boundaries, index lists on 4-byte ones.
+struct WalkRecords {
+    const EPIRec *epi;
+    const void *epj;  // EPJRec, or int in the index form
+    const void *spj;  // SPJRec, or int in the index form
+    int ni, nj, ns;
+    int io, jo, so;
+};
+// launch_pack_walks: the walks' records -> the soft kernels' arrays.  Outputs
+// whose pointer is null are left out.
+struct PackArgs {
+    const WalkRecords *walk;  // [n_walk], readable by the device; nullptr = `one`
+    WalkRecords one;
+    int n_walk;
+    int index;  // epj and spj are index lists: copied into j_idx and s_idx
+    int slices;  // CTAs per walk (set by the launch)
+    int *i_off, *j_off, *s_off;  // CSR offsets [n_walk + 1]
+    int *i_idx, *j_idx, *s_idx;
+    SoftPtcl *iptcl, *ptcl;
+    SoftSplit *isplit, *jsplit;
+    double *i_r_out, *i_r_search, *mass, *r_out, *r_search;
+    SPJRec *spj;
+    SpjPack *spjp;
+    const ForceRec *seed;  // FP64 form: the records to accumulate into, widened into acc64
+    D4 *acc64;
+    float eps2;
+    int trace_mode;
+    // optional check of a caller's CSR offsets (each starts at 0 and never
+    // decreases, the i lists end at chk_n at most): ST_BAD_INDEX into *gate
+    // and *status
+    const int *chk_i_off, *chk_j_off, *chk_s_off;
+    int chk_groups, chk_n;
+    int *gate, *status;
+};
+cudaError_t launch_pack_walks(const PackArgs &A, long long n_records, cudaStream_t st);
+cudaError_t launch_spj_pack(const SPJRec *in, int n, float eps2, int trace_mode, SpjPack *out, cudaStream_t st);
 
 // The soft launch shape last set through p3t_set_soft_tiles /
 // p3t_set_soft_occupancy: {t_ipt2, t_s1, t_s2, occ}, process-wide, for entry
 // points that run without the library context (p3t_soft_force_noalloc).
 extern int g_soft_shape[4];
 
-cudaError_t launch_pack_epj(const EPJRec *in, int n, SoftPtcl *out, double *mass, double *r_out, double *r_search,
-                            cudaStream_t st);
-cudaError_t launch_pack_epi(const EPIRec *in, int n, SoftPtcl *out, double *r_out, double *r_search, cudaStream_t st);
-cudaError_t launch_iota(int *out, int n, int base, cudaStream_t st);
 cudaError_t launch_soft(const SoftArgs &A, int precision, bool emit, cudaStream_t st);
 
 }  // namespace p3t

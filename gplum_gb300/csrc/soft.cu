@@ -454,6 +454,7 @@ __global__ void __launch_bounds__(SB, OCC) soft_mixed_kernel(SoftArgs A) {
     __shared__ int scnt[EMIT ? SB : 1];
     __shared__ float redf[SB * 8];
     __shared__ int redi[SB * 4];
+    if (A.gate && *A.gate) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     // EP-EP unroll depth: as deep as the register budget holds without spills
@@ -827,6 +828,7 @@ template <bool EMIT, int OCC>
 __global__ void __launch_bounds__(SB, OCC) soft_mixed_pipe_kernel(SoftArgs A) {
     __shared__ PipeSmem M;
     __shared__ int scnt[EMIT ? SB : 1];
+    if (A.gate && *A.gate) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     constexpr int UNR = OCC <= 4 ? 8 : 2;
@@ -1055,78 +1057,23 @@ __global__ void __launch_bounds__(SB, 4) soft_f64_kernel(SoftArgs A) {
 }
 
 // --------------------------------------------------------------------------
-// EPJGrav records -> SoftPtcl (+ FP64 side arrays for the FP64 form)
-__global__ void pack_epj_kernel(const EPJRec *__restrict__ in, int n, SoftPtcl *out, double *mass, double *r_out,
-                                double *r_search) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const EPJRec &e = in[i];
+// Records -> the pair kernels' arrays
+__device__ __forceinline__ SoftPtcl soft_ptcl(double x, double y, double z, float m, double r_out, double r_search,
+                                              int id_local, int rank) {
+    const float ro = (float)r_out, rs = (float)r_search;
     SoftPtcl r;
-    r.x = e.pos[0];
-    r.y = e.pos[1];
-    r.z = e.pos[2];
-    r.m = (float)e.mass;
-    const float ro = (float)e.r_out, rs = (float)e.r_search;
+    r.x = x;
+    r.y = y;
+    r.z = z;
+    r.m = m;
     r.ro2 = __fmul_rn(ro, ro);
     r.rs2 = __fmul_rn(__fmul_rn(rs, rs), 1.0201f);
-    r.id_local = e.id_local;
-    r.rank = e.myrank;
+    r.id_local = id_local;
+    r.rank = rank;
     r.pad = 0;
-    out[i] = r;
-    mass[i] = e.mass;
-    r_out[i] = e.r_out;
-    r_search[i] = e.r_search;
+    return r;
 }
-
-__global__ void pack_epi_kernel(const EPIRec *__restrict__ in, int n, SoftPtcl *out, double *r_out, double *r_search) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const EPIRec &e = in[i];
-    SoftPtcl r;
-    r.x = e.pos[0];
-    r.y = e.pos[1];
-    r.z = e.pos[2];
-    r.m = 0.f;
-    const float ro = (float)e.r_out, rs = (float)e.r_search;
-    r.ro2 = __fmul_rn(ro, ro);
-    r.rs2 = __fmul_rn(__fmul_rn(rs, rs), 1.0201f);
-    r.id_local = e.id_local;
-    r.rank = e.myrank;
-    r.pad = 0;
-    out[i] = r;
-    r_out[i] = e.r_out;
-    r_search[i] = e.r_search;
-}
-
-__global__ void iota_kernel(int *out, int n, int base) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = base + i;
-}
-
-cudaError_t launch_pack_epi(const EPIRec *in, int n, SoftPtcl *out, double *r_out, double *r_search, cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    { P3T_COUNT_LAUNCH(); pack_epi_kernel<<<(n + 255) / 256, 256, 0, st>>>(in, n, out, r_out, r_search); }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_iota(int *out, int n, int base, cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    { P3T_COUNT_LAUNCH(); iota_kernel<<<(n + 255) / 256, 256, 0, st>>>(out, n, base); }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_epj(const EPJRec *in, int n, SoftPtcl *out, double *mass, double *r_out, double *r_search,
-                            cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    { P3T_COUNT_LAUNCH(); pack_epj_kernel<<<(n + 255) / 256, 256, 0, st>>>(in, n, out, mass, r_out, r_search); }
-    return cudaGetLastError();
-}
-
-// Mixed-form preprocessing: per-particle splits and packed superparticles.
-__global__ void split_kernel(const SoftPtcl *__restrict__ p, int n, SoftSplit *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const SoftPtcl r = p[i];
+__device__ __forceinline__ SoftSplit soft_split(const SoftPtcl &r) {
     SoftSplit s;
     s.xh = __double2float_rn(r.x);
     s.yh = __double2float_rn(r.y);
@@ -1136,13 +1083,9 @@ __global__ void split_kernel(const SoftPtcl *__restrict__ p, int n, SoftSplit *o
     s.zl = __double2float_rn(r.z - (double)s.zh);
     s.m = r.m;
     s.ro2 = r.ro2;
-    out[i] = s;
+    return s;
 }
-
-__global__ void spj_pack_kernel(const SPJRec *__restrict__ in, int n, float eps2, int trace_mode, SpjPack *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const SPJRec &r = in[i];
+__device__ __forceinline__ SpjPack spj_pack(const SPJRec &r, float eps2, int trace_mode) {
     SpjPack s;
     s.xh = __double2float_rn(r.pos[0]);
     s.yh = __double2float_rn(r.pos[1]);
@@ -1161,7 +1104,151 @@ __global__ void spj_pack_kernel(const SPJRec *__restrict__ in, int n, float eps2
     s.nqyz = -(3.0f * (float)r.yz);
     s.nqzx = -(3.0f * (float)r.xz);
     s.pad0 = s.pad1 = 0.f;
-    out[i] = s;
+    return s;
+}
+
+// Every record of a call in one launch: offsets, identity lists, packed bodies,
+// their FP32 splits and the packed superparticles.  The work is reading the
+// records, from host memory at the link's latency (about 2 us) and rate: a CTA
+// stages 128 records with 6 to 10 independent coalesced 8-byte loads a thread
+// (of an EPJ record the 64 of 112 bytes that are used), then each thread packs
+// one from shared memory.  A launch costs the host 4 us, so one launch in place
+// of up to seven (two packs, two splits, the superparticles, three identity
+// lists) is most of a small call: with the records read in place, 3,000 bodies
+// in two dispatches 400 -> 76 us, a group's two functor calls 235 -> 82 us.
+constexpr int PK = 128, PK_IDX = 1024;  // records, list entries per turn
+template <int W, int STRIDE>
+__device__ __forceinline__ const unsigned long long *stage_records(const void *src, int first, int nt,
+                                                                   unsigned long long *raw) {
+    const unsigned long long *in = (const unsigned long long *)src + (size_t)first * STRIDE;
+    __syncthreads();
+    unsigned long long v[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const int t = threadIdx.x + k * PK;
+        if (t < nt * W) v[k] = in[(t / W) * STRIDE + t % W];
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const int t = threadIdx.x + k * PK;
+        if (t < nt * W) raw[(t / W) * (W | 1) + t % W] = v[k];
+    }
+    __syncthreads();
+    return raw + threadIdx.x * (W | 1);
+}
+__device__ __forceinline__ double as_double(unsigned long long v) { return __longlong_as_double((long long)v); }
+
+__device__ __forceinline__ void copy_indices(const void *src, int first, int n, int *out) {
+    const int *in = (const int *)src;
+#pragma unroll
+    for (int k = 0; k < PK_IDX / PK; k++) {
+        const int t = first + threadIdx.x + k * PK;
+        if (t < n) out[t] = in[t];
+    }
+}
+
+__global__ void __launch_bounds__(PK) pack_walks_kernel(PackArgs A) {
+    __shared__ unsigned long long raw[PK * 11];
+    const int w = blockIdx.x / A.slices, slice = blockIdx.x % A.slices, tid = threadIdx.x;
+    const WalkRecords W = A.walk ? A.walk[w] : A.one;
+    if (A.i_off && slice == 0 && tid == 0) {
+        A.i_off[w] = W.io; A.j_off[w] = W.jo; A.s_off[w] = W.so;
+        if (w == A.n_walk - 1) {
+            A.i_off[w + 1] = W.io + W.ni; A.j_off[w + 1] = W.jo + W.nj; A.s_off[w + 1] = W.so + W.ns;
+        }
+    }
+    const int per = A.index ? PK_IDX : PK;
+    const int ci = W.ni / PK + (W.ni % PK != 0), cj = W.nj / per + (W.nj % per != 0), cs = W.ns / per + (W.ns % per != 0);
+    for (int c = slice; c < ci + cj + cs; c += A.slices) {
+        if (c < ci) {
+            const int first = c * PK, nt = min(PK, W.ni - first);
+            const unsigned long long *v = stage_records<6, 6>(W.epi, first, nt, raw);
+            if (tid < nt) {
+                const int o = W.io + first + tid;
+                const double ro = as_double(v[4]), rs = as_double(v[5]);
+                const SoftPtcl r = soft_ptcl(as_double(v[1]), as_double(v[2]), as_double(v[3]), 0.f, ro, rs,
+                                             (int)(unsigned)v[0], (int)(v[0] >> 32));
+                A.iptcl[o] = r;
+                if (A.isplit) A.isplit[o] = soft_split(r);
+                if (A.i_r_out) { A.i_r_out[o] = ro; A.i_r_search[o] = rs; }
+                if (A.i_idx) A.i_idx[o] = o;
+                if (A.acc64) {
+                    const ForceRec &f = A.seed[o];
+                    A.acc64[o] = D4c(f.acc[0], f.acc[1], f.acc[2], f.phi);
+                }
+            }
+        } else if (A.index) {
+            if (c < ci + cj) copy_indices(W.epj, (c - ci) * PK_IDX, W.nj, A.j_idx + W.jo);
+            else copy_indices(W.spj, (c - ci - cj) * PK_IDX, W.ns, A.s_idx + W.so);
+        } else if (c < ci + cj) {
+            const int first = (c - ci) * PK, nt = min(PK, W.nj - first);
+            const unsigned long long *v = stage_records<8, 14>(W.epj, first, nt, raw);
+            if (tid < nt) {
+                const int o = W.jo + first + tid;
+                const double ro = as_double(v[4]), rs = as_double(v[5]), m = as_double(v[7]);
+                const SoftPtcl r = soft_ptcl(as_double(v[1]), as_double(v[2]), as_double(v[3]), (float)m, ro, rs,
+                                             (int)(unsigned)v[0], (int)(v[0] >> 32));
+                A.ptcl[o] = r;
+                if (A.jsplit) A.jsplit[o] = soft_split(r);
+                if (A.mass) { A.mass[o] = m; A.r_out[o] = ro; A.r_search[o] = rs; }
+                if (A.j_idx) A.j_idx[o] = o;
+            }
+        } else {
+            const int first = (c - ci - cj) * PK, nt = min(PK, W.ns - first);
+            const unsigned long long *v = stage_records<10, 10>(W.spj, first, nt, raw);
+            if (tid < nt) {
+                const int o = W.so + first + tid;
+                SPJRec r;
+                r.mass = as_double(v[0]);
+                r.pos[0] = as_double(v[1]); r.pos[1] = as_double(v[2]); r.pos[2] = as_double(v[3]);
+                r.xx = as_double(v[4]); r.yy = as_double(v[5]); r.zz = as_double(v[6]);
+                r.xy = as_double(v[7]); r.xz = as_double(v[8]); r.yz = as_double(v[9]);
+                if (A.spj) A.spj[o] = r;
+                if (A.spjp) A.spjp[o] = spj_pack(r, A.eps2, A.trace_mode);
+                if (A.s_idx) A.s_idx[o] = o;
+            }
+        }
+    }
+    if (A.chk_i_off) {
+        for (long long g = (long long)blockIdx.x * PK + tid; g <= A.chk_groups; g += (long long)gridDim.x * PK) {
+            const int i1 = A.chk_i_off[g], j1 = A.chk_j_off[g], s1 = A.chk_s_off[g];
+            bool bad = g == 0 ? i1 != 0 || j1 != 0 || s1 != 0
+                              : i1 < A.chk_i_off[g - 1] || j1 < A.chk_j_off[g - 1] || s1 < A.chk_s_off[g - 1];
+            if (g == A.chk_groups) bad = bad || i1 > A.chk_n;
+            if (bad) {
+                atomicOr(A.gate, ST_BAD_INDEX);
+                atomicOr(A.status, ST_BAD_INDEX);
+            }
+        }
+    }
+}
+
+cudaError_t launch_pack_walks(const PackArgs &Ain, long long n_records, cudaStream_t st) {
+    PackArgs A = Ain;
+    if (A.n_walk <= 0) return cudaSuccess;
+    // CTAs: one per 128 records of an average walk and one for each of its
+    // three last turns, so that every turn's loads are in flight together
+    const long long turns = n_records / A.n_walk / PK + 3;
+    A.slices = (int)(turns > 16384 ? 16384 : turns);
+    if ((long long)A.slices * A.n_walk > 2147483647LL) A.slices = 1;
+    { P3T_COUNT_LAUNCH(); pack_walks_kernel<<<A.slices * A.n_walk, PK, 0, st>>>(A); }
+    return cudaGetLastError();
+}
+
+__global__ void split_kernel(const SoftPtcl *__restrict__ p, int n, SoftSplit *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = soft_split(p[i]);
+}
+
+__global__ void spj_pack_kernel(const SPJRec *__restrict__ in, int n, float eps2, int trace_mode, SpjPack *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = spj_pack(in[i], eps2, trace_mode);
+}
+
+cudaError_t launch_spj_pack(const SPJRec *in, int n, float eps2, int trace_mode, SpjPack *out, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    { P3T_COUNT_LAUNCH(); spj_pack_kernel<<<(n + 255) / 256, 256, 0, st>>>(in, n, eps2, trace_mode, out); }
+    return cudaGetLastError();
 }
 
 namespace {
@@ -1205,27 +1292,29 @@ cudaError_t launch_soft(const SoftArgs &Ain, int precision, bool emit, cudaStrea
         A.t_s2 = 32;
     }
     if (precision == 0) {
-        const bool same = A.iptcl == A.ptcl;
-        if (!A.jsplit || !A.spjp || (!same && !A.isplit)) {
-            int dev = 0;
-            cudaError_t e = cudaGetDevice(&dev);
+        if (!A.packed) {
+            const bool same = A.iptcl == A.ptcl;
+            if (!A.jsplit || !A.spjp || (!same && !A.isplit)) {
+                int dev = 0;
+                cudaError_t e = cudaGetDevice(&dev);
+                if (e != cudaSuccess) return e;
+                if (dev < 0 || dev >= MAX_DEV) return cudaErrorInvalidDevice;
+                std::lock_guard<std::mutex> lk(g_mixed_mu);
+                MixedScratch &m = g_mixed[dev];
+                if ((e = grow(&m.jsplit, &m.jcap, (size_t)A.n_ptcl, st)) != cudaSuccess) return e;
+                if ((e = grow(&m.spj, &m.scap, (size_t)(A.n_spj > 0 ? A.n_spj : 1), st)) != cudaSuccess) return e;
+                if (!same && (e = grow(&m.isplit, &m.icap, (size_t)A.n_iptcl, st)) != cudaSuccess) return e;
+                A.jsplit = m.jsplit;
+                A.spjp = m.spj;
+                A.isplit = m.isplit;
+            }
+            if (same) A.isplit = A.jsplit;
+            if (A.n_ptcl > 0) { P3T_COUNT_LAUNCH(); split_kernel<<<(A.n_ptcl + 255) / 256, 256, 0, st>>>(A.ptcl, A.n_ptcl, A.jsplit); }
+            if (!same && A.n_iptcl > 0)
+                { P3T_COUNT_LAUNCH(); split_kernel<<<(A.n_iptcl + 255) / 256, 256, 0, st>>>(A.iptcl, A.n_iptcl, A.isplit); }
+            const cudaError_t e = launch_spj_pack(A.spj, A.n_spj, A.eps2, A.trace_mode, A.spjp, st);
             if (e != cudaSuccess) return e;
-            if (dev < 0 || dev >= MAX_DEV) return cudaErrorInvalidDevice;
-            std::lock_guard<std::mutex> lk(g_mixed_mu);
-            MixedScratch &m = g_mixed[dev];
-            if ((e = grow(&m.jsplit, &m.jcap, (size_t)A.n_ptcl, st)) != cudaSuccess) return e;
-            if ((e = grow(&m.spj, &m.scap, (size_t)(A.n_spj > 0 ? A.n_spj : 1), st)) != cudaSuccess) return e;
-            if (!same && (e = grow(&m.isplit, &m.icap, (size_t)A.n_iptcl, st)) != cudaSuccess) return e;
-            A.jsplit = m.jsplit;
-            A.spjp = m.spj;
-            A.isplit = m.isplit;
         }
-        if (same) A.isplit = A.jsplit;
-        if (A.n_ptcl > 0) { P3T_COUNT_LAUNCH(); split_kernel<<<(A.n_ptcl + 255) / 256, 256, 0, st>>>(A.ptcl, A.n_ptcl, A.jsplit); }
-        if (!same && A.n_iptcl > 0)
-            { P3T_COUNT_LAUNCH(); split_kernel<<<(A.n_iptcl + 255) / 256, 256, 0, st>>>(A.iptcl, A.n_iptcl, A.isplit); }
-        if (A.n_spj > 0)
-            { P3T_COUNT_LAUNCH(); spj_pack_kernel<<<(A.n_spj + 255) / 256, 256, 0, st>>>(A.spj, A.n_spj, A.eps2, A.trace_mode, A.spjp); }
         const int occ = A.occ ? A.occ : 5;
 #define P3T_SOFT_MIXED(OCC)                                                                               \
     do {                                                                                                  \

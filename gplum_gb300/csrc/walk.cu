@@ -1,9 +1,9 @@
 // FDPS-facing entry points of the soft force: the single-group functor
 // calls and the multiwalk dispatch/retrieve pair (pointer and index forms).
-// They stage FDPS's per-walk arrays into the same device layout the
-// resident path uses and launch the same kernels.
+// The walks' arrays are read where FDPS has them, packed into the same device
+// layout the resident path uses, and go through the same kernels.
+#include <cstdint>
 #include <cstring>
-#include <vector>
 
 #include "../../include/gplum_p3t.h"
 #include "p3t_capi_internal.cuh"
@@ -14,70 +14,11 @@ using namespace p3t;
 
 namespace {
 
-DevSet g_fun;  // buffers of the single-group functor calls
-
-int set_offsets(Context *c, DevSet &d, int n_group, const std::vector<int> &io, const std::vector<int> &jo,
-                const std::vector<int> &so) {
-    int r = 0;
-    if ((r = d.i_off.reserve(n_group + 1)) || (r = d.j_off.reserve(n_group + 1)) || (r = d.s_off.reserve(n_group + 1)))
-        return r;
-    if ((r = h2d(c, d.i_off.p, io.data(), io.size() * sizeof(int)))) return r;
-    if ((r = h2d(c, d.j_off.p, jo.data(), jo.size() * sizeof(int)))) return r;
-    return h2d(c, d.s_off.p, so.data(), so.size() * sizeof(int));
-}
-
-// Functor call: one group, accumulate into the caller's ForceGrav records.
-int functor_call(const void *epi, int ni, const void *epj, int nj, const void *spj, int ns, void *force) {
-    Context *c = ctx_get(0);
-    if (!c) return -(int)cudaErrorNoDevice;
-    if (ni <= 0) return 0;
-    if (!epi || !force || nj < 0 || ns < 0 || (nj > 0 && !epj) || (ns > 0 && !spj)) return ST_BAD_INDEX;
-    DevSet &d = g_fun;
-    int r = 0;
-    if ((r = d.epi_stage.reserve(ni)) || (r = d.iptcl.reserve(ni)) || (r = d.i_r_out.reserve(ni)) ||
-        (r = d.i_r_search.reserve(ni)) || (r = d.epj_stage.reserve(nj)) || (r = d.ptcl.reserve(nj)) ||
-        (r = d.mass.reserve(nj)) || (r = d.r_out.reserve(nj)) || (r = d.r_search.reserve(nj)) ||
-        (r = d.spj.reserve(ns)) || (r = d.i_idx.reserve(ni)) || (r = d.j_idx.reserve(nj)) ||
-        (r = d.s_idx.reserve(ns)) || (r = d.force.reserve(ni)) || (r = d.acc64.reserve(ni)))
-        return r;
-    if ((r = h2d(c, d.epi_stage.p, epi, (size_t)ni * sizeof(EPIRec)))) return r;
-    if (nj && (r = h2d(c, d.epj_stage.p, epj, (size_t)nj * sizeof(EPJRec)))) return r;
-    if (ns && (r = h2d(c, d.spj.p, spj, (size_t)ns * sizeof(SPJRec)))) return r;
-    if ((r = h2d(c, d.force.p, force, (size_t)ni * sizeof(ForceRec)))) return r;
-    std::vector<int> io = {0, ni}, jo = {0, nj}, so = {0, ns};
-    if ((r = set_offsets(c, d, 1, io, jo, so))) return r;
-    if ((r = cuda_status(launch_pack_epi((const EPIRec *)d.epi_stage.p, ni, d.iptcl.p, d.i_r_out.p, d.i_r_search.p,
-                                         c->stream))))
-        return r;
-    if ((r = cuda_status(launch_pack_epj(d.epj_stage.p, nj, d.ptcl.p, d.mass.p, d.r_out.p, d.r_search.p, c->stream))))
-        return r;
-    if ((r = cuda_status(launch_iota(d.i_idx.p, ni, 0, c->stream))) ||
-        (r = cuda_status(launch_iota(d.j_idx.p, nj, 0, c->stream))) ||
-        (r = cuda_status(launch_iota(d.s_idx.p, ns, 0, c->stream))))
-        return r;
-    d.order_valid = false;
-    SoftArgs A = make_args(c, d, 1, nj, ns, true);
-    A.iptcl = d.iptcl.p; A.i_r_out = d.i_r_out.p; A.i_r_search = d.i_r_search.p; A.n_iptcl = ni;
-    A.cand = nullptr;
-    if (c->precision == 1) {
-        // FP64 form accumulates in double: seed it from the caller's records
-        std::vector<D4> seed(ni);
-        const ForceRec *f = (const ForceRec *)force;
-        for (int k = 0; k < ni; k++) seed[k] = D4c(f[k].acc[0], f[k].acc[1], f[k].acc[2], f[k].phi);
-        if ((r = h2d(c, d.acc64.p, seed.data(), ni * sizeof(D4)))) return r;
-    }
-    if ((r = cuda_status(launch_soft(A, c->precision, false, c->stream)))) return r;
-    if ((r = cuda_status(cudaMemcpyAsync(force, d.force.p, (size_t)ni * sizeof(ForceRec), cudaMemcpyDeviceToHost,
-                                         c->stream))))
-        return r;
-    if ((r = cuda_status(cudaStreamSynchronize(c->stream)))) return r;
-    return read_status(c);
-}
-
 WalkSlot *slot_for(Context *c, int tag) {
     if (tag < 0) return nullptr;
     WalkSlot &w = c->walk[tag % MAX_TAGS];
     if (!w.done && cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+    if (!w.read && cudaEventCreateWithFlags(&w.read, cudaEventDisableTiming) != cudaSuccess) return nullptr;
     return &w;
 }
 
@@ -93,50 +34,173 @@ int check_walks(int n_walk, const int *cnt, const void *const *ptr) {
     return tot > 2147483647LL ? ST_BAD_INDEX : 0;
 }
 
-// Common tail of both dispatch forms: kernel, download, event.
-int launch_walks(Context *c, WalkSlot &w, int n_walk, int n_i, const SoftPtcl *jptcl, const double *jmass,
-                 const double *jro, const double *jrs, int n_j, const SPJRec *spj, int n_s) {
-    DevSet &d = w.d;
+// A call's walks in the slot's pinned table, which the kernels read.
+struct WalkTable {
+    WalkSlot &w;
+    int n_walk;
+    size_t size_j, size_s;  // bytes of an EPJ and SPJ entry (records or indices)
+    int ni = 0, nj = 0, ns = 0;
+    bool staged = false;  // the records lie in the slot's pinned buffer, not where the caller has them
+
+    int *status() const { return (int *)w.h_tab; }
+    WalkRecords *rec() const { return (WalkRecords *)((char *)w.h_tab + 64); }
+
+    int reserve() { return grow_host(&w.h_tab, &w.h_tab_cap, 64 + (size_t)n_walk * sizeof(WalkRecords)); }
+    void set(int k, const void *epi, int n_i, const void *epj, int n_j, const void *spj, int n_s) {
+        rec()[k] = WalkRecords{(const EPIRec *)epi, epj, spj, n_i, n_j, n_s, ni, nj, ns};
+        ni += n_i; nj += n_j; ns += n_s;
+    }
+    // Where the records are read.  The kernel reads them in the caller's memory
+    // where the device can (60,000 bodies in the index form, four dispatches: the
+    // host's copies into pinned buffers, 14-24 GB/s, were 1.2 of a pass's 1.5 ms;
+    // the link gives 150-200 GB/s; now 0.36 ms) and they are aligned as the kernel reads them;
+    // otherwise they are first copied into the slot's pinned buffer.
+    int place(bool reads_host) {
+        uintptr_t bits = 0;
+        for (int k = 0; k < n_walk; k++) {
+            const WalkRecords &r = rec()[k];
+            if (r.ni) bits |= (uintptr_t)r.epi;
+            if (r.nj) bits |= (uintptr_t)r.epj << (size_j < 8);
+            if (r.ns) bits |= (uintptr_t)r.spj << (size_s < 8);
+        }
+        if (reads_host && (bits & 7) == 0) return 0;
+        staged = true;
+        const size_t need = (size_t)ni * sizeof(EPIRec) + (size_t)nj * size_j + (size_t)ns * size_s + 16;
+        const int r = grow_host(&w.h_in, &w.h_in_cap, need);
+        if (r) return r;
+        char *h = (char *)w.h_in;
+        auto put = [&](const void *src, size_t bytes) {
+            char *to = h;
+            if (bytes) std::memcpy(h, src, bytes);
+            h += bytes;
+            return to;
+        };
+        // records of one kind after another: the 8-byte ones first
+        for (int k = 0; k < n_walk; k++) rec()[k].epi = (const EPIRec *)put(rec()[k].epi, (size_t)rec()[k].ni * sizeof(EPIRec));
+        for (int k = 0; k < n_walk; k++) rec()[k].epj = put(rec()[k].epj, (size_t)rec()[k].nj * size_j);
+        for (int k = 0; k < n_walk; k++) rec()[k].spj = put(rec()[k].spj, (size_t)rec()[k].ns * size_s);
+        return 0;
+    }
+};
+
+// Device arrays of a call's i-bodies and lists, and the pack arguments that fill them.
+int pack_args(Context *c, WalkTable &t, bool index, PackArgs &A) {
+    DevSet &d = t.w.d;
+    const bool f64 = c->precision == 1;
     int r = 0;
-    if ((r = d.force.reserve(n_i)) || (r = d.acc64.reserve(n_i))) return r;
-    d.order_valid = false;
-    SoftArgs A = make_args(c, d, n_walk, n_j, n_s, false);
-    A.ptcl = jptcl; A.mass = jmass; A.r_out = jro; A.r_search = jrs; A.n_ptcl = n_j;
-    A.spj = spj; A.n_spj = n_s;
-    A.iptcl = d.iptcl.p; A.i_r_out = d.i_r_out.p; A.i_r_search = d.i_r_search.p; A.n_iptcl = n_i;
-    A.cand = nullptr;
-    if ((r = cuda_status(launch_soft(A, c->precision, false, c->stream)))) return r;
-    if ((r = grow_host(&w.h_out, &w.h_out_cap, (size_t)n_i * sizeof(ForceRec)))) return r;
-    if ((r = cuda_status(cudaMemcpyAsync(w.h_out, d.force.p, (size_t)n_i * sizeof(ForceRec), cudaMemcpyDeviceToHost,
-                                         c->stream))))
+    if ((r = d.i_off.reserve(t.n_walk + 1)) || (r = d.j_off.reserve(t.n_walk + 1)) ||
+        (r = d.s_off.reserve(t.n_walk + 1)) || (r = d.i_idx.reserve(t.ni)) || (r = d.j_idx.reserve(t.nj)) ||
+        (r = d.s_idx.reserve(t.ns)) || (r = d.iptcl.reserve(t.ni)))
         return r;
-    if ((r = cuda_status(cudaEventRecord(w.done, c->stream)))) return r;
-    w.n_i = n_i;
-    w.busy = true;
+    A = PackArgs{};
+    A.walk = t.rec();
+    A.n_walk = t.n_walk;
+    A.index = index;
+    A.i_off = d.i_off.p; A.j_off = d.j_off.p; A.s_off = d.s_off.p;
+    A.i_idx = d.i_idx.p; A.j_idx = d.j_idx.p; A.s_idx = d.s_idx.p;
+    A.iptcl = d.iptcl.p;
+    A.eps2 = (float)c->params[0];
+    A.trace_mode = c->trace_mode;
+    if (f64) {
+        if ((r = d.i_r_out.reserve(t.ni)) || (r = d.i_r_search.reserve(t.ni))) return r;
+        A.i_r_out = d.i_r_out.p; A.i_r_search = d.i_r_search.p;
+    } else {
+        if ((r = d.isplit.reserve(t.ni))) return r;
+        A.isplit = d.isplit.p;
+    }
+    if (index) return 0;
+    if ((r = d.ptcl.reserve(t.nj))) return r;
+    A.ptcl = d.ptcl.p;
+    if (f64) {
+        if ((r = d.mass.reserve(t.nj)) || (r = d.r_out.reserve(t.nj)) || (r = d.r_search.reserve(t.nj)) ||
+            (r = d.spj.reserve(t.ns)))
+            return r;
+        A.mass = d.mass.p; A.r_out = d.r_out.p; A.r_search = d.r_search.p;
+        A.spj = d.spj.p;
+    } else {
+        if ((r = d.jsplit.reserve(t.nj)) || (r = d.spjp.reserve(t.ns))) return r;
+        A.jsplit = d.jsplit.p;
+        A.spjp = d.spjp.p;
+    }
     return 0;
 }
 
-// Gathers the walks' EPI records into slot staging and onto the device.
-int stage_epi(Context *c, WalkSlot &w, int n_walk, const void **epi, const int *n_epi, int &n_i) {
-    n_i = 0;
-    for (int k = 0; k < n_walk; k++) n_i += n_epi[k];
-    DevSet &d = w.d;
+// The soft kernel over packed walks: the j side from x (the slot's own arrays, or
+// the resident ones of the index form), the forces into the slot's pinned buffer.
+SoftArgs walk_args(Context *c, WalkTable &t, DevSet &x, int n_j, int n_s, bool accumulate) {
+    DevSet &d = t.w.d;
+    d.order_valid = false;
+    SoftArgs A = make_args(c, d, t.n_walk, n_j, n_s, accumulate);
+    A.ptcl = x.ptcl.p; A.mass = x.mass.p; A.r_out = x.r_out.p; A.r_search = x.r_search.p;
+    A.spj = x.spj.p;
+    A.iptcl = d.iptcl.p; A.i_r_out = d.i_r_out.p; A.i_r_search = d.i_r_search.p; A.n_iptcl = t.ni;
+    A.isplit = d.isplit.p; A.jsplit = x.jsplit.p; A.spjp = x.spjp.p;
+    A.packed = 1;
+    A.force = (ForceRec *)t.w.h_out;
+    A.cand = nullptr;
+    return A;
+}
+
+// Functor call: one group, accumulate into the caller's ForceGrav records.  Two
+// launches and one wait; the pack kernel reads the records where they are.
+int functor_call(const void *epi, int ni, const void *epj, int nj, const void *spj, int ns, void *force) {
+    Context *c = ctx_get(0);
+    if (!c) return -(int)cudaErrorNoDevice;
+    if (ni <= 0) return 0;
+    if (!epi || !force || nj < 0 || ns < 0 || (nj > 0 && !epj) || (ns > 0 && !spj)) return ST_BAD_INDEX;
+    WalkSlot &w = c->fun;
+    WalkTable t{w, 1, sizeof(EPJRec), sizeof(SPJRec)};
+    const size_t bytes = (size_t)ni * sizeof(ForceRec);
     int r = 0;
-    if ((r = d.epi_stage.reserve(n_i)) || (r = d.iptcl.reserve(n_i)) || (r = d.i_r_out.reserve(n_i)) ||
-        (r = d.i_r_search.reserve(n_i)) || (r = d.i_idx.reserve(n_i)))
-        return r;
-    if ((r = grow_host(&w.h_in, &w.h_in_cap, (size_t)n_i * sizeof(EPIRec)))) return r;
-    char *h = (char *)w.h_in;
-    for (int k = 0; k < n_walk; k++) {
-        std::memcpy(h, epi[k], (size_t)n_epi[k] * sizeof(EPIRec));
-        h += (size_t)n_epi[k] * sizeof(EPIRec);
+    if ((r = t.reserve()) || (r = grow_host(&w.h_out, &w.h_out_cap, bytes)) || (r = w.d.acc64.reserve(ni))) return r;
+    t.set(0, epi, ni, epj, nj, spj, ns);
+    PackArgs K;
+    if ((r = t.place(c->reads_host)) || (r = pack_args(c, t, false, K))) return r;
+    std::memcpy(w.h_out, force, bytes);
+    if (c->precision == 1) {
+        // FP64 form accumulates in double: seed it from the caller's records
+        K.seed = (const ForceRec *)w.h_out;
+        K.acc64 = w.d.acc64.p;
     }
-    if ((r = cuda_status(cudaMemcpyAsync(d.epi_stage.p, w.h_in, (size_t)n_i * sizeof(EPIRec), cudaMemcpyHostToDevice,
-                                         c->stream))))
+    if (!(r = cuda_status(launch_pack_walks(K, (long long)ni + nj + ns, c->stream))) &&
+        !(r = cuda_status(launch_soft(walk_args(c, t, w.d, nj, ns, true), c->precision, false, c->stream))))
+        r = cuda_status(cudaMemcpyAsync(t.status(), c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    // also after an error: nothing of this call may still read the caller's records
+    const int e = cuda_status(cudaStreamSynchronize(c->stream));
+    if (r || e) return r ? r : e;
+    std::memcpy(force, w.h_out, bytes);
+    return *t.status() ? read_status(c) : 0;
+}
+
+// Common tail of both dispatch forms: kernel, status copy, event.  Returns once
+// the caller's records have been read (in_place: by the kernels, where they are).
+int launch_walks(Context *c, WalkTable &t, const PackArgs &K, DevSet &x, int n_j, int n_s, long long n_records,
+                 bool in_place) {
+    WalkSlot &w = t.w;
+    int r = 0;
+    auto run = [&]() {
+        int e = 0;
+        if ((e = cuda_status(launch_pack_walks(K, n_records, c->stream)))) return e;
+        if ((e = cuda_status(cudaEventRecord(w.read, c->stream)))) return e;
+        if ((e = cuda_status(launch_soft(walk_args(c, t, x, n_j, n_s, false), c->precision, false, c->stream)))) return e;
+        if ((e = cuda_status(cudaMemcpyAsync(t.status(), c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream))))
+            return e;
+        return cuda_status(cudaEventRecord(w.done, c->stream));
+    };
+    if ((r = run())) {
+        cudaStreamSynchronize(c->stream);
         return r;
-    if ((r = cuda_status(launch_pack_epi(d.epi_stage.p, n_i, d.iptcl.p, d.i_r_out.p, d.i_r_search.p, c->stream))))
-        return r;
-    return cuda_status(launch_iota(d.i_idx.p, n_i, 0, c->stream));
+    }
+    w.n_i = t.ni;
+    w.busy = true;
+    return in_place ? cuda_status(cudaEventSynchronize(w.read)) : 0;
+}
+
+// A dispatch's slot, free of earlier work (a skipped retrieve: the slot is reused in order).
+int claim_slot(WalkSlot &w) {
+    if (!w.busy) return 0;
+    w.busy = false;
+    return cuda_status(cudaEventSynchronize(w.done));
 }
 
 }  // namespace
@@ -160,52 +224,19 @@ int p3t_soft_dispatch(int tag, int n_walk, const void **epi, const int *n_epi, c
     Context *c = ctx_get(0);
     if (!c) return -(int)cudaErrorNoDevice;
     WalkSlot *ws = slot_for(c, tag);
-    if (!ws || n_walk < 0) return ST_BAD_INDEX;
+    if (!ws) return ST_BAD_INDEX;
     WalkSlot &w = *ws;
-    if (w.busy) cudaEventSynchronize(w.done);  // a retrieve was skipped: the slot is reused in order
-    if (w.busy) w.busy = false;
-    int r = 0, n_i = 0;
-    // wait for any earlier use of this slot's pinned buffers
-    if ((r = cuda_status(cudaStreamSynchronize(c->stream)))) return r;
-    if ((r = stage_epi(c, w, n_walk, epi, n_epi, n_i))) return r;
-    int n_j = 0, n_s = 0;
-    std::vector<int> io(n_walk + 1), jo(n_walk + 1), so(n_walk + 1);
-    io[0] = jo[0] = so[0] = 0;
-    for (int k = 0; k < n_walk; k++) {
-        io[k + 1] = io[k] + n_epi[k];
-        jo[k + 1] = jo[k] + n_epj[k];
-        so[k + 1] = so[k] + n_spj[k];
-    }
-    n_j = jo[n_walk];
-    n_s = so[n_walk];
-    DevSet &d = w.d;
-    if ((r = d.epj_stage.reserve(n_j)) || (r = d.ptcl.reserve(n_j)) || (r = d.mass.reserve(n_j)) ||
-        (r = d.r_out.reserve(n_j)) || (r = d.r_search.reserve(n_j)) || (r = d.spj.reserve(n_s)) ||
-        (r = d.j_idx.reserve(n_j)) || (r = d.s_idx.reserve(n_s)))
+    WalkTable t{w, n_walk, sizeof(EPJRec), sizeof(SPJRec)};
+    int r = 0;
+    if ((r = claim_slot(w)) || (r = t.reserve())) return r;
+    for (int k = 0; k < n_walk; k++)
+        t.set(k, n_epi[k] ? epi[k] : nullptr, n_epi[k], n_epj[k] ? epj[k] : nullptr, n_epj[k], n_spj[k] ? spj[k] : nullptr,
+              n_spj[k]);
+    PackArgs K;
+    if ((r = t.place(c->reads_host)) || (r = pack_args(c, t, false, K)) || (r = w.d.acc64.reserve(t.ni)) ||
+        (r = grow_host(&w.h_out, &w.h_out_cap, (size_t)t.ni * sizeof(ForceRec))))
         return r;
-    // EPJ and SPJ records of every walk, concatenated (pageable sources are
-    // staged by h2d)
-    {
-        std::vector<char> cat((size_t)n_j * sizeof(EPJRec) + (size_t)n_s * sizeof(SPJRec));
-        char *h = cat.data();
-        for (int k = 0; k < n_walk; k++) {
-            std::memcpy(h, epj[k], (size_t)n_epj[k] * sizeof(EPJRec));
-            h += (size_t)n_epj[k] * sizeof(EPJRec);
-        }
-        char *hs = h;
-        for (int k = 0; k < n_walk; k++) {
-            std::memcpy(h, spj[k], (size_t)n_spj[k] * sizeof(SPJRec));
-            h += (size_t)n_spj[k] * sizeof(SPJRec);
-        }
-        if (n_j && (r = h2d(c, d.epj_stage.p, cat.data(), (size_t)n_j * sizeof(EPJRec)))) return r;
-        if (n_s && (r = h2d(c, d.spj.p, hs, (size_t)n_s * sizeof(SPJRec)))) return r;
-    }
-    if ((r = set_offsets(c, d, n_walk, io, jo, so))) return r;
-    if ((r = cuda_status(launch_pack_epj(d.epj_stage.p, n_j, d.ptcl.p, d.mass.p, d.r_out.p, d.r_search.p, c->stream))) ||
-        (r = cuda_status(launch_iota(d.j_idx.p, n_j, 0, c->stream))) ||
-        (r = cuda_status(launch_iota(d.s_idx.p, n_s, 0, c->stream))))
-        return r;
-    return launch_walks(c, w, n_walk, n_i, d.ptcl.p, d.mass.p, d.r_out.p, d.r_search.p, n_j, d.spj.p, n_s);
+    return launch_walks(c, t, K, w.d, t.nj, t.ns, (long long)t.ni + t.nj + t.ns, !t.staged);
 }
 
 int p3t_soft_dispatch_index(int tag, int n_walk, const void **epi, const int *n_epi, const int **id_epj,
@@ -220,47 +251,62 @@ int p3t_soft_dispatch_index(int tag, int n_walk, const void **epi, const int *n_
     Context *c = ctx_get(0);
     if (!c) return -(int)cudaErrorNoDevice;
     WalkSlot *ws = slot_for(c, tag);
-    if (!ws || n_walk < 0) return ST_BAD_INDEX;
+    if (!ws) return ST_BAD_INDEX;
     WalkSlot &w = *ws;
+    WalkTable t{w, n_walk, sizeof(int), sizeof(int)};
     int r = 0;
-    if ((r = cuda_status(cudaStreamSynchronize(c->stream)))) return r;
-    w.busy = false;
+    if ((r = claim_slot(w))) return r;
     DevSet &x = c->idx;
+    bool in_place = false;
     if (send_flag) {
-        if ((r = x.epj_stage.reserve(n_epj_tot)) || (r = x.ptcl.reserve(n_epj_tot)) || (r = x.mass.reserve(n_epj_tot)) ||
-            (r = x.r_out.reserve(n_epj_tot)) || (r = x.r_search.reserve(n_epj_tot)) || (r = x.spj.reserve(n_spj_tot)))
+        // resident for the dispatches that follow, which may switch the
+        // precision: the arrays of both forms
+        if ((r = x.ptcl.reserve(n_epj_tot)) || (r = x.mass.reserve(n_epj_tot)) || (r = x.r_out.reserve(n_epj_tot)) ||
+            (r = x.r_search.reserve(n_epj_tot)) || (r = x.jsplit.reserve(n_epj_tot)) ||
+            (r = x.spj.reserve(n_spj_tot)) || (r = x.spjp.reserve(n_spj_tot)))
             return r;
-        if (n_epj_tot && (r = h2d(c, x.epj_stage.p, epj, (size_t)n_epj_tot * sizeof(EPJRec)))) return r;
-        if (n_spj_tot && (r = h2d(c, x.spj.p, spj, (size_t)n_spj_tot * sizeof(SPJRec)))) return r;
-        if ((r = cuda_status(launch_pack_epj(x.epj_stage.p, n_epj_tot, x.ptcl.p, x.mass.p, x.r_out.p, x.r_search.p,
-                                             c->stream))))
-            return r;
+        WalkTable s{w, 1, sizeof(EPJRec), sizeof(SPJRec)};
+        if ((r = s.reserve())) return r;
+        s.set(0, nullptr, 0, n_epj_tot ? epj : nullptr, n_epj_tot, n_spj_tot ? spj : nullptr, n_spj_tot);
+        if ((r = s.place(c->reads_host))) return r;
+        PackArgs K{};
+        K.one = s.rec()[0];
+        K.n_walk = 1;
+        K.ptcl = x.ptcl.p; K.mass = x.mass.p; K.r_out = x.r_out.p; K.r_search = x.r_search.p;
+        K.jsplit = x.jsplit.p;
+        K.spj = x.spj.p; K.spjp = x.spjp.p;
+        K.eps2 = (float)c->params[0];
+        K.trace_mode = c->trace_mode;
+        if ((r = cuda_status(launch_pack_walks(K, (long long)n_epj_tot + n_spj_tot, c->stream)))) return r;
+        // the walks' records may take the same pinned buffer, and an early
+        // return leaves nothing reading the caller's arrays
+        if (s.staged && (r = cuda_status(cudaStreamSynchronize(c->stream)))) return r;
+        in_place = !s.staged;
         c->idx_nj = n_epj_tot;
         c->idx_ns = n_spj_tot;
+        c->idx_eps2 = K.eps2;
+        c->idx_trace = K.trace_mode;
+    } else if (c->idx_ns > 0 && (c->idx_eps2 != (float)c->params[0] || c->idx_trace != c->trace_mode)) {
+        c->idx_eps2 = (float)c->params[0];
+        c->idx_trace = c->trace_mode;
+        if ((r = cuda_status(launch_spj_pack(x.spj.p, c->idx_ns, c->idx_eps2, c->idx_trace, x.spjp.p, c->stream)))) return r;
     }
-    int n_i = 0;
-    if ((r = stage_epi(c, w, n_walk, epi, n_epi, n_i))) return r;
-    std::vector<int> io(n_walk + 1), jo(n_walk + 1), so(n_walk + 1);
-    io[0] = jo[0] = so[0] = 0;
-    for (int k = 0; k < n_walk; k++) {
-        io[k + 1] = io[k] + n_epi[k];
-        jo[k + 1] = jo[k] + n_epj[k];
-        so[k + 1] = so[k] + n_spj[k];
+    PackArgs K;
+    auto walks = [&]() {
+        int f = 0;
+        if ((f = t.reserve())) return f;
+        for (int k = 0; k < n_walk; k++)
+            t.set(k, n_epi[k] ? epi[k] : nullptr, n_epi[k], n_epj[k] ? id_epj[k] : nullptr, n_epj[k],
+                  n_spj[k] ? id_spj[k] : nullptr, n_spj[k]);
+        if ((f = t.place(c->reads_host)) || (f = pack_args(c, t, true, K)) || (f = w.d.acc64.reserve(t.ni))) return f;
+        return grow_host(&w.h_out, &w.h_out_cap, (size_t)t.ni * sizeof(ForceRec));
+    };
+    if ((r = walks())) {
+        cudaStreamSynchronize(c->stream);
+        return r;
     }
-    DevSet &d = w.d;
-    if ((r = d.j_idx.reserve(jo[n_walk])) || (r = d.s_idx.reserve(so[n_walk]))) return r;
-    {
-        std::vector<int> jl(jo[n_walk]), sl(so[n_walk]);
-        for (int k = 0; k < n_walk; k++) {
-            if (n_epj[k]) std::memcpy(jl.data() + jo[k], id_epj[k], n_epj[k] * sizeof(int));
-            if (n_spj[k]) std::memcpy(sl.data() + so[k], id_spj[k], n_spj[k] * sizeof(int));
-        }
-        if (!jl.empty() && (r = h2d(c, d.j_idx.p, jl.data(), jl.size() * sizeof(int)))) return r;
-        if (!sl.empty() && (r = h2d(c, d.s_idx.p, sl.data(), sl.size() * sizeof(int)))) return r;
-    }
-    if ((r = set_offsets(c, d, n_walk, io, jo, so))) return r;
-    return launch_walks(c, w, n_walk, n_i, x.ptcl.p, x.mass.p, x.r_out.p, x.r_search.p, c->idx_nj, x.spj.p,
-                        c->idx_ns);
+    return launch_walks(c, t, K, x, c->idx_nj, c->idx_ns, t.ni + ((long long)t.nj + t.ns) / 8,
+                        in_place || !t.staged);
 }
 
 int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
@@ -279,7 +325,9 @@ int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
         std::memcpy(force[k], h + off, (size_t)n_epi[k] * sizeof(ForceRec));
         off += n_epi[k];
     }
-    return read_status(c);
+    // the status word as it was behind this dispatch's kernel; the word itself
+    // is read, and cleared, only where that was not zero
+    return *(const int *)w.h_tab ? read_status(c) : 0;
 }
 
 }  // extern "C"

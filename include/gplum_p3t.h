@@ -458,7 +458,7 @@ int p3t_hard_launch_stats(double *launch_ms, long long *pairs3, double *sums5);
  * word back), so it cannot be made on a stream under CUDA-graph capture.  The
  * offsets are checked on the device before any list is read (each starts at
  * 0 and never decreases; i_off[n_group] <= n): a violation returns status 2
- * and runs no force kernel; out-of-range list entries are clamped and also
+ * and writes no force; out-of-range list entries are clamped and also
  * return 2.  All calls share the scratch: calls that overlap on the GPU race
  * and must be serialised by the caller.  The launch shape is the one
  * p3t_set_soft_tiles / p3t_set_soft_occupancy set. */
