@@ -1,10 +1,9 @@
 // C ABI of the P3T soft-force path (declarations and contracts in
 // include/gplum_p3t.h).  One process-wide context bound to one GPU.
-#include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 #include "../../include/gplum_p3t.h"
 #include "p3t_capi_internal.cuh"
@@ -121,62 +120,47 @@ bool is_pinned(const void *p) {
     return a.type == cudaMemoryTypeHost;
 }
 
-// Host->device uploads issued as one batch: pinned sources are copied by the
-// DMA engine directly, pageable ones are first gathered into the context's
-// pinned staging buffer.  flush() waits for the copies, so the caller's and
-// the staging buffers may be reused afterwards.
-struct Uploader {
-    Context *c;
-    struct Item { void *dst; const void *src; size_t bytes; bool pinned; };
-    std::vector<Item> items;
-    explicit Uploader(Context *cc) : c(cc) {}
-    void add(void *dst, const void *src, size_t bytes) {
-        if (bytes) items.push_back({dst, src, bytes, is_pinned(src)});
+// Host memory that a kernel may read in place at `align` bytes.
+static bool device_reads(Context *c, const void *p, size_t align) {
+    if ((uintptr_t)p % align) return false;
+    if (c->reads_host) return true;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    // queues the copies; returns once they are on the stream (the caller's
-    // pinned sources and the staging buffer must stay untouched until the
-    // stream has run them)
-    int issue() {
-        size_t stage = 0;
-        for (auto &it : items)
-            if (!it.pinned) stage += (it.bytes + 255) / 256 * 256;
-        int r = grow_host(&c->h_stage, &c->h_stage_cap, stage);
-        if (r) return r;
-        char *h = (char *)c->h_stage;
-        for (auto &it : items) {
-            const void *src = it.src;
-            if (!it.pinned) {
-                std::memcpy(h, it.src, it.bytes);
-                src = h;
-                h += (it.bytes + 255) / 256 * 256;
-            }
-            r = cuda_status(cudaMemcpyAsync(it.dst, src, it.bytes, cudaMemcpyHostToDevice, c->stream));
-            if (r) return r;
+    return a.type == cudaMemoryTypeHost && a.devicePointer == p;
+}
+
+void Uploader::add(void *dst, const void *src, size_t bytes) {
+    if (bytes) items.push_back({dst, src, bytes, c->reads_host || is_pinned(src)});
+}
+
+int Uploader::issue() {
+    size_t stage = 0;
+    for (auto &it : items)
+        if (!it.direct) stage += (it.bytes + 255) / 256 * 256;
+    int r = grow_host(&c->h_stage, &c->h_stage_cap, stage);
+    if (r) return r;
+    char *h = (char *)c->h_stage;
+    for (auto &it : items) {
+        const void *src = it.src;
+        if (!it.direct) {
+            std::memcpy(h, it.src, it.bytes);
+            src = h;
+            h += (it.bytes + 255) / 256 * 256;
         }
-        items.clear();
-        return 0;
-    }
-    int flush() {
-        size_t stage = 0;
-        for (auto &it : items)
-            if (!it.pinned) stage += (it.bytes + 255) / 256 * 256;
-        int r = grow_host(&c->h_stage, &c->h_stage_cap, stage);
+        r = cuda_status(cudaMemcpyAsync(it.dst, src, it.bytes, cudaMemcpyHostToDevice, c->stream));
         if (r) return r;
-        char *h = (char *)c->h_stage;
-        for (auto &it : items) {
-            const void *src = it.src;
-            if (!it.pinned) {
-                std::memcpy(h, it.src, it.bytes);
-                src = h;
-                h += (it.bytes + 255) / 256 * 256;
-            }
-            r = cuda_status(cudaMemcpyAsync(it.dst, src, it.bytes, cudaMemcpyHostToDevice, c->stream));
-            if (r) return r;
-        }
-        items.clear();
-        return cuda_status(cudaStreamSynchronize(c->stream));
     }
-};
+    items.clear();
+    return 0;
+}
+
+int Uploader::flush() {
+    const int r = issue(), e = cuda_status(cudaStreamSynchronize(c->stream));
+    return r ? r : e;
+}
 
 int d2h(Context *c, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return 0;
@@ -220,42 +204,21 @@ SoftArgs make_args(Context *c, DevSet &d, int n_group, int n_ptcl, int n_spj, bo
     return A;
 }
 
-// The staged EPJ records of a resident problem -> the soft kernels' arrays.
-static cudaError_t pack_bodies(Context *c, DevSet &d, int n) {
-    if (n <= 0) return cudaSuccess;
+// The EPJ records of a resident problem -> the soft kernels' arrays, read where
+// the caller has them if the device can, otherwise from the staged copy that
+// `u` (issued first) makes.  The caller waits for the stream before it returns.
+static const void *place(Context *c, Uploader &u, void *stage, const void *src, size_t bytes) {
+    if (device_reads(c, src, 8)) return src;
+    u.add(stage, src, bytes);
+    return stage;
+}
+static PackArgs pack_resident(DevSet &d, int n, const void *epj) {
     PackArgs A{};
-    A.one.epj = d.epj_stage.p;
+    A.one.epj = epj;
     A.one.nj = n;
     A.n_walk = 1;
     A.ptcl = d.ptcl.p; A.mass = d.mass.p; A.r_out = d.r_out.p; A.r_search = d.r_search.p;
-    return launch_pack_walks(A, n, c->stream);
-}
-
-// Launch order: largest groups first (less tail imbalance).
-// launch order of the groups: most pair work first (i-slots in whole warps x
-// list entries, a superparticle counted twice)
-static void group_order_host(int n_group, const int *i_off_h, const int *j_off_h, const int *s_off_h, int *ord) {
-    std::vector<std::pair<long long, int>> w(n_group);
-    for (int g = 0; g < n_group; g++) {
-        const long long ni = i_off_h[g + 1] - i_off_h[g];
-        const long long nj = (j_off_h[g + 1] - j_off_h[g]) + 2LL * (s_off_h[g + 1] - s_off_h[g]);
-        w[g] = {-(((ni + 31) / 32) * 32 * nj), g};
-    }
-    std::sort(w.begin(), w.end());
-    for (int g = 0; g < n_group; g++) ord[g] = w[g].second;
-}
-
-int set_group_order(Context *c, DevSet &d, int n_group, const int *i_off_h, const int *j_off_h,
-                           const int *s_off_h) {
-    std::vector<int> ord(n_group);
-    group_order_host(n_group, i_off_h, j_off_h, s_off_h, ord.data());
-    int r = d.order.reserve((size_t)n_group);
-    if (r) return r;
-    r = cuda_status(cudaMemcpyAsync(d.order.p, ord.data(), n_group * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    if (r) return r;
-    r = cuda_status(cudaStreamSynchronize(c->stream));  // ord is a host temporary
-    d.order_valid = (r == 0);
-    return r;
+    return A;
 }
 
 }  // namespace p3t
@@ -351,8 +314,12 @@ int p3t_upload_particles(int n, const void *epj) {
         (r = d.r_out.reserve(n)) || (r = d.r_search.reserve(n)) || (r = d.force.reserve(n)) ||
         (r = d.acc64.reserve(n)))
         return r;
-    if ((r = h2d(c, d.epj_stage.p, epj, (size_t)n * sizeof(EPJRec)))) return r;
-    if ((r = cuda_status(pack_bodies(c, d, n)))) return r;
+    Uploader u(c);
+    const void *src = place(c, u, d.epj_stage.p, epj, (size_t)n * sizeof(EPJRec));
+    r = u.issue();
+    if (!r && n > 0) r = cuda_status(launch_pack_walks(pack_resident(d, n, src), n, c->stream));
+    const int e = cuda_status(cudaStreamSynchronize(c->stream));  // the caller's records are read
+    if (r || e) return r ? r : e;
     c->res_n = n;
     return 0;
 }
@@ -367,21 +334,25 @@ int p3t_upload_lists(int n_group, const int *i_off, const int *i_idx, const int 
     int r = 0;
     if ((r = d.i_off.reserve(n_group + 1)) || (r = d.j_off.reserve(n_group + 1)) || (r = d.s_off.reserve(n_group + 1)) ||
         (r = d.i_idx.reserve(ni)) || (r = d.j_idx.reserve(nj)) || (r = d.s_idx.reserve(ns)) ||
-        (r = d.spj.reserve(n_spj)))
+        (r = d.spj.reserve(n_spj)) || (r = d.order.reserve(n_group)))
         return r;
     Uploader u(c);
-    u.add(d.i_off.p, i_off, (n_group + 1) * sizeof(int));
-    u.add(d.j_off.p, j_off, (n_group + 1) * sizeof(int));
-    u.add(d.s_off.p, s_off, (n_group + 1) * sizeof(int));
+    u.add(d.i_off.p, i_off, i_off ? (n_group + 1) * sizeof(int) : 0);
+    u.add(d.j_off.p, j_off, j_off ? (n_group + 1) * sizeof(int) : 0);
+    u.add(d.s_off.p, s_off, s_off ? (n_group + 1) * sizeof(int) : 0);
     u.add(d.i_idx.p, i_idx, ni * sizeof(int));
     u.add(d.j_idx.p, j_idx, nj * sizeof(int));
     u.add(d.s_idx.p, s_idx, ns * sizeof(int));
     u.add(d.spj.p, spj, (size_t)n_spj * sizeof(SPJRec));
-    if ((r = u.flush())) return r;
+    d.order_valid = false;
+    r = u.issue();
+    if (!r) r = cuda_status(launch_group_order(n_group, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p, c->stream));
+    const int e = cuda_status(cudaStreamSynchronize(c->stream));  // the caller's lists are read
+    if (r || e) return r ? r : e;
     c->res_groups = n_group;
     c->res_spj = n_spj;
-    d.order_valid = false;
-    return set_group_order(c, d, n_group, i_off, j_off, s_off);
+    d.order_valid = true;
+    return 0;
 }
 
 int p3t_soft_run(int emit_candidates) {
@@ -397,29 +368,22 @@ int p3t_soft_run(int emit_candidates) {
 int p3t_download_forces(void *force, int n) {
     CTX_OR_FAIL(c);
     if (n > c->res_n || n < 0) return ST_BAD_INDEX;
-    int r = grow_host(&c->h_out, &c->h_out_cap, (size_t)n * sizeof(ForceRec));
-    if (r) return r;
-    if (is_pinned(force)) {
-        r = cuda_status(cudaMemcpyAsync(force, c->res.force.p, (size_t)n * sizeof(ForceRec), cudaMemcpyDeviceToHost,
-                                        c->stream));
-        if (r) return r;
-        r = cuda_status(cudaStreamSynchronize(c->stream));
-        if (r) return r;
+    if (c->reads_host || is_pinned(force)) {
+        if (const int r = d2h(c, force, c->res.force.p, (size_t)n * sizeof(ForceRec))) return r;
     } else {
-        r = cuda_status(cudaMemcpyAsync(c->h_out, c->res.force.p, (size_t)n * sizeof(ForceRec),
-                                        cudaMemcpyDeviceToHost, c->stream));
-        if (r) return r;
-        r = cuda_status(cudaStreamSynchronize(c->stream));
-        if (r) return r;
+        int r = grow_host(&c->h_out, &c->h_out_cap, (size_t)n * sizeof(ForceRec));
+        if (r || (r = d2h(c, c->h_out, c->res.force.p, (size_t)n * sizeof(ForceRec)))) return r;
         std::memcpy(force, c->h_out, (size_t)n * sizeof(ForceRec));
     }
     return read_status(c);
 }
 
-// One call, host buffers in and out, with a single wait: every upload is
-// queued at once (pinned sources go straight to the copy engine), the group
-// launch order is computed on the host while they run, then the kernels and
-// the force download follow on the stream.
+// One call, host buffers in and out, with a single wait.  The link bounds what
+// the pair kernel does not: the lists go by the copy engine, one launch packs
+// bodies and superparticles from the caller's memory, the launch order is made on
+// the device, and the pair kernel writes each force into the caller's pinned
+// buffer as well as to the device.  1M bodies: 2.19 -> 1.92 ms, of which 0.99 is
+// the pair kernel and 0.88 the link at its 205 GB/s (180 MB in).
 int p3t_soft_force_host(int n, const void *epj, int n_group, const int *i_off, const int *i_idx, const int *j_off,
                         const int *j_idx, const int *s_off, const int *s_idx, const void *spj, int n_spj,
                         void *force) {
@@ -435,38 +399,50 @@ int p3t_soft_force_host(int n, const void *epj, int n_group, const int *i_off, c
         (r = d.acc64.reserve(n)) || (r = d.i_off.reserve(n_group + 1)) || (r = d.j_off.reserve(n_group + 1)) ||
         (r = d.s_off.reserve(n_group + 1)) || (r = d.i_idx.reserve(ni)) || (r = d.j_idx.reserve(nj)) ||
         (r = d.s_idx.reserve(ns)) || (r = d.spj.reserve(n_spj)) || (r = d.order.reserve((size_t)n_group)) ||
-        (r = grow_host(&c->h_order, &c->h_order_cap, (size_t)n_group * sizeof(int) + 4)))
+        (r = d.jsplit.reserve(n)) || (r = d.spjp.reserve(n_spj)))
         return r;
+    const bool f64 = c->precision == 1;
     Uploader u(c);
-    u.add(d.epj_stage.p, epj, (size_t)n * sizeof(EPJRec));
-    u.add(d.i_off.p, i_off, (n_group + 1) * sizeof(int));
-    u.add(d.j_off.p, j_off, (n_group + 1) * sizeof(int));
-    u.add(d.s_off.p, s_off, (n_group + 1) * sizeof(int));
+    u.add(d.i_off.p, i_off, i_off ? (n_group + 1) * sizeof(int) : 0);
+    u.add(d.j_off.p, j_off, j_off ? (n_group + 1) * sizeof(int) : 0);
+    u.add(d.s_off.p, s_off, s_off ? (n_group + 1) * sizeof(int) : 0);
     u.add(d.i_idx.p, i_idx, ni * sizeof(int));
     u.add(d.j_idx.p, j_idx, nj * sizeof(int));
     u.add(d.s_idx.p, s_idx, ns * sizeof(int));
-    u.add(d.spj.p, spj, (size_t)n_spj * sizeof(SPJRec));
+    PackArgs K = pack_resident(d, n, place(c, u, d.epj_stage.p, epj, (size_t)n * sizeof(EPJRec)));
+    K.one.spj = place(c, u, d.spj.p, spj, (size_t)n_spj * sizeof(SPJRec));
+    K.one.ns = n_spj;
+    if (K.one.spj != d.spj.p) K.spj = d.spj.p;  // kept for later runs on the resident lists
+    if (!f64) {
+        K.jsplit = d.jsplit.p;
+        K.spjp = d.spjp.p;
+        K.eps2 = (float)c->params[0];
+        K.trace_mode = c->trace_mode;
+    }
     // an early return leaves no copy of this call running (the caller's
-    // buffers and the staging and order buffers are reused afterwards)
+    // buffers and the staging buffer are reused afterwards)
     auto fail = [&](int e) {
         cudaStreamSynchronize(c->stream);
         return e;
     };
-    if ((r = u.issue())) return fail(r);
-    if ((r = cuda_status(pack_bodies(c, d, n)))) return fail(r);
+    if ((r = u.issue()) ||
+        (r = cuda_status(launch_group_order(n_group, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p, c->stream))) ||
+        (r = cuda_status(launch_pack_walks(K, (long long)n + n_spj, c->stream))))
+        return fail(r);
     c->res_n = n;
     c->res_groups = n_group;
     c->res_spj = n_spj;
-    if (n_group > 0) {
-        // h_order is free: every call ends with a wait on the stream
-        group_order_host(n_group, i_off, j_off, s_off, (int *)c->h_order);
-        if ((r = cuda_status(cudaMemcpyAsync(d.order.p, c->h_order, n_group * sizeof(int), cudaMemcpyHostToDevice,
-                                             c->stream))))
-            return fail(r);
-    }
     d.order_valid = true;
-    if ((r = p3t_soft_run(0))) return fail(r);
-    return p3t_download_forces(force, n);
+    SoftArgs A = make_args(c, d, n_group, n, n_spj, false);
+    A.cand = nullptr;
+    A.packed = 1;
+    A.isplit = A.jsplit = d.jsplit.p;
+    A.spjp = d.spjp.p;
+    // every body is in a group: the forces need no download of their own
+    const bool copy = ni == n && is_pinned(force) && device_reads(c, force, 4);
+    if (copy) A.force_copy = (ForceRec *)force;
+    if ((r = cuda_status(launch_soft(A, c->precision, false, c->stream)))) return fail(r);
+    return copy ? read_status(c) : p3t_download_forces(force, n);
 }
 
 }  // extern "C"

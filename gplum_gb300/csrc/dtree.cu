@@ -1073,6 +1073,12 @@ __global__ void __launch_bounds__(GO_T) k_group_order(int ng, const int *i_off, 
     for (int g = tid; g < ng; g += GO_T) order[atomicAdd(&h[bin(g)], 1)] = g;
 }
 
+cudaError_t launch_group_order(int ng, const int *i_off, const int *j_off, const int *s_off, int *order,
+                               cudaStream_t st) {
+    if (ng > 0) { P3T_COUNT_LAUNCH(); k_group_order<<<1, GO_T, 0, st>>>(ng, i_off, j_off, s_off, order); }
+    return cudaGetLastError();
+}
+
 // ---- host side ----------------------------------------------------------------------------------
 struct DTree {
     DevBuf<double> part, root;
@@ -1297,7 +1303,7 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
     }
     // 6. the soft kernel's launch order
     if ((r = d.order.reserve(ng))) return r;
-    if (ng > 0) { P3T_COUNT_LAUNCH(); k_group_order<<<1, GO_T, 0, c->stream>>>(ng, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p); }
+    if ((r = cuda_status(launch_group_order(ng, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p, c->stream)))) return r;
     d.order_valid = true;
     c->res_groups = ng;
     c->res_spj = base;

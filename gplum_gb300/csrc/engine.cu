@@ -783,10 +783,14 @@ int Engine::load(int n, const long long *id, const double *mass, const double *r
     int r = ensure(n);
     if (r) return r;
     S.n = n;
-    if ((r = h2d(c, S.id, id, n * sizeof(int64_t))) || (r = h2d(c, S.mass, mass, n * sizeof(double))) ||
-        (r = h2d(c, S.r_planet, r_planet, n * sizeof(double))) || (r = h2d(c, S.f, f, n * sizeof(double))) ||
-        (r = h2d(c, S.pos, pos, 3 * n * sizeof(double))) || (r = h2d(c, S.vel, vel, 3 * n * sizeof(double))))
-        return r;
+    Uploader u(c);
+    u.add(S.id, id, n * sizeof(int64_t));
+    u.add(S.mass, mass, n * sizeof(double));
+    u.add(S.r_planet, r_planet, n * sizeof(double));
+    u.add(S.f, f, n * sizeof(double));
+    u.add(S.pos, pos, 3 * (size_t)n * sizeof(double));
+    u.add(S.vel, vel, 3 * (size_t)n * sizeof(double));
+    if ((r = u.flush())) return r;
     // start-up reset, src/main_p3t.cpp:291-303
     for (double *p : {S.acc, S.acc_d, S.jerk_d, S.acc_s, S.jerk_s})
         cudaMemsetAsync(p, 0, 3 * (size_t)n * sizeof(double), c->stream);

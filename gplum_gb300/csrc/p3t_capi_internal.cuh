@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "p3t_common.cuh"
 #include "p3t_soft.cuh"
@@ -98,8 +99,6 @@ struct Context {
     size_t h_stage_cap = 0;
     void *h_out = nullptr;
     size_t h_out_cap = 0;
-    void *h_order = nullptr;  // group launch order on its way to the device
-    size_t h_order_cap = 0;
     WalkSlot walk[MAX_TAGS];
     WalkSlot fun;  // the single-group functor calls
 
@@ -108,9 +107,8 @@ struct Context {
         idx.release();
         if (h_stage) cudaFreeHost(h_stage);
         if (h_out) cudaFreeHost(h_out);
-        if (h_order) cudaFreeHost(h_order);
-        h_stage = h_out = h_order = nullptr;
-        h_stage_cap = h_out_cap = h_order_cap = 0;
+        h_stage = h_out = nullptr;
+        h_stage_cap = h_out_cap = 0;
         for (auto &w : walk) w.release();
         fun.release();
     }
@@ -126,15 +124,34 @@ int read_status(Context *c);
 int check_csr(int n_group, const int *off);
 int check_lists(int n_group, const int *i_off, const int *i_idx, const int *j_off, const int *j_idx,
                 const int *s_off, const int *s_idx, const void *spj, int n_spj);
-// Async host->device copy; pinned sources go straight to the DMA engine,
-// pageable ones through the context's pinned staging buffer.
+// Host->device uploads issued as one batch: sources that are pinned, or that
+// the device reads through the host's page tables, are copied by the DMA engine
+// directly (150-205 GB/s; a copy into pinned memory by a core, 14-24 GB/s),
+// others are first gathered into the context's pinned staging buffer.
+struct Uploader {
+    Context *c;
+    struct Item { void *dst; const void *src; size_t bytes; bool direct; };
+    std::vector<Item> items;
+    explicit Uploader(Context *cc) : c(cc) {}
+    void add(void *dst, const void *src, size_t bytes);
+    // queues the copies; returns once they are on the stream (the caller's
+    // sources and the staging buffer must stay untouched until the stream has
+    // run them)
+    int issue();
+    // waits for the copies as well: the caller's and the staging buffers may be
+    // reused afterwards
+    int flush();
+};
+// One upload, with its wait.
 int h2d(Context *c, void *dst, const void *src, size_t bytes);
 // Device -> host copy ordered after the work queued on the library's
 // stream (a non-blocking stream, which plain cudaMemcpy does not wait for).
 int d2h(Context *c, void *dst, const void *src, size_t bytes);
 
 SoftArgs make_args(Context *c, DevSet &d, int n_group, int n_ptcl, int n_spj, bool accumulate);
-int set_group_order(Context *c, DevSet &d, int n_group, const int *i_off_h, const int *j_off_h, const int *s_off_h);
+// Launch order of the soft kernel's groups, most pair work first.
+cudaError_t launch_group_order(int n_group, const int *i_off, const int *j_off, const int *s_off, int *order,
+                               cudaStream_t st);
 bool is_pinned(const void *p);
 
 }  // namespace p3t

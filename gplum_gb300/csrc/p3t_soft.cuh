@@ -43,6 +43,7 @@ struct SoftArgs {
     int accumulate;  // 1: add into existing ForceGrav records, 0: overwrite
     // outputs
     ForceRec *force;  // indexed like iptcl
+    ForceRec *force_copy;  // optional second place for the same records (accumulate = 0)
     D4 *acc64;   // FP64 form only: {ax, ay, az, phi}, indexed like iptcl
     int *cand;        // optional [n_iptcl x cand_cap] table of j indices
     int cand_cap;

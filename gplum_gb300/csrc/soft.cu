@@ -438,6 +438,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             r.id_max = max(idmax[k], r.id_max);
             r.id_min = min(idmin[k], r.id_min);
             o = r;
+            if (A.force_copy) A.force_copy[sQ[tid * IPT + k].z] = r;
         }
     }
 }
@@ -821,6 +822,7 @@ __device__ __forceinline__ void group_mixed_pipe(const SoftArgs &A, int g, int i
         r.id_max = max(idmax, r.id_max);
         r.id_min = min(idmin, r.id_min);
         orec = r;
+        if (A.force_copy) A.force_copy[M.sQ[tid].z] = r;
     }
 }
 
@@ -1026,6 +1028,7 @@ __device__ __forceinline__ void group_f64(const SoftArgs &A, int g, int ib, int 
             r.id_max = max(idmax[k], r.id_max);
             r.id_min = min(idmin[k], r.id_min);
             o = r;
+            if (A.force_copy) A.force_copy[pid[k]] = r;
         }
     }
 }
@@ -1111,8 +1114,8 @@ __device__ __forceinline__ SpjPack spj_pack(const SPJRec &r, float eps2, int tra
 // their FP32 splits and the packed superparticles.  The work is reading the
 // records, from host memory at the link's latency (about 2 us) and rate: a CTA
 // stages 128 records with 6 to 10 independent coalesced 8-byte loads a thread
-// (of an EPJ record the 64 of 112 bytes that are used), then each thread packs
-// one from shared memory.  A launch costs the host 4 us, so one launch in place
+// (of an EPJ record the 64 of 112 bytes that are used; the link still carries
+// whole lines), then each thread packs one from shared memory.  A launch costs the host 4 us, so one launch in place
 // of up to seven (two packs, two splits, the superparticles, three identity
 // lists) is most of a small call: with the records read in place, 3,000 bodies
 // in two dispatches 400 -> 76 us, a group's two functor calls 235 -> 82 us.
