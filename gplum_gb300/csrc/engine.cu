@@ -141,59 +141,189 @@ __global__ void k_corr_list(State S, const ForceRec *__restrict__ F, const int32
     if (!FILL) pair_n[i] = m;
 }
 
-// corr_pair's arithmetic for one pair (src/gravity_soft.h:75-242), terms out
+// corr_pair's arithmetic (src/gravity_soft.h:75-242), terms out.
+//
+// The FP64 pipe bounds this pass (85 % busy: 233 instructions a pair and
+// direction before).  So: a pair that both bodies list is taken once and its
+// terms written to both places -- the geometry only changes sign, which every
+// rounding keeps, and each side multiplies by the other's mass; roots and
+// quotients are the integer ones (p3t_exact.cuh); the cutoff polynomial's
+// coefficients are taken once per CTA; and the pairs inside r_out, which are
+// neighbours by their distance alone where that is below the critical one, go
+// apart from the others, which need the closest approach but no cutoff terms, so
+// that no warp pays for both.  A CTA takes PT * per list entries, keeps the ones
+// to compute, then sorts them into the two kinds.  1M-body crowded ring (3.2 M list
+// entries): the whole correction 1.53 -> 0.75 ms, the initial form 2.10 -> 1.15 ms
+// (with the integer roots in k_correct).
+constexpr int PT = 128, PT_MOST = 4;
+// FPGrav's cutoff polynomial, src/cutfunc.h:4-20, with cut_f's constants (the
+// same operations, once)
+struct CutCoef {
+    double c1, c2, c3, c4, c5, c6, c7;
+};
+__device__ __forceinline__ void cut_coef(const Params &P, CutCoef &c) {
+    const double g = P.gamma, g2 = g * g;
+    c.c1 = 14. * (g + 1.);
+    c.c2 = 21. * ((g + 3.) * g + 1.);
+    c.c3 = 35. / 3. * (((g + 9.) * g + 9.) * g + 1.);
+    c.c4 = 70. * ((g + 3.) * g + 1.) * g;
+    c.c5 = 210. * (g + 1.) * g2;
+    c.c6 = 140. * g2 * g;
+    c.c7 = (((g - 7.) * g + 21.) * g - 35.) * g2 * g2;
+}
+__device__ __forceinline__ double cut_W_coef(const Params &P, const CutCoef &c, double y) {
+    if (1.0 <= y) return 1.0;
+    if (y <= P.gamma) return y * P.w_y;
+    const double f = (((((((-10. / 3. * y + c.c1) * y - c.c2) * y + c.c3) * y - c.c4) * y + c.c5) * y - c.c6 * log(y)) * y +
+                      c.c7) * P.g_1_inv7;
+    return f + y * (1. - P.f1);
+}
+// is it a neighbour (NeighborList::addNeighbor, src/neighbor.h:635-670)?  rij < r_search here
 template <bool INITIAL>
-__global__ void __launch_bounds__(128) k_corr_pairs(State S, Params P, int np, const int32_t *__restrict__ pair_i,
-                                                    const int32_t *__restrict__ pair_j, PairTerms *out) {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < np; q += gridDim.x * blockDim.x) {
-        const int i = pair_i[q], j = pair_j[q];
-        PairTerms o;
-        o.flags = 0;
-        const V3 pos_i = ld3(S.pos, i), vel_i = ld3(S.vel, i), accd_i = ld3(S.acc_d, i);
-        const double mj = S.mass[j];
+__device__ __forceinline__ bool corr_near(const State &S, const Params &P, int i, int j, V3 dr, double dr2, double r_crit) {
+    const V3 dv = ld3(S.vel, j) - ld3(S.vel, i);
+    const V3 da = ld3(S.acc_d, j) - ld3(S.acc_d, i);
+    const double drdv = dot(dr, dv), dv2 = dot(dv, dv), da2 = dot(da, da);
+    const double t_min = dmin(dmax(div_rn(-drdv, sqrt_rn(dv2)), 0.), P.dt_tree);
+    const double dr2_min = dmin(dr2, dr2 + 2. * drdv * t_min + dv2 * t_min * t_min);
+    const double v_crit_a = P.R_search3 * 0.5 * P.dt_tree;
+    return dr2_min < r_crit * r_crit || dv2 < v_crit_a * v_crit_a * da2 || (INITIAL && da2 == 0.);
+}
+template <bool INITIAL>
+__global__ void __launch_bounds__(PT) k_corr_pairs(State S, Params P, int np, int per, const int32_t *__restrict__ pair_i,
+                                                   const int32_t *__restrict__ pair_j,
+                                                   const int32_t *__restrict__ pair_base,
+                                                   const int32_t *__restrict__ pair_n, PairTerms *out) {
+    __shared__ CutCoef cf;
+    __shared__ int2 task[PT * PT_MOST], kind[PT * PT_MOST];
+    __shared__ int n_task, n_in, n_out;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) n_task = n_in = n_out = 0;
+    if (tid == 32) cut_coef(P, cf);
+    __syncthreads();
+    // entries to compute: i < j, or one that the other body does not list
+    for (int k = 0; k < per; k++) {
+        const int q = (blockIdx.x * per + k) * PT + tid;
+        int rev = -1;
+        bool mine = false;
+        if (q < np) {
+            const int i = pair_i[q], j = pair_j[q];
+            const int b = pair_base[j], e = b + pair_n[j];
+            for (int u = b; u < e; u++) {
+                const int v = pair_j[u];
+                if (v >= i) {
+                    if (v == i) rev = u;
+                    break;
+                }
+            }
+            mine = i < j || rev < 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(&n_task, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (mine) task[at + __popc(m & ((1u << lane) - 1))] = make_int2(q, rev);
+    }
+    __syncthreads();
+    const int nt = n_task;
+    for (int t0 = 0; t0 < nt; t0 += PT) {
+        const int t = t0 + tid;
+        bool in = false, near = false;
+        int2 w = make_int2(0, 0);
+        if (t < nt) {
+            w = task[t];
+            const int i = pair_i[w.x], j = pair_j[w.x];
+            const double r_out = dmax(S.r_out[i], S.r_out[j]);
+            const double r_search = dmax(S.r_search[i], S.r_search[j]);
+            const V3 dr = ld3(S.pos, j) - ld3(S.pos, i);
+            double dr2 = dot(dr, dr);
+            dr2 += P.eps2;
+            const double rij = sqrt_rn(dr2);
+            in = rij < r_out;
+            near = rij < r_search;
+            if (!in && !near) {
+                out[w.x].flags = 0;
+                if (w.y >= 0) out[w.y].flags = 0;
+            }
+        }
+        // inside from the front, the others that may be neighbours from the back
+        const unsigned mi = __ballot_sync(0xffffffffu, in), mo = __ballot_sync(0xffffffffu, near && !in);
+        int ai = 0, ao = 0;
+        if (lane == 0) {
+            if (mi) ai = atomicAdd(&n_in, __popc(mi));
+            if (mo) ao = atomicAdd(&n_out, __popc(mo));
+        }
+        ai = __shfl_sync(0xffffffffu, ai, 0);
+        ao = __shfl_sync(0xffffffffu, ao, 0);
+        const unsigned below = (1u << lane) - 1;
+        // the sign of the entry says whether it is within r_search
+        if (in) kind[ai + __popc(mi & below)] = make_int2(near ? w.x : ~w.x, w.y);
+        else if (near) kind[PT * PT_MOST - 1 - (ao + __popc(mo & below))] = w;
+    }
+    __syncthreads();
+    const int no = n_out, n_all = n_in;
+    for (int t = tid; t < no; t += PT) {
+        const int2 w = kind[PT * PT_MOST - 1 - t];
+        const int i = pair_i[w.x], j = pair_j[w.x];
         const double r_out = dmax(S.r_out[i], S.r_out[j]);
-        const double r_out_inv = dmin(S.r_out_inv[i], S.r_out_inv[j]);
-        const double r_search = dmax(S.r_search[i], S.r_search[j]);
-        const V3 dr = ld3(S.pos, j) - pos_i;
+        const V3 dr = ld3(S.pos, j) - ld3(S.pos, i);
         double dr2 = dot(dr, dr);
         dr2 += P.eps2;
-        const double rij = sqrt(dr2);
-        const V3 dv = ld3(S.vel, j) - vel_i;
-        const V3 da = ld3(S.acc_d, j) - accd_i;
-        const double drdv = dot(dr, dv);
-        const double dv2 = dot(dv, dv);
-        const double da2 = dot(da, da);
-        const double t_min = dmin(dmax(-drdv / sqrt(dv2), 0.), P.dt_tree);
-        const double dr2_min = dmin(dr2, dr2 + 2. * drdv * t_min + dv2 * t_min * t_min);
+        const int near = corr_near<INITIAL>(S, P, i, j, dr, dr2, P.R_search2 * r_out);
+        out[w.x].flags = near;
+        if (near) out[w.x].acc0 = div_rn(r_out * r_out, S.mass[j]);
+        if (w.y >= 0) {
+            out[w.y].flags = near;
+            if (near) out[w.y].acc0 = div_rn(r_out * r_out, S.mass[i]);
+        }
+    }
+    for (int t = tid; t < n_all; t += PT) {
+        int2 w = kind[t];
+        bool near = w.x >= 0;
+        if (!near) w.x = ~w.x;
+        const int i = pair_i[w.x], j = pair_j[w.x];
+        const double mj = S.mass[j], mi = S.mass[i];
+        const double r_out = dmax(S.r_out[i], S.r_out[j]);
+        const double r_out_inv = dmin(S.r_out_inv[i], S.r_out_inv[j]);
+        const V3 dr = ld3(S.pos, j) - ld3(S.pos, i);
+        double dr2 = dot(dr, dr);
+        dr2 += P.eps2;
+        const double rij = sqrt_rn(dr2);
         const double r_crit = P.R_search2 * r_out;
-        const double v_crit_a = P.R_search3 * 0.5 * P.dt_tree;
-        if (dr2_min < r_crit * r_crit || dv2 < v_crit_a * v_crit_a * da2 || (INITIAL && da2 == 0.)) {
-            if (rij < r_search) {
-                // NeighborList::addNeighbor, src/neighbor.h:635-670
-                o.flags |= 1;
-                o.acc0 = r_out * r_out / mj;
-            }
+        // dr2_min <= dr2
+        if (near && !(dr2 < r_crit * r_crit)) near = corr_near<INITIAL>(S, P, i, j, dr, dr2, r_crit);
+        const double ro2 = r_out * r_out;
+        const double rinv = rcp_rn(rij);
+        const double r2inv = rinv * rinv;
+        const double r3inv = rinv * r2inv;
+        const double W = cut_W_coef(P, cf, rij * r_out_inv);
+        const double K = cut_K(P, rij, r_out_inv);
+        const double r_min = dmin(rinv, r_out_inv);
+        const double p1 = rinv * W - r_min, a1 = r3inv * K - r_min * r_min * r_min;
+        V3 jk = v3(0., 0., 0.);
+        if (INITIAL) {
+            const V3 dv = ld3(S.vel, j) - ld3(S.vel, i);
+            const double alpha = dot(dr, dv) * r2inv;
+            const double dKdt = cut_dKdt(P, rij, r_out_inv, alpha);
+            const double alpha_c = alpha * (1. - K);
+            jk = (1. - K) * dv - (3. * alpha_c + dKdt) * dr;
         }
-        if (rij < r_out) {
-            o.flags |= 2;
-            const double rinv = 1. / rij;
-            const double r2inv = rinv * rinv;
-            const double r3inv = rinv * r2inv;
-            const double W = cut_W(P, rij, r_out_inv);
-            const double K = cut_K(P, rij, r_out_inv);
-            const double r_min = dmin(rinv, r_out_inv);
-            o.phi = mj * (rinv * W - r_min);
-            o.acc = mj * (r3inv * K - r_min * r_min * r_min) * dr;
+        for (int side = 0; side < 2; side++) {
+            const int q = side ? w.y : w.x;
+            if (q < 0) break;
+            const double m = side ? mi : mj;
+            const V3 d = side ? v3(-dr.x, -dr.y, -dr.z) : dr;
+            PairTerms &o = out[q];
+            o.flags = near ? 3 : 2;
+            if (near) o.acc0 = div_rn(ro2, m);
+            o.phi = m * p1;
+            o.acc = m * a1 * d;
             if (INITIAL) {
-                const double alpha = drdv * r2inv;
-                const double dKdt = cut_dKdt(P, rij, r_out_inv, alpha);
-                const double alpha_c = alpha * (1. - K);
-                o.phi_d = mj * rinv * (1. - W);
-                o.acc_d = mj * r3inv * (1. - K) * dr;
-                o.jerk = mj * r3inv * ((1. - K) * dv - (3. * alpha_c + dKdt) * dr);
+                o.phi_d = m * rinv * (1. - W);
+                o.acc_d = m * r3inv * (1. - K) * d;
+                o.jerk = m * r3inv * (side ? v3(-jk.x, -jk.y, -jk.z) : jk);
             }
         }
-        out[q] = o;
     }
 }
 
@@ -481,12 +611,12 @@ __global__ void k_vdisp_partial(State S, double r_min, double drinv, double m_su
     const int beg = blockIdx.x * per, end = min(S.n, beg + per);
     for (int i = beg + threadIdx.x; i < end; i += blockDim.x) {
         const V3 pos = ld3(S.pos, i);
-        const double ri = sqrt(pos.x * pos.x + pos.y * pos.y);
+        const double ri = sqrt_rn(pos.x * pos.x + pos.y * pos.y);
         int b = (int)((ri - r_min) * drinv);
         if (b == NBIN) b = NBIN - 1;
         b = max(0, min(NBIN - 1, b));
-        V3 vk = v3(-pos.y / ri, pos.x / ri, 0.);
-        vk = vk * sqrt(m_sun / sqrt(pos.x * pos.x + pos.y * pos.y));
+        V3 vk = v3(div_rn(-pos.y, ri), div_rn(pos.x, ri), 0.);
+        vk = vk * sqrt_rn(div_rn(m_sun, ri));
         const V3 vr = ld3(S.vel, i) - vk;
         sv[b][threadIdx.x] += dot(vr, vr);
         sc[b][threadIdx.x] += 1;
@@ -524,7 +654,9 @@ __global__ void k_vdisp_bins(const double *part, const int *cntp, int nblk, doub
 // either side of the body's own, in FP32 beyond (their weights are below
 // exp(-(RB + 1/2)^2) ~ 1e-13 of the nearest, so FP32's 1e-6 relative error
 // there stays below 1e-19 of the sums); the sums come out within a few ulp
-// of the bin-by-bin FP64 arithmetic at a third of its FP64 work.
+// of the bin-by-bin FP64 arithmetic at a third of its FP64 work.  Roots and
+// quotients are the integer ones: with k_vdisp_partial 1.02 -> 0.80 ms at 1M
+// bodies, 1.98 -> 1.55 ms at 2M; the exponentials are the rest.
 constexpr int RB = 5;
 __global__ void k_radii(State S, Params P, double r_min, double dr, double drinv, const double *vd, const int *cnt) {
     __shared__ double s_vd[NBIN], s_on[NBIN];
@@ -540,7 +672,7 @@ __global__ void k_radii(State S, Params P, double r_min, double dr, double drinv
     if (i >= S.n) return;
     const V3 pos = ld3(S.pos, i), vel = ld3(S.vel, i);
     const double r2 = pos.x * pos.x + pos.y * pos.y;
-    const double rc = sqrt(r2);
+    const double rc = sqrt_rn(r2);
     const double x = (rc - r_min) * drinv;
     const int b0 = max(0, min(NBIN - 1, (int)floor(x)));
     const int lo = max(0, b0 - RB), hi = min(NBIN - 1, b0 + RB);
@@ -562,24 +694,24 @@ __global__ void k_radii(State S, Params P, double r_min, double dr, double drinv
     }
     vs += (double)vsf;
     ws += (double)wsf;
-    const double v_disp = vs / ws;
+    const double v_disp = div_rn(vs, ws);
     S.v_disp[i] = v_disp;
-    const double r = sqrt(dot(pos, pos));
+    const double r = sqrt_rn(dot(pos, pos));
     const double rv = dot(pos, vel);
-    double ax = 1.0 / (2.0 / r - dot(vel, vel) / P.m_sun);
-    const double ecccosu = 1. - r / ax;
-    const double eccsinu2 = rv * rv / (P.m_sun * ax);
-    if (!(sqrt(ecccosu * ecccosu + eccsinu2) < 0.6)) ax = r;
+    double ax = rcp_rn(div_rn(2.0, r) - div_rn(dot(vel, vel), P.m_sun));
+    const double ecccosu = 1. - div_rn(r, ax);
+    const double eccsinu2 = div_rn(rv * rv, P.m_sun * ax);
+    if (!(sqrt_rn(ecccosu * ecccosu + eccsinu2) < 0.6)) ax = r;
     // the cube root GPLUM takes as pow(x, 1/3.), by cbrt (within 1 ulp of it,
     // at a sixth of its cost)
-    const double rHill = cbrt(S.mass[i] / (3. * P.m_sun)) * ax;
+    const double rHill = cbrt(div_rn(S.mass[i], 3. * P.m_sun)) * ax;
     // pow(ax, -0) is 1 for every ax
     const double fac = (P.p_cut == 0.) ? 1. : pow(ax, -P.p_cut);
     const double r_out_i = dmax(P.R_cut0 * fac * rHill, P.R_cut1 * v_disp * P.dt_tree);
     double ro = dmax(r_out_i, P.r_cut_min);
     if (P.r_cut_max > 0.) ro = dmin(P.r_cut_max, ro);
     S.r_out[i] = ro;
-    S.r_out_inv[i] = 1. / ro;
+    S.r_out_inv[i] = rcp_rn(ro);
     S.r_search[i] = P.R_search0 * ro + P.R_search1 * v_disp * P.dt_tree;
 }
 
@@ -842,10 +974,17 @@ int Engine::correct(int initial) {
     { P3T_COUNT_LAUNCH(); k_corr_list<true><<<nb(S.n, 128), 128, 0, c->stream>>>(S, F, cand, cap, nullptr, pair_base.p, pair_i.p,
                                                            pair_j.p, c->status); }
     if (np > 0) {
+        // list entries per thread: up to four where that still leaves eight CTAs
+        // per SM, so that the kept ones fill whole warps
+        int sms = 152;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        const int per = std::max(1, std::min(PT_MOST, np / (PT * 8 * sms)));
         if (initial)
-            { P3T_COUNT_LAUNCH(); k_corr_pairs<true><<<nb(np, 128), 128, 0, c->stream>>>(S, P, np, pair_i.p, pair_j.p, pair_terms.p); }
+            { P3T_COUNT_LAUNCH(); k_corr_pairs<true><<<nb(np, PT * per), PT, 0, c->stream>>>(S, P, np, per, pair_i.p, pair_j.p, pair_base.p,
+                                                                       pair_n.p, pair_terms.p); }
         else
-            { P3T_COUNT_LAUNCH(); k_corr_pairs<false><<<nb(np, 128), 128, 0, c->stream>>>(S, P, np, pair_i.p, pair_j.p, pair_terms.p); }
+            { P3T_COUNT_LAUNCH(); k_corr_pairs<false><<<nb(np, PT * per), PT, 0, c->stream>>>(S, P, np, per, pair_i.p, pair_j.p, pair_base.p,
+                                                                       pair_n.p, pair_terms.p); }
     }
     if (initial)
         { P3T_COUNT_LAUNCH(); k_correct<true><<<nb(S.n, 128), 128, 0, c->stream>>>(S, P, F, cap, pair_base.p, pair_n.p, pair_j.p,

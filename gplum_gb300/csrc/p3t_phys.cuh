@@ -1,6 +1,7 @@
 // FP64 device physics of the P3T step: cutoff functions, sun force, Hermite
 // predictor/corrector and time-step criteria.  Every expression keeps the
-// operand order of the reference formula it restates (file:line beside it);
+// operand order of the reference formula it restates (file:line beside it),
+// with the roots and quotients of p3t_exact.cuh (the same doubles);
 // the translation units that include this header are compiled with
 // -fmad=false, so products and sums round separately as in GPLUM's build and
 // only the transcendental functions (log, sin, cos, atan2, pow, exp) can
@@ -8,6 +9,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "p3t_exact.cuh"
 #include "p3t_state.cuh"
 
 namespace p3t {
@@ -67,8 +69,8 @@ __device__ __forceinline__ double cut_dKdt(const Params &P, double rij, double r
 // ---- sun, src/gravity_hard.h:5-111 ---------------------------------------------
 __device__ __forceinline__ void sun_force(const Params &P, V3 x, V3 v, V3 &acc_s, V3 &jerk_s, double *phi_s) {
     const V3 dr = v3(-x.x, -x.y, -x.z), dv = v3(-v.x, -v.y, -v.z);
-    const double r2inv = 1. / (dot(dr, dr) + P.eps2_sun);
-    const double rinv = sqrt(r2inv);
+    const double r2inv = rcp_rn(dot(dr, dr) + P.eps2_sun);
+    const double rinv = sqrt_rn(r2inv);
     const double r3inv = rinv * r2inv;
     const double mr3 = P.m_sun * r3inv;
     const double alpha = dot(dr, dv) * r2inv;
@@ -81,16 +83,16 @@ __device__ __forceinline__ void sun_force(const Params &P, V3 x, V3 v, V3 &acc_s
 __device__ __forceinline__ double dt2nd(double eta, double alpha2, double acc0, V3 acc, V3 jerk) {
     const double Acc2 = dot(acc, acc) + alpha2 * acc0 * acc0;
     const double Jerk2 = dot(jerk, jerk);
-    return (Jerk2 > 0.) ? eta * sqrt(Acc2 / Jerk2) : 1.7976931348623157e308;
+    return (Jerk2 > 0.) ? eta * sqrt_rn(div_rn(Acc2, Jerk2)) : 1.7976931348623157e308;
 }
 __device__ __forceinline__ double dt4th(double eta, double alpha2, double acc0, V3 acc, V3 jerk, V3 snap, V3 crac) {
-    const double Acc = sqrt(dot(acc, acc) + alpha2 * acc0 * acc0);
+    const double Acc = sqrt_rn(dot(acc, acc) + alpha2 * acc0 * acc0);
     const double Jerk2 = dot(jerk, jerk);
-    const double Jerk = sqrt(Jerk2);
+    const double Jerk = sqrt_rn(Jerk2);
     const double Snap2 = dot(snap, snap);
-    const double Snap = sqrt(Snap2);
-    const double Crac = sqrt(dot(crac, crac));
-    return (Jerk > 0.) ? eta * sqrt((Acc * Snap + Jerk2) / (Jerk * Crac + Snap2)) : 1.7976931348623157e308;
+    const double Snap = sqrt_rn(Snap2);
+    const double Crac = sqrt_rn(dot(crac, crac));
+    return (Jerk > 0.) ? eta * sqrt_rn(div_rn(Acc * Snap + Jerk2, Jerk * Crac + Snap2)) : 1.7976931348623157e308;
 }
 
 // 1 / x, the same double as the IEEE quotient: by the exponent alone when x
