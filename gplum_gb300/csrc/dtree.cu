@@ -46,6 +46,7 @@
 #include "../../include/gplum_p3t.h"
 #include "p3t_capi_internal.cuh"
 #include "p3t_engine.cuh"
+#include "p3t_exact.cuh"
 
 namespace p3t {
 
@@ -67,35 +68,72 @@ constexpr int MAX_LEVEL = 21;                                             // lev
 constexpr int WALK_STACK = 256;
 
 // ---- bounding box and keys ------------------------------------------------------
+// doubles as integers of the same order, for minima and maxima beside the FP64 pipe
+__device__ __forceinline__ long long box_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+}
+__device__ __forceinline__ double box_value(long long k) {
+    return __longlong_as_double(k ^ (long long)((unsigned long long)(k >> 63) >> 1));
+}
+// b: box keys, the three minima and the three maxima -> the CTA's, in s[d][0]
+struct BoxSmem {
+    long long s[6][32];
+};
+__device__ __forceinline__ void box_none(long long *b) {
+    for (int d = 0; d < 3; d++) {
+        b[d] = box_key(1e300);
+        b[3 + d] = box_key(-1e300);
+    }
+}
+__device__ __forceinline__ void box_add(long long *b, int d, double x) {
+    if (x != x) return;  // as fmin and fmax, which pass over NaN
+    b[d] = min(b[d], box_key(x));
+    b[3 + d] = max(b[3 + d], box_key(x));
+}
+__device__ __forceinline__ void box_reduce(long long *b, BoxSmem &B) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int d = 0; d < 6; d++)
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long x = __shfl_xor_sync(0xffffffffu, b[d], o);
+            b[d] = d < 3 ? min(b[d], x) : max(b[d], x);
+        }
+    if (lane == 0)
+        for (int d = 0; d < 6; d++) B.s[d][w] = b[d];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int d = threadIdx.x;
+        long long x = B.s[d][0];
+        for (int k = 1; k < nw; k++) x = d < 3 ? min(x, B.s[d][k]) : max(x, B.s[d][k]);
+        B.s[d][0] = x;
+    }
+    __syncthreads();
+}
 // root cube as the host builder: out = {base.xyz, size, scale}; anchored at
-// the lower corner, so a thin axis is not cut at coarse levels.  The last CTA
-// to finish combines the partial boxes.
+// the lower corner, so a thin axis is not cut at coarse levels
+__device__ __forceinline__ void root_cube(const BoxSmem &B, double *out) {
+    double lo[3], ext = 0.;
+    for (int d = 0; d < 3; d++) {
+        lo[d] = box_value(B.s[d][0]);
+        ext = fmax(ext, box_value(B.s[3 + d][0]) - lo[d]);
+    }
+    const double size = ext * 1.0001 + 1e-300;
+    for (int d = 0; d < 3; d++) out[d] = lo[d] - 0.5 * (size - ext);
+    out[3] = size;
+    out[4] = double(1 << 21) / size;
+}
+// The last CTA to finish combines the partial boxes.
 __global__ void __launch_bounds__(256) k_bbox(const double *pos, int n, double *part, unsigned *done, double *out) {
-    __shared__ double s[6][256];
+    __shared__ BoxSmem B;
     __shared__ bool last;
     const int tid = threadIdx.x;
-    double b[6] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
-    auto reduce = [&]() {
-        for (int d = 0; d < 6; d++) s[d][tid] = b[d];
-        __syncthreads();
-        for (int o = 128; o > 0; o >>= 1) {
-            if (tid < o)
-                for (int d = 0; d < 3; d++) {
-                    s[d][tid] = fmin(s[d][tid], s[d][tid + o]);
-                    s[3 + d][tid] = fmax(s[3 + d][tid], s[3 + d][tid + o]);
-                }
-            __syncthreads();
-        }
-    };
+    long long b[6];
+    box_none(b);
     for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x)
-        for (int d = 0; d < 3; d++) {
-            const double x = pos[3 * i + d];
-            b[d] = fmin(b[d], x);
-            b[3 + d] = fmax(b[3 + d], x);
-        }
-    reduce();
+        for (int d = 0; d < 3; d++) box_add(b, d, pos[3 * i + d]);
+    box_reduce(b, B);
     if (tid < 6) {
-        __stcg(&part[6 * blockIdx.x + tid], s[tid][0]);
+        __stcg(&part[6 * blockIdx.x + tid], box_value(B.s[tid][0]));
         __threadfence();
     }
     __syncthreads();
@@ -106,20 +144,14 @@ __global__ void __launch_bounds__(256) k_bbox(const double *pos, int n, double *
     }
     __syncthreads();
     if (!last) return;
-    for (int d = 0; d < 6; d++) b[d] = d < 3 ? 1e300 : -1e300;
+    box_none(b);
     for (int k = tid; k < (int)gridDim.x; k += 256)
         for (int d = 0; d < 3; d++) {
-            b[d] = fmin(b[d], __ldcg(&part[6 * k + d]));
-            b[3 + d] = fmax(b[3 + d], __ldcg(&part[6 * k + 3 + d]));
+            b[d] = min(b[d], box_key(__ldcg(&part[6 * k + d])));
+            b[3 + d] = max(b[3 + d], box_key(__ldcg(&part[6 * k + 3 + d])));
         }
-    reduce();
-    if (tid) return;
-    double ext = 0.;
-    for (int d = 0; d < 3; d++) ext = fmax(ext, s[3 + d][0] - s[d][0]);
-    const double size = ext * 1.0001 + 1e-300;
-    for (int d = 0; d < 3; d++) out[d] = s[d][0] - 0.5 * (size - ext);
-    out[3] = size;
-    out[4] = double(1 << 21) / size;
+    box_reduce(b, B);
+    if (tid == 0) root_cube(B, out);
 }
 
 __device__ __forceinline__ unsigned long long spread21(unsigned long long v) {
@@ -130,6 +162,17 @@ __device__ __forceinline__ unsigned long long spread21(unsigned long long v) {
     v = (v | v << 4) & 0x10c30c30c30c30c3ULL;
     v = (v | v << 2) & 0x1249249249249249ULL;
     return v;
+}
+
+__device__ __forceinline__ unsigned long long morton_key(const double *pos, int i, double b0, double b1, double b2, double sc) {
+    unsigned long long c[3];
+    for (int d = 0; d < 3; d++) {
+        const double u = (pos[3 * i + d] - (d == 0 ? b0 : (d == 1 ? b1 : b2))) * sc;
+        long long v = (long long)u;
+        v = v < 0 ? 0 : (v > (1 << 21) - 1 ? (1 << 21) - 1 : v);
+        c[d] = (unsigned long long)v;
+    }
+    return (spread21(c[0]) << 2) | (spread21(c[1]) << 1) | spread21(c[2]);
 }
 
 // keys and the counts of each of their eight digits (ghist[8][256], zeroed)
@@ -144,14 +187,7 @@ __global__ void __launch_bounds__(256) k_keys(const double *pos, int n, const do
         const int i = base + tid;
         const unsigned in = __ballot_sync(0xffffffffu, i < n);
         if (i >= n) continue;
-        unsigned long long c[3];
-        for (int d = 0; d < 3; d++) {
-            const double u = (pos[3 * i + d] - (d == 0 ? b0 : (d == 1 ? b1 : b2))) * sc;
-            long long v = (long long)u;
-            v = v < 0 ? 0 : (v > (1 << 21) - 1 ? (1 << 21) - 1 : v);
-            c[d] = (unsigned long long)v;
-        }
-        const unsigned long long k = (spread21(c[0]) << 2) | (spread21(c[1]) << 1) | spread21(c[2]);
+        const unsigned long long k = morton_key(pos, i, b0, b1, b2, sc);
         key[i] = k;
         idx[i] = i;
 #pragma unroll
@@ -268,6 +304,121 @@ __global__ void __launch_bounds__(RADIX_T) k_radix_pass(const unsigned long long
         key_out[o] = k;
         idx_out[o] = si[q];
     }
+}
+
+// Root cube, keys and sort of at most SMALL_N bodies by one CTA, keys and indices
+// in shared memory: ten launches' work (box, keys, eight passes of 7 us, whose
+// tiles hold 2,048 keys: 85 us at 3,000 bodies) in one.  Eight keys a thread and
+// 132 KB of shared memory are the limit; above it the passes' tiles spread over
+// the SMs.
+constexpr int SMALL_T = 1024, SMALL_N = 8192, SMALL_W = SMALL_T / 32;
+struct SmallSmem {
+    unsigned long long k[SMALL_N];
+    int i[SMALL_N];
+    int wc[SMALL_W][256];
+    int start[256], ws[8], most;
+    double root[5];
+    BoxSmem box;
+};
+template <int K>
+__device__ __forceinline__ void small_sort(SmallSmem &M, const double *pos, int n, double *root,
+                                           unsigned long long *__restrict__ key_out, int *__restrict__ idx_out) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    long long b[6];
+    box_none(b);
+    for (int i = tid; i < n; i += SMALL_T)
+        for (int d = 0; d < 3; d++) box_add(b, d, pos[3 * i + d]);
+    box_reduce(b, M.box);
+    if (tid == 0) root_cube(M.box, M.root);
+    __syncthreads();
+    if (tid < 5) root[tid] = M.root[tid];
+    unsigned long long kv[K];
+    int iv[K], rk[K];
+#pragma unroll
+    for (int r = 0; r < K; r++) {
+        const int q = w * (32 * K) + r * 32 + lane;
+        kv[r] = q < n ? morton_key(pos, q, M.root[0], M.root[1], M.root[2], M.root[4]) : 0ULL;
+        iv[r] = q;
+    }
+#pragma unroll 1
+    for (int shift = 0; shift < 64; shift += 8) {
+        for (int j = lane; j < 256; j += 32) M.wc[w][j] = 0;
+        if (tid == 0) M.most = 0;
+        __syncwarp();
+        // as k_radix_pass: ranks among the warp's keys of the digit, in order
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            const bool valid = w * (32 * K) + r * 32 + lane < n;
+            const int d = valid ? (int)(kv[r] >> shift) & 255 : 256;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const int before = __popc(peers & ((1u << lane) - 1u));
+            int pre = 0;
+            if (valid) pre = M.wc[w][d];
+            __syncwarp();
+            if (valid && before == 0) M.wc[w][d] = pre + __popc(peers);
+            __syncwarp();
+            rk[r] = pre + before;
+        }
+        __syncthreads();
+        int total = 0, x = 0;
+        if (tid < 256) {
+            for (int j = 0; j < SMALL_W; j++) {
+                const int c = M.wc[j][tid];
+                M.wc[j][tid] = total;
+                total += c;
+            }
+            if (total == n) M.most = 1;  // one digit for all: the order stays
+            x = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += a;
+            }
+            if (lane == 31) M.ws[w] = x;
+        }
+        __syncthreads();
+        if (M.most) {
+            __syncthreads();
+            continue;
+        }
+        if (tid < 256) {
+            int s = x - total;
+            for (int k = 0; k < w; k++) s += M.ws[k];
+            M.start[tid] = s;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            if (w * (32 * K) + r * 32 + lane >= n) continue;
+            const int d = (int)(kv[r] >> shift) & 255, q = M.start[d] + M.wc[w][d] + rk[r];
+            M.k[q] = kv[r];
+            M.i[q] = iv[r];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            const int q = w * (32 * K) + r * 32 + lane;
+            if (q < n) {
+                kv[r] = M.k[q];
+                iv[r] = M.i[q];
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < K; r++) {
+        const int q = w * (32 * K) + r * 32 + lane;
+        if (q >= n) continue;
+        key_out[q] = kv[r];
+        idx_out[q] = iv[r];
+    }
+}
+__global__ void __launch_bounds__(SMALL_T) k_small_sort(const double *pos, int n, double *root, unsigned long long *key_out,
+                                                        int *idx_out) {
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    SmallSmem &M = *reinterpret_cast<SmallSmem *>(small_raw);
+    if (n <= 2 * SMALL_T) small_sort<2>(M, pos, n, root, key_out, idx_out);
+    else if (n <= 4 * SMALL_T) small_sort<4>(M, pos, n, root, key_out, idx_out);
+    else small_sort<8>(M, pos, n, root, key_out, idx_out);
 }
 
 // ---- the nodes of every level --------------------------------------------------------
@@ -431,167 +582,176 @@ __global__ void __launch_bounds__(256) k_nodes(const unsigned long long *__restr
 }
 
 // ---- moments and boxes, bottom-up -------------------------------------------------------
-constexpr int LEAF_B = 8;  // bodies of a leaf loaded at once (leaves hold at most n_leaf_limit = 8)
-// Node c's moments and boxes: a leaf sums its bodies in key order (the host
-// builder's sums), an inner node combines its children in child order by the
-// parallel-axis rule.  Children are read through L2 (ld.cg): they may have
-// been written by other CTAs of the same launch.
-__device__ void node_moments(int c, TNode *nd, TNodeF *nf, SPJRec *spj, const int *order, const double *pos,
-                             const double *mass, const double *rs) {
-    TNode &N = nd[c];
-    const int nchild = __ldcg(&N.nchild), child0 = __ldcg(&N.child0);
-    double m = 0., cx = 0., cy = 0., cz = 0., q[6] = {0., 0., 0., 0., 0., 0.};
-    double ilo[3] = {1e300, 1e300, 1e300}, ihi[3] = {-1e300, -1e300, -1e300};
-    double olo[3] = {1e300, 1e300, 1e300}, ohi[3] = {-1e300, -1e300, -1e300};
-    if (nchild == 0) {
-        const int first = N.first, count = N.count;
-        // in blocks of LEAF_B bodies, every load of a block issued before its
-        // sums (the sums stay in key order)
-        for (int k0 = first; k0 < first + count; k0 += LEAF_B) {
-            int pb[LEAF_B];
-#pragma unroll
-            for (int u = 0; u < LEAF_B; u++) pb[u] = (k0 + u < first + count) ? order[k0 + u] : -1;
-#pragma unroll
-            for (int u = 0; u < LEAF_B; u++) {
-                const int p = pb[u];
-                if (p < 0) break;
-                const double x = pos[3 * p], y = pos[3 * p + 1], z = pos[3 * p + 2], mp = mass[p];
-                m += mp;
-                cx += mp * x;
-                cy += mp * y;
-                cz += mp * z;
-                const double r = 1.1 * rs[p];
-                const double v[3] = {x, y, z};
-                for (int d = 0; d < 3; d++) {
-                    ilo[d] = fmin(ilo[d], v[d] - 0.);
-                    ihi[d] = fmax(ihi[d], v[d] + 0.);
-                    olo[d] = fmin(olo[d], v[d] - r);
-                    ohi[d] = fmax(ohi[d], v[d] + r);
-                }
-            }
-        }
-        if (m != 0.) {
-            cx /= m;
-            cy /= m;
-            cz /= m;
-        }
-        for (int k0 = first; k0 < first + count; k0 += LEAF_B) {
-            int pb[LEAF_B];
-#pragma unroll
-            for (int u = 0; u < LEAF_B; u++) pb[u] = (k0 + u < first + count) ? order[k0 + u] : -1;
-#pragma unroll
-            for (int u = 0; u < LEAF_B; u++) {
-                const int p = pb[u];
-                if (p < 0) break;
-                const double dx = pos[3 * p] - cx, dy = pos[3 * p + 1] - cy, dz = pos[3 * p + 2] - cz, mp = mass[p];
-                q[0] += mp * dx * dx; q[1] += mp * dy * dy; q[2] += mp * dz * dz;
-                q[3] += mp * dx * dy; q[4] += mp * dx * dz; q[5] += mp * dy * dz;
-            }
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (j >= nchild) break;
-            const int ch = child0 + j;
-            const double mc = __ldcg(&spj[ch].mass);
-            m += mc;
-            cx += mc * __ldcg(&spj[ch].pos[0]);
-            cy += mc * __ldcg(&spj[ch].pos[1]);
-            cz += mc * __ldcg(&spj[ch].pos[2]);
+// A node's moments and boxes by NL lanes, one body or child each: a leaf sums its
+// bodies in key order (the host builder's sums), an inner node combines its
+// children in child order by the parallel-axis rule.  What a body or child adds
+// is computed in its own lane; each component's sum then runs in key (child)
+// order in a lane of its own, from shared memory, so the sums round as one
+// thread's would.  Box bounds do not depend on the order: their minima and maxima
+// are integer comparisons of the doubles' ordered bits.
+//
+// What bounds it: in a large tree the FP64 pipe (one warp instruction per 19
+// cycles of an SM), about 10 instructions a node, as one thread per node needs
+// once the lanes its warp idles behind the fullest node are counted (with FP64
+// minima it needed 12 to 16); in a small one the chain of dependent FP64
+// operations, 64 cycles each: about 40 a level instead of 350.  The whole tree,
+// with the one-CTA sort below 8,192 bodies: 3,000 bodies 0.36 -> 0.26 ms, 50,000
+// 0.47 -> 0.37, 200,000 0.60 -> 0.51, 1M 1.48 -> 1.37, 2M 2.42 -> 2.36.
+constexpr int NL = 8, MOM_T = 128;
+struct MomentSmem {
+    double v[MOM_T / NL][6][NL];
+};
+// Lane u of node c (c < 0: no node; its lanes only keep the others company).
+// Children are read through L2 (ld.cg): other CTAs of the same launch may have
+// written them.
+__device__ void node_moments(int c, MomentSmem &M, TNode *nd, TNodeF *nf, SPJRec *spj, const int *order,
+                             const double *pos, const double *mass, const double *rs) {
+    const int u = threadIdx.x % NL, slot = threadIdx.x / NL;
+    double(*v)[NL] = M.v[slot];
+    int first = 0, count = 0, child0 = 0, nchild = 0;
+    double size = 0.;
+    if (c >= 0) {
+        const TNode &N = nd[c];
+        nchild = __ldcg(&N.nchild);
+        child0 = __ldcg(&N.child0);
+        first = N.first;
+        count = N.count;
+        size = N.size;
+    }
+    const bool leaf = nchild == 0;
+    const int items = leaf ? count : nchild;
+    int most = items;  // of the warp's nodes (a leaf at the deepest level may hold more than NL)
+    for (int o = NL; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    const long long inf = box_key(1e300), ninf = box_key(-1e300);
+    long long lo[6] = {inf, inf, inf, inf, inf, inf}, hi[6] = {ninf, ninf, ninf, ninf, ninf, ninf};  // inner, outer
+    double sum = 0.;  // lanes 0..3: mass and mass-weighted position
+    double m = 0., x = 0., y = 0., z = 0.;
+    int child = 0;
+    for (int k0 = 0; k0 < most; k0 += NL) {
+        const bool mine = k0 + u < items;
+        if (mine && leaf) {
+            const int p = order[first + k0 + u];
+            x = pos[3 * p]; y = pos[3 * p + 1]; z = pos[3 * p + 2];
+            m = mass[p];
+            const double r = 1.1 * rs[p];
+            const double w[3] = {x, y, z};
             for (int d = 0; d < 3; d++) {
-                ilo[d] = fmin(ilo[d], __ldcg(&nd[ch].ilo[d]));
-                ihi[d] = fmax(ihi[d], __ldcg(&nd[ch].ihi[d]));
-                olo[d] = fmin(olo[d], __ldcg(&nd[ch].olo[d]));
-                ohi[d] = fmax(ohi[d], __ldcg(&nd[ch].ohi[d]));
+                const double a = w[d] - r, b = w[d] + r;
+                // as fmin and fmax, which pass over NaN
+                if (w[d] == w[d]) { lo[d] = min(lo[d], box_key(w[d])); hi[d] = max(hi[d], box_key(w[d])); }
+                if (a == a) lo[3 + d] = min(lo[3 + d], box_key(a));
+                if (b == b) hi[3 + d] = max(hi[3 + d], box_key(b));
+            }
+        } else if (mine) {
+            child = child0 + u;
+            m = __ldcg(&spj[child].mass);
+            x = __ldcg(&spj[child].pos[0]); y = __ldcg(&spj[child].pos[1]); z = __ldcg(&spj[child].pos[2]);
+            for (int d = 0; d < 3; d++) {
+                lo[d] = box_key(__ldcg(&nd[child].ilo[d]));
+                hi[d] = box_key(__ldcg(&nd[child].ihi[d]));
+                lo[3 + d] = box_key(__ldcg(&nd[child].olo[d]));
+                hi[3 + d] = box_key(__ldcg(&nd[child].ohi[d]));
             }
         }
-        if (m != 0.) {
-            cx /= m;
-            cy /= m;
-            cz /= m;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (j >= nchild) break;
-            const SPJRec *S = spj + child0 + j;
-            const double mc = __ldcg(&S->mass);
-            const double dx = __ldcg(&S->pos[0]) - cx, dy = __ldcg(&S->pos[1]) - cy, dz = __ldcg(&S->pos[2]) - cz;
-            q[0] += __ldcg(&S->xx) + mc * dx * dx; q[1] += __ldcg(&S->yy) + mc * dy * dy;
-            q[2] += __ldcg(&S->zz) + mc * dz * dz;
-            q[3] += __ldcg(&S->xy) + mc * dx * dy; q[4] += __ldcg(&S->xz) + mc * dx * dz;
-            q[5] += __ldcg(&S->yz) + mc * dy * dz;
-        }
+        v[0][u] = m;  // (stale beyond the items, and not summed)
+        v[1][u] = m * x;
+        v[2][u] = m * y;
+        v[3][u] = m * z;
+        __syncwarp();
+        if (u < 4)
+            for (int k = 0; k < min(NL, items - k0); k++) sum += v[u][k];
+        __syncwarp();
     }
-    for (int d = 0; d < 3; d++) {
-        N.ilo[d] = ilo[d];
-        N.ihi[d] = ihi[d];
-        N.olo[d] = olo[d];
-        N.ohi[d] = ohi[d];
+    const int l0 = (threadIdx.x & 31) - u;
+    const double mt = __shfl_sync(0xffffffffu, sum, l0);
+    if (mt != 0. && u >= 1 && u < 4) sum = div_rn(sum, mt);
+    const double cx = __shfl_sync(0xffffffffu, sum, l0 + 1), cy = __shfl_sync(0xffffffffu, sum, l0 + 2),
+                 cz = __shfl_sync(0xffffffffu, sum, l0 + 3);
+    double q = 0.;  // lanes 0..5: the quadrupole's components
+    for (int k0 = 0; k0 < most; k0 += NL) {
+        const bool mine = k0 + u < items;
+        if (most > NL && mine && leaf) {
+            const int p = order[first + k0 + u];
+            x = pos[3 * p]; y = pos[3 * p + 1]; z = pos[3 * p + 2];
+            m = mass[p];
+        }
+        const double dx = x - cx, dy = y - cy, dz = z - cz, mx = m * dx, my = m * dy, mz = m * dz;
+        double t[6] = {mx * dx, my * dy, mz * dz, mx * dy, mx * dz, my * dz};
+        if (mine && !leaf) {
+            const double *Q = &spj[child].xx;
+            for (int k = 0; k < 6; k++) t[k] = __ldcg(Q + k) + t[k];
+        }
+        for (int k = 0; k < 6; k++) v[k][u] = t[k];
+        __syncwarp();
+        if (u < 6)
+            for (int k = 0; k < min(NL, items - k0); k++) q += v[u][k];
+        __syncwarp();
     }
-    N.com[0] = cx;
-    N.com[1] = cy;
-    N.com[2] = cz;
+    for (int d = 0; d < 6; d++)
+        for (int o = 1; o < NL; o <<= 1) {
+            lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+    if (c < 0) return;
+    TNode &N = nd[c];
     SPJRec &S = spj[c];
-    S.mass = m;
-    S.pos[0] = cx;
-    S.pos[1] = cy;
-    S.pos[2] = cz;
-    S.xx = q[0]; S.yy = q[1]; S.zz = q[2]; S.xy = q[3]; S.xz = q[4]; S.yz = q[5];
-    // the walk's FP32 copy
-    TNodeF F;
-    for (int d = 0; d < 3; d++) {
-        F.ilo[d] = (float)ilo[d];
-        F.ihi[d] = (float)ihi[d];
-        F.olo[d] = (float)olo[d];
-        F.ohi[d] = (float)ohi[d];
+    TNodeF &F = nf[c];  // the walk's FP32 copy
+    if (u < 3) {
+        auto pick = [&](const long long *a) { return box_value(u == 0 ? a[0] : u == 1 ? a[1] : a[2]); };
+        const double il = pick(lo), ih = pick(hi), ol = pick(lo + 3), oh = pick(hi + 3), cd = u == 0 ? cx : u == 1 ? cy : cz;
+        N.ilo[u] = il; N.ihi[u] = ih; N.olo[u] = ol; N.ohi[u] = oh;
+        N.com[u] = cd;
+        S.pos[u] = cd;
+        F.ilo[u] = (float)il; F.ihi[u] = (float)ih; F.olo[u] = (float)ol; F.ohi[u] = (float)oh;
+        F.com[u] = (float)cd;
     }
-    F.com[0] = (float)cx;
-    F.com[1] = (float)cy;
-    F.com[2] = (float)cz;
-    F.size = (float)N.size;
-    F.first = N.first;
-    F.count = N.count;
-    F.child0 = child0;
-    F.nchild = nchild;
-    nf[c] = F;
+    if (u < 6) (&S.xx)[u] = q;
+    if (u == 6) {
+        S.mass = mt;
+        F.size = (float)size;
+    }
+    if (u == 7) {
+        F.first = first;
+        F.count = count;
+        F.child0 = child0;
+        F.nchild = nchild;
+    }
 }
 
 // one level (nodes lo..hi-1) per launch, deepest level first
-__global__ void k_moments(int lo, int hi, TNode *nd, TNodeF *nf, SPJRec *spj, const int *order, const double *pos,
-                          const double *mass, const double *rs) {
-    const int c = lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= hi) return;
-    node_moments(c, nd, nf, spj, order, pos, mass, rs);
+__global__ void __launch_bounds__(MOM_T) k_moments(int lo, int hi, TNode *nd, TNodeF *nf, SPJRec *spj, const int *order,
+                                                   const double *pos, const double *mass, const double *rs) {
+    __shared__ MomentSmem M;
+    const int c = lo + (blockIdx.x * MOM_T + threadIdx.x) / NL;
+    node_moments(c < hi ? c : -1, M, nd, nf, spj, order, pos, mass, rs);
 }
 
-// Moments in lane-dense launches: every leaf at once from a compacted list
-// (their body sums are the bulk of the FP64 work), then the inner nodes one
-// level at a time, deepest first.  A launch over all nodes of a level, or one
-// climbing thread per finished child, left most lanes of the FP64 pipe's warp
-// instructions idle (ncu: 23 % lane efficiency for the climbing form).
-__global__ void k_moments_leaves(const int *list, const int *count, TNode *nd, TNodeF *nf, SPJRec *spj,
-                                 const int *order, const double *pos, const double *mass, const double *rs) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= *count) return;
-    node_moments(list[t], nd, nf, spj, order, pos, mass, rs);
-}
-// the inner nodes of a level (inner: their list, icnt: how many)
-__global__ void k_moments_inner(const int *inner, const int *icnt, TNode *nd, TNodeF *nf, SPJRec *spj,
-                                const int *order, const double *pos, const double *mass, const double *rs) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= *icnt) return;
-    node_moments(inner[t], nd, nf, spj, order, pos, mass, rs);
+// Moments in lane-dense launches: the nodes of a list, all leaves at once (their
+// body sums are the bulk of the FP64 work) or the inner nodes of a level, deepest
+// first.  A launch over all nodes of a level, or one climbing thread per finished
+// child, left most lanes of the FP64 pipe's warp instructions idle.
+__global__ void __launch_bounds__(MOM_T) k_moments_list(const int *list, const int *count, TNode *nd, TNodeF *nf,
+                                                        SPJRec *spj, const int *order, const double *pos,
+                                                        const double *mass, const double *rs) {
+    __shared__ MomentSmem M;
+    const int t = (int)(((long long)blockIdx.x * MOM_T + threadIdx.x) / NL), m = *count;
+    if ((t & ~(32 / NL - 1)) >= m) return;  // none of the warp's nodes
+    node_moments(t < m ? list[t] : -1, M, nd, nf, spj, order, pos, mass, rs);
 }
 // the inner nodes of levels from..to (deepest first) in one CTA, level after
 // level: runs of levels of few nodes -- the top of the tree, and the deep
-// chains around close pairs -- whose launches would cost more than their work
-constexpr int TOP_T = 128, TOP_NODES = 128;
-__global__ void __launch_bounds__(TOP_T) k_moments_run(int from, int to, const int *lstart, const int *inner, const int *icnt,
-                                                       TNode *nd, TNodeF *nf, SPJRec *spj, const int *order,
-                                                       const double *pos, const double *mass, const double *rs) {
+// chains around close pairs -- whose launches would cost more than their work.
+// TOP_NODES: the CTA's SM takes 3 us for 32 nodes, a launch 5 us.
+constexpr int TOP_NODES = 32;
+__global__ void __launch_bounds__(MOM_T) k_moments_run(int from, int to, const int *lstart, const int *inner,
+                                                       const int *icnt, TNode *nd, TNodeF *nf, SPJRec *spj,
+                                                       const int *order, const double *pos, const double *mass,
+                                                       const double *rs) {
+    __shared__ MomentSmem M;
     for (int L = from; L >= to; L--) {
-        for (int t = threadIdx.x; t < icnt[L]; t += TOP_T)
-            node_moments(inner[lstart[L] + t], nd, nf, spj, order, pos, mass, rs);
+        const int m = icnt[L], t0 = threadIdx.x / NL;
+        for (int t = t0; (t & ~(32 / NL - 1)) < m; t += MOM_T / NL)
+            node_moments(t < m ? inner[lstart[L] + t] : -1, M, nd, nf, spj, order, pos, mass, rs);
         __threadfence();
         __syncthreads();
     }
@@ -1129,16 +1289,24 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
         (r = T.lstart.reserve(MAX_LEVEL + 2)) || (r = T.gmark.reserve(n)) || (r = T.ng.reserve(1)))
         return r;
     // 1. root cube, keys, sort (the last pass writes the order into the group lists' bodies)
-    cudaMemsetAsync(T.ghist.p, 0, 8 * 256 * sizeof(unsigned), c->stream);
-    { P3T_COUNT_LAUNCH(); k_bbox<<<pb, 256, 0, c->stream>>>(E.S.pos, n, T.part.p, T.done.p, T.root.p); }
-    { P3T_COUNT_LAUNCH(); k_keys<<<rt, 256, 0, c->stream>>>(E.S.pos, n, T.root.p, T.key.p, T.idx.p, T.ghist.p); }
-    for (int p = 0; p < 8; p++) {
-        const bool odd = p & 1;
-        if ((r = E.lb.reserve(c, 256 * (size_t)rt))) return r;
-        { P3T_COUNT_LAUNCH(); k_radix_pass<<<rt, RADIX_T, 0, c->stream>>>(odd ? T.key2.p : T.key.p, odd ? T.idx2.p : T.idx.p, n, rt, 8 * p,
-                                                                     T.ghist.p + 256 * p, E.lb.st.p, E.lb.ticket.p,
-                                                                     E.lb.epoch, c->status, odd ? T.key.p : T.key2.p,
-                                                                     p == 7 ? d.i_idx.p : (odd ? T.idx.p : T.idx2.p)); }
+    if (n <= SMALL_N) {
+        // (above 48 KB of shared memory a kernel must be allowed its size)
+        if ((r = cuda_status(cudaFuncSetAttribute(k_small_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)sizeof(SmallSmem)))))
+            return r;
+        { P3T_COUNT_LAUNCH(); k_small_sort<<<1, SMALL_T, sizeof(SmallSmem), c->stream>>>(E.S.pos, n, T.root.p, T.key.p, d.i_idx.p); }
+    } else {
+        cudaMemsetAsync(T.ghist.p, 0, 8 * 256 * sizeof(unsigned), c->stream);
+        { P3T_COUNT_LAUNCH(); k_bbox<<<pb, 256, 0, c->stream>>>(E.S.pos, n, T.part.p, T.done.p, T.root.p); }
+        { P3T_COUNT_LAUNCH(); k_keys<<<rt, 256, 0, c->stream>>>(E.S.pos, n, T.root.p, T.key.p, T.idx.p, T.ghist.p); }
+        for (int p = 0; p < 8; p++) {
+            const bool odd = p & 1;
+            if ((r = E.lb.reserve(c, 256 * (size_t)rt))) return r;
+            { P3T_COUNT_LAUNCH(); k_radix_pass<<<rt, RADIX_T, 0, c->stream>>>(odd ? T.key2.p : T.key.p, odd ? T.idx2.p : T.idx.p, n, rt, 8 * p,
+                                                                         T.ghist.p + 256 * p, E.lb.st.p, E.lb.ticket.p,
+                                                                         E.lb.epoch, c->status, odd ? T.key.p : T.key2.p,
+                                                                         p == 7 ? d.i_idx.p : (odd ? T.idx.p : T.idx2.p)); }
+        }
     }
     const unsigned long long *key = T.key.p;
     const int *idx = d.i_idx.p;
@@ -1173,29 +1341,27 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
     // (or all nodes level by level), deepest first
     const int nlev_all = (int)T.level_start.size() - 1;
     if (g_moments_up) {
-        { P3T_COUNT_LAUNCH(); k_moments_leaves<<<nblocks(base, 128), 128, 0, c->stream>>>(T.list.p, icnt + MAX_LEVEL + 1, T.nd.p, T.nf.p,
-                                                                                      d.spj.p, idx, E.S.pos, E.S.mass,
-                                                                                      E.S.r_search); }
+        { P3T_COUNT_LAUNCH(); k_moments_list<<<nblocks((long long)base * NL, MOM_T), MOM_T, 0, c->stream>>>(
+            T.list.p, icnt + MAX_LEVEL + 1, T.nd.p, T.nf.p, d.spj.p, idx, E.S.pos, E.S.mass, E.S.r_search); }
         for (int L = nlev_all - 2; L >= 0;) {  // the deepest level has leaves only
             int to = L;
             while (to >= 0 && T.level_start[to + 1] - T.level_start[to] <= TOP_NODES) to--;
             const int m = T.level_start[L + 1] - T.level_start[L];
             if (to < L) {  // levels L..to + 1 are small
-                { P3T_COUNT_LAUNCH(); k_moments_run<<<1, TOP_T, 0, c->stream>>>(L, to + 1, T.lstart.p, T.list.p + base, icnt, T.nd.p, T.nf.p,
+                { P3T_COUNT_LAUNCH(); k_moments_run<<<1, MOM_T, 0, c->stream>>>(L, to + 1, T.lstart.p, T.list.p + base, icnt, T.nd.p, T.nf.p,
                                                                            d.spj.p, idx, E.S.pos, E.S.mass, E.S.r_search); }
                 L = to;
             } else {
-                { P3T_COUNT_LAUNCH(); k_moments_inner<<<nblocks(m, 128), 128, 0, c->stream>>>(T.list.p + base + T.level_start[L], icnt + L,
-                                                                                         T.nd.p, T.nf.p, d.spj.p, idx,
-                                                                                         E.S.pos, E.S.mass,
-                                                                                         E.S.r_search); }
+                { P3T_COUNT_LAUNCH(); k_moments_list<<<nblocks((long long)m * NL, MOM_T), MOM_T, 0, c->stream>>>(
+                    T.list.p + base + T.level_start[L], icnt + L, T.nd.p, T.nf.p, d.spj.p, idx, E.S.pos, E.S.mass,
+                    E.S.r_search); }
                 L--;
             }
         }
     } else {
         for (int L = nlev_all - 1; L >= 0; L--) {
             const int lo = T.level_start[L], hi = T.level_start[L + 1];
-            { P3T_COUNT_LAUNCH(); k_moments<<<nblocks(hi - lo, 128), 128, 0, c->stream>>>(lo, hi, T.nd.p, T.nf.p, d.spj.p, idx, E.S.pos,
+            { P3T_COUNT_LAUNCH(); k_moments<<<nblocks((long long)(hi - lo) * NL, MOM_T), MOM_T, 0, c->stream>>>(lo, hi, T.nd.p, T.nf.p, d.spj.p, idx, E.S.pos,
                                                                                  E.S.mass, E.S.r_search); }
         }
     }
