@@ -1,8 +1,8 @@
 // Fused EP-EP + EP-SP soft-force kernels for sm_103a.
 //
-// One CTA of 128 threads per i-group.  The group's i-particles sit in
-// registers; its EPJ list, then its SPJ list, are gathered tile by tile
-// (128 entries) into shared memory, where each entry is shifted to the
+// One CTA of 128 threads per i-group (256 or 512 where there are few groups).  The
+// group's i-particles sit in registers; its EPJ list, then its SPJ list, are gathered
+// tile by tile (128 to 512 entries) into shared memory, where each entry is shifted to the
 // group origin once (FP64 subtraction, then the FP32 rounding the functor
 // applies) and then reused by every i of the group.
 //
@@ -28,7 +28,8 @@
 //     max(rs2_i, rs2_j) -- bit-identical to the functor, so neighbour counts,
 //     rank sums and id_min/id_max match exactly;
 //   * forces: FP32 with rsqrt + one Newton step, FMA allowed; partial sums of
-//     32 pairs are folded into an error-free (TwoSum) FP32 hi/lo pair, so the
+//     32 pairs (16 where few groups share the chip) are folded into an
+//     error-free (TwoSum) FP32 hi/lo pair, so the
 //     accumulation error does not grow with the list length.
 // FP64 kernel: the same formulas with every quantity in double, the powers of
 // 1/r rounded once each -- the "plain FP64" form used as the accuracy baseline.
@@ -47,6 +48,8 @@ namespace p3t {
 constexpr int SB = 128;  // threads per CTA
 constexpr int TJ = 128;  // list entries per shared-memory tile
 constexpr int CHUNK = 32;  // pairs per FP32 partial sum before folding
+constexpr int TM = 128;        // list entries per tile of the mixed forms
+constexpr int TM_WHOLE = 256;  // and where all 128 threads take the same entries (one i each): half the barriers
 
 __device__ __forceinline__ void fold(float &hi, float &lo, float v) {
     const float s = hi + v;
@@ -80,22 +83,28 @@ __device__ __forceinline__ void fold(float &hi, float &lo, float v) {
 // No FP64 arithmetic in the staging except the functor's own local
 // coordinates of the j-particles, which the exact neighbour screen needs.
 //
-// Neighbour screen: inside the loop a pair only sets a bit when the force's
-// r^2 lies below 1.01 max(r_s,i^2, r_s,j^2) (precomputed per i and per j as
-// 1.01 r_s^2: x -> rn(1.01 x) is monotone, so the max commutes); after each
-// chunk of 32 entries the flagged pairs alone are re-screened exactly, in
-// list order, with the functor's FP32 arithmetic on its own rounded local
-// coordinates rn(x - x_epi[0]).
-constexpr int TM = 128;     // list entries per mixed-form tile
-constexpr int TP = TM / 2;  // entry pairs per tile
-
+// Neighbour screen: inside the loop two neighbouring entries only set their bits
+// when the smaller of the force's r^2 lies below 1.01 max(r_s,i^2, r_s,j^2), the
+// largest r_s,j of the chunk (precomputed per i and per j as 1.01 r_s^2: x ->
+// rn(1.01 x) is monotone, so the max commutes); after each chunk of 32 entries
+// the flagged pairs alone are re-screened exactly, in list order, with the
+// functor's FP32 arithmetic on its own rounded local coordinates
+// rn(x - x_epi[0]).  The EP-EP loop is bound by issue slots (44 for the 46 cycles
+// of its packed operations), so one comparison for two entries with the chunk's
+// threshold, tiles of 256 entries and four entry pairs unrolled count: 1M bodies,
+// EP-EP alone 553 -> 500 us, the whole pass 1.037 -> 0.979 ms.  (The pipelined form
+// compares each entry with its own threshold.)
+template <int TM>  // list entries per tile
 struct MixedTile {
+    static constexpr int TP = TM / 2;  // entry pairs
     // EP-EP: a = -(xh0,xh1,yh0,yh1) b = (-zh0,-zh1,m0,m1)
     //        c = -(xl0,xl1,yl0,yl1) d = (-zl0,-zl1,ro2_0,ro2_1) e = (t0,t1) t = 1.01 rs2_j
+    //        (the pipelined form; the others keep te)
     // EP-SP: a = -(x0,x1,y0,y1) local  b = (-z0,-z1,m0,m1)
     //        c = -(q'xx, q'yy)         d = (-q'zz, -mtr)   f = -(3qxy, 3qyz)  e = -(3qzx)
     float4 a[TP], b[TP], c[TP], d[TP], f[TP];
     float2 e[TP];
+    float te[TM / 16 + 1];  // EP-EP: the largest t of 16 entries each
     float4 r[TM];  // EP-EP exact screen: the functor's local (x, y, z) and rs2
     int2 q[TM];    // EP-EP (id_local, rank)
     int idx[TM];   // EP-EP particle index of each entry (candidate emission)
@@ -116,12 +125,28 @@ __device__ __forceinline__ void put2(float4 *arr, int t, int comp, float v) {
     reinterpret_cast<float *>(arr)[4 * (t >> 1) + 2 * comp + (t & 1)] = v;
 }
 
-template <int S, int IPT, bool EMIT, int UNR>
-__device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, int ni, MixedTile &T, float4 *sI,
-                                            int4 *sQ, int *scnt, float *redf, int *redi) {
-    // i-particles [ib, ib + ni) of group g (ni <= 2 * SB); the origin is the
-    // group's first i-particle, as in the functor
-    constexpr int W = SB / S;
+// shared memory of a CTA; the sub-blocks' sums take the tile's place at the end of a group
+template <int NT, int TM>
+struct MixedSmem {
+    union {
+        MixedTile<TM> T;
+        struct {
+            float f[8 * NT];
+            int i[4 * NT];
+        } R;
+    };
+    float4 sI[SB];
+    int4 sQ[SB];
+};
+
+template <int NT, int CAP, int TM, int S, bool EMIT, int UNR>
+__device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, int ni, MixedSmem<NT, CAP> &M, int *scnt) {
+    // i-particles [ib, ib + ni) of group g by NT threads, S sub-blocks of W; the
+    // origin is the group's first i-particle, as in the functor
+    constexpr int W = NT / S, IPT = 1, CH = NT == SB ? CHUNK : 16;
+    MixedTile<CAP> &T = M.T;
+    float4 *const sI = M.sI;
+    int4 *const sQ = M.sQ;
     const int tid = threadIdx.x;
     const int sub = tid / W, lane = tid % W;
     const int i0 = A.i_off[g];
@@ -156,8 +181,8 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
         xf[k] = __double2float_rn(r.x - ox);
         yf[k] = __double2float_rn(r.y - oy);
         zf[k] = __double2float_rn(r.z - oz);
-        sI[tid * IPT + k] = make_float4(xf[k], yf[k], zf[k], r.rs2);
-        sQ[tid * IPT + k] = make_int4(r.id_local, r.rank, p, 0);
+        sI[lane] = make_float4(xf[k], yf[k], zf[k], r.rs2);
+        sQ[lane] = make_int4(r.id_local, r.rank, p, 0);
         xh[k] = sp.xh; yh[k] = sp.yh; zh[k] = sp.zh;
         xl[k] = sp.xl; yl[k] = sp.yl; zl[k] = sp.zl;
         ro2i[k] = r.ro2;
@@ -168,7 +193,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
     // still stages tiles and meets every barrier)
     const bool wact = (lane & ~31) * IPT < ni;
     if (EMIT) {
-        for (int t = tid; t < ni; t += SB) scnt[t] = 0;
+        for (int t = tid; t < ni; t += NT) scnt[t] = 0;
     }
     // Screen prefilter.  The force's r^2 (split displacement, FMA) is within
     // 5e-7 relative of the exact r^2; the functor's differs from the exact one
@@ -183,11 +208,11 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
         for (int k = 0; k < IPT; k++)
             if (vi[k]) {
                 L = fmaxf(L, fmaxf(fabsf(xf[k]), fmaxf(fabsf(yf[k]), fabsf(zf[k]))));
-                rmin2 = fminf(rmin2, sI[tid * IPT + k].w);
+                rmin2 = fminf(rmin2, sI[lane].w);
             }
         const bool pre_ok = __syncthreads_and(L * L <= 4.0e8f * rmin2) != 0;
 #pragma unroll
-        for (int k = 0; k < IPT; k++) thi[k] = pre_ok ? 1.01f * sI[tid * IPT + k].w : 3.0e38f;
+        for (int k = 0; k < IPT; k++) thi[k] = pre_ok ? 1.01f * sI[lane].w : 3.0e38f;
     }
     const float2 c15 = dup2(1.5f), cm05 = dup2(-0.5f);
 
@@ -195,7 +220,8 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
     for (int base = 0; base < nj; base += TM) {
         const int nt = min(TM, nj - base);
         __syncthreads();
-        for (int t = tid; t < TM; t += SB) {
+        for (int t = tid; t < TM; t += NT) {
+            float th = 0.f;
             if (t < nt) {
                 int p = A.j_idx[j0 + base + t];
                 if ((unsigned)p >= (unsigned)A.n_ptcl) { atomicOr(A.status, ST_BAD_INDEX); p = 0; }
@@ -208,7 +234,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
                 put2(T.b, t, 0, -sp.zh); put2(T.b, t, 1, sp.m);
                 put2(T.c, t, 0, -sp.xl); put2(T.c, t, 1, -sp.yl);
                 put2(T.d, t, 0, -sp.zl); put2(T.d, t, 1, sp.ro2);
-                reinterpret_cast<float *>(T.e)[t] = 1.01f * rs2;
+                th = 1.01f * rs2;
                 T.r[t] = make_float4(__double2float_rn(x - ox), __double2float_rn(y - oy), __double2float_rn(z - oz),
                                      rs2);
                 T.q[t] = make_int2(id, rank);
@@ -218,30 +244,35 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
                 put2(T.b, t, 0, -1.0e18f); put2(T.b, t, 1, 0.f);
                 put2(T.c, t, 0, 0.f); put2(T.c, t, 1, 0.f);
                 put2(T.d, t, 0, 0.f); put2(T.d, t, 1, 0.f);
-                reinterpret_cast<float *>(T.e)[t] = 0.f;
                 T.r[t] = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.f);
                 T.q[t] = make_int2(-1, -1);
             }
+            float m = th;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if ((t & 15) == 0) T.te[t / 16] = m;
+            if (t == TM - 1) T.te[TM / 16] = 0.f;
         }
         __syncthreads();
         // this sub-block's share of the tile, in chunks of 32 entries (the last
         // one of a list may be 16)
-        const int jb = sub * (TM / S);
-        const int je = wact ? min(jb + TM / S, (nt + 15) & ~15) : jb;
-        for (int c0 = jb; c0 < je; c0 += CHUNK) {
-            const int nq = min(CHUNK, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
+        const int jn = (nt + 15) & ~15, per = NT == SB ? TM / S : ((nt + S - 1) / S + 15) & ~15;
+        const int jb = min(sub * per, jn), je = wact ? min(jb + per, jn) : jb;
+        for (int c0 = jb; c0 < je; c0 += CH) {
+            const int nq = min(CH, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
             float2 tx[IPT], ty[IPT], tz[IPT], tp[IPT];
             unsigned nm[IPT];
+            float thr[IPT];
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
                 tx[k] = ty[k] = tz[k] = tp[k] = dup2(0.f);
                 nm[k] = 0u;
+                thr[k] = fmaxf(thi[k], CH == 16 ? T.te[c0 / 16] : fmaxf(T.te[c0 / 16], T.te[c0 / 16 + 1]));
             }
 #pragma unroll UNR
             for (int q = 0; q < nq; q++) {
                 const int pq = (c0 >> 1) + q;
                 const float4 a = T.a[pq], b = T.b[pq], c = T.c[pq], d = T.d[pq];
-                const float2 e = T.e[pq];
 #pragma unroll
                 for (int k = 0; k < IPT; k++) {
                     const float2 rx = __fadd2_rn(__fadd2_rn(dup2(xh[k]), lo2(a)), __fadd2_rn(dup2(xl[k]), lo2(c)));
@@ -257,8 +288,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
                     ty[k] = __ffma2_rn(mr3, ry, ty[k]);
                     tz[k] = __ffma2_rn(mr3, rz, tz[k]);
                     tp[k] = __fadd2_rn(tp[k], mr);
-                    if (r2f.x < fmaxf(thi[k], e.x)) nm[k] |= 1u << (2 * q);
-                    if (r2f.y < fmaxf(thi[k], e.y)) nm[k] |= 2u << (2 * q);
+                    if (fminf(r2f.x, r2f.y) < thr[k]) nm[k] |= 3u << (2 * q);
                 }
             }
 #pragma unroll
@@ -270,8 +300,8 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
                 // exact screen of the flagged pairs, in list order
                 unsigned m = vi[k] ? nm[k] : 0u;
                 if (m) {
-                    const float4 me = sI[tid * IPT + k];
-                    const int4 mq = sQ[tid * IPT + k];
+                    const float4 me = sI[lane];
+                    const int4 mq = sQ[lane];
                     do {
                     const int jj = c0 + __ffs(m) - 1;
                     m &= m - 1;
@@ -316,7 +346,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
     for (int base = 0; base < ns; base += TM) {
         const int nt = min(TM, ns - base);
         __syncthreads();
-        for (int t = tid; t < TM; t += SB) {
+        for (int t = tid; t < TM; t += NT) {
             if (t < nt) {
                 int q = A.s_idx[s0 + base + t];
                 if ((unsigned)q >= (unsigned)A.n_spj) { atomicOr(A.status, ST_BAD_INDEX); q = 0; }
@@ -344,10 +374,10 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             }
         }
         __syncthreads();
-        const int jb = sub * (TM / S);
-        const int je = wact ? min(jb + TM / S, (nt + 15) & ~15) : jb;
-        for (int c0 = jb; c0 < je; c0 += CHUNK) {
-            const int nq = min(CHUNK, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
+        const int jn = (nt + 15) & ~15, per = NT == SB ? TM / S : ((nt + S - 1) / S + 15) & ~15;
+        const int jb = min(sub * per, jn), je = wact ? min(jb + per, jn) : jb;
+        for (int c0 = jb; c0 < je; c0 += CH) {
+            const int nq = min(CH, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
             float2 tx[IPT], ty[IPT], tz[IPT], tp[IPT];
 #pragma unroll
             for (int k = 0; k < IPT; k++) tx[k] = ty[k] = tz[k] = tp[k] = dup2(0.f);
@@ -398,30 +428,43 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
     // ---- combine sub-blocks in a fixed order and write ForceGrav ----
     if (S > 1) {
         __syncthreads();
-        float *f = redf + tid * 8;
-        f[0] = ahx[0]; f[1] = alx[0]; f[2] = ahy[0]; f[3] = aly[0];
-        f[4] = ahz[0]; f[5] = alz[0]; f[6] = ahp[0]; f[7] = alp[0];
-        int *q = redi + tid * 4;
-        q[0] = ngb[0]; q[1] = rk[0]; q[2] = idmax[0]; q[3] = idmin[0];
+        float *const rf = M.R.f + tid;
+        int *const ri = M.R.i + tid;
+        rf[0] = ahx[0]; rf[NT] = alx[0]; rf[2 * NT] = ahy[0]; rf[3 * NT] = aly[0];
+        rf[4 * NT] = ahz[0]; rf[5 * NT] = alz[0]; rf[6 * NT] = ahp[0]; rf[7 * NT] = alp[0];
+        ri[0] = ngb[0]; ri[NT] = rk[0]; ri[2 * NT] = idmax[0]; ri[3 * NT] = idmin[0];
         __syncthreads();
-        if (sub == 0) {
-            for (int s = 1; s < S; s++) {
-                const float *h = redf + (tid + s * W) * 8;
-                const int *c = redi + (tid + s * W) * 4;
-                fold(ahx[0], alx[0], h[0]); alx[0] += h[1];
-                fold(ahy[0], aly[0], h[2]); aly[0] += h[3];
-                fold(ahz[0], alz[0], h[4]); alz[0] += h[5];
-                fold(ahp[0], alp[0], h[6]); alp[0] += h[7];
-                ngb[0] += c[0]; rk[0] += c[1];
-                idmax[0] = max(idmax[0], c[2]); idmin[0] = min(idmin[0], c[3]);
+        // a component (0..3: hi and lo of x, y, z, phi; 4..7: the counts) of an i per thread
+        for (int it = tid; it < 8 * W; it += NT) {
+            const int l = it % W, c = it / W;
+            if (c < 4) {
+                float *const h = M.R.f + 2 * c * NT + l;
+                float hi = h[0], lo = h[NT];
+#pragma unroll
+                for (int s = 1; s < S; s++) {
+                    fold(hi, lo, h[s * W]);
+                    lo += h[NT + s * W];
+                }
+                h[0] = hi;
+                h[NT] = lo;
+            } else {
+                int *const h = M.R.i + (c - 4) * NT + l;
+                int v = h[0];
+#pragma unroll
+                for (int s = 1; s < S; s++) v = c < 6 ? v + h[s * W] : c == 6 ? max(v, h[s * W]) : min(v, h[s * W]);
+                h[0] = v;
             }
         }
+        __syncthreads();
+        ahx[0] = rf[0]; alx[0] = rf[NT]; ahy[0] = rf[2 * NT]; aly[0] = rf[3 * NT];
+        ahz[0] = rf[4 * NT]; alz[0] = rf[5 * NT]; ahp[0] = rf[6 * NT]; alp[0] = rf[7 * NT];
+        ngb[0] = ri[0]; rk[0] = ri[NT]; idmax[0] = ri[2 * NT]; idmin[0] = ri[3 * NT];
     }
     if (sub == 0) {
 #pragma unroll
         for (int k = 0; k < IPT; k++) {
             if (!vi[k]) continue;
-            ForceRec &o = A.force[sQ[tid * IPT + k].z];
+            ForceRec &o = A.force[sQ[lane].z];
             ForceRec r;
             if (A.accumulate) {
                 r = o;
@@ -438,7 +481,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             r.id_max = max(idmax[k], r.id_max);
             r.id_min = min(idmin[k], r.id_min);
             o = r;
-            if (A.force_copy) A.force_copy[sQ[tid * IPT + k].z] = r;
+            if (A.force_copy) A.force_copy[sQ[lane].z] = r;
         }
     }
 }
@@ -449,31 +492,55 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
 // OCC resident CTAs per SM (the autotuner picks 4, 5 or 6).
 template <bool EMIT, int OCC>
 __global__ void __launch_bounds__(SB, OCC) soft_mixed_kernel(SoftArgs A) {
-    __shared__ MixedTile T;
-    __shared__ float4 sI[SB];
-    __shared__ int4 sQ[SB];
+    __shared__ MixedSmem<SB, TM_WHOLE> M;
     __shared__ int scnt[EMIT ? SB : 1];
-    __shared__ float redf[SB * 8];
-    __shared__ int redi[SB * 4];
     if (A.gate && *A.gate) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     // EP-EP unroll depth: as deep as the register budget holds without spills
-    constexpr int UNR = OCC <= 4 ? 8 : 2;
+    constexpr int UNR = OCC <= 4 ? 8 : 4;
     for (int ib = 0; ib < ni_all; ib += SB) {
         const int ni = min(SB, ni_all - ib);
         if (ni > A.t_s1)
-            group_mixed<1, 1, EMIT, UNR>(A, g, ib, ni, T, sI, sQ, scnt, redf, redi);
+            group_mixed<SB, TM_WHOLE, TM_WHOLE, 1, EMIT, UNR>(A, g, ib, ni, M, scnt);
         else if (ni > A.t_s2)
-            group_mixed<2, 1, EMIT, UNR>(A, g, ib, ni, T, sI, sQ, scnt, redf, redi);
+            group_mixed<SB, TM_WHOLE, TM, 2, EMIT, UNR>(A, g, ib, ni, M, scnt);
         else
-            group_mixed<4, 1, EMIT, UNR>(A, g, ib, ni, T, sI, sQ, scnt, redf, redi);
+            group_mixed<SB, TM_WHOLE, TM, 4, EMIT, UNR>(A, g, ib, ni, M, scnt);
+        __syncthreads();
+    }
+}
+
+// Few groups: NT threads a group, the j list in two or four times as many parts.
+// A call of few groups is bound by one group's chain -- loads of the offsets, the
+// lists and the records one after another, then its pair loops -- and leaves most
+// of the chip idle, so more warps share the loops.  Parts end at multiples of 16
+// entries, the chunk of a partial sum here, so that the forces do not depend on
+// NT or on the parts beyond the hi/lo folds.
+// With the packing launches (9 us), groups of up to 128: 152 groups 33.9 -> 27.7 us
+// with 512 threads (256: 29.8), 304 groups 35.9 -> 31.9 with 256 (512: 33.9); groups
+// of up to 64: 456 groups 33.5 -> 31.5 with 256, 608 groups 35.6 against 36.3 (more
+// CTAs than one wave holds).
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 512 ? 1 : 3) soft_mixed_wide_kernel(SoftArgs A) {
+    __shared__ MixedSmem<NT, NT> M;
+    if (A.gate && *A.gate) return;
+    const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
+    const int ni_all = A.i_off[g + 1] - A.i_off[g];
+    for (int ib = 0; ib < ni_all; ib += SB) {
+        const int ni = min(SB, ni_all - ib);
+        if (ni > A.t_s1)
+            group_mixed<NT, NT, NT, NT / 128, false, 4>(A, g, ib, ni, M, nullptr);
+        else if (ni > A.t_s2)
+            group_mixed<NT, NT, NT, NT / 64, false, 4>(A, g, ib, ni, M, nullptr);
+        else
+            group_mixed<NT, NT, NT, NT / 32, false, 4>(A, g, ib, ni, M, nullptr);
         __syncthreads();
     }
 }
 
 // the mixed kernel's staging: pipelined (1) or gather-then-compute (0, the
-// default: at 1M bodies 1.046 ms per pass against 1.062 pipelined -- with six
+// default: at 1M bodies 0.979 ms per pass against 1.062 pipelined -- with six
 // CTAs per SM the gather's latency is already hidden, and the FMA pipe, not
 // the staging, bounds the pass)
 int g_soft_pipe = 0;
@@ -503,7 +570,7 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 struct PipeSmem {
-    MixedTile T[2];
+    MixedTile<TM> T[2];
     RawEntry raw[TM];  // also the sub-block reduction's space at the end of a group
     float4 sI[SB];
     int4 sQ[SB];
@@ -541,7 +608,7 @@ __device__ __forceinline__ int pipe_issue(const SoftArgs &A, int t, int Tep, int
 
 // entry e of tile t from its raw slot into tile buffer T (group_mixed's staging arithmetic)
 template <bool EMIT>
-__device__ __forceinline__ void pipe_convert(int t, int Tep, int e, int p, const RawEntry &R, MixedTile &T, double ox,
+__device__ __forceinline__ void pipe_convert(int t, int Tep, int e, int p, const RawEntry &R, MixedTile<TM> &T, double ox,
                                              double oy, double oz, const SoftSplit &o) {
     if (t < Tep) {
         if (p >= 0) {
@@ -667,7 +734,7 @@ __device__ __forceinline__ void group_mixed_pipe(const SoftArgs &A, int g, int i
             pn = pipe_issue(A, t + 2, Tep, j0, nj, s0, ns, tid, R);
             cp_async_commit();
         }
-        const MixedTile &T = M.T[cur];
+        const MixedTile<TM> &T = M.T[cur];
         const int jb = sub * (TM / S);
         if (t < Tep) {
             // ---- EP-EP ----
@@ -1319,6 +1386,19 @@ cudaError_t launch_soft(const SoftArgs &Ain, int precision, bool emit, cudaStrea
             if (e != cudaSuccess) return e;
         }
         const int occ = A.occ ? A.occ : 5;
+        // groups that leave SMs idle: more threads a group while a group has an SM
+        // (512) or a third of one (256) to itself.  Not where candidates are emitted:
+        // those passes drive an integration, whose roundings do not depend on the
+        // number of groups.
+        int dev = 0, sms = 0;
+        if (!emit && cudaGetDevice(&dev) == cudaSuccess)
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (!emit && A.n_group <= 3 * sms) {
+            P3T_COUNT_LAUNCH();
+            if (A.n_group <= sms) soft_mixed_wide_kernel<512><<<A.n_group, 512, 0, st>>>(A);
+            else soft_mixed_wide_kernel<256><<<A.n_group, 256, 0, st>>>(A);
+            return cudaGetLastError();
+        }
 #define P3T_SOFT_MIXED(OCC)                                                                               \
     do {                                                                                                  \
         P3T_COUNT_LAUNCH();                                                                               \

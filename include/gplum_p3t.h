@@ -90,9 +90,10 @@ int p3t_set_soft_occupancy(int ctas_per_sm);
 /* Staging of the mixed soft kernel's tiles: 1 pipelined -- each thread
  * copies the records of its entry two tiles ahead with cp.async and converts
  * the next tile into a second buffer while the CTA computes the current one,
- * one barrier per tile; 0 (default, 1.5 % faster at 1M bodies) gather,
- * barrier, compute, barrier.  Bit-identical results.  No counterpart in
- * GPLUM's interface. */
+ * one barrier per tile; 0 (default, 7 % faster at 1M bodies) gather,
+ * barrier, compute, barrier.  Bit-identical results.  Passes of at most three
+ * groups per SM that emit no candidates have a form of their own (more threads
+ * a group) under either setting.  No counterpart in GPLUM's interface. */
 int p3t_set_soft_pipe(int on);
 /* The library's CUDA stream (cudaStream_t) for callers that order their own
  * work or timing events after the library's launches. */
