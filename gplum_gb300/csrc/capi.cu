@@ -38,7 +38,8 @@ Context *ctx_get(int device) {
     int prio_lo = 0, prio_hi = 0;
     cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
     const int prio = (prio_hi < prio_lo) ? prio_hi + 1 : prio_hi;
-    if (cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, prio) != cudaSuccess) {
+    if (cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, prio) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio_hi) != cudaSuccess) {
         delete c;
         return nullptr;
     }
@@ -250,6 +251,8 @@ int p3t_finalize(void) {
     cudaStreamSynchronize(c->stream);
     c->release();
     cudaFree(c->status);
+    cudaStreamSynchronize(c->side);
+    cudaStreamDestroy(c->side);
     cudaStreamDestroy(c->stream);
     delete c;
     g_ctx = nullptr;

@@ -78,6 +78,7 @@ struct Context {
     int device = 0;
     bool reads_host = false;  // the device reads any host memory in place (it walks the host's page tables)
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;  // the multiwalk calls' reads and writes of the caller's arrays
     int *status = nullptr;  // device status bits
     double params[21];
     int params_version = 0;
