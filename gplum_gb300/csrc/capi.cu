@@ -121,8 +121,7 @@ bool is_pinned(const void *p) {
     return a.type == cudaMemoryTypeHost;
 }
 
-// Host memory that a kernel may read in place at `align` bytes.
-static bool device_reads(Context *c, const void *p, size_t align) {
+bool device_reads(Context *c, const void *p, size_t align) {
     if ((uintptr_t)p % align) return false;
     if (c->reads_host) return true;
     cudaPointerAttributes a;

@@ -13,10 +13,11 @@
 //
 // Those arrays exist once per GPU that loads this library and stay allocated
 // until the process exits (P3T_NOALLOC_MAX_BODIES x 80 B = 5 MiB,
-// P3T_NOALLOC_MAX_SPJ x 64 B = 4 MiB, plus the status word and the gate).  Their device addresses are looked up once per device, on
-// that device's first call (cudaGetSymbolAddress with the device current).
-// A call waits for its stream (it reads the status word back to the host), so
-// it cannot be made on a stream that is being captured into a CUDA graph.
+// P3T_NOALLOC_MAX_SPJ x 64 B = 4 MiB, plus the status word and the gate).  Their
+// device addresses are looked up once per device, on that device's first call
+// (cudaGetSymbolAddress with the device current).  A call waits for its stream
+// (for its status), so it cannot be made on a stream that is being captured into a
+// CUDA graph.
 // Every call shares the arrays: calls that overlap on the GPU (different
 // streams, or several host threads) race on them and must be serialised by
 // the caller.  The caller's CSR offsets are checked on the device before any
@@ -42,6 +43,8 @@ struct DeviceScratch {
     p3t::SoftSplit *split = nullptr;
     p3t::SpjPack *spj = nullptr;
     int *status = nullptr;
+    int calls = 0;             // the gate is closed for a call when it holds the call's number
+    bool writes_host = false;  // the device writes any host memory in place
 };
 constexpr int MAX_DEVICES = 64;
 DeviceScratch g_scratch[MAX_DEVICES];
@@ -50,7 +53,7 @@ std::mutex g_scratch_mu;
 // Device addresses of the static arrays for the current device.  The array
 // names are host-side stand-ins: only these looked-up addresses may be
 // passed to kernels.
-int scratch_for_current_device(DeviceScratch **out) {
+int scratch_for_current_device(DeviceScratch **out, int *call) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return -(int)e;
@@ -66,8 +69,13 @@ int scratch_for_current_device(DeviceScratch **out) {
         if (e != cudaSuccess) return -(int)e;
         e = cudaGetSymbolAddress((void **)&s.status, g_noalloc_status);
         if (e != cudaSuccess) return -(int)e;
+        int v = 0;
+        s.writes_host = cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess && v &&
+                        cudaDeviceGetAttribute(&v, cudaDevAttrHostNativeAtomicSupported, dev) == cudaSuccess && v;
         s.ready = true;
     }
+    s.calls = s.calls == 2147483647 ? 1 : s.calls + 1;
+    *call = s.calls;
     *out = &s;
     return 0;
 }
@@ -98,15 +106,20 @@ extern "C" int p3t_soft_force_noalloc(int n, const void *epj, int n_group, const
     if (!epj || !force || !i_off || !i_idx || !j_off || !j_idx || !s_off || !s_idx || (n_spj > 0 && !spj))
         return -(int)cudaErrorInvalidValue;
     DeviceScratch *s = nullptr;
-    int r = scratch_for_current_device(&s);
+    int call = 0;
+    int r = scratch_for_current_device(&s, &call);
     if (r) return r;
     cudaStream_t st = (cudaStream_t)stream;
-    // the status word and the gate keep the previous call's values: clear them
-    cudaError_t e = cudaMemsetAsync(s->status, 0, 2 * sizeof(int), st);
-    if (e != cudaSuccess) return -(int)e;
+    // The kernels set the bits in this call's own word where the device reaches the
+    // host's memory; elsewhere in the static word, which keeps the previous call's
+    // value: clear it.
+    cudaError_t e = cudaSuccess;
+    int h = 0;
+    int *const status = s->writes_host ? &h : s->status;
+    if (!s->writes_host && (e = cudaMemsetAsync(s->status, 0, sizeof(int), st)) != cudaSuccess) return -(int)e;
     // one launch packs bodies and superparticles and checks the offsets; a
     // violation closes the gate, and no list is read through a malformed offset.
-    // The host waits once, for the result: 20,000 bodies 112 -> 90 us a call
+    // The host waits once, for the result: 20,000 bodies 112 -> 73 us a call
     // against a launch for each of the check (with a wait), the bodies, their
     // splits and the superparticles.
     p3t::PackArgs K{};
@@ -125,9 +138,13 @@ extern "C" int p3t_soft_force_noalloc(int n, const void *epj, int n_group, const
     K.chk_s_off = s_off;
     K.chk_groups = n_group;
     K.chk_n = n;
-    K.status = s->status;
+    K.status = status;
+    K.gate_call = call;
     K.gate = s->status + 1;
-    if ((e = p3t::launch_pack_walks(K, (long long)n + n_spj, st)) != cudaSuccess) return -(int)e;
+    if ((e = p3t::launch_pack_walks(K, (long long)n + n_spj, st)) != cudaSuccess) {
+        cudaStreamSynchronize(st);
+        return -(int)e;
+    }
     p3t::SoftArgs A{};
     A.i_off = i_off;
     A.i_idx = i_idx;
@@ -151,20 +168,22 @@ extern "C" int p3t_soft_force_noalloc(int n, const void *epj, int n_group, const
     A.acc64 = nullptr;
     A.cand = nullptr;
     A.cand_cap = 0;
-    A.status = s->status;
+    A.status = status;
     A.jsplit = s->split;
     A.isplit = s->split;
     A.spjp = s->spj;
     A.packed = 1;
     A.gate = s->status + 1;
+    A.gate_call = call;
     // the launch shape the setters chose (the same as the allocating path's)
     A.t_ipt2 = p3t::g_soft_shape[0];
     A.t_s1 = p3t::g_soft_shape[1];
     A.t_s2 = p3t::g_soft_shape[2];
     A.occ = p3t::g_soft_shape[3];
-    if ((e = launch_soft(A, 0, false, st)) != cudaSuccess) return -(int)e;
-    int h = 0;
-    if ((e = cudaMemcpyAsync(&h, s->status, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return -(int)e;
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return -(int)e;
-    return h;
+    e = launch_soft(A, 0, false, st);
+    if (e == cudaSuccess && !s->writes_host) e = cudaMemcpyAsync(&h, s->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+    // (also after an error: nothing of this call may still write its word)
+    const cudaError_t w = cudaStreamSynchronize(st);
+    if (e != cudaSuccess || w != cudaSuccess) return -(int)(e != cudaSuccess ? e : w);
+    return *(volatile int *)&h;
 }

@@ -154,5 +154,7 @@ SoftArgs make_args(Context *c, DevSet &d, int n_group, int n_ptcl, int n_spj, bo
 cudaError_t launch_group_order(int n_group, const int *i_off, const int *j_off, const int *s_off, int *order,
                                cudaStream_t st);
 bool is_pinned(const void *p);
+// Host memory that a kernel may read in place, at `align` bytes.
+bool device_reads(Context *c, const void *p, size_t align);
 
 }  // namespace p3t

@@ -63,7 +63,8 @@ struct SoftArgs {
     SoftSplit *isplit, *jsplit;
     SpjPack *spjp;
     int packed;       // 1: the scratch is filled already (launch_pack_walks)
-    const int *gate;  // optional device word: non-zero and the mixed kernels return at once
+    const int *gate;  // optional device word: where it holds gate_call the mixed kernels return at once
+    int gate_call;
 };
 
 // One walk's records and where its packed entries start.  The records may lie
@@ -97,11 +98,12 @@ struct PackArgs {
     float eps2;
     int trace_mode;
     // optional check of a caller's CSR offsets (each starts at 0 and never
-    // decreases, the i lists end at chk_n at most): ST_BAD_INDEX into *gate
-    // and *status
+    // decreases, the i lists end at chk_n at most): gate_call into *gate and
+    // ST_BAD_INDEX into *status
     const int *chk_i_off, *chk_j_off, *chk_s_off;
     int chk_groups, chk_n;
     int *gate, *status;
+    int gate_call;
 };
 cudaError_t launch_pack_walks(const PackArgs &A, long long n_records, cudaStream_t st);
 cudaError_t launch_spj_pack(const SPJRec *in, int n, float eps2, int trace_mode, SpjPack *out, cudaStream_t st);

@@ -494,7 +494,7 @@ template <bool EMIT, int OCC>
 __global__ void __launch_bounds__(SB, OCC) soft_mixed_kernel(SoftArgs A) {
     __shared__ MixedSmem<SB, TM_WHOLE> M;
     __shared__ int scnt[EMIT ? SB : 1];
-    if (A.gate && *A.gate) return;
+    if (A.gate && *A.gate == A.gate_call) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     // EP-EP unroll depth: as deep as the register budget holds without spills
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(SB, OCC) soft_mixed_kernel(SoftArgs A) {
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 3) soft_mixed_wide_kernel(SoftArgs A) {
     __shared__ MixedSmem<NT, NT> M;
-    if (A.gate && *A.gate) return;
+    if (A.gate && *A.gate == A.gate_call) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     for (int ib = 0; ib < ni_all; ib += SB) {
@@ -897,7 +897,7 @@ template <bool EMIT, int OCC>
 __global__ void __launch_bounds__(SB, OCC) soft_mixed_pipe_kernel(SoftArgs A) {
     __shared__ PipeSmem M;
     __shared__ int scnt[EMIT ? SB : 1];
-    if (A.gate && *A.gate) return;
+    if (A.gate && *A.gate == A.gate_call) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     constexpr int UNR = OCC <= 4 ? 8 : 2;
@@ -1286,7 +1286,7 @@ __global__ void __launch_bounds__(PK) pack_walks_kernel(PackArgs A) {
                               : i1 < A.chk_i_off[g - 1] || j1 < A.chk_j_off[g - 1] || s1 < A.chk_s_off[g - 1];
             if (g == A.chk_groups) bad = bad || i1 > A.chk_n;
             if (bad) {
-                atomicOr(A.gate, ST_BAD_INDEX);
+                *A.gate = A.gate_call;
                 atomicOr(A.status, ST_BAD_INDEX);
             }
         }
