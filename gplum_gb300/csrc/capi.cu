@@ -109,6 +109,14 @@ int read_status(Context *c) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_status(e);
     if (h) cudaMemsetAsync(c->status, 0, sizeof(int), c->stream);
+    // and the walks' own words
+    auto take = [&](WalkSlot &w) {
+        if (!w.h_tab) return;
+        h |= *(volatile int *)w.h_tab;
+        *(volatile int *)w.h_tab = 0;
+    };
+    for (auto &w : c->walk) take(w);
+    take(c->fun);
     return h;
 }
 

@@ -54,7 +54,7 @@ constexpr int MAX_TAGS = 8;
 // State of one in-flight multiwalk dispatch (or of the functor calls).
 struct WalkSlot {
     DevSet d;
-    void *h_tab = nullptr;  // pinned: a copy of the status word, then the walks' records table
+    void *h_tab = nullptr;  // pinned: the kernels' status word, then the walks' records table
     size_t h_tab_cap = 0;
     void *h_in = nullptr;  // pinned: records that the device cannot read in place
     size_t h_in_cap = 0;

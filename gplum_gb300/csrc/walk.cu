@@ -34,6 +34,15 @@ int check_walks(int n_walk, const int *cnt, const void *const *ptr) {
     return tot > 2147483647LL ? ST_BAD_INDEX : 0;
 }
 
+// Room for a table behind the slot's status word, whose bits stay until they are read.
+int reserve_table(WalkSlot &w, size_t bytes) {
+    const size_t had = w.h_tab_cap;
+    const int word = had ? *(volatile int *)w.h_tab : 0;
+    const int r = grow_host(&w.h_tab, &w.h_tab_cap, 64 + bytes);
+    if (!r && w.h_tab_cap != had) *(volatile int *)w.h_tab = word;
+    return r;
+}
+
 // A call's walks in the slot's pinned table, which the kernels read.
 struct WalkTable {
     WalkSlot &w;
@@ -45,7 +54,7 @@ struct WalkTable {
     int *status() const { return (int *)w.h_tab; }
     WalkRecords *rec() const { return (WalkRecords *)((char *)w.h_tab + 64); }
 
-    int reserve() { return grow_host(&w.h_tab, &w.h_tab_cap, 64 + (size_t)n_walk * sizeof(WalkRecords)); }
+    int reserve() { return reserve_table(w, (size_t)n_walk * sizeof(WalkRecords)); }
     void set(int k, const void *epi, int n_i, const void *epj, int n_j, const void *spj, int n_s) {
         rec()[k] = WalkRecords{(const EPIRec *)epi, epj, spj, n_i, n_j, n_s, ni, nj, ns};
         ni += n_i; nj += n_j; ns += n_s;
@@ -144,6 +153,8 @@ SoftArgs walk_args(Context *c, WalkTable &t, DevSet &x, int n_j, int n_s, bool a
     A.iptcl = d.iptcl.p; A.i_r_out = d.i_r_out.p; A.i_r_search = d.i_r_search.p; A.n_iptcl = t.ni;
     A.isplit = d.isplit.p; A.jsplit = x.jsplit.p; A.spjp = x.spjp.p;
     A.packed = 1;
+    // the kernels' status bits: the slot's own pinned word (a copy behind the kernels was 4 us)
+    A.status = t.status();
     A.force = !accumulate && on_device(c, t.ni) ? d.force.p : (ForceRec *)t.w.h_out;
     A.cand = nullptr;
     return A;
@@ -183,17 +194,16 @@ int functor_call(const void *epi, int ni, const void *epj, int nj, const void *s
         K.seed = (const ForceRec *)w.h_out;
         K.acc64 = w.d.acc64.p;
     }
-    if (!(r = cuda_status(launch_pack_walks(K, (long long)ni + nj + ns, c->stream))) &&
-        !(r = cuda_status(launch_soft(walk_args(c, t, w.d, nj, ns, true), c->precision, false, c->stream))))
-        r = cuda_status(cudaMemcpyAsync(t.status(), c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (!(r = cuda_status(launch_pack_walks(K, (long long)ni + nj + ns, c->stream))))
+        r = cuda_status(launch_soft(walk_args(c, t, w.d, nj, ns, true), c->precision, false, c->stream));
     // also after an error: nothing of this call may still read the caller's records
     const int e = cuda_status(cudaStreamSynchronize(c->stream));
     if (r || e) return r ? r : e;
     std::memcpy(force, w.h_out, bytes);
-    return *t.status() ? read_status(c) : 0;
+    return *(volatile int *)t.status() ? read_status(c) : 0;
 }
 
-// Common tail of both dispatch forms: kernel, status copy, event.  Returns once
+// Common tail of both dispatch forms: kernels, events.  Returns once
 // the caller's records have been read (in_place: by the kernels, where they are).
 int launch_walks(Context *c, WalkTable &t, const PackArgs &K, DevSet &x, int n_j, int n_s, long long n_records,
                  bool in_place) {
@@ -206,8 +216,6 @@ int launch_walks(Context *c, WalkTable &t, const PackArgs &K, DevSet &x, int n_j
         if ((e = cuda_status(cudaEventRecord(w.read, c->side)))) return e;
         if ((e = cuda_status(cudaStreamWaitEvent(c->stream, w.read, 0)))) return e;
         if ((e = cuda_status(launch_soft(walk_args(c, t, x, n_j, n_s, false), c->precision, false, c->stream)))) return e;
-        if ((e = cuda_status(cudaMemcpyAsync(t.status(), c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream))))
-            return e;
         return cuda_status(cudaEventRecord(w.done, c->stream));
     };
     if ((r = run())) {
@@ -352,9 +360,7 @@ int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
     int r = cuda_status(cudaEventSynchronize(w.done));
     w.busy = false;
     if (r) return r;
-    // the status word as it was behind this dispatch's kernel; the word itself
-    // is read, and cleared, only where that was not zero
-    const int status = *(const int *)w.h_tab;
+    const int status = *(volatile int *)w.h_tab;
     uintptr_t bits = 0;
     int walks = n_walk;  // those that the dispatch covers
     long long off = 0;
@@ -367,7 +373,7 @@ int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
     }
     const bool device = on_device(c, w.n_i);
     if (device && (bits & 3) == 0) {
-        if ((r = grow_host(&w.h_tab, &w.h_tab_cap, 64 + (size_t)walks * sizeof(ForceOut)))) return r;
+        if ((r = reserve_table(w, (size_t)walks * sizeof(ForceOut)))) return r;
         ForceOut *out = (ForceOut *)((char *)w.h_tab + 64);
         off = 0;
         for (int k = 0; k < walks; k++) {

@@ -80,3 +80,32 @@ def test_retrieve_beyond_the_dispatch(gpu):
     st = lib.p3t_soft_retrieve(5, len(more), VP(more.ctypes.data), (VP * len(more))(*[out.ctypes.data + 32 * int(o) for o in off[:-1]]))
     assert st == 2
     assert lib.p3t_soft_retrieve(5, len(cnt), VP(cnt.ctypes.data), (VP * len(cnt))()) == 2  # retrieved already
+
+
+def test_status_of_dispatches_in_flight(gpu):
+    """Two dispatches in flight, the first with an index out of range: its retrieve reports it and the
+    other's does not; a status read between dispatch and retrieve reports it too, once."""
+    lib = configure(P3TParams())
+    epj, L = _problem(700, 4)
+    ng = L["n_group"]
+    cnt = np.ascontiguousarray(np.diff(L["i_off"]))
+    ei = np.ascontiguousarray(epi_records(epj)[L["i_idx"]])
+    nj, ns = np.ascontiguousarray(np.diff(L["j_off"])), np.zeros(ng, np.int32)
+    out = np.zeros(700, FORCE_DTYPE)
+    bad = L["j_idx"].copy()
+    bad[5] = len(epj)
+
+    def dispatch(tag, js, send):
+        p = [(VP * ng)(*[a.ctypes.data + int(o) * a.dtype.itemsize for o in L[k][:-1]]) for a, k in ((ei, "i_off"), (js, "j_off"))]
+        return lib.p3t_soft_dispatch_index(tag, ng, p[0], VP(cnt.ctypes.data), p[1], VP(nj.ctypes.data), (VP * ng)(),
+                                           VP(ns.ctypes.data), VP(epj.ctypes.data), len(epj), VP(L["spj"].ctypes.data), 1, send)
+
+    def retrieve(tag):
+        return lib.p3t_soft_retrieve(tag, ng, VP(cnt.ctypes.data),
+                                     (VP * ng)(*[out.ctypes.data + 32 * int(o) for o in L["i_off"][:-1]]))
+
+    assert dispatch(0, bad, 1) == 0 and dispatch(1, L["j_idx"], 0) == 0
+    assert retrieve(0) == 2 and retrieve(1) == 0
+    assert dispatch(0, bad, 0) == 0
+    assert lib.p3t_status() == 2 and lib.p3t_status() == 0
+    assert retrieve(0) == 0
