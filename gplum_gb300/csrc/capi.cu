@@ -1,5 +1,6 @@
 // C ABI of the P3T soft-force path (declarations and contracts in
 // include/gplum_p3t.h).  One process-wide context bound to one GPU.
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -39,7 +40,8 @@ Context *ctx_get(int device) {
     cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
     const int prio = (prio_hi < prio_lo) ? prio_hi + 1 : prio_hi;
     if (cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, prio) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio_hi) != cudaSuccess) {
+        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&c->pair, cudaStreamNonBlocking, prio) != cudaSuccess) {
         delete c;
         return nullptr;
     }
@@ -260,6 +262,8 @@ int p3t_finalize(void) {
     cudaFree(c->status);
     cudaStreamSynchronize(c->side);
     cudaStreamDestroy(c->side);
+    cudaStreamSynchronize(c->pair);
+    cudaStreamDestroy(c->pair);
     cudaStreamDestroy(c->stream);
     delete c;
     g_ctx = nullptr;
@@ -356,7 +360,7 @@ int p3t_upload_lists(int n_group, const int *i_off, const int *i_idx, const int 
     u.add(d.spj.p, spj, (size_t)n_spj * sizeof(SPJRec));
     d.order_valid = false;
     r = u.issue();
-    if (!r) r = cuda_status(launch_group_order(n_group, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p, c->stream));
+    if (!r) r = cuda_status(launch_group_order(n_group, d.i_off.p, d.j_off.p, d.s_off.p, nullptr, d.order.p, nullptr, c->stream));
     const int e = cuda_status(cudaStreamSynchronize(c->stream));  // the caller's lists are read
     if (r || e) return r ? r : e;
     c->res_groups = n_group;
@@ -386,6 +390,64 @@ int p3t_download_forces(void *force, int n) {
         std::memcpy(force, c->h_out, (size_t)n * sizeof(ForceRec));
     }
     return read_status(c);
+}
+
+// The pair kernel over groups as their bodies arrive.  The lists and the
+// superparticles are on the stream already; the bodies follow in up to GO_STAGES parts
+// on the side stream, and a group runs with the part that holds the last body it
+// needs, every second part on a stream of its own, so that a part's last CTAs
+// share the chip with the next part's first.  Bodies in tree order (as FDPS
+// passes them) make a group's bodies near each other; any other order is right
+// too, and ends with most groups in the last part.  The host waits once for the
+// parts' sizes, while the bodies travel.
+// A part costs its launches and the tail of its last groups (a group of 256 bodies
+// takes some 75 us alone), so it has PART_GROUPS groups or more: groups of up to
+// 256, 1M bodies (8,590 groups) 1.86 -> 1.61 ms in eight parts (four: 1.76), 800,000
+// 1.43 -> 1.29, 600,000 (5,050 groups) 1.09 -> 1.00, 400,000 (3,568) 0.74 -> 0.75: not
+// below STAGED_GROUPS or STAGED_BODIES.
+constexpr int STAGED_BODIES = 524288, STAGED_GROUPS = 4500, PART_GROUPS = 1000;
+static int run_staged(Context *c, DevSet &d, const PackArgs &K, SoftArgs A) {
+    const int n = K.one.nj, ng = A.n_group, parts = std::max(2, std::min(GO_STAGES, ng / PART_GROUPS));
+    const int per = (n + parts - 1) / parts;
+    int r = 0;
+    for (auto &e : c->stage_ev)
+        if (!e && (r = cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)))) return r;
+    cudaEvent_t *const ev = c->stage_ev, lists = ev[GO_STAGES], sizes = ev[GO_STAGES + 1];
+    if ((r = d.stage.reserve((size_t)ng + GO_STAGES)) || (r = grow_host(&c->h_out, &c->h_out_cap, GO_STAGES * sizeof(int))))
+        return r;
+    int *const start = d.stage.p + ng, *const h = (int *)c->h_out;
+    PackArgs S = K;  // the superparticles
+    S.one.nj = 0;
+    if ((r = cuda_status(launch_pack_walks(S, S.one.ns, c->stream))) || (r = cuda_status(cudaEventRecord(lists, c->stream))) ||
+        (r = cuda_status(cudaStreamWaitEvent(c->side, lists, 0))))
+        return r;
+    for (int s = 0; s < parts; s++) {
+        PackArgs B = K;
+        const int first = std::min(n, s * per);
+        B.one.ns = 0;
+        B.one.epj = (const EPJRec *)K.one.epj + first;
+        B.one.nj = std::min(per, n - first);
+        B.one.jo = first;
+        if ((r = cuda_status(launch_pack_walks(B, B.one.nj, c->side))) || (r = cuda_status(cudaEventRecord(ev[s], c->side))))
+            return r;
+    }
+    if ((r = cuda_status(launch_group_stage(ng, d.i_off.p, d.i_idx.p, d.j_off.p, d.j_idx.p, n, per, d.stage.p, c->stream))) ||
+        (r = cuda_status(launch_group_order(ng, d.i_off.p, d.j_off.p, d.s_off.p, d.stage.p, d.order.p, start, c->stream))) ||
+        (r = cuda_status(cudaMemcpyAsync(h, start, GO_STAGES * sizeof(int), cudaMemcpyDeviceToHost, c->stream))) ||
+        (r = cuda_status(cudaEventRecord(sizes, c->stream))) || (r = cuda_status(cudaStreamWaitEvent(c->pair, sizes, 0))) ||
+        (r = cuda_status(cudaEventSynchronize(sizes))))
+        return r;
+    A.n_group_all = ng;
+    for (int s = 0; s < parts; s++) {
+        const int first = h[s], last = s + 1 < parts ? h[s + 1] : ng;
+        const cudaStream_t st = s & 1 ? c->pair : c->stream;
+        A.group_order = d.order.p + first;
+        A.n_group = last - first;
+        if ((r = cuda_status(cudaStreamWaitEvent(st, ev[s], 0))) || (r = cuda_status(launch_soft(A, c->precision, false, st))))
+            return r;
+    }
+    if ((r = cuda_status(cudaEventRecord(sizes, c->pair)))) return r;
+    return cuda_status(cudaStreamWaitEvent(c->stream, sizes, 0));
 }
 
 // One call, host buffers in and out, with a single wait.  The link bounds what
@@ -432,12 +494,14 @@ int p3t_soft_force_host(int n, const void *epj, int n_group, const int *i_off, c
     // an early return leaves no copy of this call running (the caller's
     // buffers and the staging buffer are reused afterwards)
     auto fail = [&](int e) {
-        cudaStreamSynchronize(c->stream);
+        for (cudaStream_t s : {c->side, c->pair, c->stream}) cudaStreamSynchronize(s);
         return e;
     };
-    if ((r = u.issue()) ||
-        (r = cuda_status(launch_group_order(n_group, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p, c->stream))) ||
-        (r = cuda_status(launch_pack_walks(K, (long long)n + n_spj, c->stream))))
+    const bool staged = n >= STAGED_BODIES && n_group >= STAGED_GROUPS && K.one.epj == epj;
+    if ((r = u.issue())) return fail(r);
+    if (!staged &&
+        ((r = cuda_status(launch_group_order(n_group, d.i_off.p, d.j_off.p, d.s_off.p, nullptr, d.order.p, nullptr, c->stream))) ||
+         (r = cuda_status(launch_pack_walks(K, (long long)n + n_spj, c->stream)))))
         return fail(r);
     c->res_n = n;
     c->res_groups = n_group;
@@ -451,7 +515,9 @@ int p3t_soft_force_host(int n, const void *epj, int n_group, const int *i_off, c
     // every body is in a group: the forces need no download of their own
     const bool copy = ni == n && is_pinned(force) && device_reads(c, force, 4);
     if (copy) A.force_copy = (ForceRec *)force;
-    if ((r = cuda_status(launch_soft(A, c->precision, false, c->stream)))) return fail(r);
+    if (staged) r = run_staged(c, d, K, A);
+    else r = cuda_status(launch_soft(A, c->precision, false, c->stream));
+    if (r) return fail(r);
     return copy ? read_status(c) : p3t_download_forces(force, n);
 }
 

@@ -67,6 +67,8 @@ constexpr int RADIX_T = 256, RADIX_K = 8, RADIX_TILE = RADIX_T * RADIX_K;  // ke
 constexpr int MAX_LEVEL = 21;                                             // levels below the root
 constexpr int WALK_STACK = 256;
 
+static inline int nblocks(long long n, int t = 256) { return (int)std::max<long long>(1, (n + t - 1) / t); }
+
 // ---- bounding box and keys ------------------------------------------------------
 // doubles as integers of the same order, for minima and maxima beside the FP64 pipe
 __device__ __forceinline__ long long box_key(double x) {
@@ -1198,28 +1200,34 @@ __global__ void k_walk_group_off(const int *jo, const int *so, int ng, int ntop,
     s_off[g] = (g < ng) ? so[(long long)g * ntop] : ns;
 }
 
-// Launch order of the soft kernel: groups by descending weight class (eight
-// classes an octave; the order inside a class is arbitrary, and no result
-// depends on it), a counting sort by one CTA.  A full sort of the weights was 40
+// Launch order of the soft kernel: groups by the stage they belong to (`stage`, 0
+// without one), then by descending weight class (eight classes an octave; the order
+// inside a class is arbitrary, and no result depends on it), a counting sort by one
+// CTA; start[s]: the first place of stage s.  A full sort of the weights was 40
 // launches.
-constexpr int GO_T = 1024, GO_BINS = 1024;
+constexpr int GO_T = 1024, GO_CLASSES = 512, GO_PER = GO_STAGES * GO_CLASSES / GO_T;
 __global__ void __launch_bounds__(GO_T) k_group_order(int ng, const int *i_off, const int *j_off, const int *s_off,
-                                                      int *order) {
-    __shared__ int h[GO_BINS], ws[32];
+                                                      const int *stage, int *order, int *start) {
+    __shared__ int h[GO_STAGES * GO_CLASSES], ws[32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     auto bin = [&](int g) {
         const long long ni = i_off[g + 1] - i_off[g];
         const long long nj = (j_off[g + 1] - j_off[g]) + 2LL * (s_off[g + 1] - s_off[g]);
         const float wt = (float)(((ni + 31) / 32) * 32 * nj + 1);
         const int b = (int)(__float_as_uint(wt) >> 20) - (127 << 3);
-        return GO_BINS - 1 - min(max(b, 0), GO_BINS - 1);
+        return (stage ? stage[g] : 0) * GO_CLASSES + GO_CLASSES - 1 - min(max(b, 0), GO_CLASSES - 1);
     };
-    h[tid] = 0;
+    for (int k = tid; k < GO_STAGES * GO_CLASSES; k += GO_T) h[k] = 0;
     __syncthreads();
     for (int g = tid; g < ng; g += GO_T) atomicAdd(&h[bin(g)], 1);
     __syncthreads();
-    const int c = h[tid];
-    int x = c;
+    int c[GO_PER], sum = 0;
+#pragma unroll
+    for (int k = 0; k < GO_PER; k++) {
+        c[k] = h[GO_PER * tid + k];
+        sum += c[k];
+    }
+    int x = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1228,14 +1236,40 @@ __global__ void __launch_bounds__(GO_T) k_group_order(int ng, const int *i_off, 
     if (lane == 31) ws[w] = x;
     __syncthreads();
     for (int k = 0; k < w; k++) x += ws[k];
-    h[tid] = x - c;
+    x -= sum;
+#pragma unroll
+    for (int k = 0; k < GO_PER; k++) {
+        h[GO_PER * tid + k] = x;
+        x += c[k];
+    }
+    __syncthreads();
+    if (start && tid < GO_STAGES) start[tid] = h[tid * GO_CLASSES];
     __syncthreads();
     for (int g = tid; g < ng; g += GO_T) order[atomicAdd(&h[bin(g)], 1)] = g;
 }
 
-cudaError_t launch_group_order(int ng, const int *i_off, const int *j_off, const int *s_off, int *order,
-                               cudaStream_t st) {
-    if (ng > 0) { P3T_COUNT_LAUNCH(); k_group_order<<<1, GO_T, 0, st>>>(ng, i_off, j_off, s_off, order); }
+cudaError_t launch_group_order(int ng, const int *i_off, const int *j_off, const int *s_off, const int *stage, int *order,
+                               int *start, cudaStream_t st) {
+    if (ng > 0) { P3T_COUNT_LAUNCH(); k_group_order<<<1, GO_T, 0, st>>>(ng, i_off, j_off, s_off, stage, order, start); }
+    return cudaGetLastError();
+}
+
+// The stage of a group whose bodies arrive in stages of `per`: the last of its
+// bodies' and list entries' (a warp per group; entries out of range are the pair
+// kernel's to report).
+__global__ void __launch_bounds__(256) k_group_stage(int ng, const int *i_off, const int *i_idx, const int *j_off,
+                                                     const int *j_idx, int n, int per, int *stage) {
+    const int g = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (g >= ng) return;
+    int last = 0;
+    for (int k = i_off[g] + lane; k < i_off[g + 1]; k += 32) last = max(last, min(i_idx[k], n - 1));
+    for (int k = j_off[g] + lane; k < j_off[g + 1]; k += 32) last = max(last, min(j_idx[k], n - 1));
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) stage[g] = last / per;
+}
+cudaError_t launch_group_stage(int ng, const int *i_off, const int *i_idx, const int *j_off, const int *j_idx, int n,
+                               int per, int *stage, cudaStream_t st) {
+    if (ng > 0) { P3T_COUNT_LAUNCH(); k_group_stage<<<nblocks(32LL * ng), 256, 0, st>>>(ng, i_off, i_idx, j_off, j_idx, n, per, stage); }
     return cudaGetLastError();
 }
 
@@ -1264,7 +1298,6 @@ static int g_walk_last = -1;  // the form the last build's lists came from
 static int g_walk_cap = BFS_CAP;  // frontier items a group's CTA may hold (lower: more groups take the task walk)
 static int g_moments_up = 1;  // moments: leaves in one launch, then inner nodes per level (1); all nodes per level (0)
 
-static inline int nblocks(long long n, int t = 256) { return (int)std::max<long long>(1, (n + t - 1) / t); }
 
 // Builds the tree of the state's bodies and writes the group lists and the
 // SPJ array into the resident soft-force set.  *status: the status bits that the
@@ -1469,7 +1502,7 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
     }
     // 6. the soft kernel's launch order
     if ((r = d.order.reserve(ng))) return r;
-    if ((r = cuda_status(launch_group_order(ng, d.i_off.p, d.j_off.p, d.s_off.p, d.order.p, c->stream)))) return r;
+    if ((r = cuda_status(launch_group_order(ng, d.i_off.p, d.j_off.p, d.s_off.p, nullptr, d.order.p, nullptr, c->stream)))) return r;
     d.order_valid = true;
     c->res_groups = ng;
     c->res_spj = base;

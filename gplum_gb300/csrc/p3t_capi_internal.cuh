@@ -37,7 +37,7 @@ struct DevSet {
     DevBuf<SPJRec> spj;
     DevBuf<SoftSplit> isplit, jsplit;
     DevBuf<SpjPack> spjp;
-    DevBuf<int> i_off, i_idx, j_off, j_idx, s_off, s_idx, order;
+    DevBuf<int> i_off, i_idx, j_off, j_idx, s_off, s_idx, order, stage;
     DevBuf<ForceRec> force;
     DevBuf<D4> acc64;
     DevBuf<int> cand;
@@ -45,7 +45,7 @@ struct DevSet {
     void release() {
         epj_stage.release(); iptcl.release(); i_r_out.release(); i_r_search.release(); ptcl.release(); mass.release(); r_out.release();
         r_search.release(); spj.release(); isplit.release(); jsplit.release(); spjp.release(); i_off.release(); i_idx.release(); j_off.release(); j_idx.release();
-        s_off.release(); s_idx.release(); order.release(); force.release(); acc64.release(); cand.release();
+        s_off.release(); s_idx.release(); order.release(); stage.release(); force.release(); acc64.release(); cand.release();
     }
 };
 
@@ -78,7 +78,9 @@ struct Context {
     int device = 0;
     bool reads_host = false;  // the device reads any host memory in place (it walks the host's page tables)
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;  // the multiwalk calls' reads and writes of the caller's arrays
+    cudaStream_t side = nullptr;  // the soft calls' reads and writes of the caller's arrays
+    cudaStream_t pair = nullptr;  // every second stage of the host call's pair kernel
+    cudaEvent_t stage_ev[10] = {};  // the host call's stages (see p3t_soft_force_host)
     int *status = nullptr;  // device status bits
     double params[21];
     int params_version = 0;
@@ -110,6 +112,10 @@ struct Context {
         if (h_out) cudaFreeHost(h_out);
         h_stage = h_out = nullptr;
         h_stage_cap = h_out_cap = 0;
+        for (auto &e : stage_ev) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
         for (auto &w : walk) w.release();
         fun.release();
     }
@@ -150,9 +156,14 @@ int h2d(Context *c, void *dst, const void *src, size_t bytes);
 int d2h(Context *c, void *dst, const void *src, size_t bytes);
 
 SoftArgs make_args(Context *c, DevSet &d, int n_group, int n_ptcl, int n_spj, bool accumulate);
-// Launch order of the soft kernel's groups, most pair work first.
-cudaError_t launch_group_order(int n_group, const int *i_off, const int *j_off, const int *s_off, int *order,
-                               cudaStream_t st);
+// Launch order of the soft kernel's groups: by stage (optional, 0 .. GO_STAGES - 1),
+// then most pair work first; start (optional, [GO_STAGES]): the stages' first places.
+constexpr int GO_STAGES = 8;
+cudaError_t launch_group_order(int n_group, const int *i_off, const int *j_off, const int *s_off, const int *stage,
+                               int *order, int *start, cudaStream_t st);
+// stage[g]: the last body among group g's own and its EPJ list, / per.
+cudaError_t launch_group_stage(int n_group, const int *i_off, const int *i_idx, const int *j_off, const int *j_idx, int n,
+                               int per, int *stage, cudaStream_t st);
 bool is_pinned(const void *p);
 // Host memory that a kernel may read in place, at `align` bytes.
 bool device_reads(Context *c, const void *p, size_t align);

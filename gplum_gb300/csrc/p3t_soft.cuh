@@ -26,6 +26,7 @@ struct SoftArgs {
     const int *i_off, *i_idx, *j_off, *j_idx, *s_off, *s_idx;
     const int *group_order;  // optional launch order of groups (nullptr = 0..n_group-1)
     int n_group;
+    int n_group_all;  // where a call launches its groups in parts: all of them (0 = n_group)
     // particles and superparticles: i_idx indexes iptcl, j_idx indexes ptcl
     // (the same array in the device-resident form)
     const SoftPtcl *iptcl;

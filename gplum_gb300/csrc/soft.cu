@@ -37,6 +37,7 @@
 // Optional candidate emission: every screen hit (j != i) appends j's particle
 // index to the i's row of a [n x cap] candidate table; the device-side
 // cutoff correction and neighbour search read it instead of a tree query.
+#include <algorithm>
 #include <mutex>
 
 #include "p3t_common.cuh"
@@ -1393,7 +1394,7 @@ cudaError_t launch_soft(const SoftArgs &Ain, int precision, bool emit, cudaStrea
         int dev = 0, sms = 0;
         if (!emit && cudaGetDevice(&dev) == cudaSuccess)
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (!emit && A.n_group <= 3 * sms) {
+        if (!emit && std::max(A.n_group, A.n_group_all) <= 3 * sms) {
             P3T_COUNT_LAUNCH();
             if (A.n_group <= sms) soft_mixed_wide_kernel<512><<<A.n_group, 512, 0, st>>>(A);
             else soft_mixed_wide_kernel<256><<<A.n_group, 256, 0, st>>>(A);
