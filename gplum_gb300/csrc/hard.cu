@@ -1058,16 +1058,15 @@ struct IsoArgs {
 // the bodies outside every cluster (no neighbour), ascending: the drift's
 // threads take one each, every lane busy (a launch over all bodies left
 // nine lanes in ten idle on a disk whose bodies are mostly in clusters)
-__global__ void k_iso_flag(const int32_t *number, int n, int32_t *flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flag[i] = number[i] == 0;
-}
-__global__ void k_iso_list(const int32_t *flag, const int32_t *pos, int n, int32_t *list, int32_t *count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (flag[i]) list[pos[i]] = i;
-    if (i == n - 1) *count = pos[i] + flag[i];
-}
+struct IsoScan {
+    const int32_t *number;
+    int32_t *list, *count;
+    __device__ int operator()(int, int i) const { return number[i] == 0; }
+    __device__ void operator()(int, int i, int prefix, int v) const {
+        if (v) list[prefix] = i;
+    }
+    __device__ void total(int, int t) const { *count = t; }
+};
 
 __device__ void isolated_body(const IsoArgs &A, int i);
 // grid-stride over the list: the grid is sized from the host's count of
@@ -1609,11 +1608,9 @@ int p3t_hard_integrate(int istep) {
     }
     if (E.S.n > 0) {
         const int n = E.S.n;
-        if ((r = g_hb.iso.reserve(3 * (size_t)n + 1))) return r;
-        int32_t *flag = g_hb.iso.p, *pos = flag + n, *list = pos + n;
-        { P3T_COUNT_LAUNCH(); k_iso_flag<<<(n + 255) / 256, 256, 0, c->stream>>>(E.S.number, n, flag); }
-        if ((r = E.scan(flag, pos, n, nullptr))) return r;
-        { P3T_COUNT_LAUNCH(); k_iso_list<<<(n + 255) / 256, 256, 0, c->stream>>>(flag, pos, n, list, list + n); }
+        if ((r = g_hb.iso.reserve((size_t)n + 1))) return r;
+        const IsoScan is{E.S.number, g_hb.iso.p, g_hb.iso.p + n};
+        if ((r = launch_scan_lb(c, E.lb, is, is, n))) return r;
         if ((r = cuda_status(cudaEventRecord(ev_iso_ready, c->stream)))) return r;
     }
     if (nc > 0) {
@@ -1740,7 +1737,7 @@ int p3t_hard_integrate(int istep) {
         I.t0 = (istep - 1) * P.dt_tree;
         I.t1 = istep * P.dt_tree;
         I.status = c->status;
-        I.list = g_hb.iso.p + 2 * (size_t)E.S.n;
+        I.list = g_hb.iso.p;
         I.count = I.list + E.S.n;
         // the bodies outside the clusters: n - members (the device count checks it)
         const int n_iso = std::max(1, E.S.n - E.n_members);

@@ -12,7 +12,7 @@ struct Engine {
     State S;
     int cand_cap_alloc = 0;
     int n_clusters = 0, n_members = 0;
-    DevBuf<int32_t> counters, head, flag, cidx, cl_of, cl_cnt, cl_off, cl_fill, members_tmp, members, keep, kpos,
+    DevBuf<int32_t> counters, head, cidx, cl_of, cl_cnt, cl_off, cl_fill, members_tmp, members, keep, kpos,
         scan_tmp, tflag, tpos;
     DevBuf<int64_t> cmin;
     LookBack lb;
@@ -36,7 +36,7 @@ struct Engine {
     int pack_soft();
     int correct(int initial);
     int cluster();
-    int make_list();
+    int make_list(int *status = nullptr);
     int kick();
     int energy(double *out5);
     int cutoff_radii();
