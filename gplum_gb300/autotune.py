@@ -11,11 +11,12 @@ code:
 * the bundle form's heavy-cluster threshold (p3t_set_hard_heavy: clusters
   whose learned prediction of log2(1 + block steps) reaches it run alone in a
   CTA first) -- the mean hard launch over tree steps 6..25 of whole runs of
-  the hard-part disk (one restored state misjudged it: 5.5 there, 6.75 over
-  the steps, 51.3 against 47.4 ms);
-* whether the bundle form's clusters above 256 bodies run in a concurrent
-  wide launch (lone bundles of up to 512 slots) or one per CTA in the main
-  launch (p3t_set_hard_wide) -- timed from one restored state;
+  the hard-part disk (one restored state misjudges it), and the first steps of
+  four disks, where 6.0 is best in sum (csrc/hard.cu, g_heavy);
+* the bundle form's member slots and CTAs per SM (p3t_set_hard_bundle) and
+  whether its clusters above the slots run in the concurrent wide launch as lone
+  bundles of up to 512 slots or in the team form there (p3t_set_hard_wide) --
+  timed from one restored state;
 * the one-cluster-per-team form's size cutoffs of the hard launch
   (p3t_set_hard_tiers: clusters of >= cta_min members one per CTA, >= warp_min
   one per warp, smaller one per thread) -- timed from one restored state of the

@@ -1331,7 +1331,12 @@ static std::vector<ColRec> g_cols;
 static double g_edisp[2] = {0., 0.};
 static int g_warp_min = 8, g_cta_min = 64;
 static int g_hard_mode = 0;  // 0: bundles, 1: thread/warp/CTA tiers
-static float g_heavy = 6.75f;  // predicted log2(1 + block steps) from which a cluster runs alone (0: never)
+// predicted log2(1 + block steps) from which a cluster runs alone (0: never).  Mean
+// hard launch of the first six steps, ms, at 5.5 / 6.0 / 6.75 / 7.5: 2M wide disk 10.95 /
+// 10.98 / 12.12 / 14.95, 200,000 with embryos 6.7 / 6.6 / 7.2 / 7.5, 50,000 ring 8.4 /
+// 8.6 / 9.0 / 9.1, 1M ring 24.9 / 24.5 / 24.5 / 26.6 (over its steps 6-25 28.8 / 28.2 /
+// 27.5 / -): long chains of the learned order's misjudged clusters start early enough.
+static float g_heavy = 6.0f;
 static int g_wide = 1;        // clusters above 256 members: wide lone bundles (1) or one per CTA (0)
 static int g_bcap = 128;      // bundle member slots (128: three CTAs per SM, 256: one)
 static FragParams g_frag = {0., 9.426627927538057e-12, 10, 0, 0ULL};  // off (a_frag = 0)

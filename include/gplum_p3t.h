@@ -244,7 +244,7 @@ int p3t_set_hard_mode(int mode);
 /* Bundle form with the learned order: clusters whose predicted
  * log2(1 + block steps) is at least log2_steps run first, each alone in a
  * bundle CTA, so the longest chains of block steps do not wait on a full
- * bundle (default 6.75, about 110 block steps; set by the autotuner from
+ * bundle (default 6.0, about 63 block steps; set by the autotuner from
  * whole runs; 0 turns it off).  Results do not depend on it. */
 int p3t_set_hard_heavy(float log2_steps);
 /* Bundle form: clusters above the bundle's member slots run in a second,
