@@ -1337,7 +1337,7 @@ static int g_hard_mode = 0;  // 0: bundles, 1: thread/warp/CTA tiers
 // 8.6 / 9.0 / 9.1, 1M ring 24.9 / 24.5 / 24.5 / 26.6 (over its steps 6-25 28.8 / 28.2 /
 // 27.5 / -): long chains of the learned order's misjudged clusters start early enough.
 static float g_heavy = 6.0f;
-static int g_wide = 1;        // clusters above 256 members: wide lone bundles (1) or one per CTA (0)
+static int g_wide = 1;        // clusters above a bundle's slots: wide lone bundles (1) or one per CTA (0)
 static int g_bcap = 128;      // bundle member slots (128: three CTAs per SM, 256: one)
 static FragParams g_frag = {0., 9.426627927538057e-12, 10, 0, 0ULL};  // off (a_frag = 0)
 static int g_frag_cap = 0;  // fragment slots of the current launch
@@ -1664,6 +1664,7 @@ int p3t_hard_integrate(int istep) {
             static_assert(sizeof(BundleSmem<BCAP_WIDE>) <= 226 * 1024 && sizeof(BundleSmem<256>) <= 226 * 1024,
                           "a large bundle fits an SM");
             static_assert(sizeof(BundleSmem<128>) <= 75 * 1024, "three bundles of 128 slots fit an SM");
+            static_assert(sizeof(BundleSmem<128>) + LONE_EXCL_SMEM > 228 * 1024, "no bundle fits beside an exclusive lone CTA");
             static_assert(sizeof(LoneSmem<LONE_T>) <= LONE_EXCL_SMEM, "the lone state fits its request");
             const bool lone = g_lone > 0.f && g_frag.a_frag <= 0.;
             if (!attr) {

@@ -1,8 +1,8 @@
 // Lone-cluster form of the hard part: the clusters of at most LCAP members
 // that the learned cost model predicts to take the longest chains of block
-// steps, each integrated alone by one CTA whose shared memory holds the whole
-// cluster -- either a 256-thread CTA of the bundle kernel (first, before it
-// packs bundles), or a 128-thread CTA of k_hard_lone holding a whole SM.
+// steps, each integrated alone by one 128-thread CTA of k_hard_lone whose shared
+// memory holds the whole cluster; the CTA holds a whole SM, or shares it with
+// bundles.
 //
 // Such a cluster's time is its chain of block steps, and a block step is a
 // chain of FP64 operations: a warp's FP64 instruction occupies its issue slot
@@ -19,8 +19,8 @@
 // Every value is computed by the same operations in the same order as the
 // team form (run_cluster) and the bundle form, so results are bit-identical;
 // the state lives in shared memory (no global round trips) and each phase is
-// one CTA barrier.  k_hard_lone's shared memory request is large enough that
-// no bundle CTA shares its SM, so its warps have the FP64 unit to themselves.
+// one CTA barrier.  The exclusive placement's shared memory request is large enough
+// that no bundle CTA shares its SM, so its warps have the FP64 unit to themselves.
 //
 // Collisions are rare: a block step that detects one goes, as of its start,
 // to the global state of record, the team form's loop (cluster_loop,
@@ -33,9 +33,9 @@ namespace p3t {
 constexpr int LONE_T = 128;  // threads of a k_hard_lone CTA
 constexpr int LCAP = 64;     // members of a lone cluster at most
 constexpr int LRING = 256;   // live pair items per drain
-// k_hard_lone's shared memory request: large enough that no bundle CTA fits
-// beside it on its SM, so its warps have the FP64 unit to themselves
-constexpr int LONE_EXCL_SMEM = 132 * 1024;
+// k_hard_lone's shared memory request for an SM of its own: large enough that no
+// bundle CTA (74 KB) fits beside it in the SM's 228 KB
+constexpr int LONE_EXCL_SMEM = 160 * 1024;
 
 // the state of one lone cluster, for a CTA of NT threads (the last warp
 // computes the sun force beside the pair terms)
