@@ -145,6 +145,7 @@ struct Uploader {
     // sources and the staging buffer must stay untouched until the stream has
     // run them)
     int issue();
+    bool in_one_launch(int &r);
     // waits for the copies as well: the caller's and the staging buffers may be
     // reused afterwards
     int flush();
