@@ -86,11 +86,12 @@ struct FragParams {
 };
 
 // What a cluster's integration keeps for its end: start time of the log, the
-// energy its collisions dissipated, fragments and collisions made (bundle form).
+// energy its collisions dissipated, fragments and collisions made (bundle form);
+// pair sweeps and block steps so far of one that goes on in another bundle.
 struct ClusterRec {
-    long long t0, n_frag;
+    long long t0, n_frag, work;
     double ed, edd;
-    int n_col;
+    int n_col, steps;
 };
 
 // parameters at their neutral value, whose operations are exact no-ops
@@ -103,7 +104,8 @@ struct HardArgs {
     const int32_t *off, *cnt, *members, *order;
     int n_clusters;
     const int *n_tier;   // [3] clusters per tier, in `order` (device)
-    int32_t *queue;      // [3] tier queue heads
+    int32_t *queue;      // [6] tier queue heads, the lone form's; clusters left, their queue's head
+    int32_t *left;       // bundle form: clusters whose fragments outgrew their bundle
     long long *cost;     // optional [2 * n_clusters]: block steps, pair sweeps
     long long *times;    // optional [2 * n_clusters]: start, end (global timer, ns)
     double *cl_edisp;  // [2 * n_clusters]
@@ -1281,7 +1283,7 @@ __global__ void k_order_scatter(const int32_t *bin, int nc, int32_t *offs, int32
 struct HardBufs {
     DevBuf<double> d;
     DevBuf<int64_t> id;
-    DevBuf<int32_t> i32, order, queue, n_cols;
+    DevBuf<int32_t> i32, order, queue, left, n_cols;
     DevBuf<double> cl_edisp;
     DevBuf<ColRec> cols;
     DevBuf<long long> cost, times;
@@ -1523,10 +1525,10 @@ int p3t_hard_enqueue(void) {
     int r = 0;
     if (g_frag.a_frag > 0. && g_hard_mode != 0) return ST_BAD_INDEX;  // fragments need the bundle form
     g_frag_cap = (g_frag.a_frag > 0.) ? std::max(1024, g_frag.n_frag_max * 4096) : 0;
-    if ((r = B.reserve(E.n_members + g_frag_cap)) || (r = B.order.reserve(nc)) || (r = B.queue.reserve(4)) ||
+    if ((r = B.reserve(E.n_members + g_frag_cap)) || (r = B.order.reserve(nc)) || (r = B.queue.reserve(6)) ||
         (r = B.n_cols.reserve(1)) || (r = B.cl_edisp.reserve(2 * (size_t)nc + 2)) ||
         (r = B.cols.reserve(4096)) || (r = B.frags.reserve(g_frag_cap + 1)) || (r = B.n_frags.reserve(1)) ||
-        (r = B.live.reserve(2)) || (r = B.crec.reserve(nc)))
+        (r = B.live.reserve(2)) || (r = B.crec.reserve(nc)) || (r = B.left.reserve(nc)))
         return r;
     cudaMemsetAsync(B.n_frags.p, 0, sizeof(int32_t), c->stream);
     cudaMemsetAsync(B.live.p, 0, 2 * sizeof(unsigned long long), c->stream);
@@ -1573,7 +1575,7 @@ int p3t_hard_enqueue(void) {
     g_prio.clear();
     if ((r = B.cost.reserve(2 * (size_t)nc + 2)) || (r = B.times.reserve(2 * (size_t)nc + 2))) return r;
     cudaMemsetAsync(B.cost.p, 0, (2 * (size_t)nc + 2) * sizeof(long long), c->stream);
-    cudaMemsetAsync(B.queue.p, 0, 4 * sizeof(int32_t), c->stream);
+    cudaMemsetAsync(B.queue.p, 0, 6 * sizeof(int32_t), c->stream);
     cudaMemsetAsync(B.n_cols.p, 0, sizeof(int32_t), c->stream);
     g_enqueued = nc;
     return cuda_status(cudaGetLastError());
@@ -1630,6 +1632,7 @@ int p3t_hard_integrate(int istep) {
         A.n_clusters = nc;
         A.n_tier = B.ntier.p;
         A.queue = B.queue.p;
+        A.left = B.left.p;
         A.cost = B.cost.p;
         A.times = B.times.p;
         A.cl_edisp = B.cl_edisp.p;
@@ -1709,7 +1712,7 @@ int p3t_hard_integrate(int istep) {
                     return r;
             }
             if (wide_ctas > 0) {
-                { P3T_COUNT_LAUNCH(); k_hard_wide<<<wide_ctas, WT, smem_w, s_wide>>>(A); }
+                { P3T_COUNT_LAUNCH(); k_hard_wide<<<wide_ctas, WT, smem_w, s_wide>>>(A, 0); }
                 if ((r = cuda_status(cudaGetLastError()))) return r;
             }
             // persistent: as many CTAs as the SMs hold (fewer when there are few clusters)
@@ -1724,7 +1727,12 @@ int p3t_hard_integrate(int istep) {
                                   (r = cuda_status(cudaStreamWaitEvent(c->stream, ev_done, 0)))))
                 return r;
             if (lone_k && (r = cuda_status(cudaStreamWaitEvent(c->stream, ev_lone, 0)))) return r;
-            // the launch's time spans all three forms
+            // the clusters that left their bundles (rarely any: then 5 us)
+            if (g_frag.a_frag > 0.) {
+                { P3T_COUNT_LAUNCH(); k_hard_wide<<<std::min(nc, std::max(1, sms / 8)), WT, smem_w, c->stream>>>(A, 1); }
+                if ((r = cuda_status(cudaGetLastError()))) return r;
+            }
+            // the launch's time spans all forms
             if ((r = cuda_status(cudaEventRecord(g_ev_launch[1], c->stream)))) return r;
             g_launch_timed = true;
         } else {

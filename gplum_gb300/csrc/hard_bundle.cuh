@@ -76,7 +76,7 @@ __host__ __device__ constexpr int bundle_list_cap(int cap) { return cap >= 256 ?
 constexpr int BSURV = 64;    // colliding-pair candidates kept per block step
 constexpr int BCLAIM = 8;    // clusters claimed from the queue at a time
 
-enum : int { CF_COL = 1, CF_FIN = 2, CF_FRESH = 4, CF_EXACT = 8 };
+enum : int { CF_COL = 1, CF_FIN = 2, CF_GONE = 4, CF_EXACT = 8 };  // GONE: goes on in k_hard_wide
 enum : unsigned char { MF_ACT = 1, MF_TGT = 2 };
 // fields of a member slot (three components from each vector's first); F_N*:
 // the running pass's forces of a target, in the order of F_AS..F_JD
@@ -1019,7 +1019,7 @@ __device__ __noinline__ void bundle_refill(const HardArgs &A) {
                     B.c_idx[k] = c;
                     B.c_off[k] = 0;
                     B.c_n[k] = A.cnt[c];
-                    B.c_flags[k] = CF_FRESH;
+                    B.c_flags[k] = 0;
                     B.used = B.c_n[k];
                     lone = 1;
                 } else {
@@ -1071,7 +1071,7 @@ __device__ __noinline__ void bundle_refill(const HardArgs &A) {
                     B.c_idx[k] = c;
                     B.c_off[k] = B.used;
                     B.c_n[k] = n;
-                    B.c_flags[k] = CF_FRESH;
+                    B.c_flags[k] = 0;
                     B.used += n;
                     B.i_pend++;
                 }
@@ -1270,8 +1270,10 @@ __device__ __forceinline__ void bundle_move(BundleSmem<BCAP> &B, const int *mv_n
     __syncthreads();
 }
 
-// A cluster made fragments (KOMINAMI): its member range grows by them and the
-// clusters after it move up.
+// Clusters made fragments (KOMINAMI): their member ranges grow by them and the
+// clusters after them move up.  Where the bundle has no room for all, the growing
+// clusters leave it; k_hard_wide takes them up after the launch, from the state of
+// record that their collision has just written, in a bundle of BCAP_WIDE slots each.
 template <int BCAP>
 __device__ __noinline__ void bundle_grow(const HardArgs &A) {
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
@@ -1282,8 +1284,17 @@ __device__ __noinline__ void bundle_grow(const HardArgs &A) {
     const int my_n = (tid < B.ncl) ? B.c_n[tid] : 0;
     int tot;
     const int noff = bscan<BT>(my_n + add, B.ws, tot);
-    if (tot > BCAP) {  // no room: the fragments cannot be integrated here
-        if (tid == 0) atomicOr(A.status, ST_CLUSTER_TOO_BIG);
+    if (tot > BCAP) {
+        if (BCAP == BCAP_WIDE) {  // one cluster: no form has more slots
+            if (tid == 0) atomicOr(A.status, ST_CLUSTER_TOO_BIG);
+        } else if (add > 0) {
+            ClusterRec &R = A.crec[B.c_idx[tid]];
+            R.steps = B.c_steps[tid];
+            R.work = B.c_work[tid];
+            A.left[atomicAdd(&A.queue[4], 1)] = B.c_idx[tid];
+            B.c_flags[tid] = (B.c_flags[tid] & ~CF_COL) | CF_GONE;
+        }
+        __syncthreads();
         return;
     }
     if (tid < B.ncl) B.c_key[tid] = (unsigned long long)(unsigned)noff;  // new offsets, by cluster
@@ -1316,6 +1327,71 @@ __device__ __noinline__ void bundle_grow(const HardArgs &A) {
         }
     }
     if (tid == 0) B.used = tot;
+    __syncthreads();
+}
+
+// slot p of cluster k from the state of record, with its merge lists as slots:
+// twins, their owner, equal ids (every slot's gslot is set)
+template <int BCAP>
+__device__ __forceinline__ void bundle_rejoin(const HardArgs &A, BundleSmem<BCAP> &B, int p, int k) {
+    const Hard &H = A.H;
+    const int g = B.gslot[p], o = B.c_off[k], n = B.c_n[k];
+    bundle_reload(A, B, p, g, k);
+    auto slot_of = [&](int t) {
+        if (t >= 0)
+            for (int q = 0; q < n; q++)
+                if (B.gslot[o + q] == t) return o + q;
+        return -1;
+    };
+    B.twh[p] = (short)slot_of(H.tw_head[g]);
+    B.twn[p] = (short)slot_of(H.tw_next[g]);
+    const int64_t id = H.id[g];
+    int own = -1, eq = p;
+    for (int q = n - 1; q >= 0; q--) {
+        const int gj = B.gslot[o + q];
+        if (H.id[gj] == id) eq = o + q;
+        if (H.merged[gj])
+            for (int t = H.tw_head[gj], gg = 0; t >= 0 && gg < 4096; t = H.tw_next[t], gg++)
+                if (t == g) own = o + q;
+    }
+    B.owner[p] = (short)own;
+    B.eqc[p] = (short)eq;
+    if (B.dead[p]) B.any_dead = 1;
+}
+
+// the clusters of a collision, their members back from the state of record: a
+// full force and first time steps
+template <int BCAP>
+__device__ __noinline__ void bundle_restart(const HardArgs &A) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    const Params &P = A.P;
+    const Hard &H = A.H;
+#pragma unroll 1
+    FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_COL) ? MF_TGT : 0;
+    __syncthreads();
+    const int nc = bundle_full<BCAP>(A, false);
+    bundle_take(B, nc);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nc; i += BT) {
+        const int s = B.tgt[i];
+        if (B.dead[s]) continue;
+        B.d[F_DT][s] = dt_initial(P, B.d[F_TH][s], B.d[F_DT][s], H.acc0[B.gslot[s]], bld(B, F_AD, s), bld(B, F_JD, s),
+                                  bld(B, F_AS, s), bld(B, F_JS, s));
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nc; i += BT) {
+        const int s = B.tgt[i];
+        if (B.merged[s])
+            for (int t = B.twh[s], gg = 0; t >= 0 && gg < BCAP; t = B.twn[t], gg++) B.d[F_DT][t] = B.d[F_DT][s];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nc; i += BT) {
+        const int s = B.tgt[i];
+        B.d[F_TE][s] = B.d[F_TH][s] + B.d[F_DT][s];
+    }
     __syncthreads();
 }
 
@@ -1374,58 +1450,11 @@ __device__ __noinline__ void bundle_collide(const HardArgs &A) {
         const int k = B.cl[p];
         B.flag[p] = 0;
         if (!(B.c_flags[k] & CF_COL)) continue;
-        const int g = B.gslot[p], o = B.c_off[k], n = B.c_n[k];
-        bundle_reload(A, B, p, g, k);
-        // the merge lists as slots: twins, their owner, equal ids
-        auto slot_of = [&](int t) {
-            if (t >= 0)
-                for (int q = 0; q < n; q++)
-                    if (B.gslot[o + q] == t) return o + q;
-            return -1;
-        };
-        B.twh[p] = (short)slot_of(H.tw_head[g]);
-        B.twn[p] = (short)slot_of(H.tw_next[g]);
-        const int64_t id = H.id[g];
-        int own = -1, eq = p;
-        for (int q = n - 1; q >= 0; q--) {
-            const int gj = B.gslot[o + q];
-            if (H.id[gj] == id) eq = o + q;
-            if (H.merged[gj])
-                for (int t = H.tw_head[gj], gg = 0; t >= 0 && gg < 4096; t = H.tw_next[t], gg++)
-                    if (t == g) own = o + q;
-        }
-        B.owner[p] = (short)own;
-        B.eqc[p] = (short)eq;
-        if (B.dead[p]) B.any_dead = 1;
+        bundle_rejoin(A, B, p, k);
     }
     __syncthreads();
     if (B.grew) bundle_grow<BCAP>(A);
-#pragma unroll 1
-    FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_COL) ? MF_TGT : 0;
-    __syncthreads();
-    const int nc = bundle_full<BCAP>(A, false);
-    bundle_take(B, nc);
-#pragma unroll 1
-    for (int i = threadIdx.x; i < nc; i += BT) {
-        const int s = B.tgt[i];
-        if (B.dead[s]) continue;
-        B.d[F_DT][s] = dt_initial(P, B.d[F_TH][s], B.d[F_DT][s], H.acc0[B.gslot[s]], bld(B, F_AD, s), bld(B, F_JD, s),
-                                  bld(B, F_AS, s), bld(B, F_JS, s));
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int i = threadIdx.x; i < nc; i += BT) {
-        const int s = B.tgt[i];
-        if (B.merged[s])
-            for (int t = B.twh[s], gg = 0; t >= 0 && gg < BCAP; t = B.twn[t], gg++) B.d[F_DT][t] = B.d[F_DT][s];
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int i = threadIdx.x; i < nc; i += BT) {
-        const int s = B.tgt[i];
-        B.d[F_TE][s] = B.d[F_TH][s] + B.d[F_DT][s];
-    }
-    __syncthreads();
+    bundle_restart<BCAP>(A);
 }
 
 __device__ __noinline__ double dt_next_general(const HardArgs &A, double time, double dt, double dt_1) {
@@ -1537,6 +1566,55 @@ __device__ __forceinline__ void bundle_dt(const HardArgs &A, BundleSmem<BCAP> &B
     }
 }
 
+// the end of a block step (col: with collisions): each cluster's next step is opened,
+// or the cluster is finished (or gone), which sets any
+template <int BCAP>
+__device__ __forceinline__ void bundle_advance(const HardArgs &A, BundleSmem<BCAP> &B, int used, bool col) {
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    // getSystemTime (src/hermite.h:25-35) and makeActiveList's next time
+    // (src/hermite.h:4-24): the minima of th and th + dt over the alive members
+    if (threadIdx.x == 0) B.any = B.n_sv = B.moved = 0;
+    if (col) {
+#pragma unroll 1
+        FOR_CLUSTERS(k) B.c_key[k] = B.c_tm[k] = dbits(1.e10);
+        __syncthreads();
+    }
+    if (used <= 32 && B.ncl == 1 && !col) {  // one cluster: by a warp
+        if (threadIdx.x < 32) {
+            const int p = threadIdx.x;
+            const bool in = p < used && !B.dead[p];
+            const unsigned long long th = warp_min64(in ? dbits(B.d[F_TH][p]) : ~0ULL),
+                                     te = warp_min64(in ? dbits(B.d[F_TE][p]) : ~0ULL);
+            if (p == 0) {
+                B.c_tm[0] = min(th, dbits(1.e10));
+                B.c_key[0] = min(te, dbits(1.e10));
+            }
+        }
+    } else {
+#pragma unroll 1
+        FOR_SLOTS(p) {
+            if (B.dead[p]) continue;
+            const int k = B.cl[p];
+            atomicMin(&B.c_tm[k], dbits(B.d[F_TH][p]));
+            atomicMin(&B.c_key[k], dbits(B.d[F_TE][p]));
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    FOR_CLUSTERS(k) {
+        const bool going = B.c_tm[k] < dbits(A.t_end) && !(B.c_flags[k] & CF_GONE);
+        if (going && B.c_steps[k] < A.max_steps) {
+            bundle_open(B, k);
+        } else {
+            if (going) atomicOr(A.status, ST_ITER_CAP);
+            B.c_flags[k] |= CF_FIN;
+            B.any = 1;
+        }
+    }
+    __syncthreads();
+    HP_MARK(HP_TIME);
+}
+
 // one block step of every cluster in the bundle (timeIntegrate_multi body,
 // src/hermite.h:224-479), whose time bundle_open has set
 template <int BCAP>
@@ -1622,51 +1700,11 @@ __device__ __forceinline__ void bundle_step(const HardArgs &A, BundleSmem<BCAP> 
     HP_MARK(HP_DT);
     if (col) bundle_collide<BCAP>(A);
     HP_MARK(HP_COLLIDE);
-    // getSystemTime (src/hermite.h:25-35) and makeActiveList's next time
-    // (src/hermite.h:4-24): the minima of th and th + dt over the alive members
-    if (threadIdx.x == 0) B.any = B.n_sv = B.moved = 0;
-    if (col) {
-#pragma unroll 1
-        FOR_CLUSTERS(k) B.c_key[k] = B.c_tm[k] = dbits(1.e10);
-        __syncthreads();
-    }
-    if (used <= 32 && B.ncl == 1 && !col) {  // one cluster: by a warp
-        if (threadIdx.x < 32) {
-            const int p = threadIdx.x;
-            const bool in = p < used && !B.dead[p];
-            const unsigned long long th = warp_min64(in ? dbits(B.d[F_TH][p]) : ~0ULL),
-                                     te = warp_min64(in ? dbits(B.d[F_TE][p]) : ~0ULL);
-            if (p == 0) {
-                B.c_tm[0] = min(th, dbits(1.e10));
-                B.c_key[0] = min(te, dbits(1.e10));
-            }
-        }
-    } else {
-#pragma unroll 1
-        FOR_SLOTS(p) {
-            if (B.dead[p]) continue;
-            const int k = B.cl[p];
-            atomicMin(&B.c_tm[k], dbits(B.d[F_TH][p]));
-            atomicMin(&B.c_key[k], dbits(B.d[F_TE][p]));
-        }
-    }
-    __syncthreads();
-#pragma unroll 1
-    FOR_CLUSTERS(k) {
-        const bool going = B.c_tm[k] < dbits(A.t_end);
-        if (going && B.c_steps[k] < A.max_steps) {
-            bundle_open(B, k);
-        } else {
-            if (going) atomicOr(A.status, ST_ITER_CAP);
-            B.c_flags[k] |= CF_FIN;
-            B.any = 1;
-        }
-    }
-    __syncthreads();
-    HP_MARK(HP_TIME);
+    bundle_advance(A, B, used, col);
 }
 
-// final forces, write-back and removal of the finished clusters
+// final forces, write-back and removal of the finished clusters (those that are gone
+// are only removed)
 template <int BCAP>
 __device__ __noinline__ void bundle_retire(const HardArgs &A) {
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
@@ -1674,7 +1712,7 @@ __device__ __noinline__ void bundle_retire(const HardArgs &A) {
     const Hard &H = A.H;
     const int tid = threadIdx.x;
 #pragma unroll 1
-    FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & CF_FIN) ? MF_TGT : 0;
+    FOR_SLOTS(p) B.flag[p] = (B.c_flags[B.cl[p]] & (CF_FIN | CF_GONE)) == CF_FIN ? MF_TGT : 0;
     __syncthreads();
     const int nt = bundle_full<BCAP>(A, true);
     // write back to FPGrav, with resetTime (src/hard.h:768-787)
@@ -1705,7 +1743,7 @@ __device__ __noinline__ void bundle_retire(const HardArgs &A) {
     }
 #pragma unroll 1
     FOR_CLUSTERS(k) {
-        if (!(B.c_flags[k] & CF_FIN)) continue;
+        if ((B.c_flags[k] & (CF_FIN | CF_GONE)) != CF_FIN) continue;
         const int c = B.c_idx[k];
         const ClusterRec &R = A.crec[c];
         A.cl_edisp[2 * c] = (R.n_col > 0) ? R.ed : 0.;
@@ -1804,12 +1842,61 @@ __device__ __forceinline__ void bundle_close(const HardArgs &A, BundleSmem<BCAP>
         for (int k = 0; k < HP_N; k++) atomicAdd(&A.phase_cycles[k], (unsigned long long)B.ph_acc[k]);
 }
 
+// Cluster c, which a bundle left in bundle_grow, in a wide bundle of its own: members
+// and, in the order they were made, fragments from the state of record, then the rest of
+// that block step.  The bundle's prefilter bounds are not kept: every pair gets its
+// exact test.  False: too many for the wide bundle.
+template <int BCAP>
+__device__ __noinline__ bool bundle_resume(const HardArgs &A, int c) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    constexpr int BT = BundleSmem<BCAP>::NT;
+    const ClusterRec &R = A.crec[c];
+    const int tid = threadIdx.x, n0 = A.cnt[c], n = n0 + (int)R.n_frag, goff = A.off[c];
+    if (n > BCAP) {
+        if (tid == 0) atomicOr(A.status, ST_CLUSTER_TOO_BIG);
+        return false;
+    }
+    if (tid == 0) {
+        B.ncl = 1;
+        B.used = n;
+        B.any_dead = B.n_sv = B.moved = 0;
+        B.c_idx[0] = c;
+        B.c_off[0] = 0;
+        B.c_n[0] = n;
+        B.c_n0[0] = n0;
+        B.c_goff[0] = goff;
+        B.c_addn[0] = 0;
+        B.c_steps[0] = R.steps;
+        B.c_work[0] = R.work;
+        B.c_flags[0] = CF_COL | CF_EXACT;
+        B.c_thrf[0] = B.c_thrc[0] = B.c_E32[0] = 0.f;
+        const V3 r0 = ld3(A.H.pos, goff);
+        B.c_ref[0][0] = r0.x; B.c_ref[1][0] = r0.y; B.c_ref[2][0] = r0.z;
+    }
+#pragma unroll 1
+    for (int p = tid; p < n0; p += BT) B.gslot[p] = goff + p;
+    const int nf = min(*A.n_frags, A.frag_cap);
+#pragma unroll 1
+    for (int k = tid; k < nf; k += BT) {
+        const FragRec &F = A.frags[k];
+        if (F.cluster == c && F.seq >= 0 && n0 + F.seq < n) B.gslot[n0 + F.seq] = F.gslot;
+    }
+    __syncthreads();
+#pragma unroll 1
+    FOR_SLOTS(p) bundle_rejoin(A, B, p, 0);
+    __syncthreads();
+    bundle_restart<BCAP>(A);
+    bundle_advance(A, B, n, true);
+    return true;
+}
+
 // The clusters above a bundle's slots (the queue's tier 0), concurrently with
 // k_hard_bundles: one CTA takes one at a time -- up to A.wide_cap bodies
 // (fragment room included) as a lone wide bundle, larger ones in the
-// one-cluster-per-CTA form.  Same arithmetic, bit for bit, as every other form.
+// one-cluster-per-CTA form.  resume: after k_hard_bundles, the clusters whose
+// fragments outgrew their bundle.  Same arithmetic, bit for bit, as every other form.
 constexpr int WT = bundle_threads(BCAP_WIDE);  // threads of a wide CTA (it holds its SM)
-__global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ HardArgs A) {
+__global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ HardArgs A, int resume) {
     constexpr int BCAP = BCAP_WIDE;
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     __shared__ double red_d[WT / 32];
@@ -1818,36 +1905,40 @@ __global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ Har
     const int tid = threadIdx.x;
     Team<WT> tm{tid, red_d, red_l};
     const int room = (A.frag.a_frag > 0.) ? 2 * A.frag.n_frag_max : 0;
+    const int todo = resume ? A.queue[4] : A.n_tier[0];
     bundle_init(B);
     for (int guard = 0; guard < (1 << 30); guard++) {
-        if (tid == 0) q_sh = atomicAdd(&A.queue[0], 1);
+        if (tid == 0) q_sh = atomicAdd(&A.queue[resume ? 5 : 0], 1);
         __syncthreads();
         const int q = q_sh;
         __syncthreads();
-        if (q >= A.n_tier[0]) break;
-        const int c = A.order[q];
+        if (q >= todo) break;
+        const int c = resume ? A.left[q] : A.order[q];
         const int n = A.cnt[c];
-        if (n > A.wide_cap || n + room > BCAP_WIDE) {
+        if (resume) {
+            if (!bundle_resume<BCAP>(A, c)) continue;
+            if (B.any) bundle_retire<BCAP>(A);
+        } else if (n > A.wide_cap || n + room > BCAP_WIDE) {
             run_cluster<WT>(A, c, tm);
             continue;
+        } else {
+            if (tid == 0) {
+                B.ncl = 1;
+                B.c_idx[0] = c;
+                B.c_off[0] = 0;
+                B.c_n[0] = n;
+                B.c_flags[0] = 0;
+                B.used = n;
+                B.fresh_k = B.fresh_p = 0;
+                B.any_dead = 0;
+            }
+            __syncthreads();
+            bundle_load<BCAP>(A);
         }
-        if (tid == 0) {
-            B.ncl = 1;
-            B.c_idx[0] = c;
-            B.c_off[0] = 0;
-            B.c_n[0] = n;
-            B.c_flags[0] = CF_FRESH;
-            B.used = n;
-            B.fresh_k = B.fresh_p = 0;
-            B.any_dead = 0;
-        }
-        __syncthreads();
-        bundle_load<BCAP>(A);
         // bundle_step advances the cluster by one block step; it retires when done
-        for (int it = 0; it < A.max_steps + 8; it++) {
+        for (int it = 0; it < A.max_steps + 8 && B.ncl > 0; it++) {
             bundle_step(A, B);
             if (B.any) bundle_retire<BCAP>(A);
-            if (B.ncl == 0) break;
         }
         __syncthreads();
     }

@@ -312,8 +312,9 @@ int p3t_set_walk_limits(int frontier_cap, long long store_items);
  * the reference's order.  GPLUM draws the circle's phase from drand48 in
  * OpenMP order; here it is a counter-based draw keyed by (tree step,
  * impactor id, target id, seed).  Needs the bundle form of the hard launch
- * (p3t_set_hard_mode(0)); clusters above its capacity cannot fragment (status
- * bit 16). */
+ * (p3t_set_hard_mode(0)).  A cluster may hold 512 members and fragments in a
+ * tree step, wherever it began; one that would hold more, or that starts with
+ * more than 512 - 2 N_frag members, cannot fragment (status bit 16). */
 int p3t_set_fragmentation(double a_frag, int n_frag, double m_min, unsigned long long seed);
 /* The next particle id the system will hand out (src/main_p3t.cpp:233). */
 long long p3t_id_next(void);
