@@ -111,14 +111,14 @@ int read_status(Context *c) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_status(e);
     if (h) cudaMemsetAsync(c->status, 0, sizeof(int), c->stream);
-    // and the walks' own words
-    auto take = [&](WalkSlot &w) {
-        if (!w.h_tab) return;
-        h |= *(volatile int *)w.h_tab;
-        *(volatile int *)w.h_tab = 0;
-    };
-    for (auto &w : c->walk) take(w);
-    take(c->fun);
+    return h;
+}
+
+int take_word(WalkSlot &w) {
+    if (!w.h_tab) return 0;
+    volatile int *const p = (volatile int *)w.h_tab;
+    const int h = *p;
+    *p = 0;
     return h;
 }
 
@@ -370,7 +370,12 @@ int p3t_synchronize(void) {
 
 int p3t_status(void) {
     CTX_OR_FAIL(c);
-    return read_status(c);
+    int h = read_status(c);  // (drains the stream: the walks' words are complete)
+    if (h < 0) return h;
+    for (auto &w : c->walk) h |= take_word(w);
+    h |= take_word(c->fun) | c->dropped;
+    c->dropped = 0;
+    return h;
 }
 
 // ---- device-resident soft force ---------------------------------------------

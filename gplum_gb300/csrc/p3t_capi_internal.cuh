@@ -104,6 +104,7 @@ struct Context {
     size_t h_out_cap = 0;
     WalkSlot walk[MAX_TAGS];
     WalkSlot fun;  // the single-group functor calls
+    int dropped = 0;  // status bits of dispatches that were never retrieved
 
     void release() {
         res.release();
@@ -124,6 +125,8 @@ struct Context {
 extern Context *g_ctx;
 Context *ctx_get(int device);
 int read_status(Context *c);
+// The status bits that a slot's kernels have set, cleared (no kernel of the slot may run).
+int take_word(WalkSlot &w);
 // Host checks of caller lists before any copy or kernel: CSR offsets start at
 // 0 and never decrease; index arrays and records are present where the
 // offsets say there are entries.  ST_BAD_INDEX otherwise.  (GPLUM trusts

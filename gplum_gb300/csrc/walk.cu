@@ -198,9 +198,12 @@ int functor_call(const void *epi, int ni, const void *epj, int nj, const void *s
         r = cuda_status(launch_soft(walk_args(c, t, w.d, nj, ns, true), c->precision, false, c->stream));
     // also after an error: nothing of this call may still read the caller's records
     const int e = cuda_status(cudaStreamSynchronize(c->stream));
-    if (r || e) return r ? r : e;
+    if (r || e) {
+        take_word(w);
+        return r ? r : e;
+    }
     std::memcpy(force, w.h_out, bytes);
-    return *(volatile int *)t.status() ? read_status(c) : 0;
+    return take_word(w);
 }
 
 // Common tail of both dispatch forms: kernels, events.  Returns once
@@ -233,11 +236,16 @@ int reserve_force(Context *c, WalkSlot &w, int n_i) {
     return on_device(c, n_i) ? w.d.force.reserve(n_i) : grow_host(&w.h_out, &w.h_out_cap, (size_t)n_i * sizeof(ForceRec));
 }
 
-// A dispatch's slot, free of earlier work (a skipped retrieve: the slot is reused in order).
-int claim_slot(WalkSlot &w) {
-    if (!w.busy) return 0;
-    w.busy = false;
-    return cuda_status(cudaEventSynchronize(w.done));
+// A dispatch's slot, free of earlier work (a skipped retrieve: the slot is reused in
+// order, and the status bits of the dispatch that it drops are left to p3t_status).
+int claim_slot(Context *c, WalkSlot &w) {
+    int r = 0;
+    if (w.busy) {
+        w.busy = false;
+        r = cuda_status(cudaEventSynchronize(w.done));
+    }
+    c->dropped |= take_word(w);
+    return r;
 }
 
 }  // namespace
@@ -265,7 +273,7 @@ int p3t_soft_dispatch(int tag, int n_walk, const void **epi, const int *n_epi, c
     WalkSlot &w = *ws;
     WalkTable t{w, n_walk, sizeof(EPJRec), sizeof(SPJRec)};
     int r = 0;
-    if ((r = claim_slot(w)) || (r = t.reserve())) return r;
+    if ((r = claim_slot(c, w)) || (r = t.reserve())) return r;
     for (int k = 0; k < n_walk; k++)
         t.set(k, n_epi[k] ? epi[k] : nullptr, n_epi[k], n_epj[k] ? epj[k] : nullptr, n_epj[k], n_spj[k] ? spj[k] : nullptr,
               n_spj[k]);
@@ -292,7 +300,7 @@ int p3t_soft_dispatch_index(int tag, int n_walk, const void **epi, const int *n_
     WalkSlot &w = *ws;
     WalkTable t{w, n_walk, sizeof(int), sizeof(int)};
     int r = 0;
-    if ((r = claim_slot(w))) return r;
+    if ((r = claim_slot(c, w))) return r;
     DevSet &x = c->idx;
     bool sent = false;  // the resident records are being read in place, on the library's stream
     if (send_flag) {
@@ -360,7 +368,7 @@ int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
     int r = cuda_status(cudaEventSynchronize(w.done));
     w.busy = false;
     if (r) return r;
-    const int status = *(volatile int *)w.h_tab;
+    const int status = take_word(w);  // this dispatch's own bits
     uintptr_t bits = 0;
     int walks = n_walk;  // those that the dispatch covers
     long long off = 0;
@@ -398,8 +406,7 @@ int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
             h += n_epi[k];
         }
     }
-    if (walks < n_walk) return ST_BAD_INDEX;
-    return status ? read_status(c) : 0;
+    return walks < n_walk ? status | ST_BAD_INDEX : status;
 }
 
 }  // extern "C"

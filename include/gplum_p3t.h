@@ -116,7 +116,8 @@ int p3t_epsp(const void *epi, int ni, const void *spj, int nj, void *force);
  * One dispatch carries n_walk i-groups with their EPJ and SPJ lists (EP-EP
  * and EP-SP in one launch); the matching retrieve writes each group's
  * ForceGrav records as ForceGrav::clear followed by both functors.  Up to 8
- * tags may be in flight. */
+ * tags may be in flight.  A retrieve returns the status bits of its own dispatch
+ * (2: a list entry out of range), also with others in flight. */
 int p3t_soft_dispatch(int tag, int n_walk, const void **epi, const int *n_epi, const void **epj,
                       const int *n_epj, const void **spj, const int *n_spj);
 int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force);
@@ -141,7 +142,9 @@ int p3t_upload_lists(int n_group, const int *i_off, const int *i_idx, const int 
 int p3t_soft_run(int emit_candidates);
 /* Copies ForceGrav records (particle order) to the host; synchronizes. */
 int p3t_download_forces(void *force, int n);
-/* Status bits accumulated by kernels since the last call; clears them. */
+/* Status bits accumulated by kernels since the last call; clears them.  Includes the
+ * bits of dispatches not retrieved yet (their retrieve then returns 0) and of those
+ * that were never retrieved. */
 int p3t_status(void);
 /* Host buffers in, host ForceGrav records out, in one call (upload, kernel,
  * download). */
