@@ -28,9 +28,9 @@
 //     max(rs2_i, rs2_j) -- bit-identical to the functor, so neighbour counts,
 //     rank sums and id_min/id_max match exactly;
 //   * forces: FP32 with rsqrt + one Newton step, FMA allowed; partial sums of
-//     32 pairs (16 where few groups share the chip) are folded into an
-//     error-free (TwoSum) FP32 hi/lo pair, so the
-//     accumulation error does not grow with the list length.
+//     32 pairs are folded into an error-free (TwoSum) FP32 hi/lo pair, so the
+//     accumulation error does not grow with the list length.  A group's forces
+//     do not depend on the other groups of the pass, nor on their number.
 // FP64 kernel: the same formulas with every quantity in double, the powers of
 // 1/r rounded once each -- the "plain FP64" form used as the accuracy baseline.
 //
@@ -38,6 +38,7 @@
 // index to the i's row of a [n x cap] candidate table; the device-side
 // cutoff correction and neighbour search read it instead of a tree query.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "p3t_common.cuh"
@@ -141,10 +142,34 @@ struct MixedSmem {
 };
 
 template <int NT, int CAP, int TM, int S, bool EMIT, int UNR>
-__device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, int ni, MixedSmem<NT, CAP> &M, int *scnt) {
+__device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, int ni, MixedSmem<NT, CAP> &M, int *scnt,
+                                            float *P = nullptr) {
     // i-particles [ib, ib + ni) of group g by NT threads, S sub-blocks of W; the
     // origin is the group's first i-particle, as in the functor
-    constexpr int W = NT / S, IPT = 1, CH = NT == SB ? CHUNK : 16;
+    constexpr int W = NT / S, IPT = 1;
+    // More than SB threads: the sub-blocks take a tile's chunks in turn and leave
+    // their partial sums in P[chunk][component][i]; after the tile each (sub-block of
+    // the SB-thread form, component, i) is folded by one thread in that form's order,
+    // FI of them a thread, so the sums are the same bits.
+    constexpr bool WIDE = NT != SB;
+    constexpr int FS = WIDE ? SB / W : S, FI = 4 * SB / NT;
+    float fh[FI], fl[FI];
+#pragma unroll
+    for (int u = 0; u < FI; u++) fh[u] = fl[u] = 0.f;
+    auto fold_tile = [&](int jn) {  // chunks 0 .. jn / 32 of a tile, whose first is a multiple of four
+        constexpr int PER = 4 / FS;  // chunks in a row of one of the SB-thread form's sub-blocks
+        const int n = (jn + CHUNK - 1) / CHUNK;
+#pragma unroll
+        for (int u = 0; u < FI; u++) {
+            const int it = threadIdx.x + u * NT, i = it % W, c = it / W % 4, s = it / (4 * W);
+            if ((i & ~31) >= ni) continue;
+            const float *const p = P + c * W + i;
+            for (int k = s * PER; k < n; k += 4)
+#pragma unroll
+                for (int v = 0; v < PER; v++)
+                    if (k + v < n) fold(fh[u], fl[u], p[(k + v) * 4 * W]);
+        }
+    };
     MixedTile<CAP> &T = M.T;
     float4 *const sI = M.sI;
     int4 *const sQ = M.sQ;
@@ -220,7 +245,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
     // ---- EP-EP ----
     for (int base = 0; base < nj; base += TM) {
         const int nt = min(TM, nj - base);
-        __syncthreads();
+        if (!WIDE) __syncthreads();
         for (int t = tid; t < TM; t += NT) {
             float th = 0.f;
             if (t < nt) {
@@ -257,10 +282,10 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
         __syncthreads();
         // this sub-block's share of the tile, in chunks of 32 entries (the last
         // one of a list may be 16)
-        const int jn = (nt + 15) & ~15, per = NT == SB ? TM / S : ((nt + S - 1) / S + 15) & ~15;
-        const int jb = min(sub * per, jn), je = wact ? min(jb + per, jn) : jb;
-        for (int c0 = jb; c0 < je; c0 += CH) {
-            const int nq = min(CH, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
+        const int jn = (nt + 15) & ~15, jb = WIDE ? sub * CHUNK : min(sub * (TM / S), jn);
+        const int je = !wact ? jb : (WIDE ? jn : min(jb + TM / S, jn));
+        for (int c0 = jb; c0 < je; c0 += WIDE ? S * CHUNK : CHUNK) {
+            const int nq = min(CHUNK, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
             float2 tx[IPT], ty[IPT], tz[IPT], tp[IPT];
             unsigned nm[IPT];
             float thr[IPT];
@@ -268,7 +293,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             for (int k = 0; k < IPT; k++) {
                 tx[k] = ty[k] = tz[k] = tp[k] = dup2(0.f);
                 nm[k] = 0u;
-                thr[k] = fmaxf(thi[k], CH == 16 ? T.te[c0 / 16] : fmaxf(T.te[c0 / 16], T.te[c0 / 16 + 1]));
+                thr[k] = fmaxf(thi[k], fmaxf(T.te[c0 / 16], T.te[c0 / 16 + 1]));
             }
 #pragma unroll UNR
             for (int q = 0; q < nq; q++) {
@@ -294,10 +319,18 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             }
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
-                fold(ahx[k], alx[k], tx[k].x + tx[k].y);
-                fold(ahy[k], aly[k], ty[k].x + ty[k].y);
-                fold(ahz[k], alz[k], tz[k].x + tz[k].y);
-                fold(ahp[k], alp[k], tp[k].x + tp[k].y);
+                if (WIDE) {
+                    float *const p = P + c0 / CHUNK * 4 * W + lane;
+                    p[0] = tx[k].x + tx[k].y;
+                    p[W] = ty[k].x + ty[k].y;
+                    p[2 * W] = tz[k].x + tz[k].y;
+                    p[3 * W] = tp[k].x + tp[k].y;
+                } else {
+                    fold(ahx[k], alx[k], tx[k].x + tx[k].y);
+                    fold(ahy[k], aly[k], ty[k].x + ty[k].y);
+                    fold(ahz[k], alz[k], tz[k].x + tz[k].y);
+                    fold(ahp[k], alp[k], tp[k].x + tp[k].y);
+                }
                 // exact screen of the flagged pairs, in list order
                 unsigned m = vi[k] ? nm[k] : 0u;
                 if (m) {
@@ -333,6 +366,10 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
                 }
             }
         }
+        if (WIDE) {
+            __syncthreads();  // the tile is read, its sums are written
+            fold_tile(jn);
+        }
     }
 
     // ---- EP-SP (quadrupole) ----
@@ -346,7 +383,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
     const float2 c05 = dup2(-0.5f), c25 = dup2(-2.5f);
     for (int base = 0; base < ns; base += TM) {
         const int nt = min(TM, ns - base);
-        __syncthreads();
+        if (!WIDE) __syncthreads();
         for (int t = tid; t < TM; t += NT) {
             if (t < nt) {
                 int q = A.s_idx[s0 + base + t];
@@ -375,10 +412,10 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             }
         }
         __syncthreads();
-        const int jn = (nt + 15) & ~15, per = NT == SB ? TM / S : ((nt + S - 1) / S + 15) & ~15;
-        const int jb = min(sub * per, jn), je = wact ? min(jb + per, jn) : jb;
-        for (int c0 = jb; c0 < je; c0 += CH) {
-            const int nq = min(CH, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
+        const int jn = (nt + 15) & ~15, jb = WIDE ? sub * CHUNK : min(sub * (TM / S), jn);
+        const int je = !wact ? jb : (WIDE ? jn : min(jb + TM / S, jn));
+        for (int c0 = jb; c0 < je; c0 += WIDE ? S * CHUNK : CHUNK) {
+            const int nq = min(CHUNK, je - c0) >> 1;  // entry pairs in this chunk: 16, or 8 at a list's end
             float2 tx[IPT], ty[IPT], tz[IPT], tp[IPT];
 #pragma unroll
             for (int k = 0; k < IPT; k++) tx[k] = ty[k] = tz[k] = tp[k] = dup2(0.f);
@@ -418,21 +455,42 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
             }
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
-                fold(ahx[k], alx[k], tx[k].x + tx[k].y);
-                fold(ahy[k], aly[k], ty[k].x + ty[k].y);
-                fold(ahz[k], alz[k], tz[k].x + tz[k].y);
-                fold(ahp[k], alp[k], tp[k].x + tp[k].y);
+                if (WIDE) {
+                    float *const p = P + c0 / CHUNK * 4 * W + lane;
+                    p[0] = tx[k].x + tx[k].y;
+                    p[W] = ty[k].x + ty[k].y;
+                    p[2 * W] = tz[k].x + tz[k].y;
+                    p[3 * W] = tp[k].x + tp[k].y;
+                } else {
+                    fold(ahx[k], alx[k], tx[k].x + tx[k].y);
+                    fold(ahy[k], aly[k], ty[k].x + ty[k].y);
+                    fold(ahz[k], alz[k], tz[k].x + tz[k].y);
+                    fold(ahp[k], alp[k], tp[k].x + tp[k].y);
+                }
             }
+        }
+        if (WIDE) {
+            __syncthreads();  // the tile is read, its sums are written
+            fold_tile(jn);
         }
     }
 
     // ---- combine sub-blocks in a fixed order and write ForceGrav ----
     if (S > 1) {
-        __syncthreads();
+        if (!WIDE) __syncthreads();
         float *const rf = M.R.f + tid;
         int *const ri = M.R.i + tid;
-        rf[0] = ahx[0]; rf[NT] = alx[0]; rf[2 * NT] = ahy[0]; rf[3 * NT] = aly[0];
-        rf[4 * NT] = ahz[0]; rf[5 * NT] = alz[0]; rf[6 * NT] = ahp[0]; rf[7 * NT] = alp[0];
+        if (WIDE) {
+#pragma unroll
+            for (int u = 0; u < FI; u++) {
+                const int it = tid + u * NT, i = it % W, c = it / W % 4, s = it / (4 * W);
+                M.R.f[2 * c * NT + s * W + i] = fh[u];
+                M.R.f[(2 * c + 1) * NT + s * W + i] = fl[u];
+            }
+        } else {
+            rf[0] = ahx[0]; rf[NT] = alx[0]; rf[2 * NT] = ahy[0]; rf[3 * NT] = aly[0];
+            rf[4 * NT] = ahz[0]; rf[5 * NT] = alz[0]; rf[6 * NT] = ahp[0]; rf[7 * NT] = alp[0];
+        }
         ri[0] = ngb[0]; ri[NT] = rk[0]; ri[2 * NT] = idmax[0]; ri[3 * NT] = idmin[0];
         __syncthreads();
         // a component (0..3: hi and lo of x, y, z, phi; 4..7: the counts) of an i per thread
@@ -442,7 +500,7 @@ __device__ __forceinline__ void group_mixed(const SoftArgs &A, int g, int ib, in
                 float *const h = M.R.f + 2 * c * NT + l;
                 float hi = h[0], lo = h[NT];
 #pragma unroll
-                for (int s = 1; s < S; s++) {
+                for (int s = 1; s < FS; s++) {
                     fold(hi, lo, h[s * W]);
                     lo += h[NT + s * W];
                 }
@@ -512,30 +570,33 @@ __global__ void __launch_bounds__(SB, OCC) soft_mixed_kernel(SoftArgs A) {
     }
 }
 
-// Few groups: NT threads a group, the j list in two or four times as many parts.
-// A call of few groups is bound by one group's chain -- loads of the offsets, the
-// lists and the records one after another, then its pair loops -- and leaves most
-// of the chip idle, so more warps share the loops.  Parts end at multiples of 16
-// entries, the chunk of a partial sum here, so that the forces do not depend on
-// NT or on the parts beyond the hi/lo folds.
-// With the packing launches (9 us), groups of up to 128: 152 groups 33.9 -> 27.7 us
-// with 512 threads (256: 29.8), 304 groups 35.9 -> 31.9 with 256 (512: 33.9); groups
-// of up to 64: 456 groups 33.5 -> 31.5 with 256, 608 groups 35.6 against 36.3 (more
-// CTAs than one wave holds).
+// Few groups: NT threads a group, which share a tile's chunks of 32 entries.  A call of
+// few groups is bound by one group's chain -- loads of the offsets, the lists and the
+// records one after another, then its pair loops -- and leaves most of the chip idle, so
+// more warps share the loops.  With the packing launches (9 us), 128 / 256 / 512 threads:
+// groups of 47 with 190 + 150 entries, 152 groups 33.9 / 29.7 / 26.6 us, 304 groups
+// 36.0 / 31.8 / 33.9; groups of 30 with 165 + 200 entries, 456 groups 33.8 / 31.7 / 39.3,
+// 608 groups 35.7 / 36.6 / 47.8 (more CTAs than one wave holds).
+template <int NT>
+struct WideSmem {
+    MixedSmem<NT, NT> M;
+    float P[NT / CHUNK * 4 * SB];
+};
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 3) soft_mixed_wide_kernel(SoftArgs A) {
-    __shared__ MixedSmem<NT, NT> M;
+    extern __shared__ __align__(16) unsigned char soft_raw[];
+    WideSmem<NT> &B = *reinterpret_cast<WideSmem<NT> *>(soft_raw);
     if (A.gate && *A.gate == A.gate_call) return;
     const int g = A.group_order ? A.group_order[blockIdx.x] : blockIdx.x;
     const int ni_all = A.i_off[g + 1] - A.i_off[g];
     for (int ib = 0; ib < ni_all; ib += SB) {
         const int ni = min(SB, ni_all - ib);
         if (ni > A.t_s1)
-            group_mixed<NT, NT, NT, NT / 128, false, 4>(A, g, ib, ni, M, nullptr);
+            group_mixed<NT, NT, NT, NT / 128, false, 4>(A, g, ib, ni, B.M, nullptr, B.P);
         else if (ni > A.t_s2)
-            group_mixed<NT, NT, NT, NT / 64, false, 4>(A, g, ib, ni, M, nullptr);
+            group_mixed<NT, NT, NT, NT / 64, false, 4>(A, g, ib, ni, B.M, nullptr, B.P);
         else
-            group_mixed<NT, NT, NT, NT / 32, false, 4>(A, g, ib, ni, M, nullptr);
+            group_mixed<NT, NT, NT, NT / 32, false, 4>(A, g, ib, ni, B.M, nullptr, B.P);
         __syncthreads();
     }
 }
@@ -1388,16 +1449,30 @@ cudaError_t launch_soft(const SoftArgs &Ain, int precision, bool emit, cudaStrea
         }
         const int occ = A.occ ? A.occ : 5;
         // groups that leave SMs idle: more threads a group while a group has an SM
-        // (512) or a third of one (256) to itself.  Not where candidates are emitted:
-        // those passes drive an integration, whose roundings do not depend on the
-        // number of groups.
+        // (512) or a third of one (256) to itself (soft_mixed_wide_kernel: both sides of
+        // each line measured).  Candidates are emitted by the 128-thread form only.
         int dev = 0, sms = 0;
         if (!emit && cudaGetDevice(&dev) == cudaSuccess)
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (!emit && std::max(A.n_group, A.n_group_all) <= 3 * sms) {
-            P3T_COUNT_LAUNCH();
-            if (A.n_group <= sms) soft_mixed_wide_kernel<512><<<A.n_group, 512, 0, st>>>(A);
-            else soft_mixed_wide_kernel<256><<<A.n_group, 256, 0, st>>>(A);
+            constexpr int big = (int)sizeof(WideSmem<512>), small = (int)sizeof(WideSmem<256>);
+            static_assert(small <= 48 * 1024 && big <= 100 * 1024, "the partial sums fit beside the tile");
+            if (A.n_group <= sms) {
+                // (above 48 KB of shared memory a kernel must be allowed its size, on each device)
+                static std::atomic<bool> allowed[MAX_DEV];
+                if (dev < 0 || dev >= MAX_DEV) return cudaErrorInvalidDevice;
+                if (!allowed[dev]) {
+                    const cudaError_t e =
+                        cudaFuncSetAttribute(soft_mixed_wide_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+                    if (e != cudaSuccess) return e;
+                    allowed[dev] = true;
+                }
+                P3T_COUNT_LAUNCH();
+                soft_mixed_wide_kernel<512><<<A.n_group, 512, big, st>>>(A);
+            } else {
+                P3T_COUNT_LAUNCH();
+                soft_mixed_wide_kernel<256><<<A.n_group, 256, small, st>>>(A);
+            }
             return cudaGetLastError();
         }
 #define P3T_SOFT_MIXED(OCC)                                                                               \
