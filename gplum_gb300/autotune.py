@@ -10,9 +10,11 @@ code:
   disk (0.5-1.5 AU, m = 1e-10, theta = 0.5, n_group_limit = 256);
 * the bundle form's heavy-cluster threshold (p3t_set_hard_heavy: clusters
   whose learned prediction of log2(1 + block steps) reaches it run alone in a
-  CTA first) -- the mean hard launch over tree steps 6..25 of whole runs of
-  the hard-part disk (one restored state misjudges it), and the first steps of
-  four disks, where 6.0 is best in sum (csrc/hard.cu, g_heavy);
+  CTA first) -- the mean hard launch of the first five tree steps and of the
+  twenty after them (one restored state misjudges it) on five disks of the
+  workloads' kinds (heavy_disks: rings of three sizes, embryos with fragments, a
+  wide disk), by the geometric mean in which the benchmark's disk counts as much as
+  the four others together (heavy_score);
 * the bundle form's member slots and CTAs per SM (p3t_set_hard_bundle) and
   whether its clusters above the slots run in the concurrent wide launch as lone
   bundles of up to 512 slots or in the team form there (p3t_set_hard_wide) --
@@ -100,8 +102,35 @@ def tune_tiers(g, istep=1, grid=TIER_GRID):
     return best, table
 
 
-HEAVY_GRID = (0.0, 5.5, 6.0, 6.5, 6.75, 7.0, 7.5)
-HEAVY_STEPS = (5, 25)  # the hard launch's mean over tree steps 6..25 after start-up
+HEAVY_GRID = (5.0, 5.5, 5.75, 6.0, 6.25, 6.5, 6.75, 7.0, 7.5)
+HEAVY_WINDOWS = ((1, 5), (6, 25))  # tree steps after start-up, first to last
+
+
+def heavy_disks():
+    """(name, function that makes it, a_frag) of each disk the heavy threshold is
+    measured on: the hard-part ring at the benchmark's size and at a quarter and a
+    fiftieth of it, 100,000 planetesimals with embryos and fragmenting collisions, and
+    a wide disk of a million bodies (the large disk's mass)."""
+    from .disk import disk_1m_embryos, disk_1m_hard, make_disk
+
+    return (("ring 1048576", disk_1m_hard, 0.0),
+            ("ring 262144", lambda: disk_1m_hard(262144, seed=11), 0.0),
+            ("ring 20000", lambda: disk_1m_hard(20000, seed=12), 0.0),
+            ("embryos 100000", lambda: disk_1m_embryos(100000, seed=13, m=1e-9), 0.5),
+            ("wide 1048576", lambda: make_disk(1048576, 1e-10, 0.3, 3.0, ecc_hill=4.0, inc_hill=2.0, seed=14), 0.0))
+
+
+def heavy_score(table, bench="ring 1048576"):
+    """{threshold: geometric mean of its times against each row's least} of {row:
+    {threshold: ms}}; the benchmark's rows weigh half, the others half (low thresholds
+    suit small disks, whose launches wait for one chain, and slow down the benchmark's,
+    which the bundles' throughput bounds)."""
+    def loss(h, rows):
+        return np.mean([np.log(r[h] / min(r.values())) for r in rows])
+
+    own = [r for k, r in table.items() if k.startswith(bench)]
+    rest = [r for k, r in table.items() if not k.startswith(bench)]
+    return {h: float(np.exp(0.5 * (loss(h, own) + loss(h, rest)))) for h in own[0]}
 
 
 def tune_heavy(g, istep=1, grid=HEAVY_GRID):
@@ -123,37 +152,37 @@ def tune_heavy(g, istep=1, grid=HEAVY_GRID):
     return best, table
 
 
-def tune_heavy_steps(P, disk, grid=HEAVY_GRID, steps=HEAVY_STEPS):
-    """The heavy-cluster threshold by whole runs: for each threshold, start-up
-    and tree steps 1..steps[1] of `disk` with the learned order, the mean hard
-    launch over the steps after steps[0] (the distribution of chain lengths
-    changes as the disk evolves, so one state misjudges it); installs the
-    fastest.  Returns (best, {threshold: ms})."""
-    import ctypes
-
-    import numpy as np
-
+def tune_heavy_steps(P, disks=None, grid=HEAVY_GRID, windows=HEAVY_WINDOWS):
+    """The heavy-cluster threshold by whole runs with the learned order: for each disk
+    and threshold, start-up and the tree steps of the windows, the mean hard launch of
+    each window (the distribution of chain lengths changes as a disk evolves, so one
+    state misjudges it).  Returns (best by heavy_score, {disk and steps: {threshold:
+    ms}})."""
     from . import scheduler
     from .p3t import GpuSystem
 
     table = {}
-    for h in grid:
-        g = GpuSystem(P)
-        load(g.lib)
-        scheduler.load(lib=g.lib)
-        g.lib.p3t_set_schedule(1)
-        _lib.check(g.lib.p3t_set_hard_heavy(ctypes.c_float(h)), "p3t_set_hard_heavy")
-        g.load(disk)
-        g.set_r_planet()
-        g.startup()
-        hard = []
-        for istep in range(1, steps[1] + 1):
-            g.tree_step(istep)
-            if istep > steps[0]:
-                hard.append(g.step_phases_ms()["hard"])
-        table[h] = float(np.mean(hard))
-    best = min(table, key=table.get)
-    return best, table
+    for name, make, a_frag in disks or heavy_disks():
+        disk = make()
+        for h in grid:
+            g = GpuSystem(P)
+            load(g.lib)
+            scheduler.load(lib=g.lib)
+            g.lib.p3t_set_schedule(1)
+            _lib.check(g.lib.p3t_set_hard_heavy(ctypes.c_float(h)), "p3t_set_hard_heavy")
+            g.set_fragmentation(a_frag)
+            g.load(disk)
+            g.set_r_planet()
+            g.startup()
+            hard = []
+            for istep in range(1, windows[-1][1] + 1):
+                g.tree_step(istep)
+                hard.append(g.hard_launch_stats()["ms"])
+            g.set_fragmentation(0.0)
+            for lo, hi in windows:
+                table.setdefault("%s, steps %d-%d" % (name, lo, hi), {})[h] = float(np.mean(hard[lo - 1:hi]))
+    score = heavy_score(table)
+    return min(score, key=score.get), table
 
 
 # (member slots, CTAs per SM, clusters above the slots in the wide launch)
@@ -259,8 +288,8 @@ def main():
     heavy_best, heavy_table = None, {}
     wide_best, wide_table = tune_wide(g)
     if scheduler.load(lib=g.lib) is not None:
-        heavy_best, heavy_table = tune_heavy_steps(P, d)
-        heavy_best = keep_incumbent(heavy_best, heavy_table, prev.get("hard_heavy"))
+        heavy_best, heavy_table = tune_heavy_steps(P)
+        heavy_best = keep_incumbent(heavy_best, heavy_score(heavy_table), prev.get("hard_heavy"))
         _lib.check(g.lib.p3t_set_hard_heavy(ctypes.c_float(heavy_best)), "p3t_set_hard_heavy")
     if "hard_bundle" in prev and "hard_wide" in prev:
         wide_best = keep_incumbent(wide_best, wide_table, tuple(prev["hard_bundle"]) + (prev["hard_wide"],))
@@ -274,10 +303,12 @@ def main():
            "hard_bundle": list(wide_best[:2]),
            "hard_wide": wide_best[2],
            "hard_bundle_ms": {",".join(map(str, k)): v for k, v in wide_table.items()},
-           "hard_heavy_ms": {str(k): v for k, v in heavy_table.items()},
+           "hard_heavy_ms": {k: {str(h): round(v, 3) for h, v in r.items()} for k, r in heavy_table.items()},
            "hard_ms": {",".join(map(str, k)): v for k, v in hard_table.items()},
            "workloads": {"soft": "1048576-body disk 0.5-1.5 AU, m=1e-10, theta=0.5, n_group_limit=256, tree order",
-                         "hard": "1048576-body hard-part disk 0.95-1.05 AU, m=7e-11, rms e=6h, rms i=3h"}}
+                         "hard": "1048576-body hard-part disk 0.95-1.05 AU, m=7e-11, rms e=6h, rms i=3h",
+                         "hard_heavy": "mean hard launch (ms) over the named tree steps after start-up, learned order; "
+                                       "the disks of gplum_gb300/autotune.py heavy_disks"}}
     json.dump(out, open(args.out, "w"), indent=1)
     print(json.dumps({"soft_tiles": out["soft_tiles"], "soft_ms_best": soft_table[soft_best],
                       "soft_ms_default": soft_table.get((128, 64, 32, 5)), "hard_tiers": out["hard_tiers"],

@@ -1333,11 +1333,14 @@ static std::vector<ColRec> g_cols;
 static double g_edisp[2] = {0., 0.};
 static int g_warp_min = 8, g_cta_min = 64;
 static int g_hard_mode = 0;  // 0: bundles, 1: thread/warp/CTA tiers
-// predicted log2(1 + block steps) from which a cluster runs alone (0: never).  Mean
-// hard launch of the first six steps, ms, at 5.5 / 6.0 / 6.75 / 7.5: 2M wide disk 10.95 /
-// 10.98 / 12.12 / 14.95, 200,000 with embryos 6.7 / 6.6 / 7.2 / 7.5, 50,000 ring 8.4 /
-// 8.6 / 9.0 / 9.1, 1M ring 24.9 / 24.5 / 24.5 / 26.6 (over its steps 6-25 28.8 / 28.2 /
-// 27.5 / -): long chains of the learned order's misjudged clusters start early enough.
+// predicted log2(1 + block steps) from which a cluster runs alone (0: never).  A low
+// value starts the long chains of the clusters that the learned order misjudges early; a
+// high one keeps the bundles full.  Which counts depends on the disk.  Mean hard launch,
+// ms, at 5.0 / 5.75 / 6.0 / 6.75 / 7.5 over steps 1-5 and 6-25: 1,048,576-body ring 26.3 /
+// 24.5 / 24.3 / 25.3 / 30.2 and 30.3 / 27.6 / 27.5 / 26.5 / 30.9; 20,000-body ring 7.5 /
+// 10.0 / 10.0 / 11.0 / 13.6 and 7.2 / 8.0 / 8.2 / 8.4 / 8.6; 1M-body wide disk 7.4 / 8.1 /
+// 8.1 / 8.5 / 9.5 and 9.7 / 9.7 / 9.7 / 10.1 / 11.4 (autotune.py, whose score puts 5.75 and
+// 6.0 within 0.4 %; all of its disks in tuning.json).
 static float g_heavy = 6.0f;
 static int g_wide = 1;        // clusters above a bundle's slots: wide lone bundles (1) or one per CTA (0)
 static int g_bcap = 128;      // bundle member slots (128: three CTAs per SM, 256: one)
