@@ -518,8 +518,9 @@ static int run_staged(Context *c, DevSet &d, const PackArgs &K, SoftArgs A) {
 // the pair kernel does not: the lists go by the copy engine, one launch packs
 // bodies and superparticles from the caller's memory, the launch order is made on
 // the device, and the pair kernel writes each force into the caller's pinned
-// buffer as well as to the device.  1M bodies: 2.19 -> 1.92 ms, of which 0.99 is
-// the pair kernel and 0.88 the link at its 205 GB/s (180 MB in).
+// buffer as well as to the device.  1M bodies: 2.19 -> 1.92 ms with the pair kernel
+// (0.93) behind the link (0.88 at its 205 GB/s, 180 MB in), 1.63 ms with the groups run
+// as their bodies arrive (run_staged).
 int p3t_soft_force_host(int n, const void *epj, int n_group, const int *i_off, const int *i_idx, const int *j_off,
                         const int *j_idx, const int *s_off, const int *s_idx, const void *spj, int n_spj,
                         void *force) {

@@ -1366,7 +1366,7 @@ static int device_tree(Context *c, double theta, int n_leaf_limit, int n_group_l
     cudaMemsetAsync(T.gmark.p, 0, n * sizeof(int), c->stream);
     { P3T_COUNT_LAUNCH(); k_nodes<<<lbk, 256, 0, c->stream>>>(key, n, T.lev.p, T.loff.p, T.lstart.p, T.root.p, base, T.nd.p, T.parent.p,
                                                        T.nch.p, T.list.p, icnt); }
-    // 3. groups in Morton order (their count comes back while the moments run)
+    // 3. groups in Morton order (the host reads their count after the moments' launches)
     { P3T_COUNT_LAUNCH(); k_group_mark<<<nblocks(base), 256, 0, c->stream>>>(base, T.nd.p, T.parent.p, T.nch.p, n_group_limit, T.gmark.p); }
     {
         const GroupScan gs{T.gmark.p, T.gnode.p, d.i_off.p, T.ng.p, n};

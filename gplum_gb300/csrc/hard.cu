@@ -1348,7 +1348,7 @@ static FragParams g_frag = {0., 9.426627927538057e-12, 10, 0, 0ULL};  // off (a_
 static int g_frag_cap = 0;  // fragment slots of the current launch
 static int g_max_steps = MAX_BLOCK_STEPS;  // block-step cap per cluster and tree step
 // lone form: clusters predicted to take at least 2^g_lone - 1 block steps (0:
-// off), on g_lone_ctas CTAs of their own (0: in the bundle CTAs)
+// off), on g_lone_ctas CTAs that hold an SM each (0: one a SM, beside bundles)
 static int g_hard_profile = 0;  // per-phase clock counts of the bundle loop
 static float g_lone = 0.f;
 static int g_lone_ctas = 0;

@@ -343,7 +343,8 @@ __device__ __forceinline__ void bundle_lists_small(const HardArgs &A, BundleSmem
 // The live pairs from item `base` of the targets' (target, partner) items on,
 // until the items end or the list is full: B.list[0..B.ln).  Returns the next
 // item.  mode 0: full (pos of both); 1: predicted i and j; 2: corrected i,
-// predicted j.  exact: FP64 tests for every cluster.  Ends with a barrier.
+// predicted j.  exact: FP64 tests for every cluster.  Ends with the targets' runs
+// (segb, sege) being written: the caller's next barrier comes before they are read.
 template <int BCAP>
 __device__ __forceinline__ int bundle_build(const HardArgs &A, BundleSmem<BCAP> &B, int mode, int nt, int base, bool exact) {
     constexpr int BT = BundleSmem<BCAP>::NT;

@@ -26,6 +26,12 @@
 // to the global state of record, the team form's loop (cluster_loop,
 // one_step) integrates that block step, and the lone form reloads the result
 // -- dead members, merged targets and their twins included -- and goes on.
+//
+// Off by default.  The bundle form's block step has become the shorter one (11-13 us of a
+// lone pair, against 32-38 here): mean hard launch over steps 1-5 and 6-25, off / threshold
+// 8.0 beside bundles / 8.0 on 16 SMs: 1,048,576-body ring 24.6 / 30.0 / 39.8 and 27.7 /
+// 32.9 / 62.6 ms, 20,000-body ring 10.0 / 10.2 / 10.1 and 8.2 / 8.5 / 8.4, 1M-body wide disk
+// 8.1 / 9.7 / 9.7 and 9.6 / 15.2 / 15.2.
 #pragma once
 
 namespace p3t {

@@ -1247,7 +1247,7 @@ __device__ __forceinline__ SpjPack spj_pack(const SPJRec &r, float eps2, int tra
 // whole lines), then each thread packs one from shared memory.  A launch costs the host 4 us, so one launch in place
 // of up to seven (two packs, two splits, the superparticles, three identity
 // lists) is most of a small call: with the records read in place, 3,000 bodies
-// in two dispatches 400 -> 76 us, a group's two functor calls 235 -> 82 us.
+// in two dispatches 400 -> 68 us, a group's two functor calls 235 -> 63 us.
 constexpr int PK = 128, PK_IDX = 1024;  // records, list entries per turn
 template <int W, int STRIDE>
 __device__ __forceinline__ const unsigned long long *stage_records(const void *src, int first, int nt,

@@ -63,7 +63,7 @@ struct WalkTable {
     // Where the records are read.  The kernel reads them in the caller's memory
     // where the device can (60,000 bodies in the index form, four dispatches: the
     // host's copies into pinned buffers, 14-24 GB/s, were 1.2 of a pass's 1.5 ms;
-    // the link gives 150-200 GB/s; now 0.36 ms) and they are aligned as the kernel reads them;
+    // the link gives 150-200 GB/s; a pass now takes 0.28 ms) and they are aligned as the kernel reads them;
     // otherwise they are first copied into the slot's pinned buffer.
     int place(bool reads_host) {
         uintptr_t bits = 0;
@@ -138,7 +138,7 @@ int pack_args(Context *c, WalkTable &t, bool index, PackArgs &A) {
 // Forces of at least this many bytes stay on the device until the retrieve, whose
 // kernel writes them into the caller's arrays; smaller ones go to the slot's
 // pinned buffer and are copied by the host (14-24 GB/s, from a few us; the kernel
-// takes a launch and a wait, 10 us).  60,000 bodies in four dispatches: 360 -> 285 us
+// takes a launch and a wait, 10 us).  60,000 bodies in four dispatches: 360 -> 277 us
 // with the records read on the side stream.
 constexpr size_t SCATTER_BYTES = 192 << 10;
 bool on_device(Context *c, int n_i) { return c->reads_host && (size_t)n_i * sizeof(ForceRec) >= SCATTER_BYTES; }

@@ -101,6 +101,17 @@ int p3t_set_soft_pipe(int on);
 void *p3t_stream(void);
 int p3t_synchronize(void);
 
+/* Host arrays.  Where the device walks the host's page tables (GB300 with a Grace
+ * host), these calls read and write the caller's memory from the device, pinned or
+ * not, and return when they are done with it: p3t_epep, p3t_epsp,
+ * p3t_soft_dispatch and _index (records and index lists), p3t_soft_retrieve
+ * (results of 192 KB and more), p3t_upload_particles, p3t_upload_lists,
+ * p3t_download_forces, p3t_soft_force_host, p3t_state_load, p3t_state_set,
+ * p3t_state_put_fpgrav, p3t_state_get_fpgrav and the snapshot reads.  A count
+ * beyond the memory behind a pointer is then an error of the device context, not
+ * a fault of the process: the arrays must be mapped, writable where they are
+ * results, for every byte that the counts name. */
+
 /* ---- FDPS functor surface --------------------------------------------------------
  * Single-group, synchronous calls with the exact argument list and
  * accumulate-into semantics of GPLUM's functors:
@@ -268,15 +279,13 @@ int p3t_set_hard_bundle(int member_slots, int ctas_per_sm);
  * the whole cluster in shared memory for all its block steps, with the
  * independent parts of a block step (members x components, target x partner
  * pair terms, the sun force, the two time-step criteria) spread over the
- * CTA's threads -- which shortens a block step's chain of FP64 operations
- * (the longest chains of block steps set the launch's span).  ctas = 0: one
- * 128-thread CTA per SM, beside bundles; ctas > 0: that many, each holding a
- * whole SM.  Perfect accretion
- * only (with fragmentation the clusters stay in the bundles); a block step
- * with a collision runs in the one-cluster-per-CTA form's loop and the lone
- * form goes on from its result.  log2_steps = 0:
- * off (the default).  Results are bit-identical.  ctas in [0, 4096].  No
- * counterpart in GPLUM's interface. */
+ * CTA's threads.  ctas = 0: one 128-thread CTA per SM, beside bundles; ctas > 0:
+ * that many, each holding a whole SM.  Perfect accretion only (with
+ * fragmentation the clusters stay in the bundles); a block step with a
+ * collision runs in the one-cluster-per-CTA form's loop and the lone form goes
+ * on from its result.  log2_steps = 0: off (the default: the bundle form is
+ * the faster one on every disk measured).  Results are bit-identical.  ctas in
+ * [0, 4096].  No counterpart in GPLUM's interface. */
 int p3t_set_hard_lone(float log2_steps, int ctas);
 /* Device tree forms.  Bit 0, the walk of the interaction lists: 1 (default)
  * breadth first, one CTA per group, every thread testing cells of the
