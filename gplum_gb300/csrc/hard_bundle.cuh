@@ -117,6 +117,7 @@ struct BundleSmem {
     int pend_c[BCLAIM], pend_n[BCLAIM];
     int ws[NT / 32];
     int used, ncl, fresh_k, fresh_p, n_sv, n_pend, i_pend, exhausted, any, grew, phase;
+    short dn_w[32], dn_b[33];  // bundle_dense: a target's terms of a drain, their places
     int ln, nt, moved, any_dead;  // list entries, targets; a corrected position left the list's margin; dead members
     short tgt[S], cl[S], owner[S], eqc[S], twh[S], twn[S], segb[S], sege[S];
     unsigned char dead[S], merged[S], flag[S];
@@ -786,6 +787,93 @@ __device__ __noinline__ void bundle_merge(int s) {
     }
 }
 
+// The pass's listed pairs where few targets have long runs of them (a cluster of a
+// hundred members or more, all close): terms and in-order sums into the targets'
+// running forces.  A target's sum is a chain of one FP64 addition per pair and
+// component, 64 cycles each, so a drain that holds one target's pairs leaves all but six
+// lanes waiting; here the list is drained in D parts that each hold a D-th of every
+// target's run, and the chains run side by side.  Lone clusters whose pairs are all live,
+// us per block step: 300 members 1665 -> 949, 500 members 5156 -> 2560, 100 members (in
+// 128 threads) 274 -> 248.  Shorter runs lose more to the extra barriers than the chains
+// gain (64 members, runs of 17: 33.1 -> 35.7), and more targets leave too little of a run
+// to a drain.
+constexpr int DENSE_M = 32, DENSE_RUN = 20;  // targets of such a list at most, pairs a target at least
+template <int BCAP>
+__device__ __noinline__ void bundle_dense(const HardArgs &A, int fi, int fj, bool phi, int nt, bool first) {
+    BundleSmem<BCAP> &B = bundle_smem<BCAP>();
+    constexpr int BT = BundleSmem<BCAP>::NT, TC = BundleSmem<BCAP>::TC, PER = TC / BT;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int st = phi ? (6 * TC) / 7 : TC, nc = phi ? 7 : 6;  // components: acc, jerk, phi
+    const int n = B.ln, t0 = B.list[0] >> 16, m = (int)(B.list[n - 1] >> 16) - t0 + 1;
+    const int D = (n + st - m - 1) / (st - m);  // the sum of the runs' D-ths, rounded up, is at most st
+    if (first) {
+#pragma unroll 1
+        for (int i = tid; i < nc * nt; i += BT) {
+            const int c = i / nt;
+            B.d[c < 6 ? F_NAD + c : F_PHD][B.tgt[i - c * nt]] = 0.;
+        }
+        bundle_terms(A, B, fi, fj, phi, 0, 0, nt, st);  // the sun's
+    }
+    __syncthreads();  // (segb and sege)
+    // target t0 + t: its run's D-th, and where that starts among the terms
+    if (tid < 32) {
+        const int w = lane < m ? (B.sege[t0 + lane] - B.segb[t0 + lane] + D - 1) / D : 0;
+        int x = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(ALL, x, o);
+            if (lane >= o) x += y;
+        }
+        B.dn_w[lane] = (short)w;
+        B.dn_b[lane] = (short)(x - w);
+        if (lane == 31) B.dn_b[32] = (short)x;
+    }
+    __syncthreads();
+    const int total = B.dn_b[32];
+    // this thread's places among the terms: next list entry, end of its run, step
+    int q[PER], qe[PER], dq[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int it = tid + u * BT;
+        int t = 0;
+        for (int h = 16; h > 0; h >>= 1)
+            if (t + h < m && B.dn_b[t + h] <= it) t += h;
+        dq[u] = B.dn_w[t];
+        q[u] = B.segb[t0 + t] + it - B.dn_b[t];
+        qe[u] = it < total ? B.sege[t0 + t] : 0;
+    }
+#pragma unroll 1
+    for (int d = 0; d < D; d++) {
+#pragma unroll 1
+        for (int u = 0; u < PER; u++) {
+            const int qu = u == 0 ? q[0] : q[PER - 1], qeu = u == 0 ? qe[0] : qe[PER - 1], du = u == 0 ? dq[0] : dq[PER - 1];
+            const int at = qu + d * du;
+            const bool mine = at < qeu;
+            if (!__any_sync(ALL, mine)) continue;
+            const unsigned e = B.list[mine ? at : 0];
+            pair_terms(A, B, fi, fj, phi, B.tgt[e >> 16], e & 0xffffu, mine, B.term + tid + u * BT, st);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int i = tid; i < nc * m; i += BT) {
+            const int c = i / m, t = i - c * m, w = B.dn_w[t];
+            const int k = min(w, B.sege[t0 + t] - B.segb[t0 + t] - d * w);
+            double *const sum = &B.d[c < 6 ? F_NAD + c : F_PHD][B.tgt[t0 + t]];
+            const double *const p = B.term + c * st + B.dn_b[t];
+            double a = *sum;
+            if (c < 6) {
+#pragma unroll 4
+                for (int u = 0; u < k; u++) a += p[u];
+            } else {
+                for (int u = 0; u < k; u++) a -= p[u];
+            }
+            *sum = a;
+        }
+        __syncthreads();
+    }
+}
+
 // One force pass over the nt targets: list, terms, in-order sums into the
 // targets' running forces, mergeAccJerk for merged targets (in a full pass
 // those with twins).  corr 1, 2: then the first or second correction.  phi: the
@@ -813,6 +901,21 @@ __device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> 
         }
         const int n = B.ln;
         if (tid == 0) B.live[mode == 0 ? 1 : 0] += n;
+        const int m = n > st ? (int)(B.list[n - 1] >> 16) - (int)(B.list[0] >> 16) + 1 : n;
+        if (m <= DENSE_M && n >= DENSE_RUN * m && n > st) {
+            bundle_dense<BCAP>(A, fi, fj, phi, nt, first);
+            first = false;
+            if (corr && !more && !merge) {
+#pragma unroll 1
+                for (int it = tid; it < 3 * nt; it += BT) {
+                    const int t = it / 3, c = it - 3 * t, s = B.tgt[t];
+                    correct_comp(B, s, c, B.d[F_NAS + c][s], B.d[F_NJS + c][s], B.d[F_NAD + c][s], B.d[F_NJD + c][s],
+                                 corr == 2);
+                }
+                __syncthreads();
+            }
+            continue;
+        }
         int q0 = 0;
         do {
             const int np = min(n - q0, st), ns = first ? nt : 0;
