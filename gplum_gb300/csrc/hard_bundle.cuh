@@ -799,6 +799,11 @@ __device__ __noinline__ void bundle_merge(int s) {
 // to a drain.
 constexpr int DENSE_M = 32, DENSE_RUN = 20;  // targets of such a list at most, pairs a target at least
 template <int BCAP>
+__device__ __forceinline__ bool dense_list(const BundleSmem<BCAP> &B, int n) {
+    const int m = (int)(B.list[n - 1] >> 16) - (int)(B.list[0] >> 16) + 1;
+    return m <= DENSE_M && n >= DENSE_RUN * m;
+}
+template <int BCAP>
 __device__ __noinline__ void bundle_dense(const HardArgs &A, int fi, int fj, bool phi, int nt, bool first) {
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     constexpr int BT = BundleSmem<BCAP>::NT, TC = BundleSmem<BCAP>::TC, PER = TC / BT;
@@ -901,27 +906,18 @@ __device__ __forceinline__ void bundle_pass(const HardArgs &A, BundleSmem<BCAP> 
         }
         const int n = B.ln;
         if (tid == 0) B.live[mode == 0 ? 1 : 0] += n;
-        const int m = n > st ? (int)(B.list[n - 1] >> 16) - (int)(B.list[0] >> 16) + 1 : n;
-        if (m <= DENSE_M && n >= DENSE_RUN * m && n > st) {
-            bundle_dense<BCAP>(A, fi, fj, phi, nt, first);
-            first = false;
-            if (corr && !more && !merge) {
-#pragma unroll 1
-                for (int it = tid; it < 3 * nt; it += BT) {
-                    const int t = it / 3, c = it - 3 * t, s = B.tgt[t];
-                    correct_comp(B, s, c, B.d[F_NAS + c][s], B.d[F_NJS + c][s], B.d[F_NAD + c][s], B.d[F_NJD + c][s],
-                                 corr == 2);
-                }
-                __syncthreads();
-            }
-            continue;
-        }
         int q0 = 0;
         do {
-            const int np = min(n - q0, st), ns = first ? nt : 0;
+            int np = min(n - q0, st);
+            const int ns = first ? nt : 0;
             if (!FULL && np <= 8 && ns <= 8) bundle_terms_small(A, B, fi, fj, q0, np, ns, st);
             else if (!phi && ((np + 7) & ~7) + ns <= BT / 4) bundle_terms_split(A, B, fi, fj, q0, np, ns, st);
-            else bundle_terms(A, B, fi, fj, phi, q0, np, ns, st);
+            else if (q0 == 0 && n > st && dense_list(B, n)) {  // terms and sums of the whole list
+                bundle_dense<BCAP>(A, fi, fj, phi, nt, first);
+                first = false;
+                q0 = n;
+                np = 0;
+            } else bundle_terms(A, B, fi, fj, phi, q0, np, ns, st);
             __syncthreads();
             HP_MARK(HP_PAIRS);
             const bool end = q0 + np >= n && !more;
