@@ -103,8 +103,8 @@ struct HardArgs {
     Hard H;
     const int32_t *off, *cnt, *members, *order;
     int n_clusters;
-    const int *n_tier;   // [3] clusters per tier, in `order` (device)
-    int32_t *queue;      // [6] tier queue heads, the lone form's; clusters left, their queue's head
+    const int *n_tier;   // [5] clusters per tier, in `order` (device), heavy ones, k_hard_team's
+    int32_t *queue;      // [7] tier queue heads, the lone form's; clusters left, their queue's head; the team form's
     int32_t *left;       // bundle form: clusters whose fragments outgrew their bundle
     long long *cost;     // optional [2 * n_clusters]: block steps, pair sweeps
     long long *times;    // optional [2 * n_clusters]: start, end (global timer, ns)
@@ -118,7 +118,7 @@ struct HardArgs {
     FragRec *frags;      // [frag_cap] fragments of this launch
     int32_t *n_frags;    // fragments made so far
     int frag_base, frag_cap;  // hard slots frag_base + k hold fragment k
-    int wide_cap;             // bundle form: members of a cluster k_hard_wide takes as a lone wide bundle at most
+    int wide_cap;             // bundle form: members of a cluster that k_hard_wide takes at most; k_hard_team's have more
     int plain;                // PL_* bits
     ClusterRec *crec;         // [n_clusters]
     int max_steps;            // block steps a cluster may take in one tree step (ST_ITER_CAP beyond)
@@ -1205,8 +1205,8 @@ __device__ void isolated_body(const IsoArgs &A, int i) {
 constexpr int ORDER_NB = 4096;
 
 __global__ void k_order_bins(const int32_t *cnt, const float *prio, int nc, int mode, int main_cap, int warp_min, int cta_min,
-                             float pmin, float pscale, int heavy_key, int lone_key, int lone_nmax, int32_t *bin,
-                             int32_t *hist, int32_t *n_heavy) {
+                             float pmin, float pscale, int heavy_key, int lone_key, int lone_nmax, int team_min,
+                             int32_t *bin, int32_t *hist, int32_t *n_heavy) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nc) return;
     const int n = cnt[k];
@@ -1226,6 +1226,7 @@ __global__ void k_order_bins(const int32_t *cnt, const float *prio, int nc, int 
     // steps run alone in a bundle CTA first (they head tier 1, the order
     // being by prediction)
     if (mode == 0 && tier == 1 && key >= heavy_key) atomicAdd(n_heavy, 1);
+    if (mode == 0 && n >= team_min) atomicAdd(n_heavy + 1, 1);
 }
 
 // exclusive offsets of the 3 x ORDER_NB bins (one block of 1024) and the
@@ -1519,6 +1520,11 @@ int p3t_hard_times(long long *out, int n) {
 // queued on the library stream).
 static int g_enqueued = -1;  // cluster count of the enqueued lists
 
+// members of a cluster that k_hard_wide takes at most (it keeps room for a collision's fragments)
+static int wide_most() {
+    return std::min(g_wide ? BCAP_WIDE : BCAP_MAIN, BCAP_WIDE - (g_frag.a_frag > 0. ? 2 * g_frag.n_frag_max : 0));
+}
+
 int p3t_hard_enqueue(void) {
     Engine &E = g_eng;
     if (!E.c) return -(int)cudaErrorNoDevice;
@@ -1528,7 +1534,7 @@ int p3t_hard_enqueue(void) {
     int r = 0;
     if (g_frag.a_frag > 0. && g_hard_mode != 0) return ST_BAD_INDEX;  // fragments need the bundle form
     g_frag_cap = (g_frag.a_frag > 0.) ? std::max(1024, g_frag.n_frag_max * 4096) : 0;
-    if ((r = B.reserve(E.n_members + g_frag_cap)) || (r = B.order.reserve(nc)) || (r = B.queue.reserve(6)) ||
+    if ((r = B.reserve(E.n_members + g_frag_cap)) || (r = B.order.reserve(nc)) || (r = B.queue.reserve(7)) ||
         (r = B.n_cols.reserve(1)) || (r = B.cl_edisp.reserve(2 * (size_t)nc + 2)) ||
         (r = B.cols.reserve(4096)) || (r = B.frags.reserve(g_frag_cap + 1)) || (r = B.n_frags.reserve(1)) ||
         (r = B.live.reserve(2)) || (r = B.crec.reserve(nc)) || (r = B.left.reserve(nc)))
@@ -1543,9 +1549,9 @@ int p3t_hard_enqueue(void) {
     // the bundle capacity first; tier mode: CTA >= g_cta_min > warp >=
     // g_warp_min > thread), then by priority (the caller's, the learned cost
     // model's, else the size), highest first
-    if ((r = B.bin.reserve(nc + 1)) || (r = B.hist.reserve(3 * ORDER_NB)) || (r = B.ntier.reserve(4))) return r;
+    if ((r = B.bin.reserve(nc + 1)) || (r = B.hist.reserve(3 * ORDER_NB)) || (r = B.ntier.reserve(5))) return r;
     cudaMemsetAsync(B.hist.p, 0, 3 * ORDER_NB * sizeof(int32_t), c->stream);
-    cudaMemsetAsync(B.ntier.p, 0, 4 * sizeof(int32_t), c->stream);
+    cudaMemsetAsync(B.ntier.p, 0, 5 * sizeof(int32_t), c->stream);
     if (nc > 0) {
         const float *prio = nullptr;
         float pmin = 0.f, pscale = 1.f;
@@ -1561,6 +1567,7 @@ int p3t_hard_enqueue(void) {
         // members a bundle can admit (with fragmentation it keeps room for a
         // collision's fragments)
         const int main_cap = g_bcap - (g_frag.a_frag > 0. ? 2 * g_frag.n_frag_max : 0);
+        const int team_min = wide_most() + 1;
         // heavy clusters: learned prediction of log2(1 + block steps) >= g_heavy;
         // lone ones: >= g_lone (the lone form is perfect accretion only)
         int heavy_key = 2147483647, lone_key = 2147483647;
@@ -1569,7 +1576,7 @@ int p3t_hard_enqueue(void) {
         if (prio && (int)g_prio.size() != nc && g_lone > 0.f && g_frag.a_frag <= 0. && g_hard_mode == 0)
             lone_key = std::max(0, std::min(ORDER_NB - 1, (int)((g_lone - pmin) * pscale)));
         { P3T_COUNT_LAUNCH(); k_order_bins<<<(nc + 255) / 256, 256, 0, c->stream>>>(E.cl_cnt.p, prio, nc, g_hard_mode, main_cap, g_warp_min, g_cta_min,
-                                                              pmin, pscale, heavy_key, lone_key, LCAP, B.bin.p,
+                                                              pmin, pscale, heavy_key, lone_key, LCAP, team_min, B.bin.p,
                                                               B.hist.p, B.ntier.p + 3); }
         { P3T_COUNT_LAUNCH(); k_order_scan<<<1, 1024, 0, c->stream>>>(B.hist.p, B.ntier.p); }
         { P3T_COUNT_LAUNCH(); k_order_scatter<<<(nc + 255) / 256, 256, 0, c->stream>>>(B.bin.p, nc, B.hist.p, B.order.p); }
@@ -1578,7 +1585,7 @@ int p3t_hard_enqueue(void) {
     g_prio.clear();
     if ((r = B.cost.reserve(2 * (size_t)nc + 2)) || (r = B.times.reserve(2 * (size_t)nc + 2))) return r;
     cudaMemsetAsync(B.cost.p, 0, (2 * (size_t)nc + 2) * sizeof(long long), c->stream);
-    cudaMemsetAsync(B.queue.p, 0, 6 * sizeof(int32_t), c->stream);
+    cudaMemsetAsync(B.queue.p, 0, 7 * sizeof(int32_t), c->stream);
     cudaMemsetAsync(B.n_cols.p, 0, sizeof(int32_t), c->stream);
     g_enqueued = nc;
     return cuda_status(cudaGetLastError());
@@ -1650,7 +1657,7 @@ int p3t_hard_integrate(int istep) {
         A.n_frags = B.n_frags.p;
         A.frag_base = E.n_members;
         A.frag_cap = g_frag_cap;
-        A.wide_cap = g_wide ? BCAP_WIDE : BCAP_MAIN;
+        A.wide_cap = wide_most();
         A.plain = (P.eps2 == 0. ? PL_EPS2 : 0) | (P.eps2_sun == 0. ? PL_EPS2_SUN : 0) | (P.m_sun == 1. ? PL_M_SUN : 0);
         A.crec = B.crec.p;
         A.max_steps = g_max_steps;
@@ -1664,8 +1671,8 @@ int p3t_hard_integrate(int istep) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
         if (g_hard_mode == 0) {
             static bool attr = false;
-            static cudaStream_t s_wide = nullptr, s_lone = nullptr;
-            static cudaEvent_t ev_done = nullptr, ev_lone = nullptr;
+            static cudaStream_t s_wide = nullptr, s_lone = nullptr, s_team = nullptr;
+            static cudaEvent_t ev_done = nullptr, ev_lone = nullptr, ev_team = nullptr;
             const int smem_w = (int)sizeof(BundleSmem<BCAP_WIDE>);
             static_assert(sizeof(BundleSmem<BCAP_WIDE>) <= 226 * 1024 && sizeof(BundleSmem<256>) <= 226 * 1024,
                           "a large bundle fits an SM");
@@ -1687,6 +1694,8 @@ int p3t_hard_integrate(int istep) {
                     (r = cuda_status(cudaStreamCreateWithPriority(&s_lone, cudaStreamNonBlocking, -1000))) ||
                     (r = cuda_status(cudaEventCreateWithFlags(&ev_lone, cudaEventDisableTiming))) ||
                     (r = cuda_status(cudaStreamCreateWithPriority(&s_wide, cudaStreamNonBlocking, -1000))) ||
+                    (r = cuda_status(cudaStreamCreateWithPriority(&s_team, cudaStreamNonBlocking, -1000))) ||
+                    (r = cuda_status(cudaEventCreateWithFlags(&ev_team, cudaEventDisableTiming))) ||
                     (r = cuda_status(cudaEventCreateWithFlags(&ev_done, cudaEventDisableTiming))))
                     return r;
                 attr = true;
@@ -1702,9 +1711,9 @@ int p3t_hard_integrate(int istep) {
             // library stream has drained; its tier sizes then give the wide
             // grid, and both kernels are submitted before the bundle kernel
             // with no dependency left to resolve.
-            int nt[3] = {0, 0, 0};
+            int nt[5] = {0, 0, 0, 0, 0};
             if ((r = d2h(c, nt, B.ntier.p, sizeof(nt)))) return r;  // synchronizes the stream
-            const int wide_ctas = std::min(nt[0], std::max(1, sms / 8));
+            const int most = std::max(1, sms / 8), wide_ctas = std::min(nt[0] - nt[4], most), team_ctas = std::min(nt[4], most);
             if (nt[2] == 0) lone_k = false;
             if (lone_k) {
                 // CTAs of their own hold an SM each; without, they share SMs with bundles
@@ -1718,6 +1727,11 @@ int p3t_hard_integrate(int istep) {
                 { P3T_COUNT_LAUNCH(); k_hard_wide<<<wide_ctas, WT, smem_w, s_wide>>>(A, 0); }
                 if ((r = cuda_status(cudaGetLastError()))) return r;
             }
+            if (team_ctas > 0) {
+                { P3T_COUNT_LAUNCH(); k_hard_team<<<team_ctas, TEAM_T, 0, s_team>>>(A); }
+                if ((r = cuda_status(cudaGetLastError())) || (r = cuda_status(cudaEventRecord(ev_team, s_team))))
+                    return r;
+            }
             // persistent: as many CTAs as the SMs hold (fewer when there are few clusters)
             const int per_sm = g_bcap == 128 ? 3 : 1;
             const int blocks = std::max(1, std::min(sms * per_sm, (nc + 3) / 4));
@@ -1730,6 +1744,7 @@ int p3t_hard_integrate(int istep) {
                                   (r = cuda_status(cudaStreamWaitEvent(c->stream, ev_done, 0)))))
                 return r;
             if (lone_k && (r = cuda_status(cudaStreamWaitEvent(c->stream, ev_lone, 0)))) return r;
+            if (team_ctas > 0 && (r = cuda_status(cudaStreamWaitEvent(c->stream, ev_team, 0)))) return r;
             // the clusters that left their bundles (rarely any: then 5 us)
             if (g_frag.a_frag > 0.) {
                 { P3T_COUNT_LAUNCH(); k_hard_wide<<<std::min(nc, std::max(1, sms / 8)), WT, smem_w, c->stream>>>(A, 1); }

@@ -43,8 +43,8 @@
 // bit-identical to the one-cluster-per-team form; pairs beyond the cutoff
 // contribute exact +-0 terms to accumulators that start at +0.
 // Finished clusters leave the bundle and the queue refills it.  Clusters
-// larger than a bundle run concurrently in k_hard_wide: alone in a wide
-// bundle of BCAP_WIDE slots, or beyond that in the one-cluster-per-CTA form.
+// larger than a bundle run concurrently in k_hard_wide, alone in a wide bundle
+// of BCAP_WIDE slots, or beyond that in k_hard_team, the one-cluster-per-CTA form.
 //
 // Prefilter margins.  FP32 coordinates are taken relative to the cluster's
 // first member, u = fl32(x - ref).  While every stored |x - ref| component
@@ -1991,20 +1991,15 @@ __device__ __noinline__ bool bundle_resume(const HardArgs &A, int c) {
 }
 
 // The clusters above a bundle's slots (the queue's tier 0), concurrently with
-// k_hard_bundles: one CTA takes one at a time -- up to A.wide_cap bodies
-// (fragment room included) as a lone wide bundle, larger ones in the
-// one-cluster-per-CTA form.  resume: after k_hard_bundles, the clusters whose
-// fragments outgrew their bundle.  Same arithmetic, bit for bit, as every other form.
+// k_hard_bundles: one CTA takes one at a time as a lone wide bundle, up to A.wide_cap
+// bodies.  resume: after k_hard_bundles, the clusters whose fragments outgrew their
+// bundle.  Same arithmetic, bit for bit, as every other form.
 constexpr int WT = bundle_threads(BCAP_WIDE);  // threads of a wide CTA (it holds its SM)
 __global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ HardArgs A, int resume) {
     constexpr int BCAP = BCAP_WIDE;
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
-    __shared__ double red_d[WT / 32];
-    __shared__ long long red_l[WT / 32];
     __shared__ int q_sh;
     const int tid = threadIdx.x;
-    Team<WT> tm{tid, red_d, red_l};
-    const int room = (A.frag.a_frag > 0.) ? 2 * A.frag.n_frag_max : 0;
     const int todo = resume ? A.queue[4] : A.n_tier[0];
     bundle_init(B);
     for (int guard = 0; guard < (1 << 30); guard++) {
@@ -2018,8 +2013,7 @@ __global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ Har
         if (resume) {
             if (!bundle_resume<BCAP>(A, c)) continue;
             if (B.any) bundle_retire<BCAP>(A);
-        } else if (n > A.wide_cap || n + room > BCAP_WIDE) {
-            run_cluster<WT>(A, c, tm);
+        } else if (n > A.wide_cap) {  // k_hard_team's
             continue;
         } else {
             if (tid == 0) {
@@ -2043,6 +2037,26 @@ __global__ void __launch_bounds__(WT, 1) k_hard_wide(const __grid_constant__ Har
         __syncthreads();
     }
     bundle_close(A, B);
+}
+
+// The clusters above A.wide_cap (in tier 0, with k_hard_wide's): one CTA takes one at a
+// time in the one-cluster-per-CTA form.  Its pair loops are a thread a target, so it has
+// 512 threads: 600 members 8.76 ms per block step in 256, 6.58 in 512.
+constexpr int TEAM_T = 512;
+__global__ void __launch_bounds__(TEAM_T, 1) k_hard_team(const __grid_constant__ HardArgs A) {
+    __shared__ double red_d[TEAM_T / 32];
+    __shared__ long long red_l[TEAM_T / 32];
+    __shared__ int q_sh;
+    const Team<TEAM_T> tm{(int)threadIdx.x, red_d, red_l};
+    for (int guard = 0; guard < (1 << 30); guard++) {
+        if (threadIdx.x == 0) q_sh = atomicAdd(&A.queue[6], 1);
+        __syncthreads();
+        const int q = q_sh;
+        __syncthreads();
+        if (q >= A.n_tier[0]) break;
+        const int c = A.order[q];
+        if (A.cnt[c] > A.wide_cap) run_cluster<TEAM_T>(A, c, tm);
+    }
 }
 
 // bundles of BCAP member slots until the queue is empty; OCC CTAs per SM

@@ -1,6 +1,7 @@
 """The hard launch's time where clusters are large, against the same launch in another
 form on the same box (the states of both are bit-identical, tests/test_bundle_sizes_gpu.py):
-a lone cluster of 300 and of 500 bodies with all pairs live."""
+a lone cluster of 300 and of 500 bodies with all pairs live, and a lone cluster above the wide
+bundle's slots."""
 import numpy as np
 import pytest
 
@@ -52,3 +53,9 @@ def test_lone_wide_cluster(gpu, n, most):
     time 0.38 and 0.47)."""
     d = clump(n)
     assert hard_ms(d, 1) <= most * hard_ms(d, 1, mode=1)
+
+
+def test_lone_cluster_above_the_wide_bundle(gpu):
+    """In 512 threads against 128 (0.84 of their time; in 256, 0.99)."""
+    d = clump(600)
+    assert hard_ms(d, 1) <= 0.92 * hard_ms(d, 1, mode=1)
