@@ -1345,6 +1345,7 @@ static int g_hard_mode = 0;  // 0: bundles, 1: thread/warp/CTA tiers
 static float g_heavy = 6.0f;
 static int g_wide = 1;        // clusters above a bundle's slots: wide lone bundles (1) or one per CTA (0)
 static int g_bcap = 128;      // bundle member slots (128: three CTAs per SM, 256: one)
+static int g_launch_bcap = 128;  // those of the enqueued launch (few_clusters)
 static FragParams g_frag = {0., 9.426627927538057e-12, 10, 0, 0ULL};  // off (a_frag = 0)
 static int g_frag_cap = 0;  // fragment slots of the current launch
 static int g_max_steps = MAX_BLOCK_STEPS;  // block-step cap per cluster and tree step
@@ -1520,6 +1521,17 @@ int p3t_hard_times(long long *out, int n) {
 // queued on the library stream).
 static int g_enqueued = -1;  // cluster count of the enqueued lists
 
+// Whether every cluster can have an SM of its own.  Then bundles of 256 slots hold them,
+// whose 256 threads take a block step of many pairs faster (a launch of 100 clusters of
+// 60: 3.41 ms against 3.67 in bundles of 128 slots; 100 clusters of 20 0.452 against
+// 0.465; of 3 the same); above it the three smaller bundles of an SM do (300 clusters of
+// 20: 0.570 ms against 0.665, 300 of 60 3.91 against 4.11).
+static bool few_clusters(int device, int nc) {
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return nc <= sms;
+}
+
 // members of a cluster that k_hard_wide takes at most (it keeps room for a collision's fragments)
 static int wide_most() {
     return std::min(g_wide ? BCAP_WIDE : BCAP_MAIN, BCAP_WIDE - (g_frag.a_frag > 0. ? 2 * g_frag.n_frag_max : 0));
@@ -1534,6 +1546,7 @@ int p3t_hard_enqueue(void) {
     int r = 0;
     if (g_frag.a_frag > 0. && g_hard_mode != 0) return ST_BAD_INDEX;  // fragments need the bundle form
     g_frag_cap = (g_frag.a_frag > 0.) ? std::max(1024, g_frag.n_frag_max * 4096) : 0;
+    g_launch_bcap = few_clusters(c->device, nc) ? 256 : g_bcap;
     if ((r = B.reserve(E.n_members + g_frag_cap)) || (r = B.order.reserve(nc)) || (r = B.queue.reserve(7)) ||
         (r = B.n_cols.reserve(1)) || (r = B.cl_edisp.reserve(2 * (size_t)nc + 2)) ||
         (r = B.cols.reserve(4096)) || (r = B.frags.reserve(g_frag_cap + 1)) || (r = B.n_frags.reserve(1)) ||
@@ -1566,7 +1579,7 @@ int p3t_hard_enqueue(void) {
         }
         // members a bundle can admit (with fragmentation it keeps room for a
         // collision's fragments)
-        const int main_cap = g_bcap - (g_frag.a_frag > 0. ? 2 * g_frag.n_frag_max : 0);
+        const int main_cap = g_launch_bcap - (g_frag.a_frag > 0. ? 2 * g_frag.n_frag_max : 0);
         const int team_min = wide_most() + 1;
         // heavy clusters: learned prediction of log2(1 + block steps) >= g_heavy;
         // lone ones: >= g_lone (the lone form is perfect accretion only)
@@ -1732,10 +1745,14 @@ int p3t_hard_integrate(int istep) {
                 if ((r = cuda_status(cudaGetLastError())) || (r = cuda_status(cudaEventRecord(ev_team, s_team))))
                     return r;
             }
-            // persistent: as many CTAs as the SMs hold (fewer when there are few clusters)
-            const int per_sm = g_bcap == 128 ? 3 : 1;
-            const int blocks = std::max(1, std::min(sms * per_sm, (nc + 3) / 4));
-            if (g_bcap == 256)
+            // persistent: as many CTAs as the SMs hold, one a cluster where there are fewer.  (One
+            // for four clusters, of which the first CTA claimed eight, ran clusters of 65 to 128
+            // one after the other: eight of 100 34.7 ms, now 8.2.  Hard launches of eight steps,
+            // with one for four or a half bundle of members / one a cluster: 3,000-body ring, 372
+            // clusters, 24.4 / 20.9 ms; 5,000 bodies, 960 clusters, 28.0 / 27.8.)
+            const int per_sm = g_launch_bcap == 128 ? 3 : 1;
+            const int blocks = std::max(1, std::min(sms * per_sm, nc));
+            if (g_launch_bcap == 256)
                 { P3T_COUNT_LAUNCH(); k_hard_bundles<256, 1><<<blocks, bundle_threads(256), (int)sizeof(BundleSmem<256>), c->stream>>>(A); }
             else
                 { P3T_COUNT_LAUNCH(); k_hard_bundles<128, 3><<<blocks, bundle_threads(128), (int)sizeof(BundleSmem<128>), c->stream>>>(A); }

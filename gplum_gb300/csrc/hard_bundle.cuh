@@ -74,7 +74,7 @@ __host__ __device__ constexpr int bundle_threads(int cap) { return cap >= 256 ? 
 __host__ __device__ constexpr int bundle_terms_cap(int cap) { return 256; }
 __host__ __device__ constexpr int bundle_list_cap(int cap) { return cap >= 256 ? 2048 : 1024; }
 constexpr int BSURV = 64;    // colliding-pair candidates kept per block step
-constexpr int BCLAIM = 8;    // clusters claimed from the queue at a time
+constexpr int BCLAIM = 8;    // clusters claimed from the queue at a time at most
 
 enum : int { CF_COL = 1, CF_FIN = 2, CF_GONE = 4, CF_EXACT = 8 };  // GONE: goes on in k_hard_wide
 enum : unsigned char { MF_ACT = 1, MF_TGT = 2 };
@@ -1106,6 +1106,8 @@ __device__ __noinline__ void bundle_refill(const HardArgs &A) {
     BundleSmem<BCAP> &B = bundle_smem<BCAP>();
     const int lane = threadIdx.x & 31;
     const int n_heavy = A.n_tier[3];
+    // (with few clusters no CTA holds some back that others could take)
+    const int n_claim = max(1, min(BCLAIM, (A.n_tier[1] - n_heavy) / (int)gridDim.x));
     if (threadIdx.x < 32) {
         int lone = 0;
         if (lane == 0 && B.phase == 0) {
@@ -1140,10 +1142,10 @@ __device__ __noinline__ void bundle_refill(const HardArgs &A) {
             if (stop) break;
             if (claim) {
                 int q = 0;
-                if (lane == 0) q = atomicAdd(&A.queue[1], BCLAIM);
+                if (lane == 0) q = atomicAdd(&A.queue[1], n_claim);
                 q = __shfl_sync(0xffffffffu, q, 0);
                 const int qi = q + lane;
-                const bool ok = lane < BCLAIM && qi < A.n_tier[1] - n_heavy;
+                const bool ok = lane < n_claim && qi < A.n_tier[1] - n_heavy;
                 const unsigned m = __ballot_sync(0xffffffffu, ok);
                 if (ok) {
                     const int c = A.order[A.n_tier[0] + n_heavy + qi];
@@ -1154,7 +1156,7 @@ __device__ __noinline__ void bundle_refill(const HardArgs &A) {
                 if (lane == 0) {
                     B.n_pend = __popc(m);
                     B.i_pend = 0;
-                    if (__popc(m) < BCLAIM) B.exhausted = 1;
+                    if (__popc(m) < n_claim) B.exhausted = 1;
                 }
                 __syncwarp();
                 if (m == 0u) break;

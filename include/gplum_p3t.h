@@ -271,7 +271,8 @@ int p3t_set_hard_wide(int on);
 /* Bundle form: member slots per bundle and CTAs per SM asked for -- 128/3
  * (default), 128/4 or 256/2; a bundle keeps all of its members' state in
  * shared memory, so at most three CTAs of 128 slots or one of 256 fit an SM,
- * and a launch uses as many.  Results are bit-identical; set by the autotuner. */
+ * and a launch uses as many.  A launch of at most one cluster per SM always takes
+ * 256 slots.  Results are bit-identical; set by the autotuner. */
 int p3t_set_hard_bundle(int member_slots, int ctas_per_sm);
 /* Bundle form with the learned order: clusters whose predicted
  * log2(1 + block steps) is at least log2_steps and that have at most 64

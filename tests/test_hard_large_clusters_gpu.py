@@ -1,7 +1,7 @@
-"""The hard launch's time where clusters are large, against the same launch in another
+"""The hard launch's time where clusters are large or few, against the same launch in another
 form on the same box (the states of both are bit-identical, tests/test_bundle_sizes_gpu.py):
-a lone cluster of 300 and of 500 bodies with all pairs live, and a lone cluster above the wide
-bundle's slots."""
+a lone cluster of 300 and of 500 bodies with all pairs live, a lone cluster above the wide bundle's
+slots, and copies of one cluster, which run side by side where SMs are free."""
 import numpy as np
 import pytest
 
@@ -59,3 +59,8 @@ def test_lone_cluster_above_the_wide_bundle(gpu):
     """In 512 threads against 128 (0.84 of their time; in 256, 0.99)."""
     d = clump(600)
     assert hard_ms(d, 1) <= 0.92 * hard_ms(d, 1, mode=1)
+
+
+def test_copies_run_side_by_side(gpu):
+    """Eight copies of a cluster of 100 take as long as one (one after the other: eight times)."""
+    assert hard_ms(clump(100, 8), 8) <= 3.0 * hard_ms(clump(100), 1)
