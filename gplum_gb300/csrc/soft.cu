@@ -576,13 +576,15 @@ __global__ void __launch_bounds__(SB, OCC) soft_mixed_kernel(SoftArgs A) {
 // more warps share the loops.  With the packing launches (9 us), 128 / 256 / 512 threads:
 // groups of 47 with 190 + 150 entries, 152 groups 33.9 / 29.7 / 26.6 us, 304 groups
 // 36.0 / 31.8 / 33.9; groups of 30 with 165 + 200 entries, 456 groups 33.8 / 31.7 / 39.3,
-// 608 groups 35.7 / 36.6 / 47.8 (more CTAs than one wave holds).
+// 608 groups 35.7 / 36.6 / 47.8 (more CTAs than one wave holds).  With candidates emitted,
+// 128 threads against these: 60 groups of 50 32.9 -> 22.6 us, 300 groups of 67 45.1 -> 36.9.
 template <int NT>
 struct WideSmem {
     MixedSmem<NT, NT> M;
     float P[NT / CHUNK * 4 * SB];
+    int scnt[SB];
 };
-template <int NT>
+template <int NT, bool EMIT>
 __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 3) soft_mixed_wide_kernel(SoftArgs A) {
     extern __shared__ __align__(16) unsigned char soft_raw[];
     WideSmem<NT> &B = *reinterpret_cast<WideSmem<NT> *>(soft_raw);
@@ -592,11 +594,11 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 3) soft_mixed_wide_kernel(
     for (int ib = 0; ib < ni_all; ib += SB) {
         const int ni = min(SB, ni_all - ib);
         if (ni > A.t_s1)
-            group_mixed<NT, NT, NT, NT / 128, false, 4>(A, g, ib, ni, B.M, nullptr, B.P);
+            group_mixed<NT, NT, NT, NT / 128, EMIT, 4>(A, g, ib, ni, B.M, B.scnt, B.P);
         else if (ni > A.t_s2)
-            group_mixed<NT, NT, NT, NT / 64, false, 4>(A, g, ib, ni, B.M, nullptr, B.P);
+            group_mixed<NT, NT, NT, NT / 64, EMIT, 4>(A, g, ib, ni, B.M, B.scnt, B.P);
         else
-            group_mixed<NT, NT, NT, NT / 32, false, 4>(A, g, ib, ni, B.M, nullptr, B.P);
+            group_mixed<NT, NT, NT, NT / 32, EMIT, 4>(A, g, ib, ni, B.M, B.scnt, B.P);
         __syncthreads();
     }
 }
@@ -1450,11 +1452,10 @@ cudaError_t launch_soft(const SoftArgs &Ain, int precision, bool emit, cudaStrea
         const int occ = A.occ ? A.occ : 5;
         // groups that leave SMs idle: more threads a group while a group has an SM
         // (512) or a third of one (256) to itself (soft_mixed_wide_kernel: both sides of
-        // each line measured).  Candidates are emitted by the 128-thread form only.
+        // each line measured)
         int dev = 0, sms = 0;
-        if (!emit && cudaGetDevice(&dev) == cudaSuccess)
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (!emit && std::max(A.n_group, A.n_group_all) <= 3 * sms) {
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (std::max(A.n_group, A.n_group_all) <= 3 * sms) {
             constexpr int big = (int)sizeof(WideSmem<512>), small = (int)sizeof(WideSmem<256>);
             static_assert(small <= 48 * 1024 && big <= 100 * 1024, "the partial sums fit beside the tile");
             if (A.n_group <= sms) {
@@ -1462,16 +1463,19 @@ cudaError_t launch_soft(const SoftArgs &Ain, int precision, bool emit, cudaStrea
                 static std::atomic<bool> allowed[MAX_DEV];
                 if (dev < 0 || dev >= MAX_DEV) return cudaErrorInvalidDevice;
                 if (!allowed[dev]) {
-                    const cudaError_t e =
-                        cudaFuncSetAttribute(soft_mixed_wide_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+                    const auto what = cudaFuncAttributeMaxDynamicSharedMemorySize;
+                    cudaError_t e = cudaFuncSetAttribute(soft_mixed_wide_kernel<512, false>, what, big);
+                    if (e == cudaSuccess) e = cudaFuncSetAttribute(soft_mixed_wide_kernel<512, true>, what, big);
                     if (e != cudaSuccess) return e;
                     allowed[dev] = true;
                 }
                 P3T_COUNT_LAUNCH();
-                soft_mixed_wide_kernel<512><<<A.n_group, 512, big, st>>>(A);
+                if (emit) soft_mixed_wide_kernel<512, true><<<A.n_group, 512, big, st>>>(A);
+                else soft_mixed_wide_kernel<512, false><<<A.n_group, 512, big, st>>>(A);
             } else {
                 P3T_COUNT_LAUNCH();
-                soft_mixed_wide_kernel<256><<<A.n_group, 256, small, st>>>(A);
+                if (emit) soft_mixed_wide_kernel<256, true><<<A.n_group, 256, small, st>>>(A);
+                else soft_mixed_wide_kernel<256, false><<<A.n_group, 256, small, st>>>(A);
             }
             return cudaGetLastError();
         }

@@ -92,9 +92,8 @@ int p3t_set_soft_occupancy(int ctas_per_sm);
  * the next tile into a second buffer while the CTA computes the current one,
  * one barrier per tile; 0 (default, 7 % faster at 1M bodies) gather,
  * barrier, compute, barrier.  Bit-identical results.  Passes of at most three
- * groups per SM that emit no candidates have a form of their own (more threads
- * a group, the same bits) under either setting and any occupancy.  No counterpart
- * in GPLUM's interface. */
+ * groups per SM have a form of their own (more threads a group, the same bits)
+ * under either setting and any occupancy.  No counterpart in GPLUM's interface. */
 int p3t_set_soft_pipe(int on);
 /* The library's CUDA stream (cudaStream_t) for callers that order their own
  * work or timing events after the library's launches. */

@@ -1,5 +1,5 @@
 """A group's mixed soft force does not depend on the pass it is in: the forms by number of groups
-(512, 256 and 128 threads a group) and the pass that emits candidates give the same bits, over
+(512, 256 and 128 threads a group) and the passes that emit candidates give the same bits, over
 group sizes at the edges of the splits (32, 64, 128 bodies, and more than one turn) and list
 lengths at the edges of the partial sums (16, 32), of the sub-blocks' turns (128) and of the
 tiles (256, 512).  Exact equality: the same pair terms, summed in the same order."""
@@ -62,8 +62,10 @@ def test_forms_give_the_same_bits(gpu, ni):
     for g in (3, 7, 13, 18):
         got["alone"][i[g]] = _run(sf, epj, spj, i[g:g + 1], j[g:g + 1], s[g:g + 1])[i[g]]
     sf = SoftForce(P3TParams(), cand_cap=1024)
-    want = _run(sf, epj, spj, i, j, s, emit=True)
+    for name, k in (("512 threads, emitting", 0), ("256 threads, emitting", sms), ("128 threads, emitting", 3 * sms + 1)):
+        got[name] = _run(sf, epj, spj, i + more[:k], j + none[:k], s + none[:k], emit=True)
     SoftForce(P3TParams())
+    want = got.pop("128 threads")
     own = np.concatenate(i)
     assert np.any(want["acc"][own] != 0)
     for name, f in got.items():
