@@ -28,6 +28,7 @@ def clump(n, copies=1, spread=3.0, m=1e-10, seed=5):
 def hard_ms(d, clusters, mode=0):
     g = GpuSystem(P3TParams(dt_tree=2.0**-9))
     g.lib.p3t_set_schedule(0)
+    assert g.lib.p3t_set_hard_bundle(128, 3) == 0 and g.lib.p3t_set_hard_wide(1) == 0
     g.load(d)
     g.set_r_planet()
     g.startup()
