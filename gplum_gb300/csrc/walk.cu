@@ -235,19 +235,21 @@ int launch_walks(Context *c, WalkTable &t, const PackArgs &K, DevSet &x, int n_j
 // Writes a byte of every page of the walks' result arrays, as it is: a kernel's first
 // touch of fresh pages is slow, the host's is not (retrieve into an array that nobody has
 // written yet: 6,200 records 111 -> 51 us, 60,000 236 -> 111; into a used one 20 and 42).
-void touch_pages(int n_walk, const int *n_epi, void **force) {
+// The walks of one allocation lie end to end as a rule, which costs no look at each.
+void touch_range(uintptr_t a, uintptr_t e) {
     static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    uintptr_t done = 0;  // bytes below are touched
-    for (int k = 0; k < n_walk; k++) {
-        if (n_epi[k] <= 0) continue;
-        const uintptr_t a = (uintptr_t)force[k], e = a + (size_t)n_epi[k] * sizeof(ForceRec);
-        if (e <= done && a >= done - page) continue;  // on the page touched last
-        for (uintptr_t p = a; p < e; p = done) {
-            volatile char *const c = (volatile char *)p;
-            *c = *c;
-            done = (p & ~(page - 1)) + page;
-        }
+    for (uintptr_t p = a; p < e; p = (p & ~(page - 1)) + page) {
+        volatile char *const c = (volatile char *)p;
+        *c = *c;
     }
+}
+void touch_pages(int n_walk, const int *n_epi, void **force, bool end_to_end, long long n) {
+    if (end_to_end) {
+        if (n > 0) touch_range((uintptr_t)force[0], (uintptr_t)force[0] + (size_t)n * sizeof(ForceRec));
+        return;
+    }
+    for (int k = 0; k < n_walk; k++)
+        if (n_epi[k] > 0) touch_range((uintptr_t)force[k], (uintptr_t)force[k] + (size_t)n_epi[k] * sizeof(ForceRec));
 }
 
 // The forces' place: the slot's pinned buffer or device array.
@@ -384,18 +386,19 @@ int p3t_soft_retrieve(int tag, int n_walk, const int *n_epi, void **force) {
     WalkSlot *ws = slot_for(c, tag);
     if (!ws || !ws->busy) return ST_BAD_INDEX;
     WalkSlot &w = *ws;
-    uintptr_t bits = 0;
-    int walks = n_walk;  // those that the dispatch covers
+    uintptr_t bits = 0, apart = 0;  // apart: 0 while the walks' arrays lie end to end
+    int walks = n_walk;             // those that the dispatch covers
     long long off = 0;
     for (int k = 0; k < walks; k++) {
         if (off + n_epi[k] > w.n_i) walks = k;
         else {
+            apart |= (uintptr_t)force[k] - (uintptr_t)force[0] - (uintptr_t)off * sizeof(ForceRec);
             off += n_epi[k];
             if (n_epi[k] > 0) bits |= (uintptr_t)force[k];
         }
     }
     const bool device = on_device(c, w.n_i), direct = device && (bits & 3) == 0;
-    if (direct) touch_pages(walks, n_epi, force);  // while the kernels run
+    if (direct) touch_pages(walks, n_epi, force, apart == 0, off);  // while the kernels run
     int r = cuda_status(cudaEventSynchronize(w.done));
     w.busy = false;
     if (r) return r;
