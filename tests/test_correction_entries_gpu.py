@@ -1,5 +1,5 @@
 """The cutoff correction's pair pass where a CTA takes two, three or four list entries a thread
-(from 2, 3 and 4 x 1024 entries per SM on) and sorts them in as many rounds: whole CTAs of pairs
+(from 2, 3 and 4 x 1024 entries per SM on) and sorts them in as many turns: whole CTAs of pairs
 inside r_out, of pairs between r_out and r_search, and mixed ones.  Against the CPU oracle in the
 initial and the later form: neighbour pairs exactly; FP64 quantities from identical inputs 1e-12
 relative (log of the CUDA math library)."""
@@ -37,7 +37,7 @@ def bodies(n_clumps, rng):
 
 
 @pytest.mark.parametrize("per", [1, 2, 3, 4])
-def test_rounds(gpu, per):
+def test_entries_per_thread(gpu, per):
     import torch
 
     full = 128 * 8 * torch.cuda.get_device_properties(0).multi_processor_count
